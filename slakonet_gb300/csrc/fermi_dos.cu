@@ -1,4 +1,4 @@
-// Fermi level, band-gap statistics and Gaussian DOS, one CTA per structure.
+// Fermi level, band-gap statistics and Gaussian DOS, one cluster per structure.
 //
 // Fermi level.  The reference iterates mu <- mu - L / (dL/dmu + 1e-12) on
 // L = (2 sum_k w_k sum_b f(e_kb; mu, kT) - Ne)^2 from mu0 = mean(e), with
@@ -69,38 +69,129 @@ __device__ __forceinline__ void block_argext(double& v, int& idx, bool is_max, d
   }
 }
 
+// Extremes and sums of one CTA's share of a structure, combined over the cluster in rank order.
+struct GapPart {
+  double be, vbm, cbm, vmax, vmin, cmax, cmin, dgap, gv, gc;
+  int vbi, cbi, metal, nocc, nunocc;
+};
+
+SKN_DEVINL void take_max(double& v, int& i, double ov, int oi) {
+  if (ov > v || (ov == v && oi < i)) { v = ov; i = oi; }
+}
+SKN_DEVINL void take_min(double& v, int& i, double ov, int oi) {
+  if (ov < v || (ov == v && oi < i)) { v = ov; i = oi; }
+}
+SKN_DEVINL void combine(GapPart& a, const GapPart& o) {
+  a.be += o.be;
+  take_max(a.vbm, a.vbi, o.vbm, o.vbi);
+  take_min(a.cbm, a.cbi, o.cbm, o.cbi);
+  a.vmax = fmax(a.vmax, o.vmax);
+  a.vmin = fmin(a.vmin, o.vmin);
+  a.cmax = fmax(a.cmax, o.cmax);
+  a.cmin = fmin(a.cmin, o.cmin);
+  a.dgap = fmin(a.dgap, o.dgap);
+  a.gv = fmax(a.gv, o.gv);
+  a.gc = fmin(a.gc, o.gc);
+  a.metal |= o.metal;
+  a.nocc |= o.nocc;
+  a.nunocc |= o.nunocc;
+}
+SKN_DEVINL GapPart shfl_part(const GapPart& a, int o) {
+  GapPart r;
+  r.be = __shfl_down_sync(0xffffffffu, a.be, o);
+  r.vbm = __shfl_down_sync(0xffffffffu, a.vbm, o);
+  r.cbm = __shfl_down_sync(0xffffffffu, a.cbm, o);
+  r.vmax = __shfl_down_sync(0xffffffffu, a.vmax, o);
+  r.vmin = __shfl_down_sync(0xffffffffu, a.vmin, o);
+  r.cmax = __shfl_down_sync(0xffffffffu, a.cmax, o);
+  r.cmin = __shfl_down_sync(0xffffffffu, a.cmin, o);
+  r.dgap = __shfl_down_sync(0xffffffffu, a.dgap, o);
+  r.gv = __shfl_down_sync(0xffffffffu, a.gv, o);
+  r.gc = __shfl_down_sync(0xffffffffu, a.gc, o);
+  r.vbi = __shfl_down_sync(0xffffffffu, a.vbi, o);
+  r.cbi = __shfl_down_sync(0xffffffffu, a.cbi, o);
+  r.metal = __shfl_down_sync(0xffffffffu, a.metal, o);
+  r.nocc = __shfl_down_sync(0xffffffffu, a.nocc, o);
+  r.nunocc = __shfl_down_sync(0xffffffffu, a.nunocc, o);
+  return r;
+}
+
+// One cluster of FCL CTAs per structure.  The search is a chain of up to max_iter full sums, and an occupation
+// costs ~30 FP64 instructions (two per clock and SM), so one CTA's SM bounds it: 512 k-points x 18 bands took
+// 1.4 ms, 48 primitive cells of ~500 k-points 11 ms.  The eigenvalues are dealt to as many CTAs as there are
+// blocks of 256 (a rule on the structure alone); every CTA leaves its two sums in the others' shared memory,
+// alternating between two slots, so an iteration has one cluster barrier, and every CTA adds the slots in
+// rank order and takes the same step.
+constexpr int FCL = 16;
+constexpr int F_BLOCK = 256;
+
 __global__ void __launch_bounds__(NT) k_fermi_gap(const int64_t* __restrict__ eig_off, const int32_t* __restrict__ nkv,
                                                   const int32_t* __restrict__ nbv, const int64_t* __restrict__ kw_off,
                                                   const double* __restrict__ kweights, const double* __restrict__ nelec,
                                                   const double* __restrict__ eigall, double kT, double tol, int max_iter,
                                                   double* __restrict__ mu_out, double* __restrict__ stats,
                                                   int32_t* __restrict__ status) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cl = cg::this_cluster();
   __shared__ double red[4 * NT / 32];
-  __shared__ int redi[NT / 32];
-  const int s = blockIdx.x, tid = threadIdx.x;
+  __shared__ double slots[2][FCL][2];
+  __shared__ GapPart wpart[NT / 32];
+  __shared__ GapPart cpart;
+  const int s = blockIdx.x / FCL, tid = threadIdx.x, lane = tid & 31;
+  const int rank = (int)cl.block_rank();
   const int nk = nkv[s], nb = nbv[s];
   const int tot = nk * nb;
+  const int ranks = min(FCL, max(1, (tot + F_BLOCK - 1) / F_BLOCK));
+  if (rank >= ranks) return;           // its shared memory is never addressed, and barriers do not wait for it
   const double* E = eigall + eig_off[s];
   const double* w = kweights + kw_off[s];
   const double ne = nelec[s];
-  double* st = stats + (int64_t)SKN_NSTAT * s;
+  const int stride = NT * ranks, e0 = rank * NT + tid;
+  const int dk = nb > 0 ? stride / nb : 0, db = nb > 0 ? stride - dk * nb : 0;
+  const int k0 = nb > 0 ? e0 / nb : 0, b0 = nb > 0 ? e0 - k0 * nb : 0;
+  int turn = 0;
+
+  // sums of a and b over the structure, the same bits in every CTA
+  auto total2 = [&](double& a, double& b) {
+    block_sum2(a, b, red);
+    if (ranks > 1) {
+      if (tid < ranks) {
+        double* to = cl.map_shared_rank(&slots[turn][0][0], tid) + 2 * rank;
+        to[0] = a;
+        to[1] = b;
+      }
+      cl.sync();
+      a = slots[turn][0][0];
+      b = slots[turn][0][1];
+      for (int r = 1; r < ranks; ++r) {
+        a += slots[turn][r][0];
+        b += slots[turn][r][1];
+      }
+      turn ^= 1;
+    }
+  };
+  if (ranks > 1) cl.sync();            // every CTA's shared memory is there before the first remote store
 
   // mu0 = mean(e)
   double a = 0.0, b = 0.0;
-  for (int e = tid; e < tot; e += NT) a += E[e];
-  block_sum2(a, b, red);
+  for (int e = e0; e < tot; e += stride) a += E[e];
+  total2(a, b);
   double mu = a / (double)tot;
+  const double inv_kT = 1.0 / kT;
   int iters = max_iter, conv = 0;
   for (int it = 0; it < max_iter; ++it) {
     double sumo = 0.0, sumg = 0.0;
-    for (int e = tid; e < tot; e += NT) {
-      const double wk = w[e / nb];
-      const double t3 = exp((E[e] - mu) / kT);
-      const double occ = (1.0 / (t3 + 1.0)) * 1.0;
+    for (int e = e0, k = k0, bb = b0; e < tot; e += stride) {
+      const double wk = w[k];
+      const double t3 = exp((E[e] - mu) * inv_kT);
+      const double occ = 1.0 / (t3 + 1.0);
       sumo = fma(occ, wk, sumo);
       sumg += ((wk * occ) * occ) * t3;
+      k += dk;
+      bb += db;
+      if (bb >= nb) { bb -= nb; ++k; }
     }
-    block_sum2(sumo, sumg, red);
+    total2(sumo, sumg);
     const double total = 2.0 * sumo;
     const double diff = total - ne;
     const double loss = diff * diff;
@@ -109,106 +200,99 @@ __global__ void __launch_bounds__(NT) k_fermi_gap(const int64_t* __restrict__ ei
     mu = mu - loss / (grad + 1e-12);
   }
 
-  // Fermi-smeared band energy, SimpleDftb._calculate_electronic_energy (slakonet/main.py:1430-1448):
-  // sum_k w_k sum_b f(e_kb; mu, 0.025 eV) e_kb, with f = 0 where e_kb is exactly zero (fermi_smearing,
-  // slakonet/fermi.py:54-96)
-  {
-    const double kT_e = 0.025 / H2E;
-    double be = 0.0, unused = 0.0;
-    for (int e = tid; e < tot; e += NT) {
-      const double occ = (E[e] == 0.0) ? 0.0 : 1.0 / (1.0 + exp((E[e] - mu) / kT_e));
-      be += (occ * E[e]) * w[e / nb];
-    }
-    block_sum2(be, unused, red);
-    if (tid == 0) st[ST_BAND_ENERGY] = be;
-  }
-
-  // calculate_band_gap
+  GapPart P;
+  P.be = 0.0;
+  P.vbm = P.vmax = P.cmax = P.gv = -INFINITY;
+  P.cbm = P.vmin = P.cmin = P.dgap = P.gc = INFINITY;
+  P.vbi = P.cbi = 0x7fffffff;
+  P.metal = P.nocc = P.nunocc = 0;
+  const double kT_e = 0.025 / H2E, inv_kT_e = 1.0 / kT_e;
   const double f_ev = mu * H2E;
-  double vbm = -INFINITY, cbm = INFINITY;
-  int vbi = 0x7fffffff, cbi = 0x7fffffff;
-  int metal = 0, nocc = 0, nunocc = 0;
-  for (int e = tid; e < tot; e += NT) {
-    const double ev = E[e] * H2E;
-    if (fabs(ev - f_ev) < 1e-3) metal = 1;
-    if (ev < f_ev) { ++nocc; if (ev > vbm || (ev == vbm && e < vbi)) { vbm = ev; vbi = e; } }
-    if (ev >= f_ev) { ++nunocc; if (ev < cbm || (ev == cbm && e < cbi)) { cbm = ev; cbi = e; } }
+  for (int e = e0, k = k0, bb = b0; e < tot; e += stride) {
+    const double Ee = E[e];
+    // Fermi-smeared band energy, SimpleDftb._calculate_electronic_energy (slakonet/main.py:1430-1448):
+    // sum_k w_k sum_b f(e_kb; mu, 0.025 eV) e_kb, with f = 0 where e_kb is exactly zero (fermi_smearing,
+    // slakonet/fermi.py:54-96)
+    const double occ = (Ee == 0.0) ? 0.0 : 1.0 / (1.0 + exp((Ee - mu) * inv_kT_e));
+    P.be += (occ * Ee) * w[k];
+    // calculate_band_gap
+    const double ev = Ee * H2E;
+    if (fabs(ev - f_ev) < 1e-3) P.metal = 1;
+    if (ev < f_ev) { P.nocc = 1; take_max(P.vbm, P.vbi, ev, e); }
+    if (ev >= f_ev) { P.nunocc = 1; take_min(P.cbm, P.cbi, ev, e); }
+    // calculate_band_structure_properties on (e - mu) H2E
+    const double rel = (Ee - mu) * H2E;
+    if (rel < 0.0) { P.vmax = fmax(P.vmax, rel); P.vmin = fmin(P.vmin, rel); }
+    if (rel >= 0.0) { P.cmax = fmax(P.cmax, rel); P.cmin = fmin(P.cmin, rel); }
+    // get_fermi extras: occ = e <= mu, unocc = e > mu
+    if (Ee <= mu) P.gv = fmax(P.gv, Ee);
+    if (Ee > mu) P.gc = fmin(P.gc, Ee);
+    k += dk;
+    bb += db;
+    if (bb >= nb) { bb -= nb; ++k; }
   }
-  metal = __syncthreads_or(metal);
-  nocc = __syncthreads_count(nocc > 0);
-  nunocc = __syncthreads_count(nunocc > 0);
-  block_argext(vbm, vbi, true, red, redi);
-  block_argext(cbm, cbi, false, red, redi);
-
-  // calculate_band_structure_properties on (e - mu) H2E
-  double vmax = -INFINITY, vmin = INFINITY, cmax = -INFINITY, cmin = INFINITY;
-  for (int e = tid; e < tot; e += NT) {
-    const double ev = (E[e] - mu) * H2E;
-    if (ev < 0.0) { vmax = fmax(vmax, ev); vmin = fmin(vmin, ev); }
-    if (ev >= 0.0) { cmax = fmax(cmax, ev); cmin = fmin(cmin, ev); }
-  }
-  int dummy = 0;
-  block_argext(vmax, dummy, true, red, redi);
-  block_argext(vmin, dummy, false, red, redi);
-  block_argext(cmax, dummy, true, red, redi);
-  block_argext(cmin, dummy, false, red, redi);
-  double dgap = INFINITY;
-  for (int k = tid; k < nk; k += NT) {
+  // smallest direct gap: a warp per k-point
+  for (int k = rank * (NT / 32) + (tid >> 5); k < nk; k += ranks * (NT / 32)) {
     double kv = -INFINITY, kc = INFINITY;
-    int hv = 0, hc = 0;
-    for (int bb = 0; bb < nb; ++bb) {
-      const double ev = (E[k * nb + bb] - mu) * H2E;
-      if (ev < 0.0) { kv = fmax(kv, ev); hv = 1; }
-      if (ev > 0.0) { kc = fmin(kc, ev); hc = 1; }
+    for (int bb = lane; bb < nb; bb += 32) {
+      const double rel = (E[(int64_t)k * nb + bb] - mu) * H2E;
+      if (rel < 0.0) kv = fmax(kv, rel);
+      if (rel > 0.0) kc = fmin(kc, rel);
     }
-    if (hv && hc) dgap = fmin(dgap, kc - kv);
+    for (int o = 16; o > 0; o >>= 1) {
+      kv = fmax(kv, __shfl_xor_sync(0xffffffffu, kv, o));
+      kc = fmin(kc, __shfl_xor_sync(0xffffffffu, kc, o));
+    }
+    if (kv != -INFINITY && kc != INFINITY) P.dgap = fmin(P.dgap, kc - kv);
   }
-  block_argext(dgap, dummy, false, red, redi);
-
-  // get_fermi extras: occ = e <= mu, unocc = e > mu
-  double gv = -INFINITY, gc = INFINITY;
-  for (int e = tid; e < tot; e += NT) {
-    if (E[e] <= mu) gv = fmax(gv, E[e]);
-    if (E[e] > mu) gc = fmin(gc, E[e]);
-  }
-  block_argext(gv, dummy, true, red, redi);
-  block_argext(gc, dummy, false, red, redi);
-
+  for (int o = 16; o > 0; o >>= 1) combine(P, shfl_part(P, o));
+  if (lane == 0) wpart[tid >> 5] = P;
+  __syncthreads();
   if (tid == 0) {
+    for (int q = 1; q < NT / 32; ++q) combine(P, wpart[q]);
+    cpart = P;
+  }
+  if (ranks > 1) cl.sync();
+  if (rank == 0 && tid == 0) {
+    for (int r = 1; r < ranks; ++r) combine(P, *cl.map_shared_rank(&cpart, r));
+    double* st = stats + (int64_t)SKN_NSTAT * s;
+    st[ST_BAND_ENERGY] = P.be;
     mu_out[s] = mu;
-    const bool vfound = vmax != -INFINITY, cfound = cmin != INFINITY;
-    const double bs_gap = (vfound && cfound) ? (cmin - vmax) : 0.0;
-    st[ST_VWIDTH] = vfound ? (vmax - vmin) : 0.0;
-    st[ST_CWIDTH] = cfound ? (cmax - cmin) : 0.0;
-    const bool dfound = dgap != INFINITY;
-    st[ST_MIN_DGAP] = dfound ? dgap : qnan();
-    st[ST_DIRECT_SEMI] = dfound ? (fabs(bs_gap - dgap) < 0.01 ? 1.0 : 0.0) : 0.0;
+    const bool vfound = P.vmax != -INFINITY, cfound = P.cmin != INFINITY;
+    const double bs_gap = (vfound && cfound) ? (P.cmin - P.vmax) : 0.0;
+    st[ST_VWIDTH] = vfound ? (P.vmax - P.vmin) : 0.0;
+    st[ST_CWIDTH] = cfound ? (P.cmax - P.cmin) : 0.0;
+    const bool dfound = P.dgap != INFINITY;
+    st[ST_MIN_DGAP] = dfound ? P.dgap : qnan();
+    st[ST_DIRECT_SEMI] = dfound ? (fabs(bs_gap - P.dgap) < 0.01 ? 1.0 : 0.0) : 0.0;
     st[ST_CONVERGED] = conv;
     st[ST_ITERS] = iters;
-    st[ST_METAL] = metal;
-    if (metal) {
+    st[ST_METAL] = P.metal;
+    const bool none = P.nocc == 0 || P.nunocc == 0;
+    if (P.metal) {
       st[ST_MU_HA] = mu; st[ST_FERMI_EV] = mu * H2E; st[ST_GAP_EV] = 0.0;
       st[ST_VBM_EV] = f_ev; st[ST_CBM_EV] = f_ev; st[ST_DIRECT] = 0.0;
       st[ST_VBM_K] = 0; st[ST_CBM_K] = 0; st[ST_FALLBACK] = 0.0;
-    } else if (nocc == 0 || nunocc == 0) {
+    } else if (none) {
       // the reference's empty max/min raises; get_properties_dict falls back to zeros
       st[ST_MU_HA] = 0.0; st[ST_FERMI_EV] = 0.0; st[ST_GAP_EV] = 0.0;
       st[ST_VBM_EV] = 0.0; st[ST_CBM_EV] = 0.0; st[ST_DIRECT] = 1.0;
       st[ST_VBM_K] = 0; st[ST_CBM_K] = 0; st[ST_FALLBACK] = 1.0;
     } else {
-      st[ST_MU_HA] = mu; st[ST_FERMI_EV] = mu * H2E; st[ST_GAP_EV] = cbm - vbm;
-      st[ST_VBM_EV] = vbm; st[ST_CBM_EV] = cbm;
-      const int vk = vbi / nb, ck = cbi / nb;
+      st[ST_MU_HA] = mu; st[ST_FERMI_EV] = mu * H2E; st[ST_GAP_EV] = P.cbm - P.vbm;
+      st[ST_VBM_EV] = P.vbm; st[ST_CBM_EV] = P.cbm;
+      const int vk = P.vbi / nb, ck = P.cbi / nb;
       st[ST_DIRECT] = (vk == ck) ? 1.0 : 0.0;
       st[ST_VBM_K] = vk; st[ST_CBM_K] = ck; st[ST_FALLBACK] = 0.0;
     }
-    st[ST_VBM_FLAT] = (metal || nocc == 0 || nunocc == 0) ? -1.0 : (double)vbi;
-    st[ST_CBM_FLAT] = (metal || nocc == 0 || nunocc == 0) ? -1.0 : (double)cbi;
+    st[ST_VBM_FLAT] = (P.metal || none) ? -1.0 : (double)P.vbi;
+    st[ST_CBM_FLAT] = (P.metal || none) ? -1.0 : (double)P.cbi;
     st[ST_EFERMI_EV] = mu * H2E;
-    const double bg = gc - gv;
+    const double bg = P.gc - P.gv;
     st[ST_BANDGAP_EV] = (bg > 0.0 ? bg : (bg == bg ? 0.0 : bg)) * H2E;
     status[s] = conv ? SKN_OK : SKN_ERR_NO_CONVERGE;
   }
+  if (ranks > 1) cl.sync();            // rank 0 has read every part before its owner exits
 }
 
 // DOS of one structure on PTS grid points per cluster (gauss_sum.cuh).  A slice takes every 64th k-point, or,
@@ -315,8 +399,22 @@ extern "C" int skn_fermi_gap(int n_struct, const int64_t* eig_off, const int32_t
   if (n_struct == 0) return SKN_OK;
   if (!eig_off || !nk || !nb || !kw_off || !kweights || !nelec || !eig || !mu || !stats || !status)
     return SKN_ERR_ARG;
-  k_fermi_gap<<<n_struct, NT, 0, stream>>>(eig_off, nk, nb, kw_off, kweights, nelec, eig, kT, tol, max_iter, mu,
-                                           stats, status);
+  if (n_struct > INT32_MAX / FCL) return SKN_ERR_CAPACITY;
+  if (cudaFuncSetAttribute(k_fermi_gap, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)
+    return SKN_ERR_CUDA;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)n_struct * FCL);
+  cfg.blockDim = dim3(NT);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = FCL;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  if (cudaLaunchKernelEx(&cfg, k_fermi_gap, eig_off, nk, nb, kw_off, kweights, nelec, eig, kT, tol, max_iter, mu,
+                         stats, status) != cudaSuccess)
+    return SKN_ERR_CUDA;
   return cudaPeekAtLastError() == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
 }
 

@@ -1,13 +1,14 @@
-"""DOS kernel at the sizes where its splits change (needs a GB300).
+"""DOS and Fermi kernels at the sizes where their splits change (needs a GB300).
 
 The DOS kernel gives 8 grid points to a lane, 64 to a tile, 256 to a CTA, and cuts the bands into 64 slices
 (whole k-points from 64 k-points up, parts of a k-point below); fine grids take the power recurrence, coarse ones
-one exponential per point.
+one exponential per point.  The Fermi kernel deals blocks of 256 eigenvalues to up to 16 CTAs.
 """
 import numpy as np
 import pytest
 import torch
 
+from oracle import slako_oracle as O
 from slakonet_gb300._lib import call, ptr
 
 pytestmark = pytest.mark.gpu
@@ -92,3 +93,38 @@ def test_nan_fermi_level_gives_a_nan_dos():
     B = _Batch([(3, 4), (3, 4)], seed=1)
     _, dos, _ = _dos(B, [np.nan, 0.0], -20.0, 10.0, 300, 0.1, 9.0)
     assert np.isnan(dos[0]).all() and np.isfinite(dos[1]).all()
+
+
+def test_fermi_and_gap_over_the_split_sizes():
+    """Blocks of 256 eigenvalues: one below, at and above each edge, up to more than 16 blocks.  The spectra are
+    dense (metals), where the search contracts, so its level agrees with the oracle's to its own stopping
+    accuracy; the band edges are compared at the kernel's own level, where both sides do the same operations."""
+    sizes = [(1, 1), (1, 8), (15, 17), (8, 32), (1, 257), (7, 73), (27, 19), (41, 25), (63, 65), (64, 64), (97, 85), (500, 40)]
+    B = _Batch(sizes, seed=5)
+    mu = torch.empty(B.n, dtype=torch.float64, device=DEV)
+    stats = torch.zeros(B.n, 24, dtype=torch.float64, device=DEV)
+    st = torch.empty(B.n, dtype=torch.int32, device=DEV)
+    call("skn_fermi_gap", B.n, ptr(B.off), ptr(B.nk), ptr(B.nb), ptr(B.kwo), ptr(B.kw), ptr(B.nel), ptr(B.E), 0.01,
+         1e-6, 100, ptr(mu), ptr(stats), ptr(st), torch.cuda.current_stream(DEV).cuda_stream)
+    torch.cuda.synchronize()
+    stats, mu, st = stats.cpu().numpy(), mu.cpu().numpy(), st.cpu().numpy()
+    for s in range(B.n):
+        ref, it, conv = O.fermi_search(B.eig[s], B.w[s], B.ne[s])
+        assert (st[s] == 0) == conv
+        if np.isfinite(ref):
+            assert abs(mu[s] - ref) <= 1e-9 * max(1.0, abs(ref)), (sizes[s], mu[s], ref)
+        else:
+            assert not np.isfinite(mu[s])
+            continue
+        bs = O.band_structure_props(B.eig[s], mu[s])
+        be = O.band_energy(B.eig[s], B.w[s], mu[s])
+        assert abs(stats[s][23] - be) <= 1e-12 * B.eig[s].size
+        rel = (B.eig[s] - mu[s]) * H2E
+        v, c = rel[rel < 0], rel[rel >= 0]
+        assert stats[s][8] == (v.max() - v.min() if len(v) else 0.0)
+        assert stats[s][9] == (c.max() - c.min() if len(c) else 0.0)
+        kv = np.where(rel < 0, rel, -np.inf).max(1)
+        kc = np.where(rel > 0, rel, np.inf).min(1)
+        ok = np.isfinite(kv) & np.isfinite(kc)
+        assert (stats[s][10] == (kc - kv)[ok].min()) if ok.any() else np.isnan(stats[s][10])
+        assert bs is not None
