@@ -991,6 +991,8 @@ __global__ void __launch_bounds__(VNT) k_eigvec(int n_prob, const int32_t* __res
         }
         if (fabs(u1) < pivmin) u1 = (u1 < 0.0) ? -pivmin : pivmin;
         s_ru1[(n - 1) * VNT + tid] = 1.0 / u1;
+        s_u2[(n - 1) * VNT + tid] = 0.0;   // the last row has no columns to its right: the back substitution
+        s_u3[(n - 1) * VNT + tid] = 0.0;   // multiplies these by zero, and scratch may hold a NaN
         rmax = fmax(rmax, fabs(1.0 / u1));
         // A lam exact to the last bit (the Newton step can land on the eigenvalue) leaves a pivot at the
         // 1e-300 floor, and a solve then grows the vector by up to 1 / pivot: its sum of squares overflowed

@@ -99,3 +99,35 @@ def test_eigenvectors_finite_where_the_eigenvalue_is_exact():
     print(f"fitting-batch cell (n = {int(plan.nb[0])}, {len(k)} k): all {len(k)} k-points finite; "
           f"residual {r:.1e}, orthonormality {o:.1e}, direction {d:.1e}")
     assert r <= 1e-10 and o <= 1e-10 and d <= 1e-8
+
+
+@pytest.mark.parametrize("fill", [0.0, float("nan")])
+def test_eigenvectors_do_not_depend_on_what_the_scratch_held(fill):
+    """The back substitution of the last row once multiplied unwritten scratch by zero: a NaN left there by an
+    earlier use of the memory replaced the eigenvector by a unit vector."""
+    import ctypes
+    from slakonet_gb300._lib import call, ptr
+    g = golden("rand_b")
+    st, tables, sd = load_case(g)
+    ts = E.TableSet.from_synthetic(tables, sd, DEV)
+    plan = E.plan_batch([dict(st, kpoints=g["kpoints"][:3])], ts)
+    eng = E.Engine(ts)
+    db = E.DeviceBatch(plan, DEV)
+    hs = eng.execute(db, keep_hs=True, hs_only=True)
+    H, S = hs.H.clone(), hs.S.clone()
+    n, n_prob = int(plan.nb[0]), len(plan.prob_n)
+    eig = torch.empty(plan.eig_total, dtype=torch.float64, device=DEV)
+    vec, stt = torch.empty_like(H), torch.empty(n_prob, dtype=torch.int32, device=DEV)
+    tri = torch.empty(4 * plan.eig_total, dtype=torch.float64, device=DEV)
+    need = ctypes.c_int64(0)
+    call("skn_eigh_vectors_scratch_bytes", n_prob, plan.max_n, ctypes.addressof(need))
+    scratch = torch.full((need.value // 8,), fill, dtype=torch.float64, device=DEV)
+    ctr = torch.zeros(2, dtype=torch.int32, device=DEV)
+    call("skn_eigh_gen_vectors", n_prob, ptr(db.n), ptr(db.hs_off), ptr(db.eoff), ptr(db.order), ptr(H), ptr(S),
+         ptr(eig), ptr(vec), ptr(stt), ptr(tri), ptr(scratch), need.value, ptr(ctr), plan.max_n,
+         torch.cuda.current_stream(DEV).cuda_stream)
+    torch.cuda.synchronize(DEV)
+    C = torch.view_as_complex(vec.view(-1, 2)).view(n_prob, n, n).cpu().numpy()
+    Sq = torch.view_as_complex(hs.S.view(-1, 2)).view(n_prob, n, n).transpose(1, 2).cpu().numpy()
+    for q in range(n_prob):
+        assert np.abs(C[q].conj().T @ Sq[q] @ C[q] - np.eye(n)).max() <= 1e-10
