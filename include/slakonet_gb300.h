@@ -303,6 +303,47 @@ int skn_eigh_wide_scratch_bytes(int n_prob, int n, int64_t* bytes);
 int skn_eigh_gen_wide_tc(int n_prob, int n, const int32_t* prob, const int32_t* nvec, const int64_t* hs_off,
                          const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status, double* scratch,
                          int64_t scratch_bytes, int real, cudaStream_t stream);
+/*
+ * Eigenvalues (and, with `tri`, the reduced form the eigenvectors start from) of
+ * problems of up to 96 orbitals, one CTA per problem with both matrices in shared
+ * memory: B = L^-1 H beside the Cholesky factorisation, C = B L^-H, Householder
+ * tridiagonalisation, Sturm-count eigenvalues.  Replaces the same eighb call as
+ * skn_eigh_gen_batched (slakonet/utils.py:741-783).
+ *   max_n     largest n of the call (a larger problem gets SKN_ERR_CAPACITY,
+ *             untouched); up to 16, up to 32 and above run on 32, 64 and 128 threads
+ *   prob, nvec, real, hs_off, eig_off, H, S, eig, status, tri   as
+ *             skn_eigh_gen_panels; H and S are written only with `tri`
+ * Results depend only on each problem and on which of the three ranges max_n is in.
+ */
+int skn_eigh_gen_small(int n_prob, int max_n, const int32_t* prob, const int32_t* nvec, const int32_t* real,
+                       const int64_t* hs_off, const int64_t* eig_off, double* H, double* S, double* eig,
+                       int32_t* status, double* tri, cudaStream_t stream);
+/*
+ * Eigenvalues (and, with `tri`, the reduced form the eigenvectors start from) of
+ * problems of up to 1024 orbitals, in lockstep over 32-column panels: Cholesky of
+ * S, C = L^-1 H L^-H by two blocked sweeps, Householder tridiagonalisation with
+ * one cluster of CTAs per problem, Sturm-count eigenvalues.  Every trailing
+ * update runs on the bf16 tensor cores, exact products of 8 integer slices of 7
+ * bits per operand row rounded once per panel.  Replaces the same eighb call as
+ * skn_eigh_gen_batched (slakonet/utils.py:741-783).
+ *   n_prob    problems of the call (<= 65535)
+ *   max_n     largest n; every problem must have ceil(max_n / 32) panels of 32
+ *             columns (a problem that has not gets SKN_ERR_CAPACITY, untouched)
+ *   prob      [n_prob] (device) problem index of each slot, into the arrays below
+ *   real      [*] 1 where H and S are exactly real, or NULL
+ *   nvec, hs_off, eig_off, H, S, eig, status   as skn_eigh_gen_batched; only the
+ *             lower triangles are read, all of H and the lower triangle of S are
+ *             overwritten
+ *   tri       NULL, or d, e and tau per problem at 4 eig_off, as skn_eigh_gen_vectors
+ *             keeps them (reflectors in the lower triangle of H, L in S)
+ *   scratch   device scratch of skn_eigh_panels_scratch_bytes(n_prob, max_n) bytes
+ * Results depend only on each problem.
+ */
+int skn_eigh_gen_panels(int n_prob, int max_n, const int32_t* prob, const int32_t* nvec, const int32_t* real,
+                     const int64_t* hs_off, const int64_t* eig_off, double* H, double* S, double* eig,
+                     int32_t* status, double* tri, double* scratch, int64_t scratch_bytes, cudaStream_t stream);
+/* Host-side query: bytes of `scratch` skn_eigh_gen_panels needs (written to *bytes). */
+int skn_eigh_panels_scratch_bytes(int n_prob, int max_n, int64_t* bytes);
 
 /*
  * The same eigensolver compiled in more launch shapes: 32 threads per CTA with

@@ -27,8 +27,10 @@ from ._lib import call, ptr
 
 SHAPES = ["", "_t32", "_t64", "_t256", "_blk"]  # export suffixes; "" is the 128-thread default, "_blk" the blocked one
 BUCKETS = [16, 32, 64, 128, 256, 512, 1024, 2048]
-# Untuned default: the blocked Cholesky and reduction above 128 orbitals, where it measured 18-20% faster
-# on GB300 (n = 200-492); below, the unblocked kernel is faster (the panels are too short to pay).
+# Shape of the untuned default: skn_eigh_gen_small up to 96 orbitals, skn_eigh_gen_panels above (engine.route_auto).
+AUTO = "auto"
+# The one-CTA kernel's own policy: the blocked Cholesky and reduction above 128 orbitals, where it measured 18-20%
+# faster on GB300 (n = 200-492); below, its unblocked form is faster (the panels are too short to pay).
 BLOCKED_FROM_BUCKET = 256
 
 
@@ -48,11 +50,15 @@ class Tuning:
 
     @classmethod
     def default(cls) -> "Tuning":
-        """Untuned shapes: 128 threads up to 128 orbitals, the blocked shape from 256.  On the uneven batch
-        this policy runs at 692-706 ms per eigensolve on GB300, run after run.  Policies that put the small
-        problems on the 32- or 64-thread shapes are as fast at best but swing to 780-830 ms: their many
-        small CTAs, launched beside the blocked shape on other streams, can take the SMs' slots first and
-        delay the large problems, whose completion ends the step."""
+        """Untuned: the small and the panel kernels up to 1024 orbitals, the blocked one-CTA shape above."""
+        return cls({u: (AUTO if u <= 1024 else "_blk") for u in BUCKETS})
+
+    @classmethod
+    def one_cta(cls) -> "Tuning":
+        """The one-CTA kernel throughout: 128 threads up to 128 orbitals, the blocked shape from 256.  Policies that
+        put the small problems on its 32- or 64-thread shapes are as fast at best but swing by 15%: their many small
+        CTAs, launched beside the blocked shape on other streams, can take the SMs' slots first and delay the large
+        problems, whose completion ends the step."""
         return cls({u: ("_blk" if u >= BLOCKED_FROM_BUCKET else "") for u in BUCKETS})
 
 
@@ -207,13 +213,10 @@ def _merge_into_cache(path: str, key: str, tun: Tuning) -> Tuning:
 
 
 def candidate_policies(tuning: Optional[Tuning] = None) -> List[Tuning]:
-    """Whole-batch candidates: the untuned default (128 threads below 256 orbitals, blocked from 256) and
-    the blocked shape from 128.  Policies with the 32- or 64-thread shapes for the small buckets, or the
-    per-bucket winners of ``autotune`` (``tuning``, timed one shape at a time), are not offered: beside the
-    blocked launch on other streams their many small CTAs make the step swing between 690 and 830 ms.
-    ``tuning`` is accepted for its per-bucket timings only."""
+    """Whole-batch candidates: the untuned default and the one-CTA kernel's policy.  The per-bucket winners of
+    ``autotune`` (``tuning``, timed one shape at a time) are not offered; it is accepted for its timings only."""
     del tuning
-    return [Tuning.default(), Tuning({u: ("_blk" if u >= 128 else "") for u in BUCKETS})]
+    return [Tuning.default(), Tuning.one_cta()]
 
 
 def tune_batch(engine, db, candidates: Optional[List[Tuning]] = None, reps: int = 3) -> Tuning:

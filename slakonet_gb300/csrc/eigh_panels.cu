@@ -1,0 +1,1395 @@
+// Generalized Hermitian eigenvalues of problems of about 100 orbitals and more, blocked, with every O(n^3)
+// step but the Hermitian matrix-vector products on the tcgen05 tensor cores.
+//
+// The problems of one call have the same number T of 32-column panels (n from 32 T - 31 to 32 T) and go
+// through one sequence of launches together; every launch covers all of them:
+//   1. set-up: zero rows (eighb's aux option, slakonet/utils.py:741-747), the upper triangle of H;
+//   2. per panel: Cholesky of the diagonal block of S; triangular solves of the panel's rows and of the block
+//      row of B = L^-1 H; one update S22 -= L21 L21^H and H_below -= L21 B_panel on the tensor cores;
+//   3. per panel: the column block of C = B L^-H by row solves; one update of the trailing lower triangle
+//      C22 -= C_panel L21^H on the tensor cores;
+//   4. per 16 columns: Householder reflectors and the W vectors of LAPACK's zlatrd (k_tri_panel, one cluster
+//      of CTAs per problem), then A22 -= V W^H + W V^H on the tensor cores;
+//   5. eigenvalues of the tridiagonal (sturm.cuh).
+// The reference calls torch.linalg.cholesky / solve / eigh per k (slakonet/utils.py:749-783,
+// slakonet/main.py:174).
+//
+// GB300 notes.  An SM does two FP64 multiply-adds per clock, so FP64 issue bounds everything that stays on it;
+// of the 32/3 n^3 flops only the matrix-vector products (8/3 n^3) do.  The updates are exact products of
+// integer slices (below) rounded once per panel.  Every sum that crosses warps or CTAs goes to its own slot
+// and is added in a fixed order, so a problem's results depend neither on the other problems nor on the
+// number of CTAs it is given.
+#include <cooperative_groups.h>
+#include <cuda_bf16.h>
+
+#include "exact_round.cuh"
+#include "skn_common.cuh"
+#include "sturm.cuh"
+
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int NB = 32;               // panel width of the factorisations
+constexpr int NT = 16;               // columns per tridiagonalisation panel
+constexpr int LDT = NB + 1;
+constexpr int TS = 32;               // tile edge of the matrix-vector products
+constexpr int SLICES = 8;
+constexpr int KP = 64;               // inner dimension of the sliced products (32 complex columns)
+constexpr int BM = 128, BN = 16;     // output tile of the tensor-core update
+constexpr int PANELS_MAX_N = 1024;
+
+SKN_DEVINL int cdiv_d(int a, int b) { return (a + b - 1) / b; }
+inline int cdiv(int a, int b) { return (a + b - 1) / b; }
+
+// ------------------------------------------------------------------ arithmetic (R: real parts only)
+template <bool R> SKN_DEVINL double2 ld(const double2* p) {
+  if constexpr (R) return make_double2(p->x, 0.0); else return *p;
+}
+template <bool R> SKN_DEVINL double2 ldc(const double2* p) {      // written by another CTA of this launch
+  if constexpr (R) return make_double2(__ldcg(&p->x), 0.0); else return __ldcg(p);
+}
+template <bool R> SKN_DEVINL void st(double2* p, double2 v) {
+  if constexpr (R) p->x = v.x; else *p = v;
+}
+template <bool R> SKN_DEVINL double2 fma_(double2 a, double2 b, double2 c) {        // c + a b
+  if constexpr (R) { c.x = fma(a.x, b.x, c.x); return c; } else return cfma(a, b, c);
+}
+template <bool R> SKN_DEVINL double2 fma_cja(double2 a, double2 b, double2 c) {     // c + conj(a) b
+  if constexpr (R) { c.x = fma(a.x, b.x, c.x); return c; } else return cfma_conj(a, b, c);
+}
+template <bool R> SKN_DEVINL double2 fms(double2 a, double2 b, double2 c) {         // c - a b
+  c.x = fma(-a.x, b.x, c.x);
+  if constexpr (!R) {
+    c.x = fma(a.y, b.y, c.x);
+    c.y = fma(-a.x, b.y, c.y);
+    c.y = fma(-a.y, b.x, c.y);
+  }
+  return c;
+}
+template <bool R> SKN_DEVINL double2 fms_cj(double2 a, double2 b, double2 c) {      // c - a conj(b)
+  if constexpr (R) { c.x = fma(-a.x, b.x, c.x); return c; } else return cfms_conj(a, b, c);
+}
+template <bool R> SKN_DEVINL double2 mul(double2 a, double2 b) {
+  if constexpr (R) return make_double2(a.x * b.x, 0.0); else return cmul(a, b);
+}
+template <bool R> SKN_DEVINL double2 add(double2 a, double2 b) {
+  return make_double2(a.x + b.x, R ? 0.0 : a.y + b.y);
+}
+template <bool R> SKN_DEVINL double2 warp_sum(double2 s) {                          // fixed butterfly
+  for (int o = 16; o > 0; o >>= 1) {
+    s.x += __shfl_xor_sync(0xffffffffu, s.x, o);
+    if constexpr (!R) s.y += __shfl_xor_sync(0xffffffffu, s.y, o);
+  }
+  return s;
+}
+SKN_DEVINL double2 zero2() { return make_double2(0.0, 0.0); }
+
+// ------------------------------------------------------------------ scratch (per problem slot)
+struct Lay {
+  int64_t W, VW, xc, Yp, sN, sT, sD, rd, d, e2, d32, e232, bnd, flg, sa, sb, sc, ea, eb, ec, stride;   // bytes
+};
+__host__ __device__ inline int64_t take(int64_t& o, int64_t bytes) {
+  const int64_t r = o;
+  o += (bytes + 255) / 256 * 256;
+  return r;
+}
+// Rows of a slice array: a 128-row tile may start at any multiple of 16 up to n.
+__host__ __device__ inline int64_t slice_rows(int n) { return ((int64_t)n + 127) / 128 * 128 + 128; }
+__host__ __device__ inline Lay layout(int n) {
+  const int64_t nt = (n + TS - 1) / TS, nr = slice_rows(n);
+  Lay L;
+  int64_t o = 0;
+  L.W = take(o, 16 * (int64_t)NT * n);         // W panel, column q at W + q n (row index of the matrix)
+  L.VW = take(o, 16 * (int64_t)2 * NT * n);    // rows of [W V]: row r at VW + 2 NT r
+  L.xc = take(o, 16 * (int64_t)n);             // the current column before its scaling
+  L.Yp = take(o, 16 * nt * n);                 // matrix-vector partial sums: slot s at Yp + s n
+  L.sN = take(o, 8 * nt);                      // column norm, per 32-row chunk
+  L.sT = take(o, 8 * nt * (nt + 1) / 2);       // v^H A v, per tile
+  L.sD = take(o, 16 * nt * 4 * 2 * NT);        // [W V]^H v, per 8 rows
+  L.rd = take(o, 8 * (int64_t)n);              // 1 / L_kk
+  L.d = take(o, 8 * (int64_t)n);
+  L.e2 = take(o, 8 * (int64_t)n);
+  L.d32 = take(o, 4 * (int64_t)n);
+  L.e232 = take(o, 4 * (int64_t)n);
+  L.bnd = take(o, 64);
+  L.flg = take(o, 4 * 2 * (int64_t)n);
+  L.sa = take(o, 2 * SLICES * nr * KP);        // row operand
+  L.sb = take(o, 2 * 2 * SLICES * nr * KP);    // column operand from rows: form B, then B'
+  L.sc = take(o, 2 * 2 * SLICES * nr * KP);    // column operand from the block row of B
+  L.ea = take(o, 4 * nr);                      // row exponents of sa, sb, sc
+  L.eb = take(o, 4 * nr);
+  L.ec = take(o, 4 * nr);
+  L.stride = o;
+  return L;
+}
+
+struct Grp {
+  int nmax, panels, n_prob;
+  const int32_t* prob;       // [n_prob] problem of each slot
+  const int32_t* nvec;
+  const int32_t* real;       // [*] 1 where H and S are exactly real; may be null
+  const int64_t* hs_off;
+  const int64_t* eig_off;
+  double2* H;
+  double2* S;
+  double* eig;
+  int32_t* status;
+  double* tri;               // d, e, tau per problem at 4 eig_off (for eigenvectors); may be null
+  char* scratch;
+};
+
+struct WS {
+  double2 *W, *VW, *xc, *Yp, *sD;
+  double *sN, *sT, *rd, *d, *e2, *bnd;
+  float *d32, *e232;
+  int *flg, *ea, *eb, *ec;
+  uint16_t *sa, *sb, *sc;
+  int64_t nr;                // rows of a slice array
+};
+SKN_DEVINL WS ws_of(const Grp& G, int g) {
+  const Lay L = layout(G.nmax);
+  char* b = G.scratch + (int64_t)g * L.stride;
+  WS w;
+  w.W = (double2*)(b + L.W); w.VW = (double2*)(b + L.VW); w.xc = (double2*)(b + L.xc); w.Yp = (double2*)(b + L.Yp);
+  w.sD = (double2*)(b + L.sD); w.sN = (double*)(b + L.sN); w.sT = (double*)(b + L.sT); w.rd = (double*)(b + L.rd);
+  w.d = (double*)(b + L.d); w.e2 = (double*)(b + L.e2); w.bnd = (double*)(b + L.bnd);
+  w.d32 = (float*)(b + L.d32); w.e232 = (float*)(b + L.e232); w.flg = (int*)(b + L.flg);
+  w.ea = (int*)(b + L.ea); w.eb = (int*)(b + L.eb); w.ec = (int*)(b + L.ec);
+  w.sa = (uint16_t*)(b + L.sa); w.sb = (uint16_t*)(b + L.sb); w.sc = (uint16_t*)(b + L.sc);
+  w.nr = slice_rows(G.nmax);
+  return w;
+}
+SKN_DEVINL bool live(const Grp& G, int p) { return G.status[p] == SKN_OK; }
+SKN_DEVINL bool is_real(const Grp& G, int p) { return G.real != nullptr && G.real[p] != 0; }
+
+// ------------------------------------------------------------------ integer slices
+// Error-free splitting (Ozaki, Ogita and Oishi, Numer. Algorithms 59, 2012).  A row of 32 complex values is
+// scaled by its exponent ex and cut into SLICES digits of 7 bits, x = 2^ex sum_s d_s 2^(-7 (s + 1)) with
+// |d_0| <= 128 and -64 <= d_s < 64 after it, each exact in bf16; what is cut off is below 2^-57 of the
+// row's largest entry.  A slice product is an integer of at most 14 bits and a 64-term sum of the at most
+// 8 slice pairs of one level s + t stays below 2^23, exact in an FP32 accumulator.  The complex product
+// P Q^H takes A = [Pr Pi], B = [Qr Qi] for the real part and B' = [-Qi Qr] for the imaginary part.
+// The digits are taken with integer operations: the FP64 pipe would cost more than the solves.
+constexpr int EXP_NAN = INT32_MIN;       // a row with a non-finite entry: its products become NaN
+
+// Element index in a slice array, in the tensor cores' K-major core-matrix order (8-row groups of KP x 8
+// elements, each a run of 8 x 8 core matrices along K), so rows starting at a multiple of 8 are one run.
+SKN_DEVINL int64_t tc_idx(int r, int k) { return (int64_t)(r >> 3) * (8 * KP) + (k >> 3) * 64 + (r & 7) * 8 + (k & 7); }
+
+SKN_DEVINL long long fixed56(double x, int emax) {       // round(x 2^(56 - ex)), ex = emax - 1022
+  const unsigned long long b = (unsigned long long)__double_as_longlong(x);
+  const int e = (int)((b >> 52) & 0x7ff);
+  if (e == 0) return 0;
+  const long long m = (long long)((b & 0xfffffffffffffull) | 0x10000000000000ull);
+  const int d = emax - e;
+  long long f = d <= 3 ? m << (3 - d) : (d > 60 ? 0 : (m + (1LL << (d - 4))) >> (d - 3));
+  return (b >> 63) ? -f : f;
+}
+// bf16 bits of a small integer (|d| <= 128)
+SKN_DEVINL uint32_t small_bf16(int d) {
+  return __float_as_uint(__int_as_float(0x4B400000 + d) - 12582912.0f) >> 16;
+}
+SKN_DEVINL uint4 neg4(uint4 v) {
+  return make_uint4(v.x ^ 0x80008000u, v.y ^ 0x80008000u, v.z ^ 0x80008000u, v.w ^ 0x80008000u);
+}
+
+// Slices of one row r: values z_k = get(k), k < 32 (zero from K on).  A form to sa (null: none) with exponent
+// ea[r]; B and B' forms of the row with its halves swapped when `swap` (z' = [z_16.. z_31, z_0.. z_15]).
+template <class Get>
+SKN_DEVINL void slice_row(Get get, int r, int64_t nr, uint16_t* sa, int* ea, uint16_t* sb, int* eb, bool swap) {
+  int hm = 0;
+#pragma unroll 8
+  for (int k = 0; k < 32; ++k) {
+    const double2 z = get(k);
+    hm = max(hm, max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
+  }
+  const int emax = hm >> 20;
+  const int ex = emax == 0x7ff ? EXP_NAN : emax - 1022;
+  if (sa) ea[r] = ex;
+  if (sb) eb[r] = ex;
+#pragma unroll 1
+  for (int kb = 0; kb < 8; ++kb) {          // 8 entries of one part: kb < 4 real, then imaginary
+    uint32_t out[SLICES][4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      uint32_t lo[SLICES], hi[SLICES];
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const double2 z = get((kb & 3) * 8 + 2 * u + h);
+        long long f = emax == 0x7ff ? 0 : fixed56(kb < 4 ? z.x : z.y, emax);
+#pragma unroll
+        for (int s = SLICES - 1; s >= 0; --s) {
+          int dgt;
+          if (s > 0) {
+            dgt = (int)((f + 64) & 127) - 64;
+            f = (f - dgt) >> 7;
+          } else {
+            dgt = (int)f;
+          }
+          if (h == 0) lo[s] = small_bf16(dgt); else hi[s] = small_bf16(dgt);
+        }
+      }
+#pragma unroll
+      for (int s = 0; s < SLICES; ++s) out[s][u] = lo[s] | (hi[s] << 16);
+    }
+    const int pb = swap ? ((kb & 4) | ((kb + 2) & 3)) : kb;      // place of these entries in B
+    const bool im = kb >= 4;
+#pragma unroll
+    for (int s = 0; s < SLICES; ++s) {
+      const uint4 v = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
+      if (sa) *reinterpret_cast<uint4*>(sa + (int64_t)s * nr * KP + tc_idx(r, kb * 8)) = v;
+      if (sb) {
+        uint16_t* B = sb + (int64_t)s * nr * KP;
+        uint16_t* Bp = sb + (int64_t)(SLICES + s) * nr * KP;
+        *reinterpret_cast<uint4*>(B + tc_idx(r, pb * 8)) = v;
+        // B' = [-Qi Qr]: the real part of Q goes to the second half, minus the imaginary part to the first
+        *reinterpret_cast<uint4*>(Bp + tc_idx(r, (pb ^ 4) * 8)) = im ? neg4(v) : v;
+      }
+    }
+  }
+}
+
+// ------------------------------------------------------------------ set-up
+__global__ void __launch_bounds__(256) k_init(Grp G) {
+  const int g = blockIdx.y, p = G.prob[g];
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const int n = G.nvec[p];
+    const bool ok = n >= 1 && n <= G.nmax && cdiv_d(n, NB) == G.panels && G.hs_off[p] >= 0 && G.eig_off[p] >= 0;
+    G.status[p] = ok ? SKN_OK : SKN_ERR_CAPACITY;
+  }
+  const int i = blockIdx.x * 256 + threadIdx.x;
+  if (i < 2 * G.nmax) ws_of(G, g).flg[i] = 0;
+}
+
+// Rows with a nonzero entry, from 32 x 32 tiles of the lower triangles (entry (i, j) marks rows i and j), and
+// the upper triangle of H from the lower one.  One warp per tile; blockIdx.z: 0 H, 1 S.
+__global__ void __launch_bounds__(256) k_scan(Grp G) {
+  const int g = blockIdx.y, which = blockIdx.z, p = G.prob[g];
+  if (!live(G, p)) return;
+  const int n = G.nvec[p], nt = cdiv_d(n, TS), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ double2 tiles[8][TS * (TS / 8 + 1)];
+  const int t = blockIdx.x * 8 + warp;
+  if (t >= nt * nt) return;
+  const int I = t / nt, J = t % nt;
+  if (J > I) return;
+  double2* A = (which ? G.S : G.H) + G.hs_off[p];
+  int* flg = ws_of(G, g).flg + which * G.nmax;
+  const int i = I * TS + lane;
+  bool row = false;
+  double2* T = tiles[warp];
+  for (int c0 = 0; c0 < TS; c0 += 4) {
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int j = J * TS + c0 + c;
+      double2 a = zero2();
+      bool nz = false;
+      if (i < n && j <= i) {
+        a = A[i + (int64_t)j * n];
+        nz = !(is_zero_bits(a.x) && is_zero_bits(a.y));
+      }
+      row |= nz;
+      if (__any_sync(0xffffffffu, nz) && lane == 0) flg[j] = 1;
+      T[lane * 5 + c] = a;
+    }
+    __syncwarp();
+    if (which == 0) {                       // column j of the lower tile is row j of the upper one
+      const int c = lane & 3, j = J * TS + c0 + c;
+      for (int r = lane >> 2; r < TS; r += 8) {
+        const int gi = I * TS + r;
+        if (gi < n && j < gi) {
+          const double2 a = T[r * 5 + c];
+          A[j + (int64_t)gi * n] = make_double2(a.x, flip_sign(a.y));
+        }
+      }
+    }
+    __syncwarp();
+  }
+  if (row) flg[i] = 1;
+}
+
+__global__ void __launch_bounds__(256) k_fix(Grp G) {
+  const int g = blockIdx.y, p = G.prob[g];
+  if (!live(G, p)) return;
+  const int n = G.nvec[p], i = blockIdx.x * 256 + threadIdx.x;
+  if (i >= n) return;
+  const int* flg = ws_of(G, g).flg;
+  double2* H = G.H + G.hs_off[p] + (int64_t)i * (n + 1);
+  double2* S = G.S + G.hs_off[p] + (int64_t)i * (n + 1);
+  const double h = H->x + (flg[i] ? 0.0 : 1.0);
+  *H = make_double2(h, 0.0);
+  if (!flg[G.nmax + i]) S->x += 1.0;
+}
+
+// ------------------------------------------------------------------ Cholesky of a diagonal block
+// One CTA of 8 warps; warp q holds columns q, q + 8, q + 16, q + 24 (lane = row), so column k is one warp's
+// registers: that warp takes the root and scales it, all apply it.
+__global__ void __launch_bounds__(256) k_potrf(Grp G, int c0) {
+  const int g = blockIdx.x, p = G.prob[g];
+  if (!live(G, p)) return;
+  const int n = G.nvec[p], w = min(NB, n - c0), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  __shared__ double2 col[2][NB];
+  __shared__ int s_bad;
+  double2* A11 = G.S + G.hs_off[p] + c0 + (int64_t)c0 * n;
+  double* rd = ws_of(G, g).rd + c0;
+  double2 a[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int j = warp + 8 * u;
+    a[u] = (lane < w && j <= lane) ? A11[lane + (int64_t)j * n] : zero2();
+  }
+  if (threadIdx.x == 0) s_bad = 0;
+  __syncthreads();
+  for (int k = 0; k < w; ++k) {
+    if (warp == (k & 7)) {
+      double2 c = zero2();
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (u == (k >> 3)) c = a[u];
+      const double akk = __shfl_sync(0xffffffffu, c.x, k);
+      const bool ok = akk > 0.0 && is_finite_bits(akk);
+      const double q = ok ? akk : 1.0, r = rsqrt(q), r0 = q * r;
+      const double dk = fma(fma(-r0, r0, q), 0.5 * r, r0);
+      double2 l = make_double2(c.x * r, c.y * r);
+      if (lane == k) l = make_double2(dk, 0.0);
+      if (lane < k) l = zero2();
+      col[k & 1][lane] = l;
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (u == (k >> 3)) a[u] = l;
+      if (lane == 0) {
+        rd[k] = r;
+        if (!ok) s_bad = 1;
+      }
+    }
+    __syncthreads();
+    const double2 li = col[k & 1][lane];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int j = warp + 8 * u;
+      if (j > k && j < w) a[u] = cfms_conj(li, col[k & 1][j], a[u]);
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const int j = warp + 8 * u;
+    if (lane < w && j <= lane && j < w) A11[lane + (int64_t)j * n] = a[u];
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_bad) G.status[p] = SKN_ERR_NOT_SPD;
+}
+
+// ------------------------------------------------------------------ triangular solves and slicing
+constexpr int ST = 64;               // rows or columns per CTA
+
+// x L11^H = a for one row: right-looking, so the updates of a step are independent.
+template <bool R>
+SKN_DEVINL void solve_row(double2* x, const double2* Lt, const double* rd) {
+#pragma unroll
+  for (int j = 0; j < NB; ++j) {
+    x[j].x *= rd[j];
+    if constexpr (!R) x[j].y *= rd[j];
+#pragma unroll
+    for (int k = j + 1; k < NB; ++k) x[k] = fms_cj<R>(x[j], Lt[k + j * LDT], x[k]);
+  }
+}
+// L11 x = a for one column.
+template <bool R>
+SKN_DEVINL void solve_col(double2* x, const double2* Lt, const double* rd) {
+#pragma unroll
+  for (int j = 0; j < NB; ++j) {
+    x[j].x *= rd[j];
+    if constexpr (!R) x[j].y *= rd[j];
+#pragma unroll
+    for (int k = j + 1; k < NB; ++k) x[k] = fms<R>(Lt[k + j * LDT], x[j], x[k]);
+  }
+}
+
+// The diagonal block of L, unit beyond its width w (so partial panels solve as whole ones).
+SKN_DEVINL void load_diag(const double2* L11, int n, int w, const double* rd, double2* Lt, double* rds) {
+  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
+    const int i = e % NB, j = e / NB;
+    Lt[i + j * LDT] = (i < w && j < w && i >= j) ? L11[i + (int64_t)j * n] : zero2();
+  }
+  if (threadIdx.x < NB) rds[threadIdx.x] = threadIdx.x < w ? rd[threadIdx.x] : 1.0;
+  __syncthreads();
+}
+
+// MODE 1 (Cholesky sweep): CTAs [0, nrow): rows below the panel of S, x L11^H = a, sliced as both operands;
+// the others: columns of the block row of H, L11 x = a, conjugated and sliced as column operand.
+// MODE 2 (second sweep): CTAs [0, nrow): rows from the panel's own down of H, x L11^H = a, sliced as row operand;
+// the others: rows of L21 sliced as column operand.
+template <bool R, int MODE>
+SKN_DEVINL void solve_body(const Grp& G, int g, int p, int c0, int nrow, double2* Lt, double* rds) {
+  const int n = G.nvec[p], w = min(NB, n - c0);
+  const WS ws = ws_of(G, g);
+  double2* S = G.S + G.hs_off[p];
+  double2* H = G.H + G.hs_off[p];
+  load_diag(S + c0 + (int64_t)c0 * n, n, w, ws.rd + c0, Lt, rds);
+  const bool first = blockIdx.x < nrow;
+  double2 x[NB];
+  if (first) {
+    double2* A = MODE == 1 ? S : H;
+    const int r = (MODE == 1 ? c0 + NB : c0) + blockIdx.x * ST + threadIdx.x;
+    if (r >= n) return;
+    double2* row = A + r + (int64_t)c0 * n;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) x[j] = j < w ? ld<R>(row + (int64_t)j * n) : zero2();
+    solve_row<R>(x, Lt, rds);
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (j < w) row[(int64_t)j * n] = R ? make_double2(x[j].x, 0.0) : x[j];
+    if (r >= c0 + NB)
+      slice_row([&](int k) { return row[(int64_t)k * n]; }, r, ws.nr, ws.sa, ws.ea, MODE == 1 ? ws.sb : nullptr, ws.eb,
+                false);
+  } else if (MODE == 1) {
+    const int c = (blockIdx.x - nrow) * ST + threadIdx.x;
+    if (c >= n) return;
+    double2* col = H + c0 + (int64_t)c * n;
+#pragma unroll
+    for (int j = 0; j < NB; ++j) x[j] = j < w ? ld<R>(col + j) : zero2();
+    solve_col<R>(x, Lt, rds);
+#pragma unroll
+    for (int j = 0; j < NB; ++j)
+      if (j < w) col[j] = R ? make_double2(x[j].x, 0.0) : x[j];
+    if (c0 + NB < n)
+      slice_row([&](int k) { const double2 z = col[k]; return make_double2(z.x, flip_sign(z.y)); }, c, ws.nr, nullptr,
+                nullptr, ws.sc, ws.ec, false);
+  } else {
+    const int r = c0 + NB + (blockIdx.x - nrow) * ST + threadIdx.x;
+    if (r >= n) return;
+    const double2* row = S + r + (int64_t)c0 * n;
+    slice_row([&](int k) { return row[(int64_t)k * n]; }, r, ws.nr, nullptr, nullptr, ws.sb, ws.eb, false);
+  }
+}
+
+template <int MODE>
+__global__ void __launch_bounds__(ST) k_solve(Grp G, int c0, int nrow) {
+  const int g = blockIdx.y, p = G.prob[g];
+  if (!live(G, p)) return;
+  __shared__ double2 Lt[NB * LDT];
+  __shared__ double rds[NB];
+  if (is_real(G, p))
+    solve_body<true, MODE>(G, g, p, c0, nrow, Lt, rds);
+  else
+    solve_body<false, MODE>(G, g, p, c0, nrow, Lt, rds);
+}
+
+// ------------------------------------------------------------------ tensor-core update
+SKN_DEVINL uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
+
+// Shared-memory matrix descriptor: no swizzle, K-major core matrices (8 rows x 16 bytes), 128 bytes between core
+// matrices along K, KP * 16 bytes between 8-row groups.
+SKN_DEVINL uint64_t tc_desc(uint32_t addr) {
+  uint64_t d = 0;
+  d |= (uint64_t)((addr >> 4) & 0x3FFFu);
+  d |= (uint64_t)((128u >> 4) & 0x3FFFu) << 16;
+  d |= (uint64_t)(((KP * 16u) >> 4) & 0x3FFFu) << 32;
+  d |= (uint64_t)1 << 46;
+  return d;
+}
+// kind::f16: D F32, A and B BF16, both K-major, M = 128, N columns
+SKN_DEVINL uint32_t tc_idesc(int N) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+}
+SKN_DEVINL void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
+      "}\n" ::"r"(tmem_d),
+      "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
+}
+constexpr long long WAIT_LIMIT = 1LL << 26;
+SKN_DEVINL void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+SKN_DEVINL void bar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+SKN_DEVINL void tmem_ld8(uint32_t a, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(a));
+}
+
+constexpr int A_BYTES = BM * KP * 2;                 // 16 KB: one slice of a tile's rows
+constexpr int BH_BYTES = BN * KP * 2;                // 2 KB: one slice of a tile's columns, one form
+constexpr int B_BYTES = SLICES * 2 * BH_BYTES;       // 32 KB
+constexpr int UPD_SMEM = SLICES * A_BYTES + 2 * B_BYTES;       // 192 KB
+constexpr uint32_t BUF_COLS = SLICES * 2 * BN;       // TMEM columns of one tile
+constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
+constexpr int UPD_THREADS = 32 * 9;
+
+// Wait for a phase of a barrier; gives up after WAIT_LIMIT polls or once the CTA has failed.
+SKN_DEVINL bool upd_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
+  for (long long it = 0; it < WAIT_LIMIT; ++it) {
+    uint32_t done;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t"
+        "}\n"
+        : "=r"(done)
+        : "r"(bar), "r"(parity)
+        : "memory");
+    if (done) return true;
+    if ((it & 1023) == 1023 && *fail) return false;
+  }
+  return false;
+}
+
+// C -= A B^T over BM x BN tiles.  SWEEP 1: blocks [0, nlow) of S22 (lower triangle, columns from sb), the rest
+// of H below the panel over all columns (sc); SWEEP 2 and 3: the trailing lower triangle of H (sb).
+// c1: first row and column of the trailing matrix.  A CTA has one 128-row block I and up to jc column tiles: its
+// 8 row slices stay in shared memory (128 KB), the column slices and the accumulators are double-buffered.
+// Thread 256 copies and issues the products of every slice pair of level < SLICES; warps 0-3 and 4-7 take the even and
+// the odd tiles: a thread has a row, fetches its entries of C while the products run, adds the levels exactly in
+// int64 and rounds once.  At n = 492 x 300 problems a tile took 39k clocks of an SM with one tile per CTA.
+// All waits are bounded; one that runs out marks the problem SKN_ERR_CUDA and leaves the tile, and the
+// copies and products that were issued are still waited for (bounded).
+template <int SWEEP>
+__global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nlow, int chunks_low, int chunks_all,
+                                                           int jc) {
+  const int g = blockIdx.y, p = G.prob[g];
+  if (!live(G, p)) return;
+  const int n = G.nvec[p], m = n - c1;
+  if (m <= 0 || (SWEEP == 3 && m == 1)) return;      // the panel kernel has finished a lone last entry
+  const bool low = SWEEP != 1 || blockIdx.x < nlow;
+  const int bx = low ? blockIdx.x : blockIdx.x - nlow;
+  const int I = bx / (low ? chunks_low : chunks_all), ch = bx % (low ? chunks_low : chunks_all);
+  const int r0 = I * BM;
+  if (r0 >= m) return;
+  // tile columns of the block: the lower triangle ends with the block's last row
+  const int nj = low ? cdiv_d(min(m, r0 + BM), BN) : cdiv_d(n, BN);
+  const int j0 = ch * jc, ntile = min(jc, nj - j0);
+  if (ntile <= 0) return;
+  const WS w = ws_of(G, g);
+  const uint16_t* sB = low ? w.sb : w.sc;
+  const int* eB = low ? w.eb : w.ec;
+  const int boff = low ? c1 : 0;                     // matrix column (and slice row) of tile column 0
+  const int arow = c1 + r0;
+  extern __shared__ __align__(1024) uint8_t smem[];
+  const uint32_t a0 = smem_u32(smem), b0 = a0 + SLICES * A_BYTES;
+  __shared__ __align__(8) uint64_t bars[SLICES + 6];  // row slices landed; columns landed; products done; drained
+  __shared__ uint32_t tmem_slot;
+  __shared__ volatile int s_fail;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  auto bar = [&](int b) { return smem_u32(&bars[b]); };
+  constexpr int B_FULL = SLICES, T_FULL = SLICES + 2, T_EMPTY = SLICES + 4;
+  if (tid == 0) {
+    s_fail = 0;
+    for (int b = 0; b < T_EMPTY; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar(b)));
+    for (int b = T_EMPTY; b < T_EMPTY + 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(bar(b)));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  if (warp == 8) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"(TMEM_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_slot;
+  if (warp == 8) {
+    if (lane == 0) {
+      auto load_b = [&](int i) {
+        const uint32_t bb = bar(B_FULL + (i & 1)), dst = b0 + (uint32_t)((i & 1) * B_BYTES);
+        bar_expect(bb, B_BYTES);
+        const int64_t row = boff + (j0 + i) * BN;
+        for (int t = 0; t < SLICES; ++t)
+          for (int f = 0; f < 2; ++f)
+            bulk_g2s(dst + (uint32_t)((2 * t + f) * BH_BYTES), sB + ((int64_t)(f * SLICES + t) * w.nr + row) * KP, BH_BYTES,
+                     bb);
+      };
+      for (int s = 0; s < SLICES; ++s) {
+        bar_expect(bar(s), A_BYTES);
+        bulk_g2s(a0 + (uint32_t)(s * A_BYTES), w.sa + ((int64_t)s * w.nr + arow) * KP, A_BYTES, bar(s));
+        if (s == 0) load_b(0);
+      }
+      int loaded = 1, issued = 0, landed = 0, a_landed = 0, finished = 0;   // tiles (or row slices) so far
+      if (ntile > 1) {
+        load_b(1);
+        loaded = 2;
+      }
+      bool ok = true;
+      for (int i = 0; ok && i < ntile; ++i) {
+        const int b = i & 1;
+        ok = upd_wait(bar(B_FULL + b), (uint32_t)((i >> 1) & 1), &s_fail);
+        if (!ok) break;
+        ++landed;
+        if (i >= 2) ok = upd_wait(bar(T_EMPTY + b), (uint32_t)(((i >> 1) - 1) & 1), &s_fail);
+        if (!ok) break;
+        asm volatile("tcgen05.fence::after_thread_sync;");
+        const uint32_t bs = b0 + (uint32_t)(b * B_BYTES), td = tmem + (uint32_t)b * BUF_COLS;
+        for (int s = 0; s < SLICES; ++s) {
+          if (i == 0) {
+            ok = upd_wait(bar(s), 0, &s_fail);
+            if (!ok) break;
+            ++a_landed;
+            asm volatile("tcgen05.fence::after_thread_sync;");
+          }
+          // row slice s by the column slices 0 .. SLICES - 1 - s side by side: levels s .. SLICES - 1 in one product
+          const uint32_t id = tc_idesc((SLICES - s) * 2 * BN);
+#pragma unroll
+          for (int kk = 0; kk < KP / 16; ++kk)
+            tc_mma(td + (uint32_t)(s * 2 * BN), tc_desc(a0 + (uint32_t)(s * A_BYTES) + kk * 256), tc_desc(bs + kk * 256),
+                   id, (s > 0 || kk > 0) ? 1u : 0u);
+        }
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
+            bar(T_FULL + b)));
+        ++issued;
+        if (!ok) break;
+        if (i >= 1 && i + 1 < ntile) {                // the other column buffer, once tile i - 1 has been multiplied
+          ok = upd_wait(bar(T_FULL + (b ^ 1)), (uint32_t)(((i - 1) >> 1) & 1), &s_fail);
+          if (!ok) break;
+          finished = i;
+          load_b(i + 1);
+          ++loaded;
+        }
+      }
+      // whatever was issued must have completed before the CTA frees its TMEM and exits
+      if (!ok) s_fail = 1;
+      volatile int never = 0;
+      for (; a_landed < SLICES; ++a_landed)
+        if (!upd_wait(bar(a_landed), 0, &never)) ok = false;
+      for (; landed < loaded; ++landed)
+        if (!upd_wait(bar(B_FULL + (landed & 1)), (uint32_t)((landed >> 1) & 1), &never)) ok = false;
+      for (; finished < issued; ++finished)
+        if (!upd_wait(bar(T_FULL + (finished & 1)), (uint32_t)((finished >> 1) & 1), &never)) ok = false;
+      if (!ok) s_fail = 1;
+    }
+  } else {
+    const int grp = warp >> 2, wq = warp & 3;        // a warp reads TMEM lanes 32 (warp mod 4) .. + 31
+    const int i = r0 + wq * 32 + lane;               // trailing row
+    const bool rok = i < m;
+    const int er = rok ? w.ea[c1 + i] : 0;
+    double2* C = (SWEEP == 1 && low ? G.S : G.H) + G.hs_off[p] + c1 + i;
+    const uint32_t base = tmem + (uint32_t)grp * BUF_COLS + ((uint32_t)(wq * 32) << 16);
+    for (int it = grp; it < ntile; it += 2) {
+      const int q0 = (j0 + it) * BN;                 // tile's first column, counted from boff
+      double2 cv[8];
+      auto fetch = [&](int cb) {
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int gc = boff + q0 + cb + q;
+          cv[q] = zero2();
+          if (rok && gc < n && (!low || i >= q0 + cb + q)) cv[q] = C[(int64_t)gc * n];
+        }
+      };
+      fetch(0);
+      const bool ok = upd_wait(bar(T_FULL + grp), (uint32_t)((it >> 1) & 1), &s_fail);
+      if (!ok || s_fail) {
+        s_fail = 1;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;");
+#pragma unroll 1
+      for (int cb = 0; cb < BN; cb += 8) {
+        long long hr[8], lr[8], hi[8], li[8];
+        if (cb > 0) fetch(cb);
+        // integers below 2^22: the FP32 addition of 1.5 2^23 leaves them in the low bits; two levels fit 32 bits
+        auto pair = [&](int L, int part, int* out) {
+          uint32_t u[8], v[8];
+          tmem_ld8(base + (uint32_t)(L * 2 * BN + part * BN + cb), u);
+          tmem_ld8(base + (uint32_t)((L + 1) * 2 * BN + part * BN + cb), v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;");
+#pragma unroll
+          for (int q = 0; q < 8; ++q)
+            out[q] = (__float_as_int(__uint_as_float(u[q]) + 12582912.0f) - 0x4B400000) * 128 +
+                     (__float_as_int(__uint_as_float(v[q]) + 12582912.0f) - 0x4B400000);
+        };
+#pragma unroll
+        for (int part = 0; part < 2; ++part) {
+          int p0[8], p1[8];
+          pair(0, part, p0);
+          pair(2, part, p1);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) (part ? hi : hr)[q] = (long long)p0[q] * 16384 + p1[q];
+          pair(4, part, p0);
+          pair(6, part, p1);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) (part ? li : lr)[q] = (long long)p0[q] * 16384 + p1[q];
+        }
+        if (cb + 8 == BN) {                          // the accumulators have been read: the next tile may start
+          asm volatile("tcgen05.fence::before_thread_sync;");
+          if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(T_EMPTY + grp)) : "memory");
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+          const int j = q0 + cb + q, gc = boff + j;
+          if (rok && gc < n && (!low || i >= j)) {
+            double2 v = cv[q];
+            const int ec = eB[gc];
+            if (er == EXP_NAN || ec == EXP_NAN) {
+              v = make_double2(__longlong_as_double(0x7ff8000000000000LL), __longlong_as_double(0x7ff8000000000000LL));
+            } else {
+              const int e = er + ec - 63;            // the sums count units of 2^(er + ec - 63)
+              v.x -= round_sum28(hr[q], lr[q], e);
+              v.y = (low && i == j) ? 0.0 : v.y - round_sum28(hi[q], li[q], e);
+            }
+            C[(int64_t)gc * n] = v;
+          }
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (tid == 0 && s_fail) G.status[p] = SKN_ERR_CUDA;
+  if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+}
+
+// ------------------------------------------------------------------ tridiagonalisation panel
+// Columns c0 .. c0 + w - 1 by one cluster of CTAs per problem, in zlatrd order.  Rows are counted from c0;
+// 32-row chunk c belongs to CTA c mod C (a warp per chunk, lane = row); the 32 x 32 tiles of the lower triangle
+// are dealt to the cluster's warps.  A column takes two cluster barriers:
+//   after the column's update: its norm (per chunk);
+//   after the products: y = A22 v (a slot per tile row and column), [W V]^H v (per chunk), v^H A22 v (per tile).
+// Then w = tau (y - V (W^H v) - W (V^H v)) + alpha v with alpha = -|tau|^2 / 2 (v^H A22 v - 2 Re (W^H v)^H (V^H v)),
+// which needs no further reduction, and the next column's update runs on the same rows in the same pass.
+// Every CTA computes W's entry of the next pivot row itself, with the same operations.
+// A tile is read once for both products: lane = row on the way in (A v), lane = column from shared memory (A^H v).
+// The FP64 unit belongs to one of the SM's four partitions: a warp issues one FP64 instruction per 64 clocks,
+// however independent its instructions are, so a phase is as long as its busiest warp.
+// RES: a CTA's tiles and its rows of [W V] fit its shared memory and stay there for the panel's 16 columns, and
+// its four warps share every tile (8 columns each), chunk and sum: the form for few problems.  Else a warp takes
+// whole tiles, streamed, and the CTAs of other problems fill the partitions: the form for many.  Both add in the
+// same order (quarters of a tile or chunk, then (0 + 1) + (2 + 3)), so the results are the same bits.
+constexpr int PW = 4;                            // warps per CTA, one per partition
+constexpr int PT = 32 * PW;
+constexpr int TILE_LD = TS + 1;
+constexpr int TILE_EL = TS * TILE_LD;            // a resident tile, or a chunk's 32 columns of [W V]
+constexpr int QT = TS / PW;                      // columns or rows of a quarter; columns staged when streamed
+constexpr int VMAX = (PANELS_MAX_N + PT - 1) / PT;
+struct PanelSm {
+  double2 rowV[NT], rowW[NT];                    // V and W at the next pivot row
+  double2 part[PW][2 * NT];                      // [W V]^H v by quarters of the chunks
+  double2 t12[PW][2 * NT];                       // W^H v, V^H v: a copy per warp
+  double2 tau, scl, yrow, wrow;
+  double vav, alpha;
+  int triv, pad;
+};
+
+SKN_DEVINL void tile_ij(int t, int& I, int& J) {     // lower-triangle tile index, I >= J
+  int i = (int)((sqrtf(8.0f * (float)t + 1.0f) - 1.0f) * 0.5f);
+  while (i > 0 && i * (i + 1) / 2 > t) --i;
+  while ((i + 1) * (i + 2) / 2 <= t) ++i;
+  I = i;
+  J = t - i * (i + 1) / 2;
+}
+template <bool R> SKN_DEVINL double2 sum4(double2 a, double2 b, double2 c, double2 d) {
+  return add<R>(add<R>(a, b), add<R>(c, d));
+}
+
+// sv: the Householder vector; big: streamed, a quarter of a tile per warp; RES, tiles (rt), chunks of [W V] (cpc), partial
+// sums of tiles (rt x PW x 32), of diagonal tiles (rt x 32) and of chunks (2 x cpc x PW x 32).
+template <bool R, bool RES>
+SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, int cpc, PanelSm& sm, double2* sv,
+                           double2* big) {
+  cg::cluster_group cl = cg::this_cluster();
+  const int rank = (int)cl.block_rank();
+  const int n = G.nvec[p], M = n - c0, w = min(NT, n - 1 - c0);
+  const int nt = cdiv_d(M, TS), ntile = nt * (nt + 1) / 2;
+  const WS ws = ws_of(G, g);
+  double2* A = G.H + G.hs_off[p] + c0 + (int64_t)c0 * n;      // entry (r, c) of the trailing block at r + c n
+  double2* W = ws.W;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  double* tri = G.tri ? G.tri + 4 * G.eig_off[p] : nullptr;
+  double2* wvs = big + (int64_t)rt * TILE_EL;      // chunk lc, column q, row r at lc TILE_EL + q TILE_LD + r
+  double2* yps = wvs + (int64_t)cpc * TILE_EL;     // tile i, quarter q, row r at (i PW + q) TS + r
+  double2* zds = yps + (int64_t)rt * PW * TS;      // diagonal tile i, column c at i TS + c
+  double2* eps = zds + (int64_t)rt * TS;           // chunk lc, quarter q, (y, a), row r at ((lc PW + q) 2 + part) TS + r
+  auto sync = [&]() {
+    if (C > 1) cl.sync(); else __syncthreads();
+  };
+  // chunks and tiles of this CTA are rank, rank + C, ...; streamed, a warp takes every PW-th of them
+  const int first = RES ? rank : rank + C * warp, stride = RES ? C : C * PW;
+  if constexpr (RES) {
+    for (int t = rank, i = 0; t < ntile; t += C, ++i) {
+      int I, J;
+      tile_ij(t, I, J);
+      const int gi = I * TS + lane;
+      double2* T = big + (int64_t)i * TILE_EL;
+#pragma unroll
+      for (int u = 0; u < QT; ++u) {
+        const int c = warp * QT + u, gj = J * TS + c;
+        double2 a = (gi < M && gj < M && gi >= gj) ? ld<R>(A + gi + (int64_t)gj * n) : zero2();
+        if (!R && gi == gj) a.y = 0.0;
+        T[c * TILE_LD + lane] = a;
+      }
+    }
+  }
+  // first column as it stands
+  for (int ch = rank + C * warp; ch < nt; ch += C * PW) {
+    const int r = ch * 32 + lane;
+    double2 a = zero2();
+    if (r < M) {
+      a = ld<R>(A + r);
+      if (r == 0) a.y = 0.0;
+      st<R>(ws.xc + r, a);
+      if (r == 0) ws.d[c0] = a.x;
+    }
+    double s = r >= 2 && r < M ? (R ? a.x * a.x : fma(a.x, a.x, a.y * a.y)) : 0.0;
+    s = warp_sum<true>(make_double2(s, 0.0)).x;
+    if (lane == 0) ws.sN[ch] = s;
+  }
+  for (int j = 0; j < w; ++j) {
+    const int k = c0 + j;
+    sync();
+    // ---- the reflector: two warps take the norm, one the quotient by beta, one the scale of v; meanwhile the column arrives
+    double2 xv[VMAX];
+#pragma unroll
+    for (int u = 0; u < VMAX; ++u) {
+      const int r = tid + u * PT;
+      if (u * PT < nt * 32) xv[u] = (r > j + 1 && r < M) ? ldc<R>(ws.xc + r) : zero2();
+    }
+    if (warp < 2) {
+      const double2 al = ldc<R>(ws.xc + j + 1);
+      double s = 0.0;
+      for (int c = lane; c < nt; c += 32) s += __ldcg(ws.sN + c);
+      const double xnorm2 = warp_sum<true>(make_double2(s, 0.0)).x;
+      const bool triv = xnorm2 == 0.0 && al.y == 0.0;
+      const double q = triv ? 1.0 : fma(al.x, al.x, fma(al.y, al.y, xnorm2));
+      const double inv = rsqrt(q), r0 = q * inv;                 // a root and its reciprocal from one instruction chain
+      const double nrm = fma(fma(-r0, r0, q), 0.5 * inv, r0);
+      const bool up = al.x >= 0.0;
+      const double beta = triv ? al.x : (up ? -nrm : nrm), ib = up ? -inv : inv;
+      if (warp == 0) {
+        const double taur = triv ? 0.0 : (beta - al.x) * ib;
+        const double taui = (R || triv) ? 0.0 : -al.y * ib;
+        if (lane == 0) {
+          sm.tau = make_double2(taur, taui);
+          sm.triv = triv;
+          if (rank == 0) {
+            ws.e2[k] = beta * beta;
+            if (tri) {
+              tri[n + k] = beta;
+              tri[2 * n + 2 * k] = taur;
+              tri[2 * n + 2 * k + 1] = taui;
+            }
+          }
+        }
+      } else if (warp == 1) {
+        const double dr = al.x - beta, di = al.y;
+        const double den = triv ? 0.0 : 1.0 / fma(dr, dr, di * di);
+        if (lane == 0) sm.scl = make_double2(dr * den, -di * den);
+      }
+    }
+    __syncthreads();
+    const int triv = sm.triv;
+    const double2 tau = sm.tau, scl = sm.scl;
+#pragma unroll
+    for (int u = 0; u < VMAX; ++u) {
+      const int r = tid + u * PT;
+      if (u * PT < nt * 32 && r < nt * 32) {
+        double2 v = xv[u];
+        if (r == j + 1) v = make_double2(1.0, 0.0);
+        else if (!triv) v = mul<R>(v, scl);
+        sv[r] = v;
+        if (r > j && r < M && (r >> 5) % C == rank) {
+          st<R>(A + r + (int64_t)j * n, v);
+          if constexpr (RES) wvs[((r >> 5) / C) * TILE_EL + (NT + j) * TILE_LD + (r & 31)] = v;
+          st<R>(ws.VW + (int64_t)r * 2 * NT + NT + j, v);
+        }
+      }
+    }
+    __syncthreads();
+    // ---- products with v
+    // y of tile t's rows, z of its columns; lane = row, then column
+    auto put_tile = [&](int t, int I, int J, double2 y, double2 z) {
+      const int gi = I * TS + lane;
+      const bool diag = I == J;
+      if (diag) y = add<R>(y, z);
+      if (gi < M) st<R>(ws.Yp + (int64_t)J * n + gi, y);
+      const double2 vi = sv[gi];
+      double s = R ? vi.x * y.x : fma(vi.x, y.x, vi.y * y.y);   // Re conj(v) y
+      s = warp_sum<true>(make_double2(s, 0.0)).x;
+      if (lane == 0) ws.sT[t] = diag ? s : 2.0 * s;
+    };
+    if (!triv) {
+      if constexpr (RES) {
+        const int qc = lane & (QT - 1), qr = lane / QT;        // this lane's column and rows of the transposed quarter
+        for (int t = rank, i = 0; t < ntile; t += C, ++i) {
+          int I, J;
+          tile_ij(t, I, J);
+          const bool diag = I == J;
+          const double2* T = big + (int64_t)i * TILE_EL;
+          const double2 *vI = sv + I * TS, *vJ = sv + J * TS + warp * QT;
+          double2 y = zero2(), z = zero2();
+          const double2* Tq = T + warp * QT * TILE_LD;
+          const double2* Tc = Tq + qc * TILE_LD;
+          const int cc = warp * QT + qc;
+#pragma unroll
+          for (int u = 0; u < QT; ++u) {
+            y = fma_<R>(Tq[u * TILE_LD + lane], vJ[u], y);
+            const int r = qr * QT + u;
+            if (!diag || r != cc) z = fma_cja<R>(Tc[r], vI[r], z);
+          }
+          yps[(i * PW + warp) * TS + lane] = y;
+          z.x += __shfl_xor_sync(0xffffffffu, z.x, QT);
+          z.x += __shfl_xor_sync(0xffffffffu, z.x, 2 * QT);
+          if constexpr (!R) {
+            z.y += __shfl_xor_sync(0xffffffffu, z.y, QT);
+            z.y += __shfl_xor_sync(0xffffffffu, z.y, 2 * QT);
+          }
+          if (lane < QT) {
+            if (diag) zds[i * TS + cc] = z;
+            else if (J * TS + cc < M) st<R>(ws.Yp + (int64_t)I * n + J * TS + cc, z);
+          }
+        }
+      } else {
+        double2* T = big + (int64_t)warp * QT * TILE_LD;
+        const int qc = lane & (QT - 1), qr = lane / QT;
+        for (int t = first; t < ntile; t += stride) {
+          int I, J;
+          tile_ij(t, I, J);
+          const int gi = I * TS + lane;
+          const bool diag = I == J;
+          const double2 *vI = sv + I * TS + qr * QT, *vJ = sv + J * TS;
+          const double2* col = A + gi + (int64_t)(J * TS) * n;
+          double2 y01 = zero2(), y2 = zero2(), y = zero2(), z = zero2();
+#pragma unroll
+          for (int q = 0; q < PW; ++q) {
+            double2 a[QT];
+#pragma unroll
+            for (int u = 0; u < QT; ++u) {
+              const int gj = J * TS + q * QT + u;
+              a[u] = (gi < M && gj < M && gi >= gj) ? ld<R>(col + (int64_t)(q * QT + u) * n) : zero2();
+              if (!R && gi == gj) a[u].y = 0.0;
+            }
+            __syncwarp();
+            double2 yq = zero2();
+#pragma unroll
+            for (int u = 0; u < QT; ++u) {
+              yq = fma_<R>(a[u], vJ[q * QT + u], yq);
+              T[u * TILE_LD + lane] = a[u];
+            }
+            if (q == 0) y01 = yq;
+            if (q == 1) y01 = add<R>(y01, yq);
+            if (q == 2) y2 = yq;
+            if (q == 3) y = add<R>(y01, add<R>(y2, yq));
+            __syncwarp();
+            double2 zq = zero2();
+            const double2* Tc = T + qc * TILE_LD + qr * QT;
+#pragma unroll
+            for (int u = 0; u < QT; ++u)
+              if (!diag || qr * QT + u != q * QT + qc) zq = fma_cja<R>(Tc[u], vI[u], zq);
+            zq.x += __shfl_xor_sync(0xffffffffu, zq.x, QT);
+            zq.x += __shfl_xor_sync(0xffffffffu, zq.x, 2 * QT);
+            if constexpr (!R) {
+              zq.y += __shfl_xor_sync(0xffffffffu, zq.y, QT);
+              zq.y += __shfl_xor_sync(0xffffffffu, zq.y, 2 * QT);
+            }
+            if (qr == q) z = zq;
+          }
+          if (!diag && J * TS + lane < M) st<R>(ws.Yp + (int64_t)I * n + J * TS + lane, z);
+          put_tile(t, I, J, y, z);
+        }
+      }
+      if (j > 0) {
+        // lane = column of [W V]: W columns 0..j-1 and V columns NT..NT+j-1; a sum per 8 rows
+        const bool on = lane < NT ? lane < j : lane - NT < j;
+        for (int ch = first; ch < nt; ch += stride) {
+          for (int q = RES ? warp : 0; q < (RES ? warp + 1 : PW); ++q) {
+            double2 s = zero2();
+            if (on) {
+              const double2* src = RES ? wvs + (ch / C) * TILE_EL + lane * TILE_LD - ch * 32 : ws.VW + lane;
+              const int64_t step = RES ? 1 : 2 * NT;
+              const int r1 = min(M, ch * 32 + (q + 1) * QT);
+#pragma unroll 4
+              for (int r = max(ch * 32 + q * QT, j + 1); r < r1; ++r)
+                s = fma_cja<R>(ld<R>(src + (int64_t)r * step), sv[r], s);
+              st<R>(ws.sD + (ch * PW + q) * 2 * NT + lane, s);
+            }
+          }
+        }
+      }
+      if constexpr (RES) {
+        __syncthreads();
+        for (int t = rank + C * warp, i = warp; t < ntile; t += C * PW, i += PW) {
+          int I, J;
+          tile_ij(t, I, J);
+          const double2* yp = yps + i * PW * TS + lane;
+          put_tile(t, I, J, sum4<R>(yp[0], yp[TS], yp[2 * TS], yp[3 * TS]), zds[i * TS + lane]);
+        }
+      }
+    }
+    // the next column of the panel, or (last panel) the one remaining entry, the last diagonal element
+    const bool next = j + 1 < w || j + 2 == M;
+    sync();
+    // ---- W's column j; the next column
+    {
+      const bool on = lane < NT ? lane < j : lane - NT < j;
+      double2 s = zero2();
+      if (!triv && on) {
+#pragma unroll 4
+        for (int c = 0; c < nt; ++c) s = add<R>(s, ldc<R>(ws.sD + (c * PW + warp) * 2 * NT + lane));
+      }
+      sm.part[warp][lane] = s;
+      if (!triv && warp == 1) {
+        double q = 0.0;
+#pragma unroll 4
+        for (int t = lane; t < ntile; t += 32) q += __ldcg(ws.sT + t);
+        q = warp_sum<true>(make_double2(q, 0.0)).x;
+        if (lane == 0) sm.vav = q;
+      } else if (!triv && warp == 2) {
+        double2 q = zero2();
+        for (int t = lane; t < nt; t += 32) q = add<R>(q, ldc<R>(ws.Yp + (int64_t)t * n + j + 1));
+        q = warp_sum<R>(q);
+        if (lane == 0) sm.yrow = q;
+      } else if (warp == 3 && lane < j) {
+        sm.rowV[lane] = ldc<R>(A + (j + 1) + (int64_t)lane * n);
+        sm.rowW[lane] = ldc<R>(W + (int64_t)lane * n + c0 + j + 1);
+      }
+    }
+    __syncthreads();
+    double2* t12 = sm.t12[warp];
+    {
+      const double2 s = sum4<R>(sm.part[0][lane], sm.part[1][lane], sm.part[2][lane], sm.part[3][lane]);
+      t12[lane] = s;
+      if (!triv && warp == 0) {
+        // Re sum_q conj(t1_q) t2_q and the pivot row's correction: lane q < NT has t1_q, lane NT + q has t2_q
+        const double2 o = make_double2(__shfl_down_sync(0xffffffffu, s.x, NT),
+                                       R ? 0.0 : __shfl_down_sync(0xffffffffu, s.y, NT));
+        double2 c = zero2();
+        double dot = 0.0;
+        if (lane < j) {
+          dot = R ? s.x * o.x : fma(s.x, o.x, s.y * o.y);
+          c = mul<R>(sm.rowV[lane], s);
+          c = fma_<R>(sm.rowW[lane], o, c);
+        }
+        for (int q = 8; q > 0; q >>= 1) {
+          dot += __shfl_xor_sync(0xffffffffu, dot, q);
+          c.x += __shfl_xor_sync(0xffffffffu, c.x, q);
+          if constexpr (!R) c.y += __shfl_xor_sync(0xffffffffu, c.y, q);
+        }
+        if (lane == 0) {
+          const double t2 = R ? tau.x * tau.x : fma(tau.x, tau.x, tau.y * tau.y);
+          const double al = -0.5 * t2 * (sm.vav - 2.0 * dot);
+          double2 y = make_double2(sm.yrow.x - c.x, R ? 0.0 : sm.yrow.y - c.y);
+          y = mul<R>(tau, y);
+          y.x += al;
+          sm.wrow = y;
+          sm.alpha = al;
+        }
+      }
+      __syncwarp();
+    }
+    // quarter q of a row's sums: slots q, q + 4, ... of y, and columns 4 q .. 4 q + 3 of [W V]
+    auto quarter = [&](int ch, int q, double2& y, double2& a) {
+      const int r = ch * 32 + lane;
+      y = a = zero2();
+      if (r <= j || r >= M) return;
+      if (next && q == 0) a = ld<R>(A + r + (int64_t)(j + 1) * n);
+      if (!triv) {
+#pragma unroll 4
+        for (int s = q; s < nt; s += PW) y = add<R>(y, ldc<R>(ws.Yp + (int64_t)s * n + r));
+      }
+      const double2* ws_ = RES ? wvs + (ch / C) * TILE_EL + lane : W + c0 + r;
+      const double2* vs_ = RES ? ws_ + NT * TILE_LD : A + r;
+      const int64_t step = RES ? TILE_LD : n;
+#pragma unroll
+      for (int u = 0; u < NT / PW; ++u) {
+        const int c = q * (NT / PW) + u;
+        if (c < j) {
+          const double2 vq = ld<R>(vs_ + c * step), wq = ld<R>(ws_ + c * step);
+          if (!triv) {
+            y = fms<R>(vq, t12[c], y);
+            y = fms<R>(wq, t12[NT + c], y);
+          }
+          if (next) {
+            a = fms_cj<R>(vq, sm.rowW[c], a);
+            a = fms_cj<R>(wq, sm.rowV[c], a);
+          }
+        }
+      }
+    };
+    // the row's entry of W's column j and of the next column, from the sums
+    auto finish = [&](int ch, double2 y, double2 a) {
+      const int r = ch * 32 + lane;
+      const double2 wrow = triv ? zero2() : sm.wrow;
+      const double al = triv ? 0.0 : sm.alpha;
+      if (r > j && r < M) {
+        const double2 v = sv[r];
+        double2 wv = zero2();
+        if (!triv) {
+          wv = mul<R>(tau, y);
+          wv.x = fma(al, v.x, wv.x);
+          if constexpr (!R) wv.y = fma(al, v.y, wv.y);
+        }
+        st<R>(W + (int64_t)j * n + c0 + r, wv);
+        if constexpr (RES) wvs[(ch / C) * TILE_EL + j * TILE_LD + lane] = wv;
+        st<R>(ws.VW + (int64_t)r * 2 * NT + j, wv);
+        if (next) {
+          a = fms_cj<R>(v, wrow, a);
+          a.x -= wv.x;                                     // V at the pivot row is 1
+          if constexpr (!R) a.y -= wv.y;
+          if (r == j + 1) {
+            a.y = 0.0;
+            ws.d[k + 1] = a.x;
+          }
+          st<R>(ws.xc + r, a);
+        }
+      }
+      if (next) {
+        double s = r >= j + 3 && r < M ? (R ? a.x * a.x : fma(a.x, a.x, a.y * a.y)) : 0.0;
+        s = warp_sum<true>(make_double2(s, 0.0)).x;
+        if (lane == 0) ws.sN[ch] = s;
+      }
+    };
+    if constexpr (RES) {
+      for (int ch = rank; ch < nt; ch += C) {
+        double2 y, a;
+        quarter(ch, warp, y, a);
+        double2* e = eps + ((ch / C) * PW + warp) * 2 * TS + lane;
+        e[0] = y;
+        e[TS] = a;
+      }
+      __syncthreads();
+      for (int ch = rank + C * warp; ch < nt; ch += C * PW) {
+        const double2* e = eps + (ch / C) * PW * 2 * TS + lane;
+        finish(ch, sum4<R>(e[0], e[2 * TS], e[4 * TS], e[6 * TS]), sum4<R>(e[TS], e[3 * TS], e[5 * TS], e[7 * TS]));
+      }
+    } else {
+      __syncthreads();
+      for (int ch = first; ch < nt; ch += stride) {
+        double2 y0, y1, y2, y3, a0, a1, a2, a3;
+        quarter(ch, 0, y0, a0);
+        quarter(ch, 1, y1, a1);
+        y0 = add<R>(y0, y1);
+        a0 = add<R>(a0, a1);
+        quarter(ch, 2, y2, a2);
+        quarter(ch, 3, y3, a3);
+        finish(ch, add<R>(y0, add<R>(y2, y3)), add<R>(a0, add<R>(a2, a3)));
+      }
+    }
+    __syncthreads();
+  }
+  // slices of the rows below the panel: z = [V W], both operands
+  if (M - w > 1) {
+    for (int ch = rank + C * warp; ch < nt; ch += C * PW) {
+      const int r = ch * 32 + lane;
+      if (r < w || r >= M) continue;
+      const double2* vw = ws.VW + (int64_t)r * 2 * NT;
+      slice_row(
+          [&](int q) {
+            const int u = q < NT ? NT + q : q - NT;
+            if ((q & (NT - 1)) >= w) return zero2();
+            const double2 z = vw[u];
+            return R ? make_double2(z.x, 0.0) : z;
+          },
+          c0 + r, ws.nr, ws.sa, ws.ea, ws.sb, ws.eb, true);
+    }
+  }
+}
+
+template <bool RES>
+__global__ void __launch_bounds__(PT, RES ? 1 : 4) k_tri_panel(Grp G, int c0, int C, int rt, int cpc) {
+  const int g = blockIdx.x / C, p = G.prob[g];
+  if (!live(G, p)) return;
+  if (c0 >= G.nvec[p] - 1) return;
+  extern __shared__ __align__(16) char smem_raw[];
+  PanelSm& sm = *reinterpret_cast<PanelSm*>(smem_raw);
+  double2* sv = reinterpret_cast<double2*>(smem_raw + sizeof(PanelSm));
+  double2* big = sv + cdiv_d(G.nmax - c0, TS) * TS;
+  if (is_real(G, p))
+    panel_body<true, RES>(G, g, p, c0, C, rt, cpc, sm, sv, big);
+  else
+    panel_body<false, RES>(G, g, p, c0, C, rt, cpc, sm, sv, big);
+}
+
+// ------------------------------------------------------------------ eigenvalues
+__global__ void __launch_bounds__(256) k_bounds(Grp G) {
+  const int g = blockIdx.x, p = G.prob[g];
+  if (!live(G, p)) return;
+  const int n = G.nvec[p], tid = threadIdx.x;
+  const WS w = ws_of(G, g);
+  __shared__ double red[3 * 8];
+  if (n == 1 && tid == 0) w.d[0] = (G.H + G.hs_off[p])->x;     // no column, no panel
+  __syncthreads();
+  double lo = 1e300, hi = -1e300, emax = 0.0;
+  for (int i = tid; i < n; i += 256) {
+    const double ea = (i > 0) ? sqrt(w.e2[i - 1]) : 0.0;
+    const double eb = (i < n - 1) ? sqrt(w.e2[i]) : 0.0;
+    lo = fmin(lo, w.d[i] - ea - eb);
+    hi = fmax(hi, w.d[i] + ea + eb);
+    if (i < n - 1) emax = fmax(emax, w.e2[i]);
+    w.d32[i] = (float)w.d[i];
+    w.e232[i] = (i < n - 1) ? (float)w.e2[i] : 0.0f;
+  }
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmax(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+    emax = fmax(emax, __shfl_xor_sync(0xffffffffu, emax, o));
+  }
+  if ((tid & 31) == 0) {
+    red[tid >> 5] = lo;
+    red[8 + (tid >> 5)] = hi;
+    red[16 + (tid >> 5)] = emax;
+  }
+  __syncthreads();
+  if (tid == 0) {
+    for (int q = 1; q < 8; ++q) {
+      red[0] = fmin(red[0], red[q]);
+      red[8] = fmax(red[8], red[8 + q]);
+      red[16] = fmax(red[16], red[16 + q]);
+    }
+    w.bnd[0] = red[0];
+    w.bnd[1] = red[8];
+    w.bnd[2] = red[16];
+  }
+  if (G.tri) {
+    double* tri = G.tri + 4 * G.eig_off[p];
+    for (int i = tid; i < n; i += 256) tri[i] = w.d[i];
+    if (tid == 0) {
+      tri[2 * n - 1] = 0.0;
+      tri[4 * n - 2] = 0.0;
+      tri[4 * n - 1] = 0.0;
+    }
+  }
+}
+
+__global__ void __launch_bounds__(64) k_eig(Grp G) {
+  const int g = blockIdx.y, p = G.prob[g];
+  const int n = G.nvec[p], j = blockIdx.x * 64 + threadIdx.x;
+  const int st = G.status[p];
+  if (st == SKN_ERR_CAPACITY || j >= n) return;
+  double* out = G.eig + G.eig_off[p];
+  if (st != SKN_OK) {
+    if (st == SKN_ERR_NOT_SPD) out[j] = __longlong_as_double(0x7ff8000000000000LL);
+    return;
+  }
+  const WS w = ws_of(G, g);
+  const skn_sturm::Bounds B = skn_sturm::make_bounds(w.bnd[0], w.bnd[1], w.bnd[2], n);
+  out[j] = skn_sturm::eigenvalue(w.d, w.e2, w.d32, w.e232, n, j, B);
+}
+
+// ------------------------------------------------------------------ host sequence
+// CTAs per problem in the tridiagonalisation: as many as the GPU has room for, up to one per tile.
+int cluster_size(int n, int n_prob, int sms) {
+  const int nt = cdiv(n, TS);
+  const int tiles = nt * (nt + 1) / 2;
+  int c = 1;
+  while (c < 16 && 2 * c * n_prob <= sms && 2 * c <= tiles) c *= 2;
+  return c;
+}
+
+constexpr size_t SMEM_MAX = 227 * 1024;
+
+// Shared memory of a panel over m rows: streamed, or (rt > 0) resident with rt tiles and cpc chunks per CTA.
+size_t panel_smem(int m, int rt, int cpc) {
+  const size_t head = sizeof(PanelSm) + (size_t)cdiv(m, TS) * TS * sizeof(double2);
+  if (rt == 0) return head + (size_t)PW * QT * TILE_LD * sizeof(double2);
+  return head + ((size_t)(rt + cpc) * TILE_EL + (size_t)rt * (PW + 1) * TS + (size_t)cpc * PW * 2 * TS) * sizeof(double2);
+}
+
+cudaError_t launch_panel(const Grp& G, int c0, int C, int sms, cudaStream_t stream) {
+  const int m = G.nmax - c0, nt = cdiv(m, TS), cpc = cdiv(nt, C);
+  int rt = cdiv(nt * (nt + 1) / 2, C);
+  if (panel_smem(m, rt, cpc) > SMEM_MAX || (int64_t)G.n_prob * C > sms) rt = 0;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)G.n_prob * C);
+  cfg.blockDim = dim3(PT);
+  cfg.dynamicSmemBytes = panel_smem(m, rt, cpc);
+  cfg.stream = stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeClusterDimension;
+  at[0].val.clusterDim.x = C;
+  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return rt ? cudaLaunchKernelEx(&cfg, k_tri_panel<true>, G, c0, C, rt, cpc)
+            : cudaLaunchKernelEx(&cfg, k_tri_panel<false>, G, c0, C, rt, cpc);
+}
+
+// One update of every problem: jc column tiles per CTA, so that the GPU gets about two CTAs per SM at least.
+template <int SWEEP>
+void launch_update(const Grp& G, int c1, int sms, cudaStream_t stream) {
+  const int m = G.nmax - c1, nI = cdiv(m, BM);
+  const int jl = cdiv(m, BN), ja = SWEEP == 1 ? cdiv(G.nmax, BN) : 0;
+  const int64_t tiles = (int64_t)G.n_prob * nI * ((jl + BM / BN + 1) / 2 + ja);
+  int jc = (int)(tiles / (2 * (int64_t)sms));
+  jc = jc < 2 ? 2 : (jc > 32 ? 32 : jc);
+  const int cl = cdiv(jl, jc), ca = ja ? cdiv(ja, jc) : 1;
+  const int nlow = nI * cl;
+  k_update<SWEEP><<<dim3((unsigned)(nlow + (ja ? nI * ca : 0)), (unsigned)G.n_prob), UPD_THREADS, UPD_SMEM, stream>>>(
+      G, c1, nlow, cl, ca, jc);
+}
+
+cudaError_t run(const Grp& G, cudaStream_t stream) {
+  const int n = G.nmax, T = G.panels;
+  const unsigned P = (unsigned)G.n_prob;
+  int dev = 0, sms = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const int nt = cdiv(n, TS);
+  k_init<<<dim3(cdiv(2 * n, 256), P), 256, 0, stream>>>(G);
+  k_scan<<<dim3(cdiv(nt * nt, 8), P, 2), 256, 0, stream>>>(G);
+  k_fix<<<dim3(cdiv(n, 256), P), 256, 0, stream>>>(G);
+  for (int t = 0; t < T; ++t) {
+    const int c0 = t * NB, m = n - c0 - NB;
+    const int nrow = m > 0 ? cdiv(m, ST) : 0;
+    k_potrf<<<P, 256, 0, stream>>>(G, c0);
+    k_solve<1><<<dim3(nrow + cdiv(n, ST), P), ST, 0, stream>>>(G, c0, nrow);
+    if (m > 0) launch_update<1>(G, c0 + NB, sms, stream);
+  }
+  for (int t = 0; t < T; ++t) {
+    const int c0 = t * NB, m = n - c0 - NB;
+    const int nrow = cdiv(n - c0, ST), nl = m > 0 ? cdiv(m, ST) : 0;
+    k_solve<2><<<dim3(nrow + nl, P), ST, 0, stream>>>(G, c0, nrow);
+    if (m > 0) launch_update<2>(G, c0 + NB, sms, stream);
+  }
+  for (int c0 = 0; c0 < n - 1; c0 += NT) {
+    const cudaError_t e = launch_panel(G, c0, cluster_size(n - c0, G.n_prob, sms), sms, stream);
+    if (e != cudaSuccess) return e;
+    const int m = n - c0 - NT;
+    if (m > 1) launch_update<3>(G, c0 + NT, sms, stream);
+  }
+  k_bounds<<<P, 256, 0, stream>>>(G);
+  k_eig<<<dim3(cdiv(n, 64), P), 64, 0, stream>>>(G);
+  return cudaPeekAtLastError();
+}
+
+cudaError_t set_attrs() {
+  cudaError_t e = cudaFuncSetAttribute(k_tri_panel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SMEM_MAX);
+  if (e == cudaSuccess)
+    e = cudaFuncSetAttribute(k_tri_panel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)panel_smem(PANELS_MAX_N, 0, 0));
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tri_panel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tri_panel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_update<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_update<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_update<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM);
+  return e;
+}
+
+}  // namespace
+
+extern "C" int skn_eigh_panels_scratch_bytes(int n_prob, int max_n, int64_t* bytes) {
+  if (!bytes || n_prob < 0 || max_n < 1) return SKN_ERR_ARG;
+  if (max_n > PANELS_MAX_N) return SKN_ERR_CAPACITY;
+  *bytes = (int64_t)n_prob * layout(max_n).stride;
+  return SKN_OK;
+}
+
+extern "C" int skn_eigh_gen_panels(int n_prob, int max_n, const int32_t* prob, const int32_t* nvec, const int32_t* real,
+                                const int64_t* hs_off, const int64_t* eig_off, double* H, double* S, double* eig,
+                                int32_t* status, double* tri, double* scratch, int64_t scratch_bytes,
+                                cudaStream_t stream) {
+  if (n_prob < 0 || max_n < 1) return SKN_ERR_ARG;
+  if (n_prob == 0) return SKN_OK;
+  if (!prob || !nvec || !hs_off || !eig_off || !H || !S || !eig || !status || !scratch) return SKN_ERR_ARG;
+  if (max_n > PANELS_MAX_N || n_prob > 65535) return SKN_ERR_CAPACITY;
+  if (scratch_bytes < (int64_t)n_prob * layout(max_n).stride) return SKN_ERR_CAPACITY;
+  if ((reinterpret_cast<uintptr_t>(scratch) & 15) || (reinterpret_cast<uintptr_t>(H) & 15) ||
+      (reinterpret_cast<uintptr_t>(S) & 15))
+    return SKN_ERR_ARG;
+  if (set_attrs() != cudaSuccess) return SKN_ERR_CUDA;
+  Grp G{max_n, cdiv(max_n, NB), n_prob, prob, nvec, real, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, tri,
+        (char*)scratch};
+  return run(G, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
+}

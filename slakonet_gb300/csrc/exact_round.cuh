@@ -61,3 +61,27 @@ SKN_HD double exact_to_double(long long hi, long long lo, int e) {
   if (be <= 0 || be >= 2047) return fma((double)hi, 0x1p-35, (double)lo * 0x1p-56) * ldexp(1.0, e + 56);
   return skn_bits_to_double(sgn | ((unsigned long long)be << 52) | (m & 0xFFFFFFFFFFFFFull));
 }
+
+// The double nearest to (hi * 2^28 + lo) * 2^e (ties away from zero), for |hi| < 2^46 and |lo| < 2^46: the sum is
+// normalised in 64 bits (its 53 leading bits and one rounding increment), about 30 integer instructions.
+SKN_HD double round_sum28(long long hi, long long lo, int e) {
+  long long h = hi + (lo >> 28);
+  unsigned long long l = (unsigned long long)lo & 0xFFFFFFFull;
+  const bool neg = h < 0;
+  if (neg) {                                                  // negate the pair: l stays in [0, 2^28)
+    h = -h - (l != 0);
+    l = (0x10000000ull - l) & 0xFFFFFFFull;
+  }
+  const int lz = h ? skn_clz64((unsigned long long)h) - 11 : 53;
+  const int k = lz < 28 ? lz : 28;                            // bits of l that still fit below 53
+  const int d = 28 - k;
+  unsigned long long t = ((unsigned long long)h << k) + ((l + ((1ull << d) >> 1)) >> d);
+  if (t == 0) return 0.0;
+  int s = skn_clz64(t) - 11;                                  // below 2^52 only when k = 28: exact shift
+  s = s < 0 ? 0 : s;                                          // t = 2^53 after rounding up: carries into the exponent
+  t <<= s;
+  const int be = 1075 + d - s + e;                            // value = t 2^(d - s + e), t in [2^52, 2^53]
+  if (be <= 0 || be >= 2046) return ldexp((double)(neg ? -(long long)t : (long long)t), d - s + e);
+  return skn_bits_to_double((neg ? 0x8000000000000000ull : 0ull) + ((unsigned long long)be << 52) +
+                            (t - 0x10000000000000ull));
+}

@@ -474,6 +474,7 @@ class DeviceBatch:
         self.kwoff = _i64(plan.kw_off, dev)
         self.kw = _f64(plan.kweights, dev)
         self.ne = _f64(plan.nelec, dev)
+        self.real = _i32(plan.prob_real if plan.prob_real is not None else np.zeros(len(plan.prob_n)), dev)
         # work units of the Bloch-sum kernel per structure: ceil(nk_s / BLOCH_KCHUNK) k-chunks times the
         # N_s^2 ordered atom pairs (full matrices) or the N_s (N_s + 1) / 2 pairs on or below the diagonal
         # (lower triangles), numbered from an exclusive prefix sum
@@ -510,6 +511,40 @@ def wide_launches(n: int, nb: int = 32, tc: bool = False, tc_min: int = 512) -> 
         k += 6 * w + (r2k(n - c0 - w) if n - c0 - w > 0 else 0)
         c0 += nb
     return k + 2                              # bounds and eigenvalues
+
+
+PANEL = 32                  # panel width of the blocked eigensolver (csrc/eigh_panels.cu)
+PANELS_MAX_N = 1024         # its bound
+PANELS_SCRATCH = 2 << 30    # device bytes of scratch per call; a larger group goes through in parts
+
+
+def panels_launches(max_n: int) -> int:
+    """Kernel launches of one skn_eigh_gen_panels call (its host sequence)."""
+    T = -(-max_n // PANEL)
+    tri = -(-(max_n - 1) // 16)
+    upd = sum(1 for c0 in range(0, max_n - 1, 16) if max_n - c0 - 16 > 1)
+    return 3 + 2 * T + (T - 1) + T + (T - 1) + tri + upd + 2
+
+
+def panels_scratch_bytes(count: int, max_n: int) -> int:
+    need = ctypes.c_int64(0)
+    call("skn_eigh_panels_scratch_bytes", count, max_n, ctypes.addressof(need))
+    return int(need.value)
+
+
+SMALL_MAX_N = 96            # bound of the shared-memory eigensolver (csrc/eigh_small.cu)
+SMALL_CLASSES = (16, 24, 32, 40, 48, 56, 64, 80, 96)     # its calls' size classes: shared memory decides how many
+                                                         # CTAs share an SM
+
+
+def route_auto(n: int):
+    """Kernel and call of a problem of n orbitals under the untuned policy: ("small", class) or ("panels", number of
+    32-column panels).  A rule on the problem alone, as route_wide.  Measured on GB300 against the one-CTA kernel:
+    panels 432 orbitals x 8 problems 21 ms (193 ms), 160 x 27 5.4 ms (12.9), 128 x 1000 32 ms (32),
+    96 x 3000 50 ms (39), 492 x 300 220 ms (399); so the small kernel as far as shared memory holds a problem."""
+    if n <= SMALL_MAX_N:
+        return ("small", next(c for c in SMALL_CLASSES if n <= c))
+    return ("panels", -(-n // PANEL))
 
 
 _SIDE = threading.local()   # per-thread side streams of Engine._side_streams
@@ -618,6 +653,7 @@ class Engine:
             b.record()
             ev.append((name, a, b))
         self.launches += (wide_launches(args[1], tc=name.endswith("_tc")) if name.startswith("skn_eigh_gen_wide")
+                          else panels_launches(args[1]) if name == "skn_eigh_gen_panels"
                           else KERNELS_PER_CALL.get(name, 1))
 
     def run(self, plan: Plan, dos_range=(-10.0, 10.0), dos_points: int = 5000, dos_sigma: float = 0.1,
@@ -778,7 +814,9 @@ class Engine:
             need = ctypes.c_int64(0)
             if isinstance(shape, int):       # a cluster group
                 call("skn_eigh_large_scratch_bytes", count, max_n, shape, ctypes.addressof(need))
-            elif isinstance(shape, tuple):   # a device-wide group: ("wide", n, real)
+            elif isinstance(shape, tuple) and shape[0] == "panels":   # a blocked group: ("panels", number of panels)
+                need.value = panels_scratch_bytes(self._panels_part(count, max_n), max_n)
+            elif isinstance(shape, tuple) and shape[0] == "wide":   # a device-wide group: ("wide", n, real)
                 call("skn_eigh_wide_scratch_bytes", count, max_n, ctypes.addressof(need))
             else:
                 continue
@@ -786,7 +824,19 @@ class Engine:
         counters = torch.zeros(2 * len(groups), dtype=torch.int32, device=self.device)
 
         def launch(gi, sfx, order_g, count, max_n, st):
-            if isinstance(sfx, tuple):
+            if isinstance(sfx, tuple) and sfx[0] == "small":
+                self._call("skn_eigh_gen_small", count, max_n, ptr(order_g), ptr(db.n),
+                           ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk),
+                           ptr(eig), ptr(eig_status), 0, st)
+            elif isinstance(sfx, tuple) and sfx[0] == "panels":
+                part = self._panels_part(count, max_n)
+                real = db.real if self.real_path else None
+                for a in range(0, count, part):
+                    cnt = min(part, count - a)
+                    self._call("skn_eigh_gen_panels", cnt, max_n, ptr(order_g[a:]), ptr(db.n), ptr(real),
+                               ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), 0,
+                               ptr(scratch[gi]), int(scratch[gi].numel() * 8), st)
+            elif isinstance(sfx, tuple):
                 self._call("skn_eigh_gen_wide_tc" if self.wide_tc else "skn_eigh_gen_wide", count, max_n,
                            ptr(order_g), ptr(db.n), ptr(db.hs_off), ptr(db.eoff),
                            ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(scratch[gi]),
@@ -819,6 +869,11 @@ class Engine:
         for ev in joins:
             main.wait_event(ev)
 
+    @staticmethod
+    def _panels_part(count: int, max_n: int) -> int:
+        """Problems per skn_eigh_gen_panels call: as many as PANELS_SCRATCH holds."""
+        return max(1, min(count, PANELS_SCRATCH // max(1, panels_scratch_bytes(1, max_n))))
+
     def _side_streams(self, k):
         """k side streams for forked launches, cached per host thread and device (engines are
         created per batch by the server; creating streams per batch would cost more than the fork)."""
@@ -831,8 +886,9 @@ class Engine:
         return cur
 
     def _groups(self, db):
-        """[(launch shape suffix, the cluster size for the cluster path, or ("wide", n, real) for the
-        device-wide path, device order, count, max_n)], cached on the batch.
+        """[(launch shape suffix, the cluster size for the cluster path, ("wide", n, real) for the device-wide
+        path, or route_auto's ("small", class) or ("panels", panels), device order, count, max_n)], cached on the
+        batch.
 
         Empty when every problem takes the default single-CTA launch."""
         plan = db.plan
@@ -858,13 +914,18 @@ class Engine:
         small_order = plan.order[~large]
         if len(small_order):
             tuning = self.tuning if self.tuning is not None else _default_tuning()
-            shapes = [tuning.shape_for(int(n)) for n in plan.prob_n[small_order]]
-            if self.real_path and plan.prob_real is not None:
-                shapes = [("_real" + sh) if r else sh for sh, r in zip(shapes, plan.prob_real[small_order])]
-            shapes = np.array(shapes, dtype=object)
-            for sfx in dict.fromkeys(shapes.tolist()):
-                sel = small_order[shapes == sfx]
-                out.append((sfx, sel, len(sel), int(plan.prob_n[sel].max())))
+            ns, at = np.unique(plan.prob_n[small_order], return_inverse=True)
+            names = [tuning.shape_for(int(n)) for n in ns]
+            names = [route_auto(int(n)) if x == "auto" else x for n, x in zip(ns, names)]
+            kinds = list(dict.fromkeys(names))
+            kind = np.array([kinds.index(x) for x in names])[at]
+            if self.real_path and plan.prob_real is not None:     # one-CTA shapes: real problems in a call of their own
+                own = np.array([isinstance(x, str) for x in kinds])
+                kind = kind + len(kinds) * (plan.prob_real[small_order] & own[kind])
+            for i in dict.fromkeys(kind.tolist()):
+                sel = small_order[kind == i]
+                sfx = kinds[i % len(kinds)]
+                out.append(("_real" + sfx if i >= len(kinds) else sfx, sel, len(sel), int(plan.prob_n[sel].max())))
         if len(out) == 1 and out[0][0] == "" and out[0][2] == len(plan.order):
             out = []     # the default launch over the batch's own order
         real = plan.prob_real if (self.real_path and plan.prob_real is not None) else np.zeros(len(plan.prob_n), bool)
