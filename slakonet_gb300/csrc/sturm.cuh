@@ -88,13 +88,14 @@ __device__ __forceinline__ double secant_step(double x0, double p0, int e0, doub
   return (x1 - x0) * (1.0 / (s - 1.0));
 }
 
-// FP32 count on the rounded tridiagonal (LDL^T pivots; FP32 division is cheap).
+// FP32 count on the rounded tridiagonal (LDL^T pivots).  The bracket it gives is checked in FP64, so the quotient's
+// last bits do not matter: the two-instruction division.
 __device__ __forceinline__ int count32(const float* d, const float* e2, int n, float x, float pivmin) {
   float q = d[0] - x;
   int c = q < 0.0f;
   for (int i = 1; i < n; ++i) {
     if (fabsf(q) < pivmin) q = -pivmin;
-    q = (d[i] - x) - __fdiv_rn(e2[i - 1], q);
+    q = (d[i] - x) - __fdividef(e2[i - 1], q);
     c += q < 0.0f;
   }
   return c;
