@@ -320,30 +320,36 @@ int skn_eigh_gen_small(int n_prob, int max_n, const int32_t* prob, const int32_t
                        int32_t* status, double* tri, cudaStream_t stream);
 /*
  * Eigenvalues (and, with `tri`, the reduced form the eigenvectors start from) of
- * problems of up to 1024 orbitals, in lockstep over 32-column panels: Cholesky of
+ * problems of up to 2048 orbitals, in lockstep over 32-column panels: Cholesky of
  * S, C = L^-1 H L^-H by two blocked sweeps, Householder tridiagonalisation with
  * one cluster of CTAs per problem, Sturm-count eigenvalues.  Every trailing
  * update runs on the bf16 tensor cores, exact products of 8 integer slices of 7
  * bits per operand row rounded once per panel.  Replaces the same eighb call as
  * skn_eigh_gen_batched (slakonet/utils.py:741-783).
  *   n_prob    problems of the call (<= 65535)
- *   max_n     largest n; every problem must have ceil(max_n / 32) panels of 32
- *             columns (a problem that has not gets SKN_ERR_CAPACITY, untouched)
+ *   sizes     [n_prob] (host) n of each slot's problem, descending, at most 2048
  *   prob      [n_prob] (device) problem index of each slot, into the arrays below
+ *   ws_off    [n_prob] (device) byte offset of each slot's scratch, a multiple of 256;
+ *             a slot takes skn_eigh_panels_scratch_bytes(n) bytes (a problem that is
+ *             larger than sizes[0] or whose scratch ends past scratch_bytes gets
+ *             SKN_ERR_CAPACITY, untouched)
  *   real      [*] 1 where H and S are exactly real, or NULL
  *   nvec, hs_off, eig_off, H, S, eig, status   as skn_eigh_gen_batched; only the
  *             lower triangles are read, all of H and the lower triangle of S are
  *             overwritten
  *   tri       NULL, or d, e and tau per problem at 4 eig_off, as skn_eigh_gen_vectors
  *             keeps them (reflectors in the lower triangle of H, L in S)
- *   scratch   device scratch of skn_eigh_panels_scratch_bytes(n_prob, max_n) bytes
+ *   scratch   device scratch of scratch_bytes bytes
+ *   sms       SMs to plan for, as when other calls run beside this one (0: all); the
+ *             results do not depend on it
  * Results depend only on each problem.
  */
-int skn_eigh_gen_panels(int n_prob, int max_n, const int32_t* prob, const int32_t* nvec, const int32_t* real,
-                     const int64_t* hs_off, const int64_t* eig_off, double* H, double* S, double* eig,
-                     int32_t* status, double* tri, double* scratch, int64_t scratch_bytes, cudaStream_t stream);
-/* Host-side query: bytes of `scratch` skn_eigh_gen_panels needs (written to *bytes). */
-int skn_eigh_panels_scratch_bytes(int n_prob, int max_n, int64_t* bytes);
+int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
+                        const int32_t* nvec, const int32_t* real, const int64_t* hs_off, const int64_t* eig_off,
+                        double* H, double* S, double* eig, int32_t* status, double* tri, double* scratch,
+                        int64_t scratch_bytes, int sms, cudaStream_t stream);
+/* Host-side query: scratch bytes of one problem of n orbitals in skn_eigh_gen_panels (written to *bytes). */
+int skn_eigh_panels_scratch_bytes(int n, int64_t* bytes);
 
 /*
  * The same eigensolver compiled in more launch shapes: 32 threads per CTA with

@@ -50,8 +50,8 @@ class Tuning:
 
     @classmethod
     def default(cls) -> "Tuning":
-        """Untuned: the small and the panel kernels up to 1024 orbitals, the blocked one-CTA shape above."""
-        return cls({u: (AUTO if u <= 1024 else "_blk") for u in BUCKETS})
+        """Untuned: the small and the panel kernels (engine.route_auto)."""
+        return cls({u: AUTO for u in BUCKETS})
 
     @classmethod
     def one_cta(cls) -> "Tuning":

@@ -1,8 +1,8 @@
 // Generalized Hermitian eigenvalues of problems of about 100 orbitals and more, blocked, with every O(n^3)
 // step but the Hermitian matrix-vector products on the tcgen05 tensor cores.
 //
-// The problems of one call have the same number T of 32-column panels (n from 32 T - 31 to 32 T) and go
-// through one sequence of launches together; every launch covers all of them:
+// The problems of one call go through one sequence of launches together, largest first; every launch covers all that
+// still have columns at its panel:
 //   1. set-up: zero rows (eighb's aux option, slakonet/utils.py:741-747), the upper triangle of H;
 //   2. per panel: Cholesky of the diagonal block of S; triangular solves of the panel's rows and of the block
 //      row of B = L^-1 H; one update S22 -= L21 L21^H and H_below -= L21 B_panel on the tensor cores;
@@ -19,6 +19,8 @@
 // integer slices (below) rounded once per panel.  Every sum that crosses warps or CTAs goes to its own slot
 // and is added in a fixed order, so a problem's results depend neither on the other problems nor on the
 // number of CTAs it is given.
+#include <algorithm>
+
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
 
@@ -37,7 +39,7 @@ constexpr int TS = 32;               // tile edge of the matrix-vector products
 constexpr int SLICES = 8;
 constexpr int KP = 64;               // inner dimension of the sliced products (32 complex columns)
 constexpr int BM = 128, BN = 16;     // output tile of the tensor-core update
-constexpr int PANELS_MAX_N = 1024;
+constexpr int PANELS_MAX_N = 2048;
 
 SKN_DEVINL int cdiv_d(int a, int b) { return (a + b - 1) / b; }
 inline int cdiv(int a, int b) { return (a + b - 1) / b; }
@@ -87,7 +89,7 @@ SKN_DEVINL double2 zero2() { return make_double2(0.0, 0.0); }
 
 // ------------------------------------------------------------------ scratch (per problem slot)
 struct Lay {
-  int64_t W, VW, xc, Yp, sN, sT, sD, rd, d, e2, d32, e232, bnd, flg, sa, sb, sc, ea, eb, ec, stride;   // bytes
+  int64_t W, VW, xc, Yp, sN, sT, sD, li, d, e2, d32, e232, bnd, flg, bar, sa, sb, sc, ea, eb, ec, stride;   // bytes
 };
 __host__ __device__ inline int64_t take(int64_t& o, int64_t bytes) {
   const int64_t r = o;
@@ -107,13 +109,14 @@ __host__ __device__ inline Lay layout(int n) {
   L.sN = take(o, 8 * nt);                      // column norm, per 32-row chunk
   L.sT = take(o, 8 * nt * (nt + 1) / 2);       // v^H A v, per tile
   L.sD = take(o, 16 * nt * 4 * 2 * NT);        // [W V]^H v, per 8 rows
-  L.rd = take(o, 8 * (int64_t)n);              // 1 / L_kk
+  L.li = take(o, 16 * (int64_t)NB * NB * ((n + NB - 1) / NB));   // inverses of the diagonal blocks, row-major
   L.d = take(o, 8 * (int64_t)n);
   L.e2 = take(o, 8 * (int64_t)n);
   L.d32 = take(o, 4 * (int64_t)n);
   L.e232 = take(o, 4 * (int64_t)n);
   L.bnd = take(o, 64);
   L.flg = take(o, 4 * 2 * (int64_t)n);
+  L.bar = take(o, 4 * ((int64_t)n / NT + 1));  // arrivals at a grid team's barriers, per tridiagonalisation panel
   L.sa = take(o, 2 * SLICES * nr * KP);        // row operand
   L.sb = take(o, 2 * 2 * SLICES * nr * KP);    // column operand from rows: form B, then B'
   L.sc = take(o, 2 * 2 * SLICES * nr * KP);    // column operand from the block row of B
@@ -125,8 +128,9 @@ __host__ __device__ inline Lay layout(int n) {
 }
 
 struct Grp {
-  int nmax, panels, n_prob;
-  const int32_t* prob;       // [n_prob] problem of each slot
+  int nmax, n_prob;
+  const int32_t* prob;       // [n_prob] problem of each slot, sizes descending
+  const int64_t* ws_off;     // [n_prob] byte offset of each slot's scratch
   const int32_t* nvec;
   const int32_t* real;       // [*] 1 where H and S are exactly real; may be null
   const int64_t* hs_off;
@@ -137,27 +141,31 @@ struct Grp {
   int32_t* status;
   double* tri;               // d, e, tau per problem at 4 eig_off (for eigenvectors); may be null
   char* scratch;
+  int64_t scratch_bytes;
 };
 
 struct WS {
-  double2 *W, *VW, *xc, *Yp, *sD;
-  double *sN, *sT, *rd, *d, *e2, *bnd;
+  double2 *W, *VW, *xc, *Yp, *sD, *li;
+  double *sN, *sT, *d, *e2, *bnd;
   float *d32, *e232;
   int *flg, *ea, *eb, *ec;
+  unsigned* bar;
   uint16_t *sa, *sb, *sc;
   int64_t nr;                // rows of a slice array
 };
 SKN_DEVINL WS ws_of(const Grp& G, int g) {
-  const Lay L = layout(G.nmax);
-  char* b = G.scratch + (int64_t)g * L.stride;
+  const int n = G.nvec[G.prob[g]];
+  const Lay L = layout(n);
+  char* b = G.scratch + G.ws_off[g];
   WS w;
   w.W = (double2*)(b + L.W); w.VW = (double2*)(b + L.VW); w.xc = (double2*)(b + L.xc); w.Yp = (double2*)(b + L.Yp);
-  w.sD = (double2*)(b + L.sD); w.sN = (double*)(b + L.sN); w.sT = (double*)(b + L.sT); w.rd = (double*)(b + L.rd);
+  w.sD = (double2*)(b + L.sD); w.sN = (double*)(b + L.sN); w.sT = (double*)(b + L.sT); w.li = (double2*)(b + L.li);
   w.d = (double*)(b + L.d); w.e2 = (double*)(b + L.e2); w.bnd = (double*)(b + L.bnd);
   w.d32 = (float*)(b + L.d32); w.e232 = (float*)(b + L.e232); w.flg = (int*)(b + L.flg);
+  w.bar = (unsigned*)(b + L.bar);
   w.ea = (int*)(b + L.ea); w.eb = (int*)(b + L.eb); w.ec = (int*)(b + L.ec);
   w.sa = (uint16_t*)(b + L.sa); w.sb = (uint16_t*)(b + L.sb); w.sc = (uint16_t*)(b + L.sc);
-  w.nr = slice_rows(G.nmax);
+  w.nr = slice_rows(n);
   return w;
 }
 SKN_DEVINL bool live(const Grp& G, int p) { return G.status[p] == SKN_OK; }
@@ -179,19 +187,44 @@ SKN_DEVINL int64_t tc_idx(int r, int k) { return (int64_t)(r >> 3) * (8 * KP) + 
 
 SKN_DEVINL long long fixed56(double x, int emax) {       // round(x 2^(56 - ex)), ex = emax - 1022
   const unsigned long long b = (unsigned long long)__double_as_longlong(x);
-  const int e = (int)((b >> 52) & 0x7ff);
-  if (e == 0) return 0;
-  const long long m = (long long)((b & 0xfffffffffffffull) | 0x10000000000000ull);
-  const int d = emax - e;
-  long long f = d <= 3 ? m << (3 - d) : (d > 60 ? 0 : (m + (1LL << (d - 4))) >> (d - 3));
-  return (b >> 63) ? -f : f;
+  const int e = (int)((b >> 52) & 0x7ff), d = emax - e;
+  const unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+  // m 2^3 is the value at d = 0; one bit more is kept for the rounding
+  unsigned long long f = d <= 59 ? (m << 4) >> d : 0;
+  f = (f + 1) >> 1;
+  const long long sg = (long long)b >> 63;
+  return e == 0 ? 0 : ((long long)f ^ sg) - sg;
 }
-// bf16 bits of a small integer (|d| <= 128)
-SKN_DEVINL uint32_t small_bf16(int d) {
-  return __float_as_uint(__int_as_float(0x4B400000 + d) - 12582912.0f) >> 16;
+// 64 at each of the seven low digits: the digits of f + DIGIT_BIAS are its bit fields, each 64 too large
+constexpr long long DIGIT_BIAS = 64LL * (1 + (1LL << 7) + (1LL << 14) + (1LL << 21) + (1LL << 28) + (1LL << 35) + (1LL << 42));
+// Digit s of a biased value as a float, exact in its upper 16 bits (bf16).
+SKN_DEVINL uint32_t digit_bf16(long long fb, int s) {
+  if (s == 0)                                             // the leading digit, unbiased, |d| <= 128
+    return __float_as_uint(__int_as_float(0x4B400000 + (int)(fb >> 49)) - 12582912.0f);
+  const int sh = 7 * (SLICES - 1 - s);
+  const uint32_t v = sh + 7 <= 32 ? (uint32_t)fb >> sh
+                     : sh >= 32   ? (uint32_t)(fb >> 32) >> (sh - 32)
+                                  : __funnelshift_r((uint32_t)fb, (uint32_t)(fb >> 32), sh);
+  return __float_as_uint(__uint_as_float(0x4B400000u | (v & 127u)) - 12582976.0f);
 }
 SKN_DEVINL uint4 neg4(uint4 v) {
   return make_uint4(v.x ^ 0x80008000u, v.y ^ 0x80008000u, v.z ^ 0x80008000u, v.w ^ 0x80008000u);
+}
+
+// The digits of 8 entries of one part of a row: kb < 4 the real parts of z_(8 kb) .., then the imaginary ones.
+template <class Get>
+SKN_DEVINL void slice_block(Get get, int kb, int emax, uint4* out) {
+  uint32_t w[SLICES][4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const double2 z0 = get((kb & 3) * 8 + 2 * u), z1 = get((kb & 3) * 8 + 2 * u + 1);
+    const long long f0 = fixed56(kb < 4 ? z0.x : z0.y, emax) + DIGIT_BIAS;
+    const long long f1 = fixed56(kb < 4 ? z1.x : z1.y, emax) + DIGIT_BIAS;
+#pragma unroll
+    for (int s = 0; s < SLICES; ++s) w[s][u] = __byte_perm(digit_bf16(f0, s), digit_bf16(f1, s), 0x7632);
+  }
+#pragma unroll
+  for (int s = 0; s < SLICES; ++s) out[s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
 }
 
 // Slices of one row r: values z_k = get(k), k < 32 (zero from K on).  A form to sa (null: none) with exponent
@@ -204,40 +237,19 @@ SKN_DEVINL void slice_row(Get get, int r, int64_t nr, uint16_t* sa, int* ea, uin
     const double2 z = get(k);
     hm = max(hm, max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
   }
-  const int emax = hm >> 20;
+  const int emax = hm >> 20;                // 0x7ff: the digits mean nothing, the exponent says so
   const int ex = emax == 0x7ff ? EXP_NAN : emax - 1022;
   if (sa) ea[r] = ex;
   if (sb) eb[r] = ex;
 #pragma unroll 1
   for (int kb = 0; kb < 8; ++kb) {          // 8 entries of one part: kb < 4 real, then imaginary
-    uint32_t out[SLICES][4];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      uint32_t lo[SLICES], hi[SLICES];
-#pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const double2 z = get((kb & 3) * 8 + 2 * u + h);
-        long long f = emax == 0x7ff ? 0 : fixed56(kb < 4 ? z.x : z.y, emax);
-#pragma unroll
-        for (int s = SLICES - 1; s >= 0; --s) {
-          int dgt;
-          if (s > 0) {
-            dgt = (int)((f + 64) & 127) - 64;
-            f = (f - dgt) >> 7;
-          } else {
-            dgt = (int)f;
-          }
-          if (h == 0) lo[s] = small_bf16(dgt); else hi[s] = small_bf16(dgt);
-        }
-      }
-#pragma unroll
-      for (int s = 0; s < SLICES; ++s) out[s][u] = lo[s] | (hi[s] << 16);
-    }
+    uint4 out[SLICES];
+    slice_block(get, kb, emax, out);
     const int pb = swap ? ((kb & 4) | ((kb + 2) & 3)) : kb;      // place of these entries in B
     const bool im = kb >= 4;
 #pragma unroll
     for (int s = 0; s < SLICES; ++s) {
-      const uint4 v = make_uint4(out[s][0], out[s][1], out[s][2], out[s][3]);
+      const uint4 v = out[s];
       if (sa) *reinterpret_cast<uint4*>(sa + (int64_t)s * nr * KP + tc_idx(r, kb * 8)) = v;
       if (sb) {
         uint16_t* B = sb + (int64_t)s * nr * KP;
@@ -250,16 +262,42 @@ SKN_DEVINL void slice_row(Get get, int r, int64_t nr, uint16_t* sa, int* ea, uin
   }
 }
 
+// The same into shared memory for a product of this CTA: slice s of row r at dst + s * slice_el, form A; with prime >
+// 0 form B, and form B' at row r + prime.
+template <class Get>
+SKN_DEVINL void slice_row_to(Get get, int r, uint16_t* dst, int slice_el, int prime, int& ex) {
+  int hm = 0;
+#pragma unroll 8
+  for (int k = 0; k < 32; ++k) {
+    const double2 z = get(k);
+    hm = max(hm, max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
+  }
+  const int emax = hm >> 20;
+  ex = emax == 0x7ff ? EXP_NAN : emax - 1022;
+#pragma unroll 1
+  for (int kb = 0; kb < 8; ++kb) {
+    uint4 v[SLICES];
+    slice_block(get, kb, emax, v);
+#pragma unroll
+    for (int s = 0; s < SLICES; ++s) {
+      uint16_t* D = dst + (int64_t)s * slice_el;
+      *reinterpret_cast<uint4*>(D + tc_idx(r, kb * 8)) = v[s];
+      if (prime) *reinterpret_cast<uint4*>(D + tc_idx(r + prime, (kb ^ 4) * 8)) = kb >= 4 ? neg4(v[s]) : v[s];
+    }
+  }
+}
+
 // ------------------------------------------------------------------ set-up
 __global__ void __launch_bounds__(256) k_init(Grp G) {
-  const int g = blockIdx.y, p = G.prob[g];
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    const int n = G.nvec[p];
-    const bool ok = n >= 1 && n <= G.nmax && cdiv_d(n, NB) == G.panels && G.hs_off[p] >= 0 && G.eig_off[p] >= 0;
-    G.status[p] = ok ? SKN_OK : SKN_ERR_CAPACITY;
-  }
+  const int g = blockIdx.y, p = G.prob[g], n = G.nvec[p];
+  const bool ok = n >= 1 && n <= G.nmax && G.hs_off[p] >= 0 && G.eig_off[p] >= 0 && G.ws_off[g] >= 0 &&
+                  G.ws_off[g] % 256 == 0 && G.ws_off[g] + layout(n).stride <= G.scratch_bytes;
+  if (blockIdx.x == 0 && threadIdx.x == 0) G.status[p] = ok ? SKN_OK : SKN_ERR_CAPACITY;
+  if (!ok) return;
+  const WS w = ws_of(G, g);
   const int i = blockIdx.x * 256 + threadIdx.x;
-  if (i < 2 * G.nmax) ws_of(G, g).flg[i] = 0;
+  if (i < 2 * n) w.flg[i] = 0;
+  if (i <= n / NT) w.bar[i] = 0;
 }
 
 // Rows with a nonzero entry, from 32 x 32 tiles of the lower triangles (entry (i, j) marks rows i and j), and
@@ -274,7 +312,7 @@ __global__ void __launch_bounds__(256) k_scan(Grp G) {
   const int I = t / nt, J = t % nt;
   if (J > I) return;
   double2* A = (which ? G.S : G.H) + G.hs_off[p];
-  int* flg = ws_of(G, g).flg + which * G.nmax;
+  int* flg = ws_of(G, g).flg + which * n;
   const int i = I * TS + lane;
   bool row = false;
   double2* T = tiles[warp];
@@ -318,164 +356,81 @@ __global__ void __launch_bounds__(256) k_fix(Grp G) {
   double2* S = G.S + G.hs_off[p] + (int64_t)i * (n + 1);
   const double h = H->x + (flg[i] ? 0.0 : 1.0);
   *H = make_double2(h, 0.0);
-  if (!flg[G.nmax + i]) S->x += 1.0;
+  if (!flg[n + i]) S->x += 1.0;
 }
 
 // ------------------------------------------------------------------ Cholesky of a diagonal block
-// One CTA of 8 warps; warp q holds columns q, q + 8, q + 16, q + 24 (lane = row), so column k is one warp's
-// registers: that warp takes the root and scales it, all apply it.
+// One CTA of 8 warps; warp q holds columns q, q + 8, q + 16, q + 24 of the block and of its inverse (lane = row), so
+// column k is one warp's registers: that warp takes the root and scales it, all apply it to both.  The inverse X
+// starts as the unit matrix: step k scales its row k and subtracts l_i times it from the rows below.
 __global__ void __launch_bounds__(256) k_potrf(Grp G, int c0) {
   const int g = blockIdx.x, p = G.prob[g];
   if (!live(G, p)) return;
   const int n = G.nvec[p], w = min(NB, n - c0), warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (w <= 0) return;
   __shared__ double2 col[2][NB];
+  __shared__ double s_rd[2];
   __shared__ int s_bad;
   double2* A11 = G.S + G.hs_off[p] + c0 + (int64_t)c0 * n;
-  double* rd = ws_of(G, g).rd + c0;
-  double2 a[4];
+  double2 a[4], x[4];
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int j = warp + 8 * u;
     a[u] = (lane < w && j <= lane) ? A11[lane + (int64_t)j * n] : zero2();
+    x[u] = make_double2(lane == j ? 1.0 : 0.0, 0.0);
   }
   if (threadIdx.x == 0) s_bad = 0;
   __syncthreads();
-  for (int k = 0; k < w; ++k) {
-    if (warp == (k & 7)) {
-      double2 c = zero2();
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (u == (k >> 3)) c = a[u];
-      const double akk = __shfl_sync(0xffffffffu, c.x, k);
-      const bool ok = akk > 0.0 && is_finite_bits(akk);
-      const double q = ok ? akk : 1.0, r = rsqrt(q), r0 = q * r;
-      const double dk = fma(fma(-r0, r0, q), 0.5 * r, r0);
-      double2 l = make_double2(c.x * r, c.y * r);
-      if (lane == k) l = make_double2(dk, 0.0);
-      if (lane < k) l = zero2();
-      col[k & 1][lane] = l;
+  for (int kb = 0; kb < 4; ++kb) {          // columns 8 kb .. 8 kb + 7: static register indices
+#pragma unroll 1
+    for (int kq = 0; kq < 8; ++kq) {
+      const int k = kb * 8 + kq;
+      if (k >= w) break;
+      if (warp == kq) {
+        const double akk = __shfl_sync(0xffffffffu, a[kb].x, k);
+        const bool ok = akk > 0.0 && is_finite_bits(akk);
+        const double q = ok ? akk : 1.0, r = rsqrt(q), r0 = q * r;
+        const double dk = fma(fma(-r0, r0, q), 0.5 * r, r0);
+        double2 l = make_double2(a[kb].x * r, a[kb].y * r);
+        if (lane == k) l = make_double2(dk, 0.0);
+        if (lane < k) l = zero2();
+        col[k & 1][lane] = l;
+        a[kb] = l;
+        if (lane == 0) {
+          s_rd[k & 1] = r;
+          if (!ok) s_bad = 1;
+        }
+      }
+      __syncthreads();
+      const double2 li = col[k & 1][lane];
+      const double r = s_rd[k & 1];
 #pragma unroll
-      for (int u = 0; u < 4; ++u)
-        if (u == (k >> 3)) a[u] = l;
-      if (lane == 0) {
-        rd[k] = r;
-        if (!ok) s_bad = 1;
+      for (int u = 0; u < 4; ++u) {
+        const int j = warp + 8 * u;
+        if (u >= kb && j > k && j < w) a[u] = cfms_conj(li, col[k & 1][j], a[u]);
+        if (u <= kb && j <= k) {
+          if (lane == k) x[u] = make_double2(x[u].x * r, x[u].y * r);
+          double2 xk;
+          xk.x = __shfl_sync(0xffffffffu, x[u].x, k);
+          xk.y = __shfl_sync(0xffffffffu, x[u].y, k);
+          if (lane > k) x[u] = fms<false>(li, xk, x[u]);
+        }
       }
     }
-    __syncthreads();
-    const double2 li = col[k & 1][lane];
-#pragma unroll
-    for (int u = 0; u < 4; ++u) {
-      const int j = warp + 8 * u;
-      if (j > k && j < w) a[u] = cfms_conj(li, col[k & 1][j], a[u]);
-    }
   }
+  double2* li = ws_of(G, g).li + (int64_t)(c0 / NB) * NB * NB;
 #pragma unroll
   for (int u = 0; u < 4; ++u) {
     const int j = warp + 8 * u;
     if (lane < w && j <= lane && j < w) A11[lane + (int64_t)j * n] = a[u];
+    li[lane * NB + j] = (lane < w && j <= lane) ? x[u] : zero2();
   }
   __syncthreads();
   if (threadIdx.x == 0 && s_bad) G.status[p] = SKN_ERR_NOT_SPD;
 }
 
-// ------------------------------------------------------------------ triangular solves and slicing
-constexpr int ST = 64;               // rows or columns per CTA
-
-// x L11^H = a for one row: right-looking, so the updates of a step are independent.
-template <bool R>
-SKN_DEVINL void solve_row(double2* x, const double2* Lt, const double* rd) {
-#pragma unroll
-  for (int j = 0; j < NB; ++j) {
-    x[j].x *= rd[j];
-    if constexpr (!R) x[j].y *= rd[j];
-#pragma unroll
-    for (int k = j + 1; k < NB; ++k) x[k] = fms_cj<R>(x[j], Lt[k + j * LDT], x[k]);
-  }
-}
-// L11 x = a for one column.
-template <bool R>
-SKN_DEVINL void solve_col(double2* x, const double2* Lt, const double* rd) {
-#pragma unroll
-  for (int j = 0; j < NB; ++j) {
-    x[j].x *= rd[j];
-    if constexpr (!R) x[j].y *= rd[j];
-#pragma unroll
-    for (int k = j + 1; k < NB; ++k) x[k] = fms<R>(Lt[k + j * LDT], x[j], x[k]);
-  }
-}
-
-// The diagonal block of L, unit beyond its width w (so partial panels solve as whole ones).
-SKN_DEVINL void load_diag(const double2* L11, int n, int w, const double* rd, double2* Lt, double* rds) {
-  for (int e = threadIdx.x; e < NB * NB; e += blockDim.x) {
-    const int i = e % NB, j = e / NB;
-    Lt[i + j * LDT] = (i < w && j < w && i >= j) ? L11[i + (int64_t)j * n] : zero2();
-  }
-  if (threadIdx.x < NB) rds[threadIdx.x] = threadIdx.x < w ? rd[threadIdx.x] : 1.0;
-  __syncthreads();
-}
-
-// MODE 1 (Cholesky sweep): CTAs [0, nrow): rows below the panel of S, x L11^H = a, sliced as both operands;
-// the others: columns of the block row of H, L11 x = a, conjugated and sliced as column operand.
-// MODE 2 (second sweep): CTAs [0, nrow): rows from the panel's own down of H, x L11^H = a, sliced as row operand;
-// the others: rows of L21 sliced as column operand.
-template <bool R, int MODE>
-SKN_DEVINL void solve_body(const Grp& G, int g, int p, int c0, int nrow, double2* Lt, double* rds) {
-  const int n = G.nvec[p], w = min(NB, n - c0);
-  const WS ws = ws_of(G, g);
-  double2* S = G.S + G.hs_off[p];
-  double2* H = G.H + G.hs_off[p];
-  load_diag(S + c0 + (int64_t)c0 * n, n, w, ws.rd + c0, Lt, rds);
-  const bool first = blockIdx.x < nrow;
-  double2 x[NB];
-  if (first) {
-    double2* A = MODE == 1 ? S : H;
-    const int r = (MODE == 1 ? c0 + NB : c0) + blockIdx.x * ST + threadIdx.x;
-    if (r >= n) return;
-    double2* row = A + r + (int64_t)c0 * n;
-#pragma unroll
-    for (int j = 0; j < NB; ++j) x[j] = j < w ? ld<R>(row + (int64_t)j * n) : zero2();
-    solve_row<R>(x, Lt, rds);
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-      if (j < w) row[(int64_t)j * n] = R ? make_double2(x[j].x, 0.0) : x[j];
-    if (r >= c0 + NB)
-      slice_row([&](int k) { return row[(int64_t)k * n]; }, r, ws.nr, ws.sa, ws.ea, MODE == 1 ? ws.sb : nullptr, ws.eb,
-                false);
-  } else if (MODE == 1) {
-    const int c = (blockIdx.x - nrow) * ST + threadIdx.x;
-    if (c >= n) return;
-    double2* col = H + c0 + (int64_t)c * n;
-#pragma unroll
-    for (int j = 0; j < NB; ++j) x[j] = j < w ? ld<R>(col + j) : zero2();
-    solve_col<R>(x, Lt, rds);
-#pragma unroll
-    for (int j = 0; j < NB; ++j)
-      if (j < w) col[j] = R ? make_double2(x[j].x, 0.0) : x[j];
-    if (c0 + NB < n)
-      slice_row([&](int k) { const double2 z = col[k]; return make_double2(z.x, flip_sign(z.y)); }, c, ws.nr, nullptr,
-                nullptr, ws.sc, ws.ec, false);
-  } else {
-    const int r = c0 + NB + (blockIdx.x - nrow) * ST + threadIdx.x;
-    if (r >= n) return;
-    const double2* row = S + r + (int64_t)c0 * n;
-    slice_row([&](int k) { return row[(int64_t)k * n]; }, r, ws.nr, nullptr, nullptr, ws.sb, ws.eb, false);
-  }
-}
-
-template <int MODE>
-__global__ void __launch_bounds__(ST) k_solve(Grp G, int c0, int nrow) {
-  const int g = blockIdx.y, p = G.prob[g];
-  if (!live(G, p)) return;
-  __shared__ double2 Lt[NB * LDT];
-  __shared__ double rds[NB];
-  if (is_real(G, p))
-    solve_body<true, MODE>(G, g, p, c0, nrow, Lt, rds);
-  else
-    solve_body<false, MODE>(G, g, p, c0, nrow, Lt, rds);
-}
-
-// ------------------------------------------------------------------ tensor-core update
+// ------------------------------------------------------------------ tensor-core building blocks
 SKN_DEVINL uint32_t smem_u32(const void* p) { return static_cast<uint32_t>(__cvta_generic_to_shared(p)); }
 
 // Shared-memory matrix descriptor: no swizzle, K-major core matrices (8 rows x 16 bytes), 128 bytes between core
@@ -500,29 +455,34 @@ SKN_DEVINL void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, 
       "}\n" ::"r"(tmem_d),
       "l"(a), "l"(b), "r"(idesc), "r"(accumulate));
 }
-constexpr long long WAIT_LIMIT = 1LL << 26;
-SKN_DEVINL void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-SKN_DEVINL void bar_expect(uint32_t bar, uint32_t bytes) {
-  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+SKN_DEVINL void tc_commit(uint32_t bar) {
+  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
 }
 SKN_DEVINL void tmem_ld8(uint32_t a, uint32_t* v) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(a));
 }
+// Exact sums of 8 columns over the levels: hi counts units of 2^28 of lo.  The level sums are integers below 2^22:
+// the FP32 addition of 1.5 2^23 leaves them in the low bits, and two levels fit 32 bits.
+SKN_DEVINL void level_sums(uint32_t base, int level_cols, long long* hi, long long* lo) {
+  auto quad = [&](int L, long long* out) {
+    uint32_t t[8], u[8], v[8], w[8];
+    tmem_ld8(base + (uint32_t)(L * level_cols), t);
+    tmem_ld8(base + (uint32_t)((L + 1) * level_cols), u);
+    tmem_ld8(base + (uint32_t)((L + 2) * level_cols), v);
+    tmem_ld8(base + (uint32_t)((L + 3) * level_cols), w);
+    asm volatile("tcgen05.wait::ld.sync.aligned;");
+    auto whole = [](uint32_t x) { return __float_as_int(__uint_as_float(x) + 12582912.0f) - 0x4B400000; };
+#pragma unroll
+    for (int q = 0; q < 8; ++q)
+      out[q] = (long long)(whole(t[q]) * 128 + whole(u[q])) * 16384 + (whole(v[q]) * 128 + whole(w[q]));
+  };
+  quad(0, hi);
+  quad(4, lo);
+}
 
-constexpr int A_BYTES = BM * KP * 2;                 // 16 KB: one slice of a tile's rows
-constexpr int BH_BYTES = BN * KP * 2;                // 2 KB: one slice of a tile's columns, one form
-constexpr int B_BYTES = SLICES * 2 * BH_BYTES;       // 32 KB
-constexpr int UPD_SMEM = SLICES * A_BYTES + 2 * B_BYTES;       // 192 KB
-constexpr uint32_t BUF_COLS = SLICES * 2 * BN;       // TMEM columns of one tile
-constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
-constexpr int UPD_THREADS = 32 * 9;
-
+constexpr long long WAIT_LIMIT = 1LL << 26;
 // Wait for a phase of a barrier; gives up after WAIT_LIMIT polls or once the CTA has failed.
 SKN_DEVINL bool upd_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
   for (long long it = 0; it < WAIT_LIMIT; ++it) {
@@ -540,6 +500,154 @@ SKN_DEVINL bool upd_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
   }
   return false;
 }
+SKN_DEVINL void bulk_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
+               : "memory");
+}
+SKN_DEVINL void bar_expect(uint32_t bar, uint32_t bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+constexpr int A_BYTES = BM * KP * 2;                 // 16 KB: one slice of 128 rows
+
+// ------------------------------------------------------------------ triangular solves
+// Rows x of x L11^H = a and columns of L11 x = a, through the inverse X of the diagonal block: x = a X^H, and for a
+// column conj(x) = conj(a) X^H, on the tensor cores (a substitution in FP64 kept one warp per 32 rows busy for 85 us
+// a panel, and was a quarter of the FP64 work at n = 400).  MODE 1 (Cholesky sweep): blocks [0, nrow): rows below
+// the panel of S, sliced as both operands of the update; the others: columns of the block row of H, sliced as column
+// operand.  MODE 2 (second sweep): blocks [0, nrow): rows from the panel's own down of H, sliced as row operand; the
+// others: rows of L21, sliced as column operand without a solve.
+// One CTA per 128 rows: a thread slices its row into shared memory, warp 4 the rows of X, thread 128 issues the
+// products, a thread rounds its row's 32 sums and slices the result.
+constexpr int SV_THREADS = 160;
+constexpr int X_BYTES = 2 * NB * KP * 2;             // 8 KB: one slice of X, both forms
+constexpr int SV_SMEM = SLICES * (A_BYTES + X_BYTES);              // 192 KB
+constexpr uint32_t SV_COLS = SLICES * 2 * NB;        // 512 TMEM columns
+
+template <int MODE>
+__global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow) {
+  const int g = blockIdx.y, p = G.prob[g];
+  if (!live(G, p)) return;
+  const int n = G.nvec[p], w = min(NB, n - c0);
+  const bool rows = blockIdx.x < nrow;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int first = rows ? (MODE == 1 ? c0 + NB : c0) : (MODE == 1 ? 0 : c0 + NB);
+  const int base = first + (rows ? blockIdx.x : blockIdx.x - nrow) * BM;
+  if (c0 >= n || base >= n) return;
+  const WS ws = ws_of(G, g);
+  double2* S = G.S + G.hs_off[p];
+  double2* H = G.H + G.hs_off[p];
+  const int r = base + tid;                          // row, or column of the block row (threads below 128)
+  if (MODE == 2 && !rows) {
+    if (tid >= BM || r >= n) return;
+    const double2* row = S + r + (int64_t)c0 * n;
+    slice_row([&](int k) { return row[(int64_t)k * n]; }, r, ws.nr, nullptr, nullptr, ws.sb, ws.eb, false);
+    return;
+  }
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ __align__(8) uint64_t s_bar;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_ex[NB];
+  __shared__ volatile int s_fail;
+  const uint32_t a0 = smem_u32(smem), x0 = a0 + SLICES * A_BYTES, bar = smem_u32(&s_bar);
+  if (tid == 0) {
+    s_fail = 0;
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
+    asm volatile("fence.mbarrier_init.release.cluster;");
+  }
+  if (warp == 4) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"(SV_COLS));
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+  }
+  // entry k of this thread's row; a column's entries are taken conjugate
+  const bool conj_in = !rows;
+  double2* src = rows ? (MODE == 1 ? S : H) + r + (int64_t)c0 * n : H + c0 + (int64_t)r * n;
+  const int64_t step = rows ? n : 1;
+  int er = 0;
+  if (warp < 4) {
+    auto in = [&](int k) {
+      if (r >= n || k >= w || (MODE == 2 && k > r - c0)) return zero2();   // above the diagonal: not updated, not needed
+      double2 z = src[k * step];
+      if (conj_in) z.y = flip_sign(z.y);
+      return z;
+    };
+    slice_row_to(in, tid, reinterpret_cast<uint16_t*>(smem), A_BYTES / 2, 0, er);
+  } else {
+    const double2* X = ws.li + (int64_t)(c0 / NB) * NB * NB + lane * NB;
+    int ex = 0;
+    // slice s: rows 0 .. 31 form B, rows 32 .. 63 form B'
+    slice_row_to([&](int k) { return X[k]; }, lane, reinterpret_cast<uint16_t*>(smem + SLICES * A_BYTES), X_BYTES / 2,
+                 NB, ex);
+    s_ex[lane] = ex;
+  }
+  asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the products read what the threads wrote
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  const uint32_t tmem = tmem_slot;
+  if (tid == 128) {
+    for (int s = 0; s < SLICES; ++s) {
+      // column slices 0 .. SLICES - 1 - s side by side give levels s .. SLICES - 1; at most 256 columns a product
+      for (int t0 = 0; t0 < SLICES - s; t0 += 4) {
+        const int cnt = min(4, SLICES - s - t0);
+        const uint32_t id = tc_idesc(cnt * 2 * NB);
+#pragma unroll
+        for (int kk = 0; kk < KP / 16; ++kk)
+          tc_mma(tmem + (uint32_t)((s + t0) * 2 * NB), tc_desc(a0 + (uint32_t)(s * A_BYTES) + kk * 256),
+                 tc_desc(x0 + (uint32_t)(t0 * X_BYTES) + kk * 256), id, (s > 0 || kk > 0) ? 1u : 0u);
+      }
+    }
+    tc_commit(bar);
+  }
+  if (!upd_wait(bar, 0, &s_fail)) s_fail = 1;
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;");
+  if (!s_fail && warp < 4) {
+    const uint32_t tb = tmem + ((uint32_t)(warp * 32) << 16);
+#pragma unroll 1
+    for (int cb = 0; cb < NB; cb += 8) {
+      long long hr[8], lr[8], hi[8], li[8];
+      level_sums(tb + cb, 2 * NB, hr, lr);
+      level_sums(tb + NB + cb, 2 * NB, hi, li);
+#pragma unroll
+      for (int q = 0; q < 8; ++q) {
+        const int k = cb + q, ex = s_ex[k];
+        if (r < n && k < w) {
+          double2 v;
+          if (er == EXP_NAN || ex == EXP_NAN) {
+            v = make_double2(__longlong_as_double(0x7ff8000000000000LL), __longlong_as_double(0x7ff8000000000000LL));
+          } else {
+            v = make_double2(round_sum28(hr[q], lr[q], er + ex - 63), round_sum28(hi[q], li[q], er + ex - 63));
+          }
+          if (conj_in) v.y = flip_sign(v.y);
+          src[k * step] = v;
+        }
+      }
+    }
+    if (r < n) {
+      if (rows && r >= c0 + NB)
+        slice_row([&](int k) { return src[k * step]; }, r, ws.nr, ws.sa, ws.ea, MODE == 1 ? ws.sb : nullptr, ws.eb,
+                  false);
+      if (!rows && c0 + NB < n)
+        slice_row([&](int k) { const double2 z = src[k]; return make_double2(z.x, flip_sign(z.y)); }, r, ws.nr, nullptr,
+                  nullptr, ws.sc, ws.ec, false);
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;");
+  __syncthreads();
+  if (tid == 0 && s_fail) G.status[p] = SKN_ERR_CUDA;
+  if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(SV_COLS));
+}
+
+// ------------------------------------------------------------------ tensor-core update
+constexpr int BH_BYTES = BN * KP * 2;                // 2 KB: one slice of a tile's columns, one form
+constexpr int B_BYTES = SLICES * 2 * BH_BYTES;       // 32 KB
+constexpr int UPD_SMEM = SLICES * A_BYTES + 2 * B_BYTES;       // 192 KB
+constexpr uint32_t BUF_COLS = SLICES * 2 * BN;       // TMEM columns of one tile
+constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
+constexpr int UPD_THREADS = 32 * 9;
 
 // C -= A B^T over BM x BN tiles.  SWEEP 1: blocks [0, nlow) of S22 (lower triangle, columns from sb), the rest
 // of H below the panel over all columns (sc); SWEEP 2 and 3: the trailing lower triangle of H (sb).
@@ -639,8 +747,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
             tc_mma(td + (uint32_t)(s * 2 * BN), tc_desc(a0 + (uint32_t)(s * A_BYTES) + kk * 256), tc_desc(bs + kk * 256),
                    id, (s > 0 || kk > 0) ? 1u : 0u);
         }
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
-            bar(T_FULL + b)));
+        tc_commit(bar(T_FULL + b));
         ++issued;
         if (!ok) break;
         if (i >= 1 && i + 1 < ntile) {                // the other column buffer, once tile i - 1 has been multiplied
@@ -691,29 +798,8 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
       for (int cb = 0; cb < BN; cb += 8) {
         long long hr[8], lr[8], hi[8], li[8];
         if (cb > 0) fetch(cb);
-        // integers below 2^22: the FP32 addition of 1.5 2^23 leaves them in the low bits; two levels fit 32 bits
-        auto pair = [&](int L, int part, int* out) {
-          uint32_t u[8], v[8];
-          tmem_ld8(base + (uint32_t)(L * 2 * BN + part * BN + cb), u);
-          tmem_ld8(base + (uint32_t)((L + 1) * 2 * BN + part * BN + cb), v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;");
-#pragma unroll
-          for (int q = 0; q < 8; ++q)
-            out[q] = (__float_as_int(__uint_as_float(u[q]) + 12582912.0f) - 0x4B400000) * 128 +
-                     (__float_as_int(__uint_as_float(v[q]) + 12582912.0f) - 0x4B400000);
-        };
-#pragma unroll
-        for (int part = 0; part < 2; ++part) {
-          int p0[8], p1[8];
-          pair(0, part, p0);
-          pair(2, part, p1);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) (part ? hi : hr)[q] = (long long)p0[q] * 16384 + p1[q];
-          pair(4, part, p0);
-          pair(6, part, p1);
-#pragma unroll
-          for (int q = 0; q < 8; ++q) (part ? li : lr)[q] = (long long)p0[q] * 16384 + p1[q];
-        }
+        level_sums(base + cb, 2 * BN, hr, lr);
+        level_sums(base + BN + cb, 2 * BN, hi, li);
         if (cb + 8 == BN) {                          // the accumulators have been read: the next tile may start
           asm volatile("tcgen05.fence::before_thread_sync;");
           if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(T_EMPTY + grp)) : "memory");
@@ -764,14 +850,14 @@ constexpr int PT = 32 * PW;
 constexpr int TILE_LD = TS + 1;
 constexpr int TILE_EL = TS * TILE_LD;            // a resident tile, or a chunk's 32 columns of [W V]
 constexpr int QT = TS / PW;                      // columns or rows of a quarter; columns staged when streamed
-constexpr int VMAX = (PANELS_MAX_N + PT - 1) / PT;
+constexpr int VMAX = 8;                          // column entries a thread fetches ahead (1024 rows)
 struct PanelSm {
   double2 rowV[NT], rowW[NT];                    // V and W at the next pivot row
   double2 part[PW][2 * NT];                      // [W V]^H v by quarters of the chunks
   double2 t12[PW][2 * NT];                       // W^H v, V^H v: a copy per warp
   double2 tau, scl, yrow, wrow;
   double vav, alpha;
-  int triv, pad;
+  int triv, dead;
 };
 
 SKN_DEVINL void tile_ij(int t, int& I, int& J) {     // lower-triangle tile index, I >= J
@@ -785,13 +871,50 @@ template <bool R> SKN_DEVINL double2 sum4(double2 a, double2 b, double2 c, doubl
   return add<R>(add<R>(a, b), add<R>(c, d));
 }
 
+// The CTAs of one problem: a cluster, or (more than 16) CTAs of a cooperative launch that meet at a counter.  A
+// wait is bounded; once one has run out the problem is marked SKN_ERR_CUDA and its CTAs no longer wait.
+constexpr int TEAM_LIMIT = 1 << 22;              // polls of about half a microsecond
+struct Team {
+  int rank, C;
+  bool grid;
+  unsigned* count;
+  unsigned target;
+  int32_t* status;
+  int* dead;                                     // shared: a wait has run out
+  SKN_DEVINL void sync() {
+    if (C == 1) {
+      __syncthreads();
+    } else if (!grid) {
+      cg::this_cluster().sync();
+    } else {
+      target += (unsigned)C;
+      __syncthreads();
+      if (threadIdx.x == 0 && !*dead) {
+        __threadfence();
+        atomicAdd(count, 1u);
+        int it = 0;
+        for (; it < TEAM_LIMIT; ++it) {
+          unsigned v;
+          asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
+          if (v >= target) break;
+        }
+        if (it == TEAM_LIMIT) {
+          *dead = 1;
+          *status = SKN_ERR_CUDA;
+        }
+        __threadfence();
+      }
+      __syncthreads();
+    }
+  }
+};
+
 // sv: the Householder vector; big: streamed, a quarter of a tile per warp; RES, tiles (rt), chunks of [W V] (cpc), partial
-// sums of tiles (rt x PW x 32), of diagonal tiles (rt x 32) and of chunks (2 x cpc x PW x 32).
+// sums of tiles (rt x PW x 32) and of chunks (2 x cpc x PW x 32).
 template <bool R, bool RES>
-SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, int cpc, PanelSm& sm, double2* sv,
+SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int rt, int cpc, PanelSm& sm, double2* sv,
                            double2* big) {
-  cg::cluster_group cl = cg::this_cluster();
-  const int rank = (int)cl.block_rank();
+  const int rank = team.rank, C = team.C;
   const int n = G.nvec[p], M = n - c0, w = min(NT, n - 1 - c0);
   const int nt = cdiv_d(M, TS), ntile = nt * (nt + 1) / 2;
   const WS ws = ws_of(G, g);
@@ -801,10 +924,14 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
   double* tri = G.tri ? G.tri + 4 * G.eig_off[p] : nullptr;
   double2* wvs = big + (int64_t)rt * TILE_EL;      // chunk lc, column q, row r at lc TILE_EL + q TILE_LD + r
   double2* yps = wvs + (int64_t)cpc * TILE_EL;     // tile i, quarter q, row r at (i PW + q) TS + r
-  double2* zds = yps + (int64_t)rt * PW * TS;      // diagonal tile i, column c at i TS + c
-  double2* eps = zds + (int64_t)rt * TS;           // chunk lc, quarter q, (y, a), row r at ((lc PW + q) 2 + part) TS + r
-  auto sync = [&]() {
-    if (C > 1) cl.sync(); else __syncthreads();
+  double2* eps = yps + (int64_t)rt * PW * TS;      // chunk lc, quarter q, (y, a), row r at ((lc PW + q) 2 + part) TS + r
+  auto sync = [&]() { team.sync(); };
+  // entry (i, j) of the Hermitian trailing block, from its lower triangle
+  auto entry = [&](int i, int j) {
+    if (i >= M || j >= M) return zero2();
+    double2 a = ld<R>(i >= j ? A + i + (int64_t)j * n : A + j + (int64_t)i * n);
+    if constexpr (!R) a.y = i == j ? 0.0 : cond_flip(a.y, i < j);
+    return a;
   };
   // chunks and tiles of this CTA are rank, rank + C, ...; streamed, a warp takes every PW-th of them
   const int first = RES ? rank : rank + C * warp, stride = RES ? C : C * PW;
@@ -812,15 +939,9 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
     for (int t = rank, i = 0; t < ntile; t += C, ++i) {
       int I, J;
       tile_ij(t, I, J);
-      const int gi = I * TS + lane;
       double2* T = big + (int64_t)i * TILE_EL;
 #pragma unroll
-      for (int u = 0; u < QT; ++u) {
-        const int c = warp * QT + u, gj = J * TS + c;
-        double2 a = (gi < M && gj < M && gi >= gj) ? ld<R>(A + gi + (int64_t)gj * n) : zero2();
-        if (!R && gi == gj) a.y = 0.0;
-        T[c * TILE_LD + lane] = a;
-      }
+      for (int u = 0; u < QT; ++u) T[(warp * QT + u) * TILE_LD + lane] = entry(I * TS + lane, J * TS + warp * QT + u);
     }
   }
   // first column as it stands
@@ -882,6 +1003,13 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
     __syncthreads();
     const int triv = sm.triv;
     const double2 tau = sm.tau, scl = sm.scl;
+    auto put_v = [&](int r, double2 v) {
+      if (r > j && r < M && (r >> 5) % C == rank) {
+        st<R>(A + r + (int64_t)j * n, v);
+        if constexpr (RES) wvs[((r >> 5) / C) * TILE_EL + (NT + j) * TILE_LD + (r & 31)] = v;
+        st<R>(ws.VW + (int64_t)r * 2 * NT + NT + j, v);
+      }
+    };
 #pragma unroll
     for (int u = 0; u < VMAX; ++u) {
       const int r = tid + u * PT;
@@ -890,20 +1018,21 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
         if (r == j + 1) v = make_double2(1.0, 0.0);
         else if (!triv) v = mul<R>(v, scl);
         sv[r] = v;
-        if (r > j && r < M && (r >> 5) % C == rank) {
-          st<R>(A + r + (int64_t)j * n, v);
-          if constexpr (RES) wvs[((r >> 5) / C) * TILE_EL + (NT + j) * TILE_LD + (r & 31)] = v;
-          st<R>(ws.VW + (int64_t)r * 2 * NT + NT + j, v);
-        }
+        put_v(r, v);
       }
+    }
+    for (int r = tid + VMAX * PT; r < nt * 32; r += PT) {
+      double2 v = r < M ? ldc<R>(ws.xc + r) : zero2();      // r > j + 1: past the entries above
+      if (!triv) v = mul<R>(v, scl);
+      sv[r] = v;
+      put_v(r, v);
     }
     __syncthreads();
     // ---- products with v
-    // y of tile t's rows, z of its columns; lane = row, then column
-    auto put_tile = [&](int t, int I, int J, double2 y, double2 z) {
+    // y of tile t's rows (lane = row); a diagonal tile is whole, another one stands for its transpose too
+    auto put_tile = [&](int t, int I, int J, double2 y) {
       const int gi = I * TS + lane;
       const bool diag = I == J;
-      if (diag) y = add<R>(y, z);
       if (gi < M) st<R>(ws.Yp + (int64_t)J * n + gi, y);
       const double2 vi = sv[gi];
       double s = R ? vi.x * y.x : fma(vi.x, y.x, vi.y * y.y);   // Re conj(v) y
@@ -913,33 +1042,36 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
     if (!triv) {
       if constexpr (RES) {
         const int qc = lane & (QT - 1), qr = lane / QT;        // this lane's column and rows of the transposed quarter
+#pragma unroll 2
         for (int t = rank, i = 0; t < ntile; t += C, ++i) {
           int I, J;
           tile_ij(t, I, J);
           const bool diag = I == J;
           const double2* T = big + (int64_t)i * TILE_EL;
           const double2 *vI = sv + I * TS, *vJ = sv + J * TS + warp * QT;
-          double2 y = zero2(), z = zero2();
+          double2 y = zero2();
           const double2* Tq = T + warp * QT * TILE_LD;
-          const double2* Tc = Tq + qc * TILE_LD;
-          const int cc = warp * QT + qc;
+          if (diag) {
 #pragma unroll
-          for (int u = 0; u < QT; ++u) {
-            y = fma_<R>(Tq[u * TILE_LD + lane], vJ[u], y);
-            const int r = qr * QT + u;
-            if (!diag || r != cc) z = fma_cja<R>(Tc[r], vI[r], z);
+            for (int u = 0; u < QT; ++u) y = fma_<R>(Tq[u * TILE_LD + lane], vJ[u], y);
+          } else {
+            double2 z = zero2();
+            const double2* Tc = Tq + qc * TILE_LD;
+            const int cc = warp * QT + qc;
+#pragma unroll
+            for (int u = 0; u < QT; ++u) {
+              y = fma_<R>(Tq[u * TILE_LD + lane], vJ[u], y);
+              z = fma_cja<R>(Tc[qr * QT + u], vI[qr * QT + u], z);
+            }
+            z.x += __shfl_xor_sync(0xffffffffu, z.x, QT);
+            z.x += __shfl_xor_sync(0xffffffffu, z.x, 2 * QT);
+            if constexpr (!R) {
+              z.y += __shfl_xor_sync(0xffffffffu, z.y, QT);
+              z.y += __shfl_xor_sync(0xffffffffu, z.y, 2 * QT);
+            }
+            if (lane < QT && J * TS + cc < M) st<R>(ws.Yp + (int64_t)I * n + J * TS + cc, z);
           }
           yps[(i * PW + warp) * TS + lane] = y;
-          z.x += __shfl_xor_sync(0xffffffffu, z.x, QT);
-          z.x += __shfl_xor_sync(0xffffffffu, z.x, 2 * QT);
-          if constexpr (!R) {
-            z.y += __shfl_xor_sync(0xffffffffu, z.y, QT);
-            z.y += __shfl_xor_sync(0xffffffffu, z.y, 2 * QT);
-          }
-          if (lane < QT) {
-            if (diag) zds[i * TS + cc] = z;
-            else if (J * TS + cc < M) st<R>(ws.Yp + (int64_t)I * n + J * TS + cc, z);
-          }
         }
       } else {
         double2* T = big + (int64_t)warp * QT * TILE_LD;
@@ -958,26 +1090,26 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
 #pragma unroll
             for (int u = 0; u < QT; ++u) {
               const int gj = J * TS + q * QT + u;
-              a[u] = (gi < M && gj < M && gi >= gj) ? ld<R>(col + (int64_t)(q * QT + u) * n) : zero2();
-              if (!R && gi == gj) a[u].y = 0.0;
+              if (diag) a[u] = entry(gi, gj);
+              else a[u] = gi < M ? ld<R>(col + (int64_t)(q * QT + u) * n) : zero2();   // gj < I TS < M
             }
             __syncwarp();
             double2 yq = zero2();
 #pragma unroll
             for (int u = 0; u < QT; ++u) {
               yq = fma_<R>(a[u], vJ[q * QT + u], yq);
-              T[u * TILE_LD + lane] = a[u];
+              if (!diag) T[u * TILE_LD + lane] = a[u];
             }
             if (q == 0) y01 = yq;
             if (q == 1) y01 = add<R>(y01, yq);
             if (q == 2) y2 = yq;
             if (q == 3) y = add<R>(y01, add<R>(y2, yq));
+            if (diag) continue;
             __syncwarp();
             double2 zq = zero2();
             const double2* Tc = T + qc * TILE_LD + qr * QT;
 #pragma unroll
-            for (int u = 0; u < QT; ++u)
-              if (!diag || qr * QT + u != q * QT + qc) zq = fma_cja<R>(Tc[u], vI[u], zq);
+            for (int u = 0; u < QT; ++u) zq = fma_cja<R>(Tc[u], vI[u], zq);
             zq.x += __shfl_xor_sync(0xffffffffu, zq.x, QT);
             zq.x += __shfl_xor_sync(0xffffffffu, zq.x, 2 * QT);
             if constexpr (!R) {
@@ -986,8 +1118,8 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
             }
             if (qr == q) z = zq;
           }
-          if (!diag && J * TS + lane < M) st<R>(ws.Yp + (int64_t)I * n + J * TS + lane, z);
-          put_tile(t, I, J, y, z);
+          if (!diag) st<R>(ws.Yp + (int64_t)I * n + J * TS + lane, z);
+          put_tile(t, I, J, y);
         }
       }
       if (j > 0) {
@@ -1014,7 +1146,7 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
           int I, J;
           tile_ij(t, I, J);
           const double2* yp = yps + i * PW * TS + lane;
-          put_tile(t, I, J, sum4<R>(yp[0], yp[TS], yp[2 * TS], yp[3 * TS]), zds[i * TS + lane]);
+          put_tile(t, I, J, sum4<R>(yp[0], yp[TS], yp[2 * TS], yp[3 * TS]));
         }
       }
     }
@@ -1026,13 +1158,13 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
       const bool on = lane < NT ? lane < j : lane - NT < j;
       double2 s = zero2();
       if (!triv && on) {
-#pragma unroll 4
+#pragma unroll 8
         for (int c = 0; c < nt; ++c) s = add<R>(s, ldc<R>(ws.sD + (c * PW + warp) * 2 * NT + lane));
       }
       sm.part[warp][lane] = s;
       if (!triv && warp == 1) {
         double q = 0.0;
-#pragma unroll 4
+#pragma unroll 8
         for (int t = lane; t < ntile; t += 32) q += __ldcg(ws.sT + t);
         q = warp_sum<true>(make_double2(q, 0.0)).x;
         if (lane == 0) sm.vav = q;
@@ -1051,31 +1183,25 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
     {
       const double2 s = sum4<R>(sm.part[0][lane], sm.part[1][lane], sm.part[2][lane], sm.part[3][lane]);
       t12[lane] = s;
-      if (!triv && warp == 0) {
-        // Re sum_q conj(t1_q) t2_q and the pivot row's correction: lane q < NT has t1_q, lane NT + q has t2_q
-        const double2 o = make_double2(__shfl_down_sync(0xffffffffu, s.x, NT),
-                                       R ? 0.0 : __shfl_down_sync(0xffffffffu, s.y, NT));
+      // lane q < NT has t1_q, lane NT + q has t2_q
+      const double2 o = make_double2(__shfl_down_sync(0xffffffffu, s.x, NT),
+                                     R ? 0.0 : __shfl_down_sync(0xffffffffu, s.y, NT));
+      if (!triv && warp == 0) {                            // the pivot row's tau (y - V t1 - W t2)
         double2 c = zero2();
-        double dot = 0.0;
         if (lane < j) {
-          dot = R ? s.x * o.x : fma(s.x, o.x, s.y * o.y);
           c = mul<R>(sm.rowV[lane], s);
           c = fma_<R>(sm.rowW[lane], o, c);
         }
         for (int q = 8; q > 0; q >>= 1) {
-          dot += __shfl_xor_sync(0xffffffffu, dot, q);
           c.x += __shfl_xor_sync(0xffffffffu, c.x, q);
           if constexpr (!R) c.y += __shfl_xor_sync(0xffffffffu, c.y, q);
         }
-        if (lane == 0) {
-          const double t2 = R ? tau.x * tau.x : fma(tau.x, tau.x, tau.y * tau.y);
-          const double al = -0.5 * t2 * (sm.vav - 2.0 * dot);
-          double2 y = make_double2(sm.yrow.x - c.x, R ? 0.0 : sm.yrow.y - c.y);
-          y = mul<R>(tau, y);
-          y.x += al;
-          sm.wrow = y;
-          sm.alpha = al;
-        }
+        if (lane == 0) sm.wrow = mul<R>(tau, make_double2(sm.yrow.x - c.x, R ? 0.0 : sm.yrow.y - c.y));
+      } else if (!triv && warp == 1) {                     // alpha, with Re sum_q conj(t1_q) t2_q
+        double dot = lane < j ? (R ? s.x * o.x : fma(s.x, o.x, s.y * o.y)) : 0.0;
+        for (int q = 8; q > 0; q >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, q);
+        const double t2 = R ? tau.x * tau.x : fma(tau.x, tau.x, tau.y * tau.y);
+        if (lane == 0) sm.alpha = -0.5 * t2 * (sm.vav - 2.0 * dot);
       }
       __syncwarp();
     }
@@ -1111,8 +1237,8 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
     // the row's entry of W's column j and of the next column, from the sums
     auto finish = [&](int ch, double2 y, double2 a) {
       const int r = ch * 32 + lane;
-      const double2 wrow = triv ? zero2() : sm.wrow;
       const double al = triv ? 0.0 : sm.alpha;
+      const double2 wrow = triv ? zero2() : make_double2(sm.wrow.x + al, sm.wrow.y);
       if (r > j && r < M) {
         const double2 v = sv[r];
         double2 wv = zero2();
@@ -1188,7 +1314,7 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, int C, int rt, in
 }
 
 template <bool RES>
-__global__ void __launch_bounds__(PT, RES ? 1 : 4) k_tri_panel(Grp G, int c0, int C, int rt, int cpc) {
+__global__ void __launch_bounds__(PT, RES ? 1 : 4) k_tri_panel(Grp G, int c0, int C, int rt, int cpc, int grid) {
   const int g = blockIdx.x / C, p = G.prob[g];
   if (!live(G, p)) return;
   if (c0 >= G.nvec[p] - 1) return;
@@ -1196,10 +1322,12 @@ __global__ void __launch_bounds__(PT, RES ? 1 : 4) k_tri_panel(Grp G, int c0, in
   PanelSm& sm = *reinterpret_cast<PanelSm*>(smem_raw);
   double2* sv = reinterpret_cast<double2*>(smem_raw + sizeof(PanelSm));
   double2* big = sv + cdiv_d(G.nmax - c0, TS) * TS;
+  if (threadIdx.x == 0) sm.dead = 0;
+  Team team{(int)(blockIdx.x % C), C, grid != 0, ws_of(G, g).bar + c0 / NT, 0u, G.status + p, &sm.dead};
   if (is_real(G, p))
-    panel_body<true, RES>(G, g, p, c0, C, rt, cpc, sm, sv, big);
+    panel_body<true, RES>(G, g, p, c0, team, rt, cpc, sm, sv, big);
   else
-    panel_body<false, RES>(G, g, p, c0, C, rt, cpc, sm, sv, big);
+    panel_body<false, RES>(G, g, p, c0, team, rt, cpc, sm, sv, big);
 }
 
 // ------------------------------------------------------------------ eigenvalues
@@ -1269,85 +1397,110 @@ __global__ void __launch_bounds__(64) k_eig(Grp G) {
 }
 
 // ------------------------------------------------------------------ host sequence
-// CTAs per problem in the tridiagonalisation: as many as the GPU has room for, up to one per tile.
-int cluster_size(int n, int n_prob, int sms) {
-  const int nt = cdiv(n, TS);
-  const int tiles = nt * (nt + 1) / 2;
-  int c = 1;
-  while (c < 16 && 2 * c * n_prob <= sms && 2 * c <= tiles) c *= 2;
-  return c;
-}
-
 constexpr size_t SMEM_MAX = 227 * 1024;
 
 // Shared memory of a panel over m rows: streamed, or (rt > 0) resident with rt tiles and cpc chunks per CTA.
 size_t panel_smem(int m, int rt, int cpc) {
   const size_t head = sizeof(PanelSm) + (size_t)cdiv(m, TS) * TS * sizeof(double2);
   if (rt == 0) return head + (size_t)PW * QT * TILE_LD * sizeof(double2);
-  return head + ((size_t)(rt + cpc) * TILE_EL + (size_t)rt * (PW + 1) * TS + (size_t)cpc * PW * 2 * TS) * sizeof(double2);
+  return head + ((size_t)(rt + cpc) * TILE_EL + (size_t)rt * PW * TS + (size_t)cpc * PW * 2 * TS) * sizeof(double2);
 }
 
-cudaError_t launch_panel(const Grp& G, int c0, int C, int sms, cudaStream_t stream) {
-  const int m = G.nmax - c0, nt = cdiv(m, TS), cpc = cdiv(nt, C);
-  int rt = cdiv(nt * (nt + 1) / 2, C);
-  if (panel_smem(m, rt, cpc) > SMEM_MAX || (int64_t)G.n_prob * C > sms) rt = 0;
+inline int pow2_below(int v, int most) {
+  int c = 1;
+  while (c < most && 2 * c <= v) c *= 2;
+  return c;
+}
+
+// CTAs per problem over m rows, and the tiles of each when they are resident (0: streamed).  Resident: one CTA per SM,
+// up to one per tile, if shared memory holds its part.  A cluster's barrier takes about 1200 clocks, a counter's
+// 5000, so a grid team only from GRID_FROM CTAs.  Streamed: STREAM_PER_SM CTAs for each SM (three are resident; the
+// rest wait) even out the mixed batch's calls, which run beside one another: 305 ms at 3, 300 at 4, 289 at 6, 284 at 10.
+constexpr int GRID_FROM = 24, STREAM_PER_SM = 10;
+void plan_panel(int m, int n_prob, int sms, int& C, int& rt) {
+  const int nt = cdiv(m, TS), tiles = nt * (nt + 1) / 2;
+  const int most = std::min(tiles, std::max(1, sms / n_prob));
+  C = most >= GRID_FROM ? most : pow2_below(most, 16);
+  rt = cdiv(tiles, C);
+  if ((int64_t)n_prob * C <= sms && panel_smem(m, rt, cdiv(nt, C)) <= SMEM_MAX) return;
+  rt = 0;
+  C = pow2_below(std::min(std::max(1, STREAM_PER_SM * sms / n_prob), std::max(1, tiles / (2 * PW))), 16);
+}
+
+cudaError_t launch_panel(const Grp& G, int count, int c0, int sms, cudaStream_t stream) {
+  const int m = G.nmax - c0;
+  int C, rt;
+  plan_panel(m, count, sms, C, rt);
+  const int cpc = cdiv(cdiv(m, TS), C);
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)G.n_prob * C);
+  cfg.gridDim = dim3((unsigned)count * C);
   cfg.blockDim = dim3(PT);
   cfg.dynamicSmemBytes = panel_smem(m, rt, cpc);
   cfg.stream = stream;
+  const int grid = C > 16;
   cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeClusterDimension;
-  at[0].val.clusterDim.x = C;
-  at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  if (grid) {
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+  } else {
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+  }
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return rt ? cudaLaunchKernelEx(&cfg, k_tri_panel<true>, G, c0, C, rt, cpc)
-            : cudaLaunchKernelEx(&cfg, k_tri_panel<false>, G, c0, C, rt, cpc);
+  return rt ? cudaLaunchKernelEx(&cfg, k_tri_panel<true>, G, c0, C, rt, cpc, grid)
+            : cudaLaunchKernelEx(&cfg, k_tri_panel<false>, G, c0, C, rt, cpc, grid);
 }
 
-// One update of every problem: jc column tiles per CTA, so that the GPU gets about two CTAs per SM at least.
+// One update of the first `count` problems: jc column tiles per CTA, so that the GPU gets about two CTAs per SM at
+// least.
 template <int SWEEP>
-void launch_update(const Grp& G, int c1, int sms, cudaStream_t stream) {
+void launch_update(const Grp& G, int count, int c1, int sms, cudaStream_t stream) {
   const int m = G.nmax - c1, nI = cdiv(m, BM);
   const int jl = cdiv(m, BN), ja = SWEEP == 1 ? cdiv(G.nmax, BN) : 0;
-  const int64_t tiles = (int64_t)G.n_prob * nI * ((jl + BM / BN + 1) / 2 + ja);
+  const int64_t tiles = (int64_t)count * nI * ((jl + BM / BN + 1) / 2 + ja);
   int jc = (int)(tiles / (2 * (int64_t)sms));
   jc = jc < 2 ? 2 : (jc > 32 ? 32 : jc);
   const int cl = cdiv(jl, jc), ca = ja ? cdiv(ja, jc) : 1;
   const int nlow = nI * cl;
-  k_update<SWEEP><<<dim3((unsigned)(nlow + (ja ? nI * ca : 0)), (unsigned)G.n_prob), UPD_THREADS, UPD_SMEM, stream>>>(
+  k_update<SWEEP><<<dim3((unsigned)(nlow + (ja ? nI * ca : 0)), (unsigned)count), UPD_THREADS, UPD_SMEM, stream>>>(
       G, c1, nlow, cl, ca, jc);
 }
 
-cudaError_t run(const Grp& G, cudaStream_t stream) {
-  const int n = G.nmax, T = G.panels;
+// sizes: the slots' n, descending.  A launch covers the slots that have columns at its panel.
+cudaError_t run(const Grp& G, const int32_t* sizes, int budget, cudaStream_t stream) {
+  const int n = G.nmax, T = cdiv(n, NB);
   const unsigned P = (unsigned)G.n_prob;
   int dev = 0, sms = 0;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (budget > 0 && budget < sms) sms = budget;
+  auto above = [&](int m) {                    // slots with more than m orbitals
+    return (int)(std::lower_bound(sizes, sizes + G.n_prob, m, [](int a, int b) { return a > b; }) - sizes);
+  };
   const int nt = cdiv(n, TS);
   k_init<<<dim3(cdiv(2 * n, 256), P), 256, 0, stream>>>(G);
   k_scan<<<dim3(cdiv(nt * nt, 8), P, 2), 256, 0, stream>>>(G);
   k_fix<<<dim3(cdiv(n, 256), P), 256, 0, stream>>>(G);
   for (int t = 0; t < T; ++t) {
     const int c0 = t * NB, m = n - c0 - NB;
-    const int nrow = m > 0 ? cdiv(m, ST) : 0;
-    k_potrf<<<P, 256, 0, stream>>>(G, c0);
-    k_solve<1><<<dim3(nrow + cdiv(n, ST), P), ST, 0, stream>>>(G, c0, nrow);
-    if (m > 0) launch_update<1>(G, c0 + NB, sms, stream);
+    const int nrow = m > 0 ? cdiv(m, BM) : 0;
+    const unsigned A = (unsigned)above(c0);
+    k_potrf<<<A, 256, 0, stream>>>(G, c0);
+    k_solve<1><<<dim3(nrow + cdiv(n, BM), A), SV_THREADS, SV_SMEM, stream>>>(G, c0, nrow);
+    if (m > 0) launch_update<1>(G, above(c0 + NB), c0 + NB, sms, stream);
   }
   for (int t = 0; t < T; ++t) {
     const int c0 = t * NB, m = n - c0 - NB;
-    const int nrow = cdiv(n - c0, ST), nl = m > 0 ? cdiv(m, ST) : 0;
-    k_solve<2><<<dim3(nrow + nl, P), ST, 0, stream>>>(G, c0, nrow);
-    if (m > 0) launch_update<2>(G, c0 + NB, sms, stream);
+    const int nrow = cdiv(n - c0, BM), nl = m > 0 ? cdiv(m, BM) : 0;
+    k_solve<2><<<dim3(nrow + nl, (unsigned)above(c0)), SV_THREADS, SV_SMEM, stream>>>(G, c0, nrow);
+    if (m > 0) launch_update<2>(G, above(c0 + NB), c0 + NB, sms, stream);
   }
   for (int c0 = 0; c0 < n - 1; c0 += NT) {
-    const cudaError_t e = launch_panel(G, c0, cluster_size(n - c0, G.n_prob, sms), sms, stream);
+    const cudaError_t e = launch_panel(G, above(c0 + 1), c0, sms, stream);
     if (e != cudaSuccess) return e;
-    const int m = n - c0 - NT;
-    if (m > 1) launch_update<3>(G, c0 + NT, sms, stream);
+    if (n - c0 - NT > 1) launch_update<3>(G, above(c0 + NT + 1), c0 + NT, sms, stream);
   }
   k_bounds<<<P, 256, 0, stream>>>(G);
   k_eig<<<dim3(cdiv(n, 64), P), 64, 0, stream>>>(G);
@@ -1361,6 +1514,8 @@ cudaError_t set_attrs() {
                              (int)panel_smem(PANELS_MAX_N, 0, 0));
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tri_panel<true>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_tri_panel<false>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_solve<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(k_solve<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, SV_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_update<1>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_update<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM);
   if (e == cudaSuccess) e = cudaFuncSetAttribute(k_update<3>, cudaFuncAttributeMaxDynamicSharedMemorySize, UPD_SMEM);
@@ -1369,27 +1524,28 @@ cudaError_t set_attrs() {
 
 }  // namespace
 
-extern "C" int skn_eigh_panels_scratch_bytes(int n_prob, int max_n, int64_t* bytes) {
-  if (!bytes || n_prob < 0 || max_n < 1) return SKN_ERR_ARG;
-  if (max_n > PANELS_MAX_N) return SKN_ERR_CAPACITY;
-  *bytes = (int64_t)n_prob * layout(max_n).stride;
+extern "C" int skn_eigh_panels_scratch_bytes(int n, int64_t* bytes) {
+  if (!bytes || n < 1) return SKN_ERR_ARG;
+  if (n > PANELS_MAX_N) return SKN_ERR_CAPACITY;
+  *bytes = layout(n).stride;
   return SKN_OK;
 }
 
-extern "C" int skn_eigh_gen_panels(int n_prob, int max_n, const int32_t* prob, const int32_t* nvec, const int32_t* real,
-                                const int64_t* hs_off, const int64_t* eig_off, double* H, double* S, double* eig,
-                                int32_t* status, double* tri, double* scratch, int64_t scratch_bytes,
-                                cudaStream_t stream) {
-  if (n_prob < 0 || max_n < 1) return SKN_ERR_ARG;
+extern "C" int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
+                                   const int32_t* nvec, const int32_t* real, const int64_t* hs_off,
+                                   const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status,
+                                   double* tri, double* scratch, int64_t scratch_bytes, int sms, cudaStream_t stream) {
+  if (n_prob < 0 || sms < 0) return SKN_ERR_ARG;
   if (n_prob == 0) return SKN_OK;
-  if (!prob || !nvec || !hs_off || !eig_off || !H || !S || !eig || !status || !scratch) return SKN_ERR_ARG;
-  if (max_n > PANELS_MAX_N || n_prob > 65535) return SKN_ERR_CAPACITY;
-  if (scratch_bytes < (int64_t)n_prob * layout(max_n).stride) return SKN_ERR_CAPACITY;
+  if (!sizes || !prob || !ws_off || !nvec || !hs_off || !eig_off || !H || !S || !eig || !status || !scratch)
+    return SKN_ERR_ARG;
+  if (sizes[0] < 1 || !std::is_sorted(sizes, sizes + n_prob, [](int a, int b) { return a > b; })) return SKN_ERR_ARG;
+  if (sizes[0] > PANELS_MAX_N || n_prob > 65535 || scratch_bytes < layout(sizes[0]).stride) return SKN_ERR_CAPACITY;
   if ((reinterpret_cast<uintptr_t>(scratch) & 15) || (reinterpret_cast<uintptr_t>(H) & 15) ||
       (reinterpret_cast<uintptr_t>(S) & 15))
     return SKN_ERR_ARG;
   if (set_attrs() != cudaSuccess) return SKN_ERR_CUDA;
-  Grp G{max_n, cdiv(max_n, NB), n_prob, prob, nvec, real, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, tri,
-        (char*)scratch};
-  return run(G, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
+  Grp G{sizes[0], n_prob, prob, ws_off, nvec, real, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, tri,
+        (char*)scratch, scratch_bytes};
+  return run(G, sizes, sms, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
 }

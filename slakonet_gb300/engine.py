@@ -514,8 +514,8 @@ def wide_launches(n: int, nb: int = 32, tc: bool = False, tc_min: int = 512) -> 
 
 
 PANEL = 32                  # panel width of the blocked eigensolver (csrc/eigh_panels.cu)
-PANELS_MAX_N = 1024         # its bound
-PANELS_SCRATCH = 2 << 30    # device bytes of scratch per call; a larger group goes through in parts
+PANELS_MAX_N = 2048         # its bound
+PANELS_SCRATCH = 4 << 30    # device bytes of scratch per call; a larger group goes through in parts
 
 
 def panels_launches(max_n: int) -> int:
@@ -526,10 +526,26 @@ def panels_launches(max_n: int) -> int:
     return 3 + 2 * T + (T - 1) + T + (T - 1) + tri + upd + 2
 
 
-def panels_scratch_bytes(count: int, max_n: int) -> int:
+def panels_scratch_bytes(n: int) -> int:
     need = ctypes.c_int64(0)
-    call("skn_eigh_panels_scratch_bytes", count, max_n, ctypes.addressof(need))
+    call("skn_eigh_panels_scratch_bytes", int(n), ctypes.addressof(need))
     return int(need.value)
+
+
+def panels_parts(sizes: np.ndarray, budget: int):
+    """[(first, last, scratch offsets, scratch bytes)]: the calls of a group of ``sizes`` (descending), each within
+    ``budget`` bytes of scratch."""
+    uniq, at = np.unique(sizes, return_inverse=True)
+    per = np.array([panels_scratch_bytes(n) for n in uniq], np.int64)[at]
+    end = np.cumsum(per)
+    parts, first = [], 0
+    while first < len(sizes):
+        base = int(end[first] - per[first])
+        last = max(first + 1, int(np.searchsorted(end, base + budget, side="right")))
+        last = min(last, first + 65535)
+        parts.append((first, last, end[first:last] - per[first:last] - base, int(end[last - 1]) - base))
+        first = last
+    return parts
 
 
 SMALL_MAX_N = 96            # bound of the shared-memory eigensolver (csrc/eigh_small.cu)
@@ -538,10 +554,12 @@ SMALL_CLASSES = (16, 24, 32, 40, 48, 56, 64, 80, 96)     # its calls' size class
 
 
 def route_auto(n: int):
-    """Kernel and call of a problem of n orbitals under the untuned policy: ("small", class) or ("panels", number of
-    32-column panels).  A rule on the problem alone, as route_wide.  Measured on GB300 against the one-CTA kernel:
-    panels 432 orbitals x 8 problems 21 ms (193 ms), 160 x 27 5.4 ms (12.9), 128 x 1000 32 ms (32),
-    96 x 3000 50 ms (39), 492 x 300 220 ms (399); so the small kernel as far as shared memory holds a problem."""
+    """Kernel and call of a problem of n orbitals under the untuned policy: ("small", class) or ("panels", panel
+    count).  A rule on the problem alone, as route_wide.  Measured on GB300 against the one-CTA kernel:
+    panels 432 orbitals x 8 problems 18.8 ms (191 ms), 160 x 27 4.6 ms (12.6), 128 x 1000 28 ms (31),
+    200 x 500 44 ms (62), 492 x 300 208 ms (393), 96 x 3000 45 ms (38); so the small kernel as far as shared memory
+    holds a problem.  One panel call per panel count: the 600 problems of 57 to 492 orbitals of a mixed batch take
+    284 ms so, on one stream each, and 297 ms as one call that drops the smaller ones on the way."""
     if n <= SMALL_MAX_N:
         return ("small", next(c for c in SMALL_CLASSES if n <= c))
     return ("panels", -(-n // PANEL))
@@ -618,8 +636,8 @@ class Engine:
     """Runs the whole path for a planned batch on one CUDA stream."""
 
     def __init__(self, tables: TableSet, cutoff: float = CUTOFF_BOHR, stream: Optional[torch.cuda.Stream] = None,
-                 tuning=None, large_threshold: Optional[int] = 1024, large_cluster: Optional[int] = None,
-                 real_path: bool = True, wide_threshold: Optional[int] = 1024, wide_tc: bool = True):
+                 tuning=None, large_threshold: Optional[int] = 2048, large_cluster: Optional[int] = None,
+                 real_path: bool = True, wide_threshold: Optional[int] = 2048, wide_tc: bool = True):
         _dev(tables.device)
         self.tables = tables
         self.tuning = tuning          # autotune.Tuning: eigensolver launch shape per problem-size bucket
@@ -628,7 +646,8 @@ class Engine:
         self.large_threshold = large_threshold
         self.large_cluster = large_cluster
         # problems above wide_threshold orbitals run on the device-wide eigensolver instead (route_wide):
-        # measured on GB300 it is 4.6x the 4-CTA cluster at n = 1024 and 6-7x at n = 2048-4096
+        # measured on GB300 it is 4.6x the 4-CTA cluster at n = 1024 and 6-7x at n = 2048-4096.  Up to the panel
+        # kernels' bound of 2048 orbitals those are faster: 2 problems of 1152 take 51 ms, 125 on this path
         self.wide_threshold = wide_threshold
         # the device-wide path's rank-2k updates on the tensor cores (skn_eigh_gen_wide_tc): measured on
         # GB300, the 1000-atom structure (n = 9000, 8 real k-points) solves in 13.2 s instead of 18.9 s
@@ -653,7 +672,6 @@ class Engine:
             b.record()
             ev.append((name, a, b))
         self.launches += (wide_launches(args[1], tc=name.endswith("_tc")) if name.startswith("skn_eigh_gen_wide")
-                          else panels_launches(args[1]) if name == "skn_eigh_gen_panels"
                           else KERNELS_PER_CALL.get(name, 1))
 
     def run(self, plan: Plan, dos_range=(-10.0, 10.0), dos_points: int = 5000, dos_sigma: float = 0.1,
@@ -814,14 +832,15 @@ class Engine:
             need = ctypes.c_int64(0)
             if isinstance(shape, int):       # a cluster group
                 call("skn_eigh_large_scratch_bytes", count, max_n, shape, ctypes.addressof(need))
-            elif isinstance(shape, tuple) and shape[0] == "panels":   # a blocked group: ("panels", number of panels)
-                need.value = panels_scratch_bytes(self._panels_part(count, max_n), max_n)
+            elif isinstance(shape, tuple) and shape[0] == "panels":
+                need.value = max(part[3] for part in db._panel_parts[gi])
             elif isinstance(shape, tuple) and shape[0] == "wide":   # a device-wide group: ("wide", n, real)
                 call("skn_eigh_wide_scratch_bytes", count, max_n, ctypes.addressof(need))
             else:
                 continue
             scratch[gi] = torch.empty(max(need.value // 8, 1), dtype=torch.float64, device=self.device)
         counters = torch.zeros(2 * len(groups), dtype=torch.int32, device=self.device)
+        share = self._sm_shares(db, groups)
 
         def launch(gi, sfx, order_g, count, max_n, st):
             if isinstance(sfx, tuple) and sfx[0] == "small":
@@ -829,13 +848,11 @@ class Engine:
                            ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk),
                            ptr(eig), ptr(eig_status), 0, st)
             elif isinstance(sfx, tuple) and sfx[0] == "panels":
-                part = self._panels_part(count, max_n)
-                real = db.real if self.real_path else None
-                for a in range(0, count, part):
-                    cnt = min(part, count - a)
-                    self._call("skn_eigh_gen_panels", cnt, max_n, ptr(order_g[a:]), ptr(db.n), ptr(real),
-                               ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), 0,
-                               ptr(scratch[gi]), int(scratch[gi].numel() * 8), st)
+                for first, last, ws_off, nbytes, sizes in db._panel_parts[gi]:
+                    self._call("skn_eigh_gen_panels", last - first, sizes.ctypes.data, ptr(order_g[first:]), ptr(ws_off),
+                               ptr(db.n), ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff),
+                               ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), 0, ptr(scratch[gi]), nbytes, share[gi], st)
+                    self.launches += panels_launches(int(sizes[0])) - 1
             elif isinstance(sfx, tuple):
                 self._call("skn_eigh_gen_wide_tc" if self.wide_tc else "skn_eigh_gen_wide", count, max_n,
                            ptr(order_g), ptr(db.n), ptr(db.hs_off), ptr(db.eoff),
@@ -869,10 +886,14 @@ class Engine:
         for ev in joins:
             main.wait_event(ev)
 
-    @staticmethod
-    def _panels_part(count: int, max_n: int) -> int:
-        """Problems per skn_eigh_gen_panels call: as many as PANELS_SCRATCH holds."""
-        return max(1, min(count, PANELS_SCRATCH // max(1, panels_scratch_bytes(1, max_n))))
+    def _sm_shares(self, db, groups):
+        """SMs each group plans for: its part of the batch's n^3, as the groups run beside one another."""
+        cached = getattr(db, "_shares", None)
+        if cached is None or cached[0] is not groups:
+            cost = [float((db.plan.prob_n[sel].astype(np.float64) ** 3).sum()) for sel in db._group_problems]
+            sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+            cached = db._shares = (groups, [max(1, round(sms * c / max(sum(cost), 1.0))) for c in cost])
+        return cached[1]
 
     def _side_streams(self, k):
         """k side streams for forked launches, cached per host thread and device (engines are
@@ -887,8 +908,7 @@ class Engine:
 
     def _groups(self, db):
         """[(launch shape suffix, the cluster size for the cluster path, ("wide", n, real) for the device-wide
-        path, or route_auto's ("small", class) or ("panels", panels), device order, count, max_n)], cached on the
-        batch.
+        path, or route_auto's ("small", class) or ("panels", panel count), device order, count, max_n)], cached on the batch.
 
         Empty when every problem takes the default single-CTA launch."""
         plan = db.plan
@@ -925,11 +945,19 @@ class Engine:
             for i in dict.fromkeys(kind.tolist()):
                 sel = small_order[kind == i]
                 sfx = kinds[i % len(kinds)]
-                out.append(("_real" + sfx if i >= len(kinds) else sfx, sel, len(sel), int(plan.prob_n[sel].max())))
+                sfx = "_real" + sfx if i >= len(kinds) else sfx
+                out.append((sfx, sel, len(sel), int(plan.prob_n[sel].max())))
         if len(out) == 1 and out[0][0] == "" and out[0][2] == len(plan.order):
             out = []     # the default launch over the batch's own order
         real = plan.prob_real if (self.real_path and plan.prob_real is not None) else np.zeros(len(plan.prob_n), bool)
         out = [out[i] for i in launch_order([g[1] for g in out], plan.prob_n, real)]
+        db._group_problems = [g[1] for g in out]
+        db._panel_parts = {}
+        for gi, (sh, sel, _, _) in enumerate(out):
+            if isinstance(sh, tuple) and sh[0] == "panels":
+                sizes = np.ascontiguousarray(plan.prob_n[sel].astype(np.int32))
+                db._panel_parts[gi] = [(a, b, _i64(w, self.device), nbytes, sizes[a:b])
+                                       for a, b, w, nbytes in panels_parts(sizes, PANELS_SCRATCH)]
         out = [(sh, _i32(sel, self.device), cnt, mx) for sh, sel, cnt, mx in out]     # problem lists on the device
         db._groups = (key, out)
         return out

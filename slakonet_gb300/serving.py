@@ -15,9 +15,10 @@ batch ends only when its largest eigensolve ends.  So requests are sorted
 into two lanes by orbital count (``large_orbitals``).  ``small_workers`` of
 the workers take small requests only; the others take large requests first
 and small ones when no large one waits.  Within a lane a worker takes the
-cheapest requests first (n^3 x k-points), and problems above
-``wide_threshold`` orbitals run on the device-wide eigensolver (every SM on
-one structure's k-points), which shortens the longest eigensolve of a batch.
+cheapest requests first (n^3 x k-points).  A large request's eigensolve runs on
+as many SMs as it can use (the panel kernels' teams of CTAs; above
+``wide_threshold`` orbitals the device-wide eigensolver), which shortens the
+longest eigensolve of a batch.
 
 The reference serves one structure per call (slakonet/optim.py:949-1075 via
 predict_slakonet.py); there is no queue, batch or stream there.
@@ -40,10 +41,12 @@ from .model import MultiElementSkfParameterOptimizer, properties_dict
 MAX_N = E.LARGE_MAX_N   # cluster eigensolver bound (csrc/eigh_cluster.cu)
 
 
-def request_bytes(n_orb: int, nk: int, dos_points: int, wide_threshold: Optional[int] = None) -> int:
+def request_bytes(n_orb: int, nk: int, dos_points: int, wide_threshold: Optional[int] = None,
+                  panels: bool = False) -> int:
     """Device bytes one request holds while in flight (H, S, eigenvalues, DOS, slack for bonds), plus the
     device-wide eigensolver's scratch when its problems are above ``wide_threshold`` orbitals (panels,
-    partial sums and the tensor-core update's integer slices: about 5.5 KB per orbital and k-point)."""
+    partial sums and the tensor-core update's integer slices: about 5.5 KB per orbital and k-point), or with
+    ``panels`` the panel kernels' scratch below it (as much again, at most PANELS_SCRATCH at a time)."""
     nb = int(2 * 16 * n_orb * n_orb * nk + 8 * n_orb * nk + 8 * dos_points + (8 << 20))
     if wide_threshold is not None and wide_threshold < n_orb <= MAX_N and nk > 0:
         import ctypes
@@ -51,6 +54,8 @@ def request_bytes(n_orb: int, nk: int, dos_points: int, wide_threshold: Optional
         need = ctypes.c_int64(0)
         _lib.call("skn_eigh_wide_scratch_bytes", nk, n_orb, ctypes.addressof(need))
         nb += int(need.value)
+    elif panels and E.SMALL_MAX_N < n_orb <= E.PANELS_MAX_N:
+        nb += min(nk * E.panels_scratch_bytes(n_orb), 2 * E.PANELS_SCRATCH)
     return nb
 
 
@@ -95,8 +100,8 @@ class Server:
                  n_workers: int = 2, max_batch_problems: int = 8192, dos_range=(-20.0, 10.0),
                  dos_points: int = 1000, dos_sigma: float = 0.1, dos_window: float = 9.0,
                  executor: Optional[Callable] = None, large_orbitals: Optional[int] = 256,
-                 small_workers: Optional[int] = None, large_threshold: Optional[int] = 512,
-                 wide_threshold: Optional[int] = 512):
+                 small_workers: Optional[int] = None, large_threshold: Optional[int] = 2048,
+                 wide_threshold: Optional[int] = 2048):
         self.model = model
         self.sd = shell_dict
         self.device = torch.device(device)
@@ -144,7 +149,8 @@ class Server:
         with self.cv:
             self.rid += 1
             req = Request(self.rid, structure, n_orb, nk,
-                          request_bytes(n_orb, nk, self.dos["dos_points"], self.wide_threshold), time.perf_counter())
+                          request_bytes(n_orb, nk, self.dos["dos_points"], self.wide_threshold,
+                                    panels=self.tables is not None), time.perf_counter())
         err = None
         if missing:
             err = ValueError(f"no shells for element Z={missing[0]}")

@@ -2,7 +2,7 @@
 
 Sizes sit at the edges of its panels (32 columns in the factorisations, 16 in the tridiagonalisation), of the
 32-wide tiles of the matrix-vector products and of the 128 x 16 tiles of the tensor-core updates; a call mixes
-the sizes of one panel count.
+sizes.  The scratch starts as NaN.
 """
 import ctypes
 
@@ -39,19 +39,27 @@ def _setup(Hs, Ss):
     return sizes, H, S, dev(sizes.astype(np.int32)), dev(off), dev(eo), eo
 
 
-def _panels(Hs, Ss, real=None, slots=None, max_n=None):
+def _panels(Hs, Ss, real=None, slots=None, max_n=None, sms=0):
     sizes, H, S, nv, off, eod, eo = _setup(Hs, Ss)
     slots = np.arange(len(sizes)) if slots is None else np.asarray(slots)
-    prob = torch.as_tensor(slots.astype(np.int32), device=DEV)
     rl = None if real is None else torch.as_tensor(np.asarray(real, np.int32), device=DEV)
     eig = torch.full((int(sizes.sum()),), -7.0, dtype=torch.float64, device=DEV)
     st = torch.full((len(sizes),), -1, dtype=torch.int32, device=DEV)
-    mx = int(max_n or sizes[slots].max())
-    need = ctypes.c_int64(0)
-    call("skn_eigh_panels_scratch_bytes", len(slots), mx, ctypes.addressof(need))
-    scratch = torch.empty(need.value // 8, dtype=torch.float64, device=DEV)
-    call("skn_eigh_gen_panels", len(slots), mx, ptr(prob), ptr(nv), ptr(rl), ptr(off), ptr(eod), ptr(H), ptr(S), ptr(eig),
-         ptr(st), 0, ptr(scratch), need.value, torch.cuda.current_stream(DEV).cuda_stream)
+    host = np.ascontiguousarray(np.sort(sizes[slots])[::-1].astype(np.int32))
+    order = slots[np.argsort(-sizes[slots], kind="stable")]
+    prob = torch.as_tensor(order.astype(np.int32), device=DEV)
+    if max_n is not None:
+        host = np.minimum(host, max_n).astype(np.int32)
+    need, at = ctypes.c_int64(0), []
+    total = 0
+    for n in host:
+        at.append(total)
+        call("skn_eigh_panels_scratch_bytes", int(n), ctypes.addressof(need))
+        total += need.value
+    ws = torch.as_tensor(np.array(at, np.int64), device=DEV)
+    scratch = torch.full((total // 8,), float("nan"), dtype=torch.float64, device=DEV)
+    call("skn_eigh_gen_panels", len(slots), host.ctypes.data, ptr(prob), ptr(ws), ptr(nv), ptr(rl), ptr(off), ptr(eod),
+         ptr(H), ptr(S), ptr(eig), ptr(st), 0, ptr(scratch), total, sms, torch.cuda.current_stream(DEV).cuda_stream)
     torch.cuda.synchronize(DEV)
     e = eig.cpu().numpy()
     return [e[o:o + n] for o, n in zip(eo, sizes)], st.cpu().numpy()
@@ -77,7 +85,8 @@ def _bound(n, ref):
 
 
 @pytest.mark.parametrize("sizes", [(1, 2, 17, 32), (33, 34, 48, 49, 50, 64), (65, 80, 81, 82, 96), (97, 113, 128),
-                                   (129, 145, 160), (257, 272, 288), (385, 400, 401, 402, 416), (513, 534, 544), (1000,)])
+                                   (129, 145, 160), (257, 272, 288), (385, 400, 401, 402, 416), (513, 534, 544), (1000,), (1300,),
+                                   (3, 40, 97, 128, 129, 210, 256, 300)])
 def test_blocked_solver_agrees_with_lapack(sizes):
     Hs, Ss = _pairs(sizes, seed=sum(sizes))
     got, st = _panels(Hs, Ss)
@@ -101,27 +110,29 @@ def test_real_problems_in_a_mixed_call():
         assert np.abs(a - r).max() <= _bound(n, r) and np.abs(b - r).max() <= _bound(n, r)
 
 
-def test_results_do_not_depend_on_the_group():
-    """Alone a problem gets a cluster of CTAs; among 200 it gets one."""
-    sizes = (150, 129, 160)
+@pytest.mark.parametrize("sizes", [(150, 129, 160), (300, 289, 320)])
+def test_results_do_not_depend_on_the_group(sizes):
+    """Alone a problem gets many CTAs (a grid team, or a cluster where fewer SMs are planned for, resident in shared
+    memory); among 200 it gets one, streamed."""
     Hs, Ss = _pairs(sizes, seed=9)
     many, _ = _panels(Hs * 70, Ss * 70, slots=np.random.default_rng(1).permutation(210))
     for i in range(3):
-        alone, st = _panels([Hs[i]], [Ss[i]], max_n=160)
-        assert st[0] == 0
-        for q in range(0, 210, 3):
-            assert np.array_equal(alone[0], many[q + i])
+        for sms in (0, 20, 8, 2, 1):
+            alone, st = _panels([Hs[i]], [Ss[i]], sms=sms)
+            assert st[0] == 0
+            for q in range(0, 210, 21):
+                assert np.array_equal(alone[0], many[q + i]), (i, sms)
 
 
 def test_indefinite_overlap_and_zero_rows_and_other_sizes():
-    sizes = (100, 120, 128, 90)
+    sizes = (100, 120, 128, 150)
     Hs, Ss = _pairs(sizes, seed=2)
     Ss[1] = Ss[1] - 2.0 * np.eye(120) * np.abs(Ss[1]).max()
     for m in (Hs[2], Ss[2]):                     # an all-zero row and column counts as a unit diagonal
         m[40, :] = 0.0
         m[:, 40] = 0.0
     got, st = _panels(Hs, Ss, max_n=128)
-    assert st.tolist() == [0, 2, 0, 5]           # 90 orbitals are three panels, not four
+    assert st.tolist() == [0, 2, 0, 5]           # 150 orbitals in a call for at most 128
     assert np.isnan(got[1]).all() and (got[3] == -7.0).all()
     for i in (0, 2):
         h, s = Hs[i].copy(), Ss[i].copy()
