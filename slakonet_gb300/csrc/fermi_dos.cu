@@ -363,12 +363,24 @@ __global__ void __cluster_dims__(1, 1, skn_gauss::Z) __launch_bounds__(skn_gauss
 // and trapezoid integral, as get_properties_dict (slakonet/main.py:1766-1782).
 constexpr int DS_NT = 512;
 
-__global__ void __launch_bounds__(DS_NT) k_dos_stats(const double* __restrict__ grid, const double* __restrict__ dos,
-                                                     int npts, double* __restrict__ stats) {
+//
+// In the middle of a gap of more than about 75 sigma the unwindowed DOS runs through the subnormal numbers to zero, and
+// the minimum's place, the first point that is zero, hangs on the rounding of each term there. Those points (a sigma's
+// width at each edge, and the zeros next to it) are therefore summed again term by term, exponential first, as the
+// reference's expression is written; every other point keeps k_dos's value. A warp takes a point, a lane a k-point.
+constexpr double SUBNORMAL_BELOW = 1e-307, GONE_T = 39.0;      // exp(-t^2 / 2) is zero past t = 38.7
+
+__global__ void __launch_bounds__(DS_NT) k_dos_stats(const int64_t* __restrict__ eig_off, const int32_t* __restrict__ nkv,
+                                                     const int32_t* __restrict__ nbv, const int64_t* __restrict__ kw_off,
+                                                     const double* __restrict__ kweights, const double* __restrict__ eigall,
+                                                     const double* __restrict__ muv, double sigma, int windowed,
+                                                     const double* __restrict__ grid, double* dos, int npts,
+                                                     double* __restrict__ stats) {
   __shared__ double red[2 * DS_NT / 32];
   __shared__ int redi[DS_NT / 32];
-  const int s = blockIdx.x, tid = threadIdx.x;
-  const double* D = dos + (int64_t)s * npts;
+  __shared__ int again[DS_NT], n_again;
+  const int s = blockIdx.x, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  double* D = dos + (int64_t)s * npts;
   double av = INFINITY, mv = INFINITY, tr = 0.0, dummy = 0.0;
   int ai = 0x7fffffff, mi = 0x7fffffff;
   for (int i = tid; i < npts; i += DS_NT) {
@@ -381,6 +393,53 @@ __global__ void __launch_bounds__(DS_NT) k_dos_stats(const double* __restrict__ 
   block_argext(av, ai, false, red, redi);
   block_argext(mv, mi, false, red, redi);
   block_sum2(tr, dummy, red);
+  if (mv < SUBNORMAL_BELOW && !windowed && npts > 1) {
+    const int nk = nkv[s], nb = nbv[s];
+    const double* E = eigall + eig_off[s];
+    const double* w = kweights + kw_off[s];
+    const double mu = muv[s], inv_sigma = 1.0 / sigma;
+    const double inv_norm = 1.0 / (sigma * sqrt(2.0 * 3.141592653589793));
+    const double step = fabs(grid[1] - grid[0]);
+    const int reach = step > 0.0 && 0.2 * sigma < 64.0 * step ? 1 + (int)(0.2 * sigma / step) : 64;
+    for (int base = 0; base < npts; base += DS_NT) {
+      const int i = base + tid;
+      if (tid == 0) n_again = 0;
+      __syncthreads();
+      if (i < npts && fabs(grid[i]) < 2.0 && D[i] < SUBNORMAL_BELOW) {
+        bool take = D[i] != 0.0;
+        for (int q = max(0, i - reach); q <= min(npts - 1, i + reach) && !take; ++q) take = D[q] != 0.0;
+        if (take) again[atomicAdd(&n_again, 1)] = i;       // their order does not matter
+      }
+      __syncthreads();
+      for (int c = warp; c < n_again; c += DS_NT / 32) {
+        const int i0 = again[c];
+        const double x = grid[i0];
+        double acc = 0.0;
+        for (int k0 = 0; k0 < nk; k0 += 32) {
+          double sk = 0.0;
+          const double wk = k0 + lane < nk ? w[k0 + lane] : 0.0;
+          if (k0 + lane < nk) {
+            const double* Ek = E + (int64_t)(k0 + lane) * nb;
+            for (int b = 0; b < nb; ++b) {
+              const double t = (x - (Ek[b] - mu) * H2E) * inv_sigma;
+              if (fabs(t) < GONE_T) sk += exp(-0.5 * (t * t)) * inv_norm;
+            }
+          }
+          for (unsigned any = __ballot_sync(0xffffffffu, sk != 0.0); any; any &= any - 1) {
+            const int l = __ffs(any) - 1;
+            acc = fma(__shfl_sync(0xffffffffu, wk, l), __shfl_sync(0xffffffffu, sk, l), acc);
+          }
+        }
+        if (lane == 0) D[i0] = acc;
+      }
+      __syncthreads();
+    }
+    mv = INFINITY;
+    mi = 0x7fffffff;
+    for (int i = tid; i < npts; i += DS_NT)
+      if (fabs(grid[i]) < 2.0 && (D[i] < mv || (D[i] == mv && i < mi))) { mv = D[i]; mi = i; }
+    block_argext(mv, mi, false, red, redi);
+  }
   if (tid == 0) {
     double* st = stats + (int64_t)SKN_NSTAT * s;
     st[ST_DOS_FERMI] = D[ai];
@@ -434,7 +493,8 @@ extern "C" int skn_dos(int n_struct, const int64_t* eig_off, const int32_t* nk, 
     k_dos<false><<<g, skn_gauss::THREADS, 0, stream>>>(eig_off, nk, nb, kw_off, kweights, eig, mu, e_lo, e_hi, npts,
                                                        sigma, 0.0, grid, dos);
   if (cudaPeekAtLastError() != cudaSuccess) return SKN_ERR_CUDA;
-  k_dos_stats<<<n_struct, DS_NT, 0, stream>>>(grid, dos, npts, stats);
+  k_dos_stats<<<n_struct, DS_NT, 0, stream>>>(eig_off, nk, nb, kw_off, kweights, eig, mu, sigma, window_sigmas > 0.0,
+                                              grid, dos, npts, stats);
   return cudaPeekAtLastError() == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
 }
 

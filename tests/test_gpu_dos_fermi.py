@@ -128,3 +128,39 @@ def test_fermi_and_gap_over_the_split_sizes():
         ok = np.isfinite(kv) & np.isfinite(kc)
         assert (stats[s][10] == (kc - kv)[ok].min()) if ok.any() else np.isnan(stats[s][10])
         assert bs is not None
+
+
+@pytest.mark.parametrize("npts", [5000, 1001])
+def test_gap_centre_of_a_wide_gap_is_the_first_zero_of_the_summed_terms(npts):
+    """Through the subnormal numbers the minimum's place hangs on each term's rounding: the point must be the one of the
+    DOS summed term by term (the same exponential, on the GPU), gap by gap.  Weights that make no ties."""
+    B = _Batch([(1, 4), (3, 6)] * 40, seed=11)
+    rng = np.random.default_rng(5)
+    sigma, lo, hi = 0.1, -10.0, 10.0
+    for s, e in enumerate(B.eig):
+        half = rng.uniform(3.4, 4.6, 2) / H2E
+        nb = e.shape[1]
+        e[:, : nb // 2] = -half[0] - rng.uniform(0.0, 0.02, (len(e), nb // 2))
+        e[:, nb // 2:] = half[1] + rng.uniform(0.0, 0.02, (len(e), nb - nb // 2))
+        e.sort(axis=1)
+        B.w[s] = np.ones(1) if len(e) == 1 else np.array([0.3, 0.34, 0.36])
+    B.E, B.kw = _dev(np.concatenate([e.reshape(-1) for e in B.eig]), torch.float64), _dev(np.concatenate(B.w), torch.float64)
+    grid, dos, stats = _dos(B, np.zeros(B.n), lo, hi, npts, sigma, 0.0)
+    g = torch.as_tensor(grid, device=DEV)
+    inside = np.abs(grid) < 2.0
+    flat = 0
+    for s, e in enumerate(B.eig):
+        ref = torch.zeros_like(g)
+        for k in range(len(e)):
+            sk = torch.zeros_like(g)
+            for ev in e[k]:
+                t = (g - ev * H2E) * (1.0 / sigma)
+                sk = sk + torch.exp(-0.5 * (t * t)) * (1.0 / (sigma * np.sqrt(2.0 * np.pi)))
+            ref = ref + float(B.w[s][k]) * sk
+        r = np.where(inside, ref.cpu().numpy(), np.inf)
+        assert stats[s, 17] == grid[r.argmin()], (s, stats[s, 17], grid[r.argmin()])
+        small = inside & (r < 1e-307)
+        flat += int(small.any())
+        # 2e-11 of the sum, as above, and the last place of each subnormal term
+        assert (np.abs(dos[s][small] - r[small]) <= 2e-11 * r[small] + e.size * 4.0 * 4.95e-324).all()
+    assert flat > 20
