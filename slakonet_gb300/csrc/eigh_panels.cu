@@ -1417,20 +1417,20 @@ inline int pow2_below(int v, int most) {
 // 5000, so a grid team only from GRID_FROM CTAs.  Streamed: STREAM_PER_SM CTAs for each SM (three are resident; the
 // rest wait) even out the mixed batch's calls, which run beside one another: 305 ms at 3, 300 at 4, 289 at 6, 284 at 10.
 constexpr int GRID_FROM = 24, STREAM_PER_SM = 10;
-void plan_panel(int m, int n_prob, int sms, int& C, int& rt) {
+void plan_panel(int m, int n_prob, int sms, int all, int& C, int& rt) {
   const int nt = cdiv(m, TS), tiles = nt * (nt + 1) / 2;
   const int most = std::min(tiles, std::max(1, sms / n_prob));
   C = most >= GRID_FROM ? most : pow2_below(most, 16);
   rt = cdiv(tiles, C);
-  if ((int64_t)n_prob * C <= sms && panel_smem(m, rt, cdiv(nt, C)) <= SMEM_MAX) return;
+  if ((int64_t)n_prob * C <= all && panel_smem(m, rt, cdiv(nt, C)) <= SMEM_MAX) return;
   rt = 0;
   C = pow2_below(std::min(std::max(1, STREAM_PER_SM * sms / n_prob), std::max(1, tiles / (2 * PW))), 16);
 }
 
-cudaError_t launch_panel(const Grp& G, int count, int c0, int sms, cudaStream_t stream) {
+cudaError_t launch_panel(const Grp& G, int count, int c0, int sms, int all, cudaStream_t stream) {
   const int m = G.nmax - c0;
   int C, rt;
-  plan_panel(m, count, sms, C, rt);
+  plan_panel(m, count, sms, all, C, rt);
   const int cpc = cdiv(cdiv(m, TS), C);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)count * C);
@@ -1472,10 +1472,10 @@ void launch_update(const Grp& G, int count, int c1, int sms, cudaStream_t stream
 cudaError_t run(const Grp& G, const int32_t* sizes, int budget, cudaStream_t stream) {
   const int n = G.nmax, T = cdiv(n, NB);
   const unsigned P = (unsigned)G.n_prob;
-  int dev = 0, sms = 0;
+  int dev = 0, all = 0;
   cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (budget > 0 && budget < sms) sms = budget;
+  cudaDeviceGetAttribute(&all, cudaDevAttrMultiProcessorCount, dev);
+  const int sms = budget > 0 && budget < all ? budget : all;
   auto above = [&](int m) {                    // slots with more than m orbitals
     return (int)(std::lower_bound(sizes, sizes + G.n_prob, m, [](int a, int b) { return a > b; }) - sizes);
   };
@@ -1498,7 +1498,7 @@ cudaError_t run(const Grp& G, const int32_t* sizes, int budget, cudaStream_t str
     if (m > 0) launch_update<2>(G, above(c0 + NB), c0 + NB, sms, stream);
   }
   for (int c0 = 0; c0 < n - 1; c0 += NT) {
-    const cudaError_t e = launch_panel(G, above(c0 + 1), c0, sms, stream);
+    const cudaError_t e = launch_panel(G, above(c0 + 1), c0, sms, all, stream);
     if (e != cudaSuccess) return e;
     if (n - c0 - NT > 1) launch_update<3>(G, above(c0 + NT + 1), c0 + NT, sms, stream);
   }
