@@ -352,6 +352,23 @@ int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32_t* prob, c
 int skn_eigh_panels_scratch_bytes(int n, int64_t* bytes);
 
 /*
+ * Eigenvectors of problems that skn_eigh_gen_small or skn_eigh_gen_panels solved
+ * with `tri`: inverse iteration on the tridiagonal, then the reflectors and L^-H.
+ *   prob      [n_prob] problem indices, the largest first; max_n bounds their n (<= 2048)
+ *   H, S, eig, tri, status, real   as that call left them (real: as it was given)
+ *   vec       row-major per problem at hs_off, as skn_eigh_gen_vectors; NaN where
+ *             status is SKN_ERR_NOT_SPD, untouched where it is SKN_ERR_CAPACITY
+ *   scratch   at least the query's bytes for one problem of max_n; up to the query's for n_prob
+ *             lets more problems run at once, with the same results
+ *   counter   one int32
+ */
+int skn_eigvec(int n_prob, int max_n, const int32_t* prob, const int32_t* n, const int32_t* real, const int64_t* hs_off,
+               const int64_t* eig_off, const double* H, const double* S, const double* eig, const double* tri,
+               const int32_t* status, double* vec, double* scratch, int64_t scratch_bytes, int32_t* counter,
+               cudaStream_t stream);
+int skn_eigvec_scratch_bytes(int n_prob, int max_n, int64_t* bytes);
+
+/*
  * The same eigensolver compiled in more launch shapes: 32 threads per CTA with
  * up to 16 CTAs per SM (suffix _t32), 64 threads with up to 8 (_t64), 256
  * threads with up to 3 (_t256), and 128 threads with up to 3 whose Cholesky and

@@ -61,6 +61,8 @@ SIGNATURES = {
     "skn_eigh_gen_small": [I32, I32, P, P, P, P, P, P, P, P, P, P, P],
     "skn_eigh_gen_panels": [I32, P, P, P, P, P, P, P, P, P, P, P, P, P, I64, I32, P],
     "skn_eigh_panels_scratch_bytes": [I32, P],
+    "skn_eigvec": [I32, I32, P, P, P, P, P, P, P, P, P, P, P, P, I64, P, P],
+    "skn_eigvec_scratch_bytes": [I32, I32, P],
     "skn_adj_projectors": [I32, P, P, P, P, P, P, P, P, P, P],
     "skn_adj_bloch": [I64] + [P] * 18 + [P],
     "skn_adj_tables": [I64, P, P, P, P, P, P, I32, P, P, P, P, P, P, P, P, P, P, P, P],

@@ -23,16 +23,21 @@ namespace {
 
 constexpr double H2E = 27.211;
 
-// G, F per problem, 16x16 output tiles staged through shared memory.
+// G and F of every problem.  What bounds it: FP64 issue, 8 multiply-adds per (a, b, band).  Both are Hermitian, so only
+// the tiles on and below the diagonal are summed and the others mirrored; bands of zero weight (outside the DOS
+// window's reach, sorted to the ends) are passed over 16 at a time; the tiles of a problem go to gridDim.y CTAs, each
+// thread with 2 x 2 entries so that a shared-memory read feeds two of them.  One CTA per problem with one entry per
+// thread over the full square took 8.4 ms for the 484 problems of 30 to 116 orbitals of a training step.
+constexpr int AT = 32, AJ = 16;
 __global__ void __launch_bounds__(256) k_adj_projectors(int n_prob, const int32_t* __restrict__ nvec,
                                                         const int64_t* __restrict__ hs_off,
                                                         const int64_t* __restrict__ eig_off,
                                                         const double2* __restrict__ C, const double* __restrict__ eig,
                                                         const double* __restrict__ g, const int32_t* __restrict__ status,
                                                         double2* __restrict__ G, double2* __restrict__ F) {
-  __shared__ double2 ca[16][17], cb[16][17];
-  __shared__ double gj[16], gej[16];
-  const int tx = threadIdx.x & 15, ty = threadIdx.x >> 4;
+  __shared__ double2 ca[AT][AJ + 1], cb[AT][AJ + 1];
+  __shared__ double gj[AJ], gej[AJ];
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
   for (int p = blockIdx.x; p < n_prob; p += gridDim.x) {
     const int n = nvec[p];
     const double2* Cp = C + hs_off[p];
@@ -41,44 +46,67 @@ __global__ void __launch_bounds__(256) k_adj_projectors(int n_prob, const int32_
     double2* Gp = G + hs_off[p];
     double2* Fp = F + hs_off[p];
     if (status != nullptr && status[p] != SKN_OK) {   // failed problem: NaN vectors carry no gradient
-      for (int e = threadIdx.x; e < n * n; e += blockDim.x) {
+      for (int64_t e = blockIdx.y * 256 + tid; e < (int64_t)n * n; e += gridDim.y * 256) {
         Gp[e] = make_double2(0.0, 0.0);
         Fp[e] = make_double2(0.0, 0.0);
       }
       continue;
     }
-    for (int a0 = 0; a0 < n; a0 += 16) {
-      for (int b0 = 0; b0 < n; b0 += 16) {
-        const int a = a0 + tx, b = b0 + ty;
-        double2 accG = make_double2(0.0, 0.0), accF = make_double2(0.0, 0.0);
-        for (int j0 = 0; j0 < n; j0 += 16) {
-          const int jc = j0 + tx;
-          ca[ty][tx] = (a0 + ty < n && jc < n) ? Cp[(int64_t)(a0 + ty) * n + jc] : make_double2(0.0, 0.0);
-          cb[ty][tx] = (b0 + ty < n && jc < n) ? Cp[(int64_t)(b0 + ty) * n + jc] : make_double2(0.0, 0.0);
-          if (threadIdx.x < 16) {
-            const int j = j0 + threadIdx.x;
-            gj[threadIdx.x] = j < n ? gp[j] : 0.0;
-            gej[threadIdx.x] = j < n ? gp[j] * ep[j] : 0.0;
-          }
-          __syncthreads();
-#pragma unroll 4
-          for (int c = 0; c < 16; ++c) {
-            const double2 x = ca[tx][c], y = cb[ty][c];
-            // conj(x) * y
-            const double pr = fma(x.x, y.x, x.y * y.y);
-            const double pi = fma(x.x, y.y, -x.y * y.x);
-            accG.x = fma(gj[c], pr, accG.x);
-            accG.y = fma(gj[c], pi, accG.y);
-            accF.x = fma(gej[c], pr, accF.x);
-            accF.y = fma(gej[c], pi, accF.y);
-          }
-          __syncthreads();
+    const int T = (n + AT - 1) / AT;
+    for (int t = blockIdx.y; t < T * (T + 1) / 2; t += gridDim.y) {
+      int ta = (int)((sqrtf(8.0f * t + 1.0f) - 1.0f) * 0.5f);
+      while (ta * (ta + 1) / 2 > t) --ta;
+      while ((ta + 1) * (ta + 2) / 2 <= t) ++ta;
+      const int a0 = ta * AT, b0 = (t - ta * (ta + 1) / 2) * AT;
+      double2 accG[2][2], accF[2][2];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) accG[q >> 1][q & 1] = accF[q >> 1][q & 1] = make_double2(0.0, 0.0);
+      for (int j0 = 0; j0 < n; j0 += AJ) {
+        const int jc = j0 + tx;
+        const double gv = jc < n ? gp[jc] : 0.0;
+        if (!__syncthreads_or(gv != 0.0)) continue;      // also: the last chunk has been read
+        if (tid < AJ) {
+          gj[tid] = gv;
+          gej[tid] = jc < n ? gv * ep[jc] : 0.0;
         }
-        if (a < n && b < n) {
-          Gp[(int64_t)b * n + a] = accG;
-          Fp[(int64_t)b * n + a] = accF;
+#pragma unroll
+        for (int h = 0; h < AT; h += 16) {
+          const int a = a0 + h + ty, b = b0 + h + ty;
+          ca[h + ty][tx] = a < n && jc < n ? Cp[(int64_t)a * n + jc] : make_double2(0.0, 0.0);
+          cb[h + ty][tx] = b < n && jc < n ? Cp[(int64_t)b * n + jc] : make_double2(0.0, 0.0);
+        }
+        __syncthreads();
+#pragma unroll 4
+        for (int c = 0; c < AJ; ++c) {
+          const double2 x[2] = {ca[tx][c], ca[tx + 16][c]}, y[2] = {cb[ty][c], cb[ty + 16][c]};
+          const double w = gj[c], we = gej[c];
+#pragma unroll
+          for (int u = 0; u < 2; ++u)
+#pragma unroll
+            for (int v = 0; v < 2; ++v) {                // conj(x) * y
+              const double pr = fma(x[u].x, y[v].x, x[u].y * y[v].y);
+              const double pi = fma(x[u].x, y[v].y, -x[u].y * y[v].x);
+              accG[u][v].x = fma(w, pr, accG[u][v].x);
+              accG[u][v].y = fma(w, pi, accG[u][v].y);
+              accF[u][v].x = fma(we, pr, accF[u][v].x);
+              accF[u][v].y = fma(we, pi, accF[u][v].y);
+            }
         }
       }
+#pragma unroll
+      for (int u = 0; u < 2; ++u)
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          const int a = a0 + tx + 16 * u, b = b0 + ty + 16 * v;
+          if (a >= n || b >= n) continue;
+          const double2 cg = accG[u][v], cf = accF[u][v];
+          Gp[(int64_t)b * n + a] = cg;
+          Fp[(int64_t)b * n + a] = cf;
+          if (a0 != b0) {
+            Gp[(int64_t)a * n + b] = make_double2(cg.x, -cg.y);
+            Fp[(int64_t)a * n + b] = make_double2(cf.x, -cf.y);
+          }
+        }
     }
   }
 }
@@ -264,7 +292,9 @@ extern "C" int skn_adj_projectors(int n_prob, const int32_t* n, const int64_t* h
   if (n_prob < 0) return SKN_ERR_ARG;
   if (n_prob == 0) return SKN_OK;
   if (!n || !hs_off || !eig_off || !vec || !eig || !grad_eig || !G || !F) return SKN_ERR_ARG;
-  const int grid = n_prob < 152 * 8 ? n_prob : 152 * 8;
+  // CTAs per problem: 8 cover a problem of 116 orbitals' 10 tiles in two rounds; more for fewer problems
+  const int split = n_prob < 152 ? (152 * 8 / n_prob < 256 ? 152 * 8 / n_prob : 256) : 8;
+  const dim3 grid(n_prob < 152 * 64 ? n_prob : 152 * 64, split);
   k_adj_projectors<<<grid, 256, 0, stream>>>(n_prob, n, hs_off, eig_off, (const double2*)vec, eig, grad_eig,
                                              status, (double2*)G, (double2*)F);
   return cudaPeekAtLastError() == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;

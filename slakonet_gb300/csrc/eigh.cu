@@ -20,6 +20,7 @@
 // problems share every SM; several CTAs per SM hide the latency of the
 // per-column scalar steps.  Problems with n <= SMEM_N are staged in shared
 // memory; larger ones are factorised in place in global memory (L2-resident).
+#include "eigvec.cuh"
 #include "skn_common.cuh"
 #include "sturm.cuh"
 
@@ -871,256 +872,6 @@ __global__ void __launch_bounds__(NT, SKN_EIG_MINB) k_eigh_gen(int n_prob, const
 }
 
 
-// ============================================================= eigenvectors
-// Eigenvectors of H x = e S x for problems whose values kernel kept the
-// reflectors (lower triangle of H), tau, the tridiagonal (d, e) and L (in S):
-//   1. inverse iteration on T - e_j I (Gaussian elimination with partial
-//      pivoting on the tridiagonal, two solves from a pseudo-random start),
-//      one thread per eigenvalue; vectors of eigenvalues closer than 1e-9 of
-//      the spectrum's scale are re-orthogonalised (modified Gram-Schmidt, twice);
-//   2. y = Q z with Q = H_0 H_1 ... H_{n-2} (reflectors applied last first);
-//   3. x = L^-H y, so x^H S x = 1.
-// Vectors are written row-major per problem: vec[i*n + j] is component i of
-// eigenvector j (the reference's eigh column convention).
-constexpr int VNT = 128;
-constexpr int VNW = VNT / 32;
-
-__device__ __forceinline__ double hash_unit(unsigned a, unsigned b) {
-  unsigned h = a * 0x9E3779B1u ^ (b + 0x7F4A7C15u) * 0x85EBCA77u;
-  h ^= h >> 15; h *= 0x2C1B3C6Du; h ^= h >> 12; h *= 0x297A2D39u; h ^= h >> 15;
-  return (double)((int)(h & 0xFFFFFF) - 0x800000) * (1.0 / 8388608.0);   // [-1, 1)
-}
-
-__device__ double vblock_sum(double v, double* red) {
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  __syncthreads();
-  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
-  __syncthreads();
-  double t = 0.0;
-  for (int i = 0; i < VNW; ++i) t += red[i];
-  return t;
-}
-
-__global__ void __launch_bounds__(VNT) k_eigvec(int n_prob, const int32_t* __restrict__ nvec,
-                                                const int64_t* __restrict__ hs_off, const int64_t* __restrict__ eig_off,
-                                                const int32_t* __restrict__ order, const double2* __restrict__ H,
-                                                const double2* __restrict__ S, const double* __restrict__ eig,
-                                                const double* __restrict__ tri_all, const int32_t* __restrict__ status,
-                                                double2* __restrict__ vec, double* __restrict__ scratch,
-                                                int32_t* __restrict__ counter, int max_n) {
-  extern __shared__ double smem[];
-  double* red = smem;                                      // 2*VNW
-  double* d = smem + 2 * VNW;                              // max_n
-  double* e = d + max_n;                                   // max_n
-  double2* col = reinterpret_cast<double2*>(e + max_n);  // max_n (offset 2*VNW + 2*max_n doubles: even)
-  __shared__ int s_idx;
-  const int tid = threadIdx.x;
-  const int64_t sstride = (int64_t)max_n * VNT;
-  double* su = scratch + (int64_t)blockIdx.x * 5 * sstride;   // rows i: [i*VNT + tid]
-  double* s_ru1 = su;                 // 1 / u1
-  double* s_u2 = su + sstride;
-  double* s_u3 = su + 2 * sstride;
-  double* s_m = su + 3 * sstride;
-  double* s_pv = su + 4 * sstride;    // 1.0 where rows were swapped
-  for (;;) {
-    if (tid == 0) s_idx = atomicAdd(counter, 1);
-    __syncthreads();
-    const int idx = s_idx;
-    __syncthreads();
-    if (idx >= n_prob) break;
-    const int p = order[idx];
-    const int n = nvec[p];
-    double2* Y = vec + hs_off[p];
-    if (status[p] != SKN_OK) {
-      // a problem the values kernel refused for its size keeps its buffers untouched
-      if (status[p] != SKN_ERR_CAPACITY)
-        for (int q = tid; q < n * n; q += VNT) Y[q] = make_double2(__longlong_as_double(0x7ff8000000000000LL), 0.0);
-      __syncthreads();
-      continue;
-    }
-    const double* tri = tri_all + 4 * eig_off[p];
-    const double* w = eig + eig_off[p];
-    const double2* A = H + hs_off[p];
-    const double2* L = S + hs_off[p];
-    for (int i = tid; i < n; i += VNT) {
-      d[i] = tri[i];
-      e[i] = tri[n + i];
-    }
-    __syncthreads();
-    double scale = 0.0;
-    for (int i = tid; i < n; i += VNT) scale = fmax(scale, fabs(w[i]));
-    for (int o = 16; o > 0; o >>= 1) scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
-    __syncthreads();
-    if ((tid & 31) == 0) red[tid >> 5] = scale;
-    __syncthreads();
-    scale = red[0];
-    for (int q = 1; q < VNW; ++q) scale = fmax(scale, red[q]);
-    scale = fmax(scale, 1e-300);
-    const double pivmin = 1e-300 * fmax(1.0, scale);
-
-    // ---- 1. inverse iteration, one eigenvalue per thread
-    for (int j0 = 0; j0 < n; j0 += VNT) {
-      const int j = j0 + tid;
-      if (j < n) {
-        const double lam = w[j];
-        double u1 = d[0] - lam, u2 = (n > 1) ? e[0] : 0.0;
-        double rmax = 0.0;                 // largest |1 / pivot|
-        for (int i = 0; i < n - 1; ++i) {
-          const double c = e[i];
-          const double a1 = d[i + 1] - lam;
-          const double b1 = (i + 1 < n - 1) ? e[i + 1] : 0.0;
-          double m, r1, r2, r3, pv;
-          if (fabs(u1) >= fabs(c)) {
-            if (fabs(u1) < pivmin) u1 = (u1 < 0.0) ? -pivmin : pivmin;
-            m = c / u1;
-            r1 = u1; r2 = u2; r3 = 0.0; pv = 0.0;
-            u1 = a1 - m * u2;
-            u2 = b1;
-          } else {
-            m = u1 / c;
-            r1 = c; r2 = a1; r3 = b1; pv = 1.0;
-            u1 = u2 - m * a1;
-            u2 = -m * b1;
-          }
-          s_ru1[i * VNT + tid] = 1.0 / r1;
-          rmax = fmax(rmax, fabs(1.0 / r1));
-          s_u2[i * VNT + tid] = r2;
-          s_u3[i * VNT + tid] = r3;
-          s_m[i * VNT + tid] = m;
-          s_pv[i * VNT + tid] = pv;
-        }
-        if (fabs(u1) < pivmin) u1 = (u1 < 0.0) ? -pivmin : pivmin;
-        s_ru1[(n - 1) * VNT + tid] = 1.0 / u1;
-        s_u2[(n - 1) * VNT + tid] = 0.0;   // the last row has no columns to its right: the back substitution
-        s_u3[(n - 1) * VNT + tid] = 0.0;   // multiplies these by zero, and scratch may hold a NaN
-        rmax = fmax(rmax, fabs(1.0 / u1));
-        // A lam exact to the last bit (the Newton step can land on the eigenvalue) leaves a pivot at the
-        // 1e-300 floor, and a solve then grows the vector by up to 1 / pivot: its sum of squares overflowed
-        // and the eigenvector came out NaN.  Every solve's right-hand side is therefore scaled by
-        // ysc = 2^-e with 2^e >= rmax, which keeps the solution near unit size; a power of two scales
-        // exactly, so without a tiny pivot the normalised vectors are bitwise what they were unscaled.
-        int rex = 0;
-        frexp(rmax, &rex);
-        const double ysc = rex > 0 ? ldexp(1.0, -rex) : 1.0;
-        // y lives in the real parts of column j of Y
-        for (int i = 0; i < n; ++i) Y[(int64_t)i * n + j] = make_double2(hash_unit(j, i) * ysc, 0.0);
-        for (int it = 0; it < 2; ++it) {
-          for (int i = 0; i < n - 1; ++i) {
-            const double m = s_m[i * VNT + tid];
-            const double yi = Y[(int64_t)i * n + j].x, yn = Y[(int64_t)(i + 1) * n + j].x;
-            if (s_pv[i * VNT + tid] != 0.0) {
-              Y[(int64_t)i * n + j].x = yn;
-              Y[(int64_t)(i + 1) * n + j].x = yi - m * yn;
-            } else {
-              Y[(int64_t)(i + 1) * n + j].x = yn - m * yi;
-            }
-          }
-          double x2 = 0.0, x1 = 0.0, nrm = 0.0;
-          for (int i = n - 1; i >= 0; --i) {
-            const double xi = (Y[(int64_t)i * n + j].x - s_u2[i * VNT + tid] * x1 - s_u3[i * VNT + tid] * x2) *
-                              s_ru1[i * VNT + tid];
-            Y[(int64_t)i * n + j].x = xi;
-            nrm = fma(xi, xi, nrm);
-            x2 = x1;
-            x1 = xi;
-          }
-          if (!(nrm > 0.0 && nrm <= 1.7976931348623157e308)) {   // vanished, overflowed or NaN: restart from e_j
-            for (int i = 0; i < n; ++i) Y[(int64_t)i * n + j].x = (i == j) ? ysc : 0.0;
-            nrm = ysc * ysc;
-          }
-          // normalised, and scaled by ysc again when it is the next solve's right-hand side
-          const double inv = (it == 0 ? ysc : 1.0) / sqrt(nrm);
-          for (int i = 0; i < n; ++i) Y[(int64_t)i * n + j].x *= inv;
-        }
-      }
-    }
-    __syncthreads();
-    // ---- clusters: modified Gram-Schmidt (twice) within runs of close eigenvalues
-    {
-      const double ctol = 1e-9 * scale;
-      int j = 1;
-      while (j < n) {
-        if (w[j] - w[j - 1] > ctol) { ++j; continue; }
-        int j0 = j - 1, j1 = j + 1;
-        while (j1 < n && w[j1] - w[j1 - 1] <= ctol) ++j1;
-        for (int pass = 0; pass < 2; ++pass) {
-          for (int q = j0; q < j1; ++q) {
-            for (int r = j0; r < q; ++r) {
-              double dp = 0.0;
-              for (int i = tid; i < n; i += VNT) dp = fma(Y[(int64_t)i * n + r].x, Y[(int64_t)i * n + q].x, dp);
-              dp = vblock_sum(dp, red);
-              for (int i = tid; i < n; i += VNT) Y[(int64_t)i * n + q].x -= dp * Y[(int64_t)i * n + r].x;
-              __syncthreads();
-            }
-            double nn = 0.0;
-            for (int i = tid; i < n; i += VNT) nn = fma(Y[(int64_t)i * n + q].x, Y[(int64_t)i * n + q].x, nn);
-            nn = vblock_sum(nn, red);
-            const double inv = 1.0 / sqrt(nn);
-            for (int i = tid; i < n; i += VNT) Y[(int64_t)i * n + q].x *= inv;
-            __syncthreads();
-          }
-        }
-        j = j1;
-      }
-    }
-    __syncthreads();
-    // ---- 2. back-transformation y = Q z
-    for (int k = n - 2; k >= 0; --k) {
-      const double2 tau = make_double2(tri[2 * n + 2 * k], tri[2 * n + 2 * k + 1]);
-      if (tau.x == 0.0 && tau.y == 0.0) continue;
-      const int m = n - k - 1;
-      for (int r = tid; r < m; r += VNT)
-        col[r] = (r == 0) ? make_double2(1.0, 0.0) : A[(k + 1 + r) + (int64_t)k * n];
-      __syncthreads();
-      for (int jj = tid; jj < n; jj += VNT) {
-        double2 s0 = make_double2(0.0, 0.0), s1 = s0, s2 = s0, s3 = s0;
-        int r = 0;
-        for (; r + 3 < m; r += 4) {
-          const double2 y0 = Y[(int64_t)(k + 1 + r) * n + jj], y1 = Y[(int64_t)(k + 2 + r) * n + jj];
-          const double2 y2 = Y[(int64_t)(k + 3 + r) * n + jj], y3 = Y[(int64_t)(k + 4 + r) * n + jj];
-          s0 = cfma_conj(col[r], y0, s0);
-          s1 = cfma_conj(col[r + 1], y1, s1);
-          s2 = cfma_conj(col[r + 2], y2, s2);
-          s3 = cfma_conj(col[r + 3], y3, s3);
-        }
-        for (; r < m; ++r) s0 = cfma_conj(col[r], Y[(int64_t)(k + 1 + r) * n + jj], s0);
-        s0.x += s1.x + (s2.x + s3.x);
-        s0.y += s1.y + (s2.y + s3.y);
-        const double2 ts = cmul(tau, s0);          // y -= tau v (v^H y)
-        for (int q = 0; q < m; ++q) {
-          double2 y = Y[(int64_t)(k + 1 + q) * n + jj];
-          y = cfms_conj(col[q], make_double2(ts.x, -ts.y), y);
-          Y[(int64_t)(k + 1 + q) * n + jj] = y;
-        }
-      }
-      __syncthreads();
-    }
-    // ---- 3. x = L^-H y (backward substitution, one column per thread)
-    for (int i = n - 1; i >= 0; --i) {
-      const int m = n - i - 1;
-      for (int r = tid; r < m; r += VNT) col[r] = L[(i + 1 + r) + (int64_t)i * n];
-      if (tid == 0) col[max_n - 1] = L[i + (int64_t)i * n];
-      __syncthreads();
-      const double rl = 1.0 / col[max_n - 1].x;
-      for (int jj = tid; jj < n; jj += VNT) {
-        double2 acc0 = Y[(int64_t)i * n + jj], acc1 = make_double2(0.0, 0.0), acc2 = acc1, acc3 = acc1;
-        int r = 0;
-        for (; r + 3 < m; r += 4) {
-          const double2 y0 = Y[(int64_t)(i + 1 + r) * n + jj], y1 = Y[(int64_t)(i + 2 + r) * n + jj];
-          const double2 y2 = Y[(int64_t)(i + 3 + r) * n + jj], y3 = Y[(int64_t)(i + 4 + r) * n + jj];
-          acc0 = cfms_conj_l(col[r], y0, acc0);
-          acc1 = cfms_conj_l(col[r + 1], y1, acc1);
-          acc2 = cfms_conj_l(col[r + 2], y2, acc2);
-          acc3 = cfms_conj_l(col[r + 3], y3, acc3);
-        }
-        for (; r < m; ++r) acc0 = cfms_conj_l(col[r], Y[(int64_t)(i + 1 + r) * n + jj], acc0);
-        Y[(int64_t)i * n + jj] = make_double2((acc0.x + acc1.x + (acc2.x + acc3.x)) * rl,
-                                              (acc0.y + acc1.y + (acc2.y + acc3.y)) * rl);
-      }
-      __syncthreads();
-    }
-  }
-}
 }  // namespace
 }  // namespace SKN_EIG_NS
 using namespace SKN_EIG_NS;
@@ -1132,16 +883,12 @@ static size_t eig_smem_bytes(int mn) {
   return sizeof(double) * (16 + 4 * NW + 2 * NT + 3 * (size_t)mn + (mn & 1) + 4 * (size_t)mn) +
          (SMEM_REGION + (SKN_EIG_BLOCKED ? NB * LDT : 0)) * sizeof(double2);
 }
-static size_t vec_smem_bytes(int mn) {
-  return sizeof(double) * (2 * VNW + 2 * (size_t)mn + 2) + sizeof(double2) * (size_t)mn;
-}
 static cudaError_t set_smem_limit_once() {
   cudaError_t e = cudaFuncSetAttribute(k_eigh_gen<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        (int)eig_smem_bytes(MAX_N));
   if (e != cudaSuccess) return e;
-  e = cudaFuncSetAttribute(k_eigh_gen<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)eig_smem_bytes(MAX_N));
-  if (e != cudaSuccess) return e;
-  return cudaFuncSetAttribute(k_eigvec, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)vec_smem_bytes(MAX_N));
+  return cudaFuncSetAttribute(k_eigh_gen<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)eig_smem_bytes(MAX_N));
 }
 
 // Values-only launch of k_eigh_gen<R> over a persistent grid (all problems of the call).
@@ -1185,33 +932,9 @@ extern "C" int SKN_EXPORT(skn_eigh_gen_batched_real)(int n_prob, const int32_t* 
   return launch_values<true>(n_prob, n, hs_off, eig_off, order, H, S, eig, status, work_counter, max_n, stream);
 }
 
-// CTAs of the vector stage: as many as fit on the GPU at once (the stage is latency-bound, so
-// occupancy matters), but no more than the problems, and no more than keep the inverse-iteration
-// scratch (5 * max_n * VNT doubles per CTA) within VEC_SCRATCH_BUDGET.  Each problem is solved by
-// one CTA, so the results do not depend on the grid.
-constexpr int64_t VEC_SCRATCH_BUDGET = (int64_t)2 << 30;
-static int vec_grid(int n_prob, int max_n) {
-  int dev = 0, sms = 0, per_sm = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (sms < 1) sms = 1;
-  const int mn = max_n < 1 ? 1 : max_n;
-  if (set_smem_limit_once() != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_eigvec, VNT, vec_smem_bytes(mn)) != cudaSuccess ||
-      per_sm < 1)
-    per_sm = 2;
-  int64_t g = (int64_t)sms * per_sm;
-  const int64_t per_cta = (int64_t)5 * mn * VNT * (int64_t)sizeof(double);
-  const int64_t cap = VEC_SCRATCH_BUDGET / per_cta;
-  if (g > cap) g = cap;
-  if (g < sms) g = sms < n_prob ? sms : n_prob;      // never fewer than one CTA per SM (or per problem)
-  if (g > n_prob) g = n_prob;
-  return g > 0 ? (int)g : 1;
-}
-
 extern "C" int SKN_EXPORT(skn_eigh_vectors_scratch_bytes)(int n_prob, int max_n, int64_t* bytes) {
   if (!bytes || max_n < 0 || n_prob < 0) return SKN_ERR_ARG;
-  *bytes = (int64_t)vec_grid(n_prob, max_n) * 5 * (int64_t)(max_n < 1 ? 1 : max_n) * VNT * (int64_t)sizeof(double);
+  *bytes = skn_vec::grid(n_prob, max_n) * skn_vec::cta_bytes(max_n);
   return SKN_OK;
 }
 
@@ -1244,11 +967,7 @@ extern "C" int SKN_EXPORT(skn_eigh_gen_vectors)(int n_prob, const int32_t* n, co
   k_eigh_gen<false><<<grid, NT, smem, stream>>>(n_prob, n, hs_off, eig_off, order, (double2*)H, (double2*)S, eig, status,
                                          work_counter, mn, use_smem_mats, tri, INT64_MAX);
   if (cudaPeekAtLastError() != cudaSuccess) return SKN_ERR_CUDA;
-  const size_t vsmem = sizeof(double) * (2 * VNW + 2 * (size_t)mn + 2) + sizeof(double2) * (size_t)mn;
-
-  k_eigvec<<<vec_grid(n_prob, mn), VNT, vsmem, stream>>>(n_prob, n, hs_off, eig_off, order, (const double2*)H,
-                                                     (const double2*)S, eig, tri, status, (double2*)vec, scratch,
-                                                     work_counter + 1, mn);
-  return cudaPeekAtLastError() == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
+  return skn_vec::launch(n_prob, n, hs_off, eig_off, order, nullptr, H, S, eig, tri, status, vec, scratch,
+                         skn_vec::grid(n_prob, mn), work_counter + 1, mn, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
 }
 #endif  // SKN_EIG_KERNELS_ONLY

@@ -24,7 +24,7 @@ constexpr int64_t NA_SCRATCH_DOUBLES = SKN_NOALLOC_SCRATCH_DOUBLES;
 constexpr int64_t NA_TOTAL_DOUBLES = NA_COUNTER_DOUBLES + NA_TRI_DOUBLES + NA_SCRATCH_DOUBLES;
 static_assert(SKN_NOALLOC_MAX_N <= MAX_N, "the static variant cannot exceed the eigensolver's bound");
 static_assert(NA_TRI_DOUBLES % 32 == 0, "keep the scratch section 256-byte aligned");
-static_assert((int64_t)5 * SKN_NOALLOC_MAX_N * VNT <= NA_SCRATCH_DOUBLES, "one vector CTA must fit");
+static_assert((int64_t)5 * SKN_NOALLOC_MAX_N * skn_vec::VNT <= NA_SCRATCH_DOUBLES, "one vector CTA must fit");
 
 // [counters | tri: 4 doubles per eigenvalue row | inverse-iteration scratch]
 static __device__ __align__(256) double g_noalloc[NA_TOTAL_DOUBLES];
@@ -69,7 +69,7 @@ extern "C" int skn_eigh_gen_vectors_noalloc(int n_prob, const int32_t* n, const 
   int grid = sms * per_sm;
   if (grid > n_prob) grid = n_prob;
   // the vector stage takes as many CTAs as the fixed workspace holds (at most 2 per SM)
-  int vgrid = (int)(NA_SCRATCH_DOUBLES / ((int64_t)5 * mn * VNT));
+  int vgrid = (int)(NA_SCRATCH_DOUBLES * (int64_t)sizeof(double) / skn_vec::cta_bytes(mn));
   if (vgrid > 2 * sms) vgrid = 2 * sms;
   if (vgrid > n_prob) vgrid = n_prob;
   // only the queue counters must start at zero; every tri row and scratch entry is written before it is read
@@ -77,8 +77,6 @@ extern "C" int skn_eigh_gen_vectors_noalloc(int n_prob, const int32_t* n, const 
   k_eigh_gen<false><<<grid, NT, smem, stream>>>(n_prob, n, hs_off, eig_off, order, (double2*)H, (double2*)S, eig, status,
                                          counter, mn, use_smem_mats, tri, n_rows);
   if (cudaPeekAtLastError() != cudaSuccess) return SKN_ERR_CUDA;
-  k_eigvec<<<vgrid, VNT, vec_smem_bytes(mn), stream>>>(n_prob, n, hs_off, eig_off, order, (const double2*)H,
-                                                       (const double2*)S, eig, tri, status, (double2*)vec, scratch,
-                                                       counter + 1, mn);
-  return cudaPeekAtLastError() == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
+  return skn_vec::launch(n_prob, n, hs_off, eig_off, order, nullptr, H, S, eig, tri, status, vec, scratch, vgrid,
+                         counter + 1, mn, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
 }

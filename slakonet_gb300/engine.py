@@ -494,7 +494,7 @@ class DeviceBatch:
 # kernels each ABI call launches (for the launch count the bench reports)
 KERNELS_PER_CALL = {"skn_bond_counts": 1, "skn_bond_fill": 1, "skn_image_phases": 1, "skn_sk_blocks": 1,
                     "skn_bloch": 1, "skn_bloch_pairs": 1, "skn_eigh_gen_batched": 1, "skn_eigh_gen_vectors": 2, "skn_fermi_gap": 1,
-                    "skn_dos": 2, "skn_eigh_gen_large": 1, "skn_eigh_gen_vectors_noalloc": 2}
+                    "skn_dos": 2, "skn_eigvec": 2, "skn_eigh_gen_large": 1, "skn_eigh_gen_vectors_noalloc": 2}
 
 def wide_launches(n: int, nb: int = 32, tc: bool = False, tc_min: int = 512) -> int:
     """Kernel launches of one skn_eigh_gen_wide(_tc) call for problems of n orbitals (its host sequence);
@@ -546,6 +546,9 @@ def panels_parts(sizes: np.ndarray, budget: int):
         parts.append((first, last, end[first:last] - per[first:last] - base, int(end[last - 1]) - base))
         first = last
     return parts
+
+
+VEC_SCRATCH = 512 << 20      # device bytes of the inverse iteration's scratch per group
 
 
 SMALL_MAX_N = 96            # bound of the shared-memory eigensolver (csrc/eigh_small.cu)
@@ -777,29 +780,25 @@ class Engine:
         eig = torch.empty(max(plan.eig_total, 1), dtype=torch.float64, device=dev)
         eig_status = torch.empty(max(n_prob, 1), dtype=torch.int32, device=dev)
         counter = torch.zeros(2, dtype=torch.int32, device=dev)
-        vec = None
+        vec = tri = None
         if vectors:
+            if plan.max_n > PANELS_MAX_N:
+                raise _lib.SknError(f"eigenvectors: problems of up to {PANELS_MAX_N} orbitals")
             vec = torch.empty(2 * max(plan.hs_total, 1), dtype=torch.float64, device=dev)
             tri = torch.empty(4 * max(plan.eig_total, 1), dtype=torch.float64, device=dev)
-            need = ctypes.c_int64(0)
-            call("skn_eigh_vectors_scratch_bytes", n_prob, plan.max_n, ctypes.addressof(need))
-            scratch = torch.empty(max(need.value // 8, 1), dtype=torch.float64, device=dev)
-            self._call("skn_eigh_gen_vectors", n_prob, ptr(db.n), ptr(db.hs_off), ptr(db.eoff), ptr(db.order),
-                       ptr(Hk), ptr(Sk), ptr(eig), ptr(vec), ptr(eig_status), ptr(tri), ptr(scratch),
-                       int(need.value), ptr(counter), plan.max_n, stream)
+        ev = self.event_log
+        if ev is not None:
+            a = torch.cuda.Event(enable_timing=True)
+            b = torch.cuda.Event(enable_timing=True)
+            a.record()
+            self.event_log = None        # the phase is timed as a whole (groups run on forked streams)
+        self._eig_values(db, Hk, Sk, eig, eig_status, counter, stream, tri, vec)
+        if ev is not None:
+            b.record()
+            self.event_log = ev
+            ev.append(("eigensolve", a, b))
+        if vectors:
             vec = torch.view_as_complex(vec.view(-1, 2))
-        else:
-            ev = self.event_log
-            if ev is not None:
-                a = torch.cuda.Event(enable_timing=True)
-                b = torch.cuda.Event(enable_timing=True)
-                a.record()
-                self.event_log = None        # the phase is timed as a whole (groups run on forked streams)
-            self._eig_values(db, Hk, Sk, eig, eig_status, counter, stream)
-            if ev is not None:
-                b.record()
-                self.event_log = ev
-                ev.append(("eigensolve", a, b))
         mu = torch.empty(S, dtype=torch.float64, device=dev)
         stats = torch.zeros(S * _lib.SKN_NSTAT, dtype=torch.float64, device=dev)
         fst = torch.empty(S, dtype=torch.int32, device=dev)
@@ -819,10 +818,11 @@ class Engine:
                                        float(dos_window)))
         return out
 
-    def _eig_values(self, db, Hk, Sk, eig, eig_status, counter, stream):
+    def _eig_values(self, db, Hk, Sk, eig, eig_status, counter, stream, tri=None, vec=None):
+        """Eigenvalues, and the eigenvectors into ``vec`` where it is given (``tri``: 4 doubles per eigenvalue)."""
         plan = db.plan
         n_prob = len(plan.prob_n)
-        groups = self._groups(db)
+        groups = self._groups(db, vec is not None)
         if not groups:
             self._call("skn_eigh_gen_batched", n_prob, ptr(db.n), ptr(db.hs_off), ptr(db.eoff), ptr(db.order),
                        ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counter), plan.max_n, stream)
@@ -839,6 +839,14 @@ class Engine:
             else:
                 continue
             scratch[gi] = torch.empty(max(need.value // 8, 1), dtype=torch.float64, device=self.device)
+        vec_scratch = []
+        if vec is not None:                  # the inverse iteration takes what it is given, at least one CTA's part
+            for _, _, count, max_n in groups:
+                need, one = ctypes.c_int64(0), ctypes.c_int64(0)
+                call("skn_eigvec_scratch_bytes", count, max_n, ctypes.addressof(need))
+                call("skn_eigvec_scratch_bytes", 1, max_n, ctypes.addressof(one))
+                nbytes = min(need.value, max(VEC_SCRATCH, one.value))
+                vec_scratch.append(torch.empty(nbytes // 8, dtype=torch.float64, device=self.device))
         counters = torch.zeros(2 * len(groups), dtype=torch.int32, device=self.device)
         share = self._sm_shares(db, groups)
 
@@ -846,12 +854,13 @@ class Engine:
             if isinstance(sfx, tuple) and sfx[0] == "small":
                 self._call("skn_eigh_gen_small", count, max_n, ptr(order_g), ptr(db.n),
                            ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk),
-                           ptr(eig), ptr(eig_status), 0, st)
+                           ptr(eig), ptr(eig_status), ptr(tri), st)
             elif isinstance(sfx, tuple) and sfx[0] == "panels":
                 for first, last, ws_off, nbytes, sizes in db._panel_parts[gi]:
                     self._call("skn_eigh_gen_panels", last - first, sizes.ctypes.data, ptr(order_g[first:]), ptr(ws_off),
                                ptr(db.n), ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff),
-                               ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), 0, ptr(scratch[gi]), nbytes, share[gi], st)
+                               ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(tri), ptr(scratch[gi]), nbytes, share[gi],
+                               st)
                     self.launches += panels_launches(int(sizes[0])) - 1
             elif isinstance(sfx, tuple):
                 self._call("skn_eigh_gen_wide_tc" if self.wide_tc else "skn_eigh_gen_wide", count, max_n,
@@ -866,6 +875,10 @@ class Engine:
                 self._call("skn_eigh_gen_batched" + sfx, count, ptr(db.n), ptr(db.hs_off), ptr(db.eoff),
                            ptr(order_g), ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counters[2 * gi:]),
                            max_n, st)
+            if vec is not None:
+                self._call("skn_eigvec", count, max_n, ptr(order_g), ptr(db.n), ptr(db.real if self.real_path else None),
+                           ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk), ptr(eig), ptr(tri), ptr(eig_status), ptr(vec),
+                           ptr(vec_scratch[gi]), int(vec_scratch[gi].numel() * 8), ptr(counters[2 * gi + 1:]), st)
 
         if len(groups) == 1:
             launch(0, *groups[0], stream)
@@ -906,18 +919,20 @@ class Engine:
             cur.append(torch.cuda.Stream(self.device))
         return cur
 
-    def _groups(self, db):
+    def _groups(self, db, vectors: bool = False):
         """[(launch shape suffix, the cluster size for the cluster path, ("wide", n, real) for the device-wide
         path, or route_auto's ("small", class) or ("panels", panel count), device order, count, max_n)], cached on the batch.
 
-        Empty when every problem takes the default single-CTA launch."""
+        Empty when every problem takes the default single-CTA launch.  With ``vectors`` every problem takes route_auto's
+        kernel: the others keep no reflectors."""
         plan = db.plan
-        key = (id(self.tuning), self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
+        key = (vectors, id(self.tuning), self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
         cache = getattr(db, "_groups", None)
         if cache is not None and cache[0] == key:
             return cache[1]
-        wide = route_wide(plan.prob_n, self.wide_threshold)[plan.order]
-        csize = route_large(plan.prob_n, self.large_threshold, self.large_cluster)[plan.order]
+        wide = route_wide(plan.prob_n, None if vectors else self.wide_threshold)[plan.order]
+        csize = (np.zeros(len(plan.order), int) if vectors
+                 else route_large(plan.prob_n, self.large_threshold, self.large_cluster)[plan.order])
         csize[wide] = 0
         large = (csize > 0) | wide
         out = []
@@ -935,7 +950,7 @@ class Engine:
         if len(small_order):
             tuning = self.tuning if self.tuning is not None else _default_tuning()
             ns, at = np.unique(plan.prob_n[small_order], return_inverse=True)
-            names = [tuning.shape_for(int(n)) for n in ns]
+            names = ["auto" if vectors else tuning.shape_for(int(n)) for n in ns]
             names = [route_auto(int(n)) if x == "auto" else x for n, x in zip(ns, names)]
             kinds = list(dict.fromkeys(names))
             kind = np.array([kinds.index(x) for x in names])[at]
