@@ -74,11 +74,10 @@ def adjoint(eng: "E.Engine", res: "E.BatchResult", g_eig=None, g_dos=None, g_gap
         ok = (vf >= 0) & (cf >= 0)
         base = db.eos
         gg = g_gap.to(torch.float64) * H2E
-        iv = (base + vf.clamp(min=0).long())[ok]
-        ic = (base + cf.clamp(min=0).long())[ok]
-        g.index_add_(0, iv, -gg[ok])
-        g.index_add_(0, ic, gg[ok])
-    st["degenerate_pairs"] = _degenerate_pairs(plan, res.eig, g)
+        gg = torch.where(ok, gg, 0.0)             # a zero added, not a selection: that would wait for the device
+        g.index_add_(0, base + vf.clamp(min=0).long(), -gg)
+        g.index_add_(0, base + cf.clamp(min=0).long(), gg)
+    pairs = _degenerate_pairs(plan, res.eig, g)
     n_prob = len(plan.prob_n)
     Gm = torch.empty(2 * max(plan.hs_total, 1), dtype=torch.float64, device=dev)
     Fm = torch.empty_like(Gm)
@@ -104,31 +103,55 @@ def adjoint(eng: "E.Engine", res: "E.BatchResult", g_eig=None, g_dos=None, g_gap
              ptr(st["bond_blk"]), ptr(db.species), len(T.species), ptr(T.sp_nshell), ptr(T.sp_shell_l),
              ptr(T.sp_norb), ptr(T.tab_index), ptr(T.tab_off), ptr(T.tab_ngrid), ptr(T.tab_step), ptr(gbH), ptr(gbS),
              ptr(dtab_H), ptr(dtab_S), stream)
-    grads = []
-    for tensor, kind, off, numel in T.param_slices:
-        src = dtab_H if kind == "H" else dtab_S
-        grads.append(src[off: off + numel].view(tensor.shape).to(tensor.device))
-    return grads
+    st["degenerate_pairs"] = pairs()                    # waits for the count alone, behind the launches
+    pieces = {"H": _pieces(dtab_H, "H", T.param_slices), "S": _pieces(dtab_S, "S", T.param_slices)}
+    grads = [next(pieces[kind]).view(tensor.shape) for tensor, kind, _, _ in T.param_slices]
+    return [x if x.device == t[0].device else x.to(t[0].device) for x, t in zip(grads, T.param_slices)]
 
 
-def _degenerate_pairs(plan, eig, g, tol: float = 1e-8) -> int:
+def _pieces(flat, kind, param_slices):
+    """The parts of ``flat`` that belong to the parameters of one kind, in their order: one split, not a slice each
+    (the several hundred tables of a training model took 1.8 ms of host time)."""
+    sizes, keep, at = [], [], 0
+    for _, k, off, numel in param_slices:
+        if k == kind:
+            if off > at:
+                sizes.append(off - at)
+            keep.append(len(sizes))
+            sizes.append(numel)
+            at = off + numel
+    parts = flat.split(sizes + [flat.numel() - at])
+    return iter([parts[i] for i in keep])
+
+
+def _degenerate_pairs(plan, eig, g, tol: float = 1e-8):
     """Adjacent bands at one k closer than ``tol`` Hartree whose loss weights differ.
 
     For such a pair the derivative of each eigenvalue separately is not
     defined; the projector form used here returns the derivative of the
     weighted sum over the degenerate subspace, which is exact only when the
-    weights agree.  The count is reported so callers can tell.
+    weights agree.  The count is reported so callers can tell: a function that
+    waits for it and returns it, so that what follows it on the stream need not wait.
     """
     if plan.eig_total < 2:
-        return 0
-    nb = np.repeat(plan.nb, plan.nk.astype(np.int64) * plan.nb)
-    pos = np.concatenate([np.arange(int(k) * int(b)) % int(b) for k, b in zip(plan.nk, plan.nb)])
-    valid = torch.as_tensor((pos[:-1] < nb[:-1] - 1), device=eig.device)
+        return lambda: 0
+    last = np.concatenate([np.cumsum(np.full(int(k), int(b))) for k, b in zip(plan.nk, plan.nb)])
+    last = last + np.repeat(plan.eig_off_struct, plan.nk) - 1            # the last band of every k-point
+    valid = np.ones(plan.eig_total, dtype=bool)
+    valid[last] = False
+    valid = torch.from_numpy(valid[:-1]).to(eig.device, non_blocking=True)
     de = (eig[1:plan.eig_total] - eig[:plan.eig_total - 1]).abs()
     dg = (g[1:plan.eig_total] - g[:plan.eig_total - 1]).abs()
-    gscale = float(g.abs().max()) if plan.eig_total else 0.0
-    flag = valid & (de < tol) & (dg > 1e-9 * max(gscale, 1e-300))
-    return int(flag.sum())
+    flag = valid & (de < tol) & (dg > 1e-9 * g.abs().max().clamp(min=1e-300))
+    host = torch.empty((), dtype=torch.int64, pin_memory=True)
+    host.copy_(flag.sum(), non_blocking=True)
+    done = torch.cuda.Event()
+    done.record()
+
+    def count():
+        done.synchronize()
+        return int(host)
+    return count
 
 
 def differentiable_properties(model, structures: Sequence[dict], shell_dict=None, device="cuda",

@@ -247,7 +247,7 @@ def tune_batch(engine, db, candidates: Optional[List[Tuning]] = None, reps: int 
                 a = torch.cuda.Event(enable_timing=True)
                 b = torch.cuda.Event(enable_timing=True)
                 a.record()
-                engine._eig_values(db, H, S, eig, st, ctr, torch.cuda.current_stream(dev).cuda_stream)
+                engine._eig_values(db, H, S, eig, st, torch.cuda.current_stream(dev).cuda_stream)
                 b.record()
                 torch.cuda.synchronize(dev)
                 trials.append(a.elapsed_time(b) * 1e-3)

@@ -54,6 +54,35 @@ def _f64(a, device):
     return torch.as_tensor(np.ascontiguousarray(a, dtype=np.float64)).to(device, non_blocking=True)
 
 
+_TORCH = {np.int32: (torch.int32, 4), np.int64: (torch.int64, 8), np.float64: (torch.float64, 8)}
+_ZEROS = bytes(256)
+
+
+def _to_device(arrays, device) -> list:
+    """[(array, np.int32 / np.int64 / np.float64)] on the device, flat, in one copy: views of one buffer, each on a
+    256-byte boundary as an allocation of its own would be.  A copy each took 290 us of a one-k-point cell's call for
+    its 30 descriptor arrays, and every one waited for those before it."""
+    chunks, sections, first = [], [], 0
+    for dtype, (tdtype, size) in _TORCH.items():          # by type: one view and one split each
+        idx, sizes, start = [], [], first
+        for i, (a, t) in enumerate(arrays):
+            if t is dtype:
+                raw = np.asarray(a, dtype).tobytes()
+                pad = -len(raw) % 256
+                chunks += (raw, _ZEROS[:pad])
+                sizes += (len(raw) // size, pad // size)
+                first += len(raw) + pad
+                idx.append(i)
+        sections.append((tdtype, idx, sizes, start, first))
+    buf = torch.frombuffer(bytearray().join(chunks), dtype=torch.uint8).to(device, non_blocking=True)
+    out = [None] * len(arrays)
+    for tdtype, idx, sizes, start, end in sections:
+        if idx:
+            for i, v in zip(idx, buf[start:end].view(tdtype).split(sizes)[::2]):
+                out[i] = v
+    return out
+
+
 # ------------------------------------------------------------------ tables
 
 class TableSet:
@@ -446,46 +475,28 @@ class DeviceBatch:
     """A planned batch with its descriptor arrays resident on the device."""
 
     def __init__(self, plan: Plan, device):
-        dev = device
         self.plan = plan
-        self.atom_ptr = _i32(plan.atom_ptr, dev)
-        self.pos = _f64(plan.positions, dev)
-        self.cells = _f64(plan.cells, dev)
-        self.rng = _i32(plan.image_range, dev)
-        self.pair_base = _i64(plan.pair_base, dev)
-        self.norb = _i32(plan.atom_norb, dev)
-        self.kptr = _i32(plan.k_ptr, dev)
-        self.kp = _f64(plan.kpoints, dev)
-        self.phb = _i64(plan.phase_base, dev)
-        self.species = _i32(plan.atom_species, dev)
-        self.ps = _i32(plan.prob_struct, dev)
-        self.pk = _i32(plan.prob_k, dev)
-        self.hs_off = _i64(plan.hs_off, dev)
-        self.orb_ptr = _i32(plan.orb_ptr, dev)
-        self.orb_atom = _i32(plan.orb_atom, dev)
-        self.aoff = _i32(plan.atom_orb_off, dev)
-        self.onsite = _f64(plan.onsite_H, dev)
-        self.n = _i32(plan.prob_n, dev)
-        self.eoff = _i64(plan.eig_off_prob, dev)
-        self.order = _i32(plan.order, dev)
-        self.eos = _i64(plan.eig_off_struct, dev)
-        self.nk = _i32(plan.nk, dev)
-        self.nb = _i32(plan.nb, dev)
-        self.kwoff = _i64(plan.kw_off, dev)
-        self.kw = _f64(plan.kweights, dev)
-        self.ne = _f64(plan.nelec, dev)
-        self.real = _i32(plan.prob_real if plan.prob_real is not None else np.zeros(len(plan.prob_n)), dev)
         # work units of the Bloch-sum kernel per structure: ceil(nk_s / BLOCH_KCHUNK) k-chunks times the
         # N_s^2 ordered atom pairs (full matrices) or the N_s (N_s + 1) / 2 pairs on or below the diagonal
         # (lower triangles), numbered from an exclusive prefix sum
         na = np.diff(plan.atom_ptr).astype(np.int64)
         kch = (plan.nk.astype(np.int64) + BLOCH_KCHUNK - 1) // BLOCH_KCHUNK
-
-        def base(units):
-            return _i64(np.concatenate([[0], np.cumsum(units)[:-1]]) if len(units) else np.zeros(1), dev), \
-                int(units.sum())
-        self.bloch_unit_base, self.bloch_units = base(na * na * kch)
-        self.bloch_unit_base_lower, self.bloch_units_lower = base(na * (na + 1) // 2 * kch)
+        full, lower = na * na * kch, na * (na + 1) // 2 * kch
+        self.bloch_units, self.bloch_units_lower = int(full.sum()), int(lower.sum())
+        i32, i64, f64 = np.int32, np.int64, np.float64
+        arrays = dict(
+            atom_ptr=(plan.atom_ptr, i32), pos=(plan.positions, f64), cells=(plan.cells, f64),
+            rng=(plan.image_range, i32), pair_base=(plan.pair_base, i64), norb=(plan.atom_norb, i32),
+            kptr=(plan.k_ptr, i32), kp=(plan.kpoints, f64), phb=(plan.phase_base, i64),
+            species=(plan.atom_species, i32), ps=(plan.prob_struct, i32), pk=(plan.prob_k, i32),
+            hs_off=(plan.hs_off, i64), orb_ptr=(plan.orb_ptr, i32), orb_atom=(plan.orb_atom, i32),
+            aoff=(plan.atom_orb_off, i32), onsite=(plan.onsite_H, f64), n=(plan.prob_n, i32),
+            eoff=(plan.eig_off_prob, i64), order=(plan.order, i32), eos=(plan.eig_off_struct, i64),
+            nk=(plan.nk, i32), nb=(plan.nb, i32), kwoff=(plan.kw_off, i64), kw=(plan.kweights, f64),
+            ne=(plan.nelec, f64),
+            real=(plan.prob_real if plan.prob_real is not None else np.zeros(len(plan.prob_n)), i32),
+            bloch_unit_base=(np.cumsum(full) - full, i64), bloch_unit_base_lower=(np.cumsum(lower) - lower, i64))
+        self.__dict__.update(zip(arrays, _to_device(list(arrays.values()), device)))
 
     def h2d_bytes(self) -> int:
         return sum(int(v.numel() * v.element_size()) for v in vars(self).values() if isinstance(v, torch.Tensor))
@@ -721,8 +732,7 @@ class Engine:
             d_pair_blk = _i64(pair_blk[:-1] if plan.n_pairs else np.zeros(1), dev)
             d_pair_ptr = b["pair_ptr"]
         else:
-            d_pair_ptr = _i64(pair_ptr, dev)
-            d_pair_blk = _i64(pair_blk[:-1] if plan.n_pairs else np.zeros(1), dev)
+            d_pair_ptr, d_pair_blk = _i64(np.stack([pair_ptr, pair_blk]), dev)
             nb1 = max(nbond, 1)
             b = dict(nbond=nbond, nblk=nblk, pair_ptr=d_pair_ptr,
                      bond_i=torch.empty(nb1, dtype=torch.int32, device=dev),
@@ -779,7 +789,6 @@ class Engine:
             return BatchResult(plan, None, None, None, None, None, None, None, hs_copy[0], hs_copy[1])
         eig = torch.empty(max(plan.eig_total, 1), dtype=torch.float64, device=dev)
         eig_status = torch.empty(max(n_prob, 1), dtype=torch.int32, device=dev)
-        counter = torch.zeros(2, dtype=torch.int32, device=dev)
         vec = tri = None
         if vectors:
             if plan.max_n > PANELS_MAX_N:
@@ -792,7 +801,7 @@ class Engine:
             b = torch.cuda.Event(enable_timing=True)
             a.record()
             self.event_log = None        # the phase is timed as a whole (groups run on forked streams)
-        self._eig_values(db, Hk, Sk, eig, eig_status, counter, stream, tri, vec)
+        self._eig_values(db, Hk, Sk, eig, eig_status, stream, tri, vec)
         if ev is not None:
             b.record()
             self.event_log = ev
@@ -818,14 +827,15 @@ class Engine:
                                        float(dos_window)))
         return out
 
-    def _eig_values(self, db, Hk, Sk, eig, eig_status, counter, stream, tri=None, vec=None):
+    def _eig_values(self, db, Hk, Sk, eig, eig_status, stream, tri=None, vec=None):
         """Eigenvalues, and the eigenvectors into ``vec`` where it is given (``tri``: 4 doubles per eigenvalue)."""
         plan = db.plan
         n_prob = len(plan.prob_n)
         groups = self._groups(db, vec is not None)
+        counters = torch.empty(2 * max(len(groups), 1), dtype=torch.int32, device=self.device)     # each call zeroes its own
         if not groups:
             self._call("skn_eigh_gen_batched", n_prob, ptr(db.n), ptr(db.hs_off), ptr(db.eoff), ptr(db.order),
-                       ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counter), plan.max_n, stream)
+                       ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counters), plan.max_n, stream)
             return
         scratch = {}
         for gi, (shape, _, count, max_n) in enumerate(groups):
@@ -847,8 +857,7 @@ class Engine:
                 call("skn_eigvec_scratch_bytes", 1, max_n, ctypes.addressof(one))
                 nbytes = min(need.value, max(VEC_SCRATCH, one.value))
                 vec_scratch.append(torch.empty(nbytes // 8, dtype=torch.float64, device=self.device))
-        counters = torch.zeros(2 * len(groups), dtype=torch.int32, device=self.device)
-        share = self._sm_shares(db, groups)
+        share = self._sm_shares(db, groups) if db._panel_parts else None
 
         def launch(gi, sfx, order_g, count, max_n, st):
             if isinstance(sfx, tuple) and sfx[0] == "small":
@@ -967,13 +976,20 @@ class Engine:
         real = plan.prob_real if (self.real_path and plan.prob_real is not None) else np.zeros(len(plan.prob_n), bool)
         out = [out[i] for i in launch_order([g[1] for g in out], plan.prob_n, real)]
         db._group_problems = [g[1] for g in out]
-        db._panel_parts = {}
+        parts = {}
         for gi, (sh, sel, _, _) in enumerate(out):
             if isinstance(sh, tuple) and sh[0] == "panels":
                 sizes = np.ascontiguousarray(plan.prob_n[sel].astype(np.int32))
-                db._panel_parts[gi] = [(a, b, _i64(w, self.device), nbytes, sizes[a:b])
-                                       for a, b, w, nbytes in panels_parts(sizes, PANELS_SCRATCH)]
-        out = [(sh, _i32(sel, self.device), cnt, mx) for sh, sel, cnt, mx in out]     # problem lists on the device
+                parts[gi] = [(a, b, w, nbytes, sizes[a:b]) for a, b, w, nbytes in panels_parts(sizes, PANELS_SCRATCH)]
+        if out:                              # problem lists and scratch offsets to the device
+            lists = [(sel, np.int32) for _, sel, _, _ in out] + [(p[2], np.int64) for g in parts.values() for p in g]
+            if len(lists) == 1 and len(lists[0][0]) == len(plan.order):      # the batch's own order
+                lists = iter([db.order])
+            else:
+                lists = iter(_to_device(lists, self.device))
+            out = [(sh, next(lists), cnt, mx) for sh, _, cnt, mx in out]
+            parts = {gi: [(a, b, next(lists), nbytes, sizes) for a, b, _, nbytes, sizes in g] for gi, g in parts.items()}
+        db._panel_parts = parts
         db._groups = (key, out)
         return out
 

@@ -552,12 +552,13 @@ def _default_shell_dict():
 def properties_dict(res: "E.BatchResult", s: int, get_fermi: bool = False) -> dict:
     """The reference's properties dict for structure ``s`` of a batch result."""
     plan = res.plan
-    st = res.stats[s].detach().cpu().numpy()
+    st = res.stats[s].detach().cpu().tolist()
     I = E.STAT
-    dev = res.eig.device
     eig = res.eigenvalues(s).unsqueeze(0)
     metal_or_fallback = st[I["metal"]] > 0 or st[I["fallback"]] > 0
-    gap_t = torch.tensor(float(st[I["gap_ev"]]), dtype=torch.float64, device="cpu" if metal_or_fallback else dev)
+    # on the device by a copy there: a tensor made from the host's value waits for its transfer
+    gap_t = torch.tensor(st[I["gap_ev"]], dtype=torch.float64) if metal_or_fallback \
+        else res.stats[s, I["gap_ev"]].clone()
     mdg = st[I["min_dgap"]]
     dos = res.dos[s]
     props = {
