@@ -8,18 +8,25 @@
 //      row of B = L^-1 H; one update S22 -= L21 L21^H and H_below -= L21 B_panel on the tensor cores;
 //   3. per panel: the column block of C = B L^-H by row solves; one update of the trailing lower triangle
 //      C22 -= C_panel L21^H on the tensor cores;
-//   4. per 16 columns: Householder reflectors and the W vectors of LAPACK's zlatrd (k_tri_panel, one cluster
-//      of CTAs per problem), then A22 -= V W^H + W V^H on the tensor cores;
+//   4. per 16 columns: the trailing tiles in 56-bit fixed point (k_fixed), Householder reflectors and the W vectors of
+//      LAPACK's zlatrd (k_tri_panel, a team of CTAs per problem), then A22 -= V W^H + W V^H on the tensor cores;
 //   5. eigenvalues of the tridiagonal (sturm.cuh).
 // The reference calls torch.linalg.cholesky / solve / eigh per k (slakonet/utils.py:749-783,
 // slakonet/main.py:174).
 //
-// GB300 notes.  An SM does two FP64 multiply-adds per clock, so FP64 issue bounds everything that stays on it;
-// of the 32/3 n^3 flops only the matrix-vector products (8/3 n^3) do.  The updates are exact products of
-// integer slices (below) rounded once per panel.  Every sum that crosses warps or CTAs goes to its own slot
-// and is added in a fixed order, so a problem's results depend neither on the other problems nor on the
-// number of CTAs it is given.
+// GB300 notes.  An SM does two FP64 multiply-adds per clock, so what stays on that unit bounds everything.  The updates
+// are exact products of integer slices on the tensor cores, rounded once per panel; the matrix-vector products of the
+// tridiagonalisation are exact products of 28-bit limbs on the integer units, rounded once per tile; FP64 keeps the
+// reflectors, the O(n) work of a column and the diagonal blocks.  Every sum that crosses warps or CTAs goes to its own
+// slot and is added in a fixed order, or is an integer, so a problem's results depend neither on the other problems nor
+// on the number of CTAs it is given.
+// Measured (random pencils): 492 orbitals x 300 problems 393 ms with one CTA per problem, 208 with the products in FP64,
+// 130 now (tridiagonalisation 63, updates 40, solves 16, eigenvalues 6); 432 x 8 190, 18.8, 11.6 ms (6.4 of them the
+// tridiagonalisation, 15 us a column); 1152 x 2 47, 35.8 ms.
 #include <algorithm>
+#include <map>
+#include <mutex>
+#include <utility>
 
 #include <cooperative_groups.h>
 #include <cuda_bf16.h>
@@ -89,7 +96,7 @@ SKN_DEVINL double2 zero2() { return make_double2(0.0, 0.0); }
 
 // ------------------------------------------------------------------ scratch (per problem slot)
 struct Lay {
-  int64_t W, VW, xc, Yp, sN, sT, sD, li, d, e2, d32, e232, bnd, flg, bar, sa, sb, sc, ea, eb, ec, stride;   // bytes
+  int64_t W, VW, xc, Yp, sN, sT, sD, li, d, e2, d32, e232, bnd, flg, bar, sa, sb, sc, ea, eb, ec, fx, fe, vf, ve, stride;   // bytes
 };
 __host__ __device__ inline int64_t take(int64_t& o, int64_t bytes) {
   const int64_t r = o;
@@ -108,7 +115,7 @@ __host__ __device__ inline Lay layout(int n) {
   L.Yp = take(o, 16 * nt * n);                 // matrix-vector partial sums: slot s at Yp + s n
   L.sN = take(o, 8 * nt);                      // column norm, per 32-row chunk
   L.sT = take(o, 8 * nt * (nt + 1) / 2);       // v^H A v, per tile
-  L.sD = take(o, 16 * nt * 4 * 2 * NT);        // [W V]^H v, per 8 rows
+  L.sD = take(o, 16 * nt * 2 * NT);            // [W V]^H v, per 32-row chunk
   L.li = take(o, 16 * (int64_t)NB * NB * ((n + NB - 1) / NB));   // inverses of the diagonal blocks, row-major
   L.d = take(o, 8 * (int64_t)n);
   L.e2 = take(o, 8 * (int64_t)n);
@@ -123,6 +130,10 @@ __host__ __device__ inline Lay layout(int n) {
   L.ea = take(o, 4 * nr);                      // row exponents of sa, sb, sc
   L.eb = take(o, 4 * nr);
   L.ec = take(o, 4 * nr);
+  L.fx = take(o, 16 * (int64_t)TS * TS * (nt * (nt + 1) / 2));   // the trailing block's tiles in 56-bit fixed point
+  L.fe = take(o, 4 * (nt * (nt + 1) / 2));                       // their exponents
+  L.vf = take(o, 16 * (int64_t)TS * 2 * NT * nt);                // chunks of [W V] in fixed point, column by column
+  L.ve = take(o, 4 * (int64_t)2 * NT * nt);                      // the exponent of each of their columns
   L.stride = o;
   return L;
 }
@@ -151,6 +162,8 @@ struct WS {
   int *flg, *ea, *eb, *ec;
   unsigned* bar;
   uint16_t *sa, *sb, *sc;
+  int4 *fx, *vf;
+  int *fe, *ve;
   int64_t nr;                // rows of a slice array
 };
 SKN_DEVINL WS ws_of(const Grp& G, int g) {
@@ -165,6 +178,8 @@ SKN_DEVINL WS ws_of(const Grp& G, int g) {
   w.bar = (unsigned*)(b + L.bar);
   w.ea = (int*)(b + L.ea); w.eb = (int*)(b + L.eb); w.ec = (int*)(b + L.ec);
   w.sa = (uint16_t*)(b + L.sa); w.sb = (uint16_t*)(b + L.sb); w.sc = (uint16_t*)(b + L.sc);
+  w.fx = (int4*)(b + L.fx); w.fe = (int*)(b + L.fe);
+  w.vf = (int4*)(b + L.vf); w.ve = (int*)(b + L.ve);
   w.nr = slice_rows(n);
   return w;
 }
@@ -838,15 +853,18 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
 // Then w = tau (y - V (W^H v) - W (V^H v)) + alpha v with alpha = -|tau|^2 / 2 (v^H A22 v - 2 Re (W^H v)^H (V^H v)),
 // which needs no further reduction, and the next column's update runs on the same rows in the same pass.
 // Every CTA computes W's entry of the next pivot row itself, with the same operations.
-// A tile is read once for both products: lane = row on the way in (A v), lane = column from shared memory (A^H v).
-// The FP64 unit belongs to one of the SM's four partitions: a warp issues one FP64 instruction per 64 clocks,
-// however independent its instructions are, so a phase is as long as its busiest warp.
-// RES: a CTA's tiles and its rows of [W V] fit its shared memory and stay there for the panel's 16 columns, and
-// its four warps share every tile (8 columns each), chunk and sum: the form for few problems.  Else a warp takes
-// whole tiles, streamed, and the CTAs of other problems fill the partitions: the form for many.  Both add in the
-// same order (quarters of a tile or chunk, then (0 + 1) + (2 + 3)), so the results are the same bits.
-constexpr int PW = 4;                            // warps per CTA, one per partition
-constexpr int PT = 32 * PW;
+// A tile is read once for both products: lane = row (A v), then lane = column (A^H v); both, and the products with [W V],
+// in fixed point (below).  The FP64 unit belongs to one of the SM's four partitions: a warp issues one FP64 instruction
+// per 64 clocks, however independent its instructions are, so the FP64 work of a phase is spread over the warps.
+// RES: a CTA's tiles and its rows of [W V] fit its shared memory and stay there for the panel's 16 columns; eight warps
+// take a tile each.  The form for few problems, bound by the latency of a column: 29,700 clocks at 432 orbitals on
+// clusters of 12, 5,500 of them the products (20,000 in FP64), the rest two barriers, the reflector, the sums and the
+// row's update.  Else a warp takes whole tiles, streamed, and the CTAs of other problems fill the partitions: the form for
+// many, bound by the integer multiply-adds (4 to 5 clocks each and partition) and what FP64 is left.  Integer sums do not
+// depend on their order and FP64 sums keep theirs, so both forms give the same bits.
+constexpr int PW = 4;                            // warps per CTA when streamed, one per partition
+constexpr int PWR = 8;                           // and when resident: two per partition hide each other's latency
+constexpr int PT = 32 * PW, PTR = 32 * PWR;
 constexpr int TILE_LD = TS + 1;
 constexpr int TILE_EL = TS * TILE_LD;            // a resident tile, or a chunk's 32 columns of [W V]
 constexpr int QT = TS / PW;                      // columns or rows of a quarter; columns staged when streamed
@@ -854,7 +872,7 @@ constexpr int VMAX = 8;                          // column entries a thread fetc
 struct PanelSm {
   double2 rowV[NT], rowW[NT];                    // V and W at the next pivot row
   double2 part[PW][2 * NT];                      // [W V]^H v by quarters of the chunks
-  double2 t12[PW][2 * NT];                       // W^H v, V^H v: a copy per warp
+  int4 tf[PW][2 * NT], qf[PW][2 * NT];           // multipliers of [W V]'s columns for a warp's chunk
   double2 tau, scl, yrow, wrow;
   double vav, alpha;
   int triv, dead;
@@ -867,8 +885,156 @@ SKN_DEVINL void tile_ij(int t, int& I, int& J) {     // lower-triangle tile inde
   I = i;
   J = t - i * (i + 1) / 2;
 }
+constexpr int EPS = TS * PW * (16 + 64);         // a chunk's partial sums: four of y's slots, four of the two integer sums
 template <bool R> SKN_DEVINL double2 sum4(double2 a, double2 b, double2 c, double2 d) {
   return add<R>(add<R>(a, b), add<R>(c, d));
+}
+
+// ------------------------------------------------------------------ fixed-point products
+// A tile and a chunk of v are held as integers of 56 bits under one exponent, each in two limbs of 28 (balanced, so the
+// low one has a sign).  Of a product's four partial products the lowest, 2^-58 of the largest, is left out; the others are
+// exact in 64-bit accumulators over the 32 terms of a tile, and a tile's sum is rounded once.  The error per term is that
+// of the operands' last bit, 2^-57 of the largest, against 2^-53 of each product for FP64: it stays below FP64's own as
+// long as the entries of a tile are within 2^4 of each other, and relative to the matrix's norm always.
+// A partition issues a multiply-add of two 32-bit integers into 64 bits every 4.8 clocks and an FP64 instruction every 64:
+// three of the one replace one of the other.
+struct alignas(8) Limb { int h, l; };
+SKN_DEVINL Limb limbs(long long f) {
+  const long long h = (f + (1LL << 27)) >> 28;
+  return {(int)h, (int)(f - (h << 28))};
+}
+template <bool R> SKN_DEVINL int4 fixed_point(double2 a, int emax) {
+  const Limb x = limbs(fixed56(a.x, emax));
+  if constexpr (R) return make_int4(x.h, x.l, 0, 0);
+  const Limb y = limbs(fixed56(a.y, emax));
+  return make_int4(x.h, x.l, y.h, y.l);
+}
+template <bool R> SKN_DEVINL int high_word(double2 a) {         // orders magnitudes; its upper bits are the exponent
+  const int x = __double2hiint(a.x) & 0x7fffffff;
+  if constexpr (R) return x;
+  return max(x, __double2hiint(a.y) & 0x7fffffff);
+}
+constexpr int EXP_BAD = 1 << 20;                                // an infinity or a NaN among the operands
+SKN_DEVINL int exp_sum(int a, int b) { return a == 0x7ff || b == 0x7ff ? EXP_BAD : a + b; }
+SKN_DEVINL long long wide(int a, int b, long long c) { return c + (long long)a * b; }
+// sums of a v (or conj(a) v): real and imaginary parts, high (2^56) and middle (2^28) weights
+template <bool R> struct Dot {
+  long long rh = 0, rm = 0, ih = 0, im = 0, qh = 0, qm = 0;
+  SKN_DEVINL void add(int4 a, int4 v) {                         // a v
+    rh = wide(a.x, v.x, rh);
+    rm = wide(a.x, v.y, wide(a.y, v.x, rm));
+    if constexpr (!R) {
+      qh = wide(a.z, v.z, qh);
+      qm = wide(a.z, v.w, wide(a.w, v.z, qm));
+      ih = wide(a.x, v.z, wide(a.z, v.x, ih));
+      im = wide(a.x, v.w, wide(a.y, v.z, wide(a.z, v.y, wide(a.w, v.x, im))));
+    }
+  }
+  SKN_DEVINL void add_conj(int4 a, int4 v) {                    // conj(a) v
+    rh = wide(a.x, v.x, rh);
+    rm = wide(a.x, v.y, wide(a.y, v.x, rm));
+    if constexpr (!R) {
+      rh = wide(a.z, v.z, rh);
+      rm = wide(a.z, v.w, wide(a.w, v.z, rm));
+      ih = wide(a.x, v.z, ih);
+      im = wide(a.x, v.w, wide(a.y, v.z, im));
+      qh = wide(a.z, v.x, qh);
+      qm = wide(a.z, v.y, wide(a.w, v.x, qm));
+    }
+  }
+  SKN_DEVINL void close(bool conj) {                            // then (rh, rm) + i (ih, im)
+    if constexpr (!R) {
+      if (conj) { ih -= qh; im -= qm; } else { rh -= qh; rm -= qm; }
+    }
+  }
+  SKN_DEVINL void sum_lanes(int o) {
+    rh += __shfl_xor_sync(0xffffffffu, rh, o);
+    rm += __shfl_xor_sync(0xffffffffu, rm, o);
+    if constexpr (!R) {
+      ih += __shfl_xor_sync(0xffffffffu, ih, o);
+      im += __shfl_xor_sync(0xffffffffu, im, o);
+    }
+  }
+  SKN_DEVINL void put(long long* p, int stride) const {
+    p[0] = rh;
+    p[stride] = rm;
+    if constexpr (!R) {
+      p[2 * stride] = ih;
+      p[3 * stride] = im;
+    }
+  }
+  SKN_DEVINL void take(const long long* p, int stride) {
+    rh += p[0];
+    rm += p[stride];
+    if constexpr (!R) {
+      ih += p[2 * stride];
+      im += p[3 * stride];
+    }
+  }
+  // the rounded sum; ke: the sum of the operands' exponent fields
+  SKN_DEVINL double2 value(int ke) const {
+    if (ke == EXP_BAD) {
+      const double q = __longlong_as_double(0x7ff8000000000000LL);
+      return make_double2(q, R ? 0.0 : q);
+    }
+    const int k = ke - 2 * (1022 + 56);
+    return make_double2(round_wide28(rh, rm, k + 28), R ? 0.0 : round_wide28(ih, im, k + 28));
+  }
+};
+
+// entry (i, j) of the Hermitian block of M rows at A, from its lower triangle
+template <bool R> SKN_DEVINL double2 trailing_entry(const double2* A, int n, int M, int i, int j) {
+  if (i >= M || j >= M) return zero2();
+  double2 a = ld<R>(i >= j ? A + i + (int64_t)j * n : A + j + (int64_t)i * n);
+  if constexpr (!R) a.y = i == j ? 0.0 : cond_flip(a.y, i < j);
+  return a;
+}
+
+// The tiles of the trailing block at c0 in fixed point, for the 16 columns of a panel: a CTA per tile, a warp per 8
+// columns.  Bound by its reads and writes, 32 bytes an entry.
+template <bool R>
+SKN_DEVINL void fixed_body(const Grp& G, int g, int p, int c0, int* red) {
+  const int n = G.nvec[p], M = n - c0, nt = cdiv_d(M, TS), t = blockIdx.x;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (t >= nt * (nt + 1) / 2) return;
+  int I, J;
+  tile_ij(t, I, J);
+  const WS ws = ws_of(G, g);
+  const double2* A = G.H + G.hs_off[p] + c0 + (int64_t)c0 * n;
+  double2 a[QT];
+  int hm = 0;
+#pragma unroll
+  for (int u = 0; u < QT; ++u) {
+    a[u] = trailing_entry<R>(A, n, M, I * TS + lane, J * TS + warp * QT + u);
+    hm = max(hm, high_word<R>(a[u]));
+  }
+  hm = __reduce_max_sync(0xffffffffu, hm);
+  if (lane == 0) red[warp] = hm;
+  __syncthreads();
+  const int emax = max(max(red[0], red[1]), max(red[2], red[3])) >> 20;
+  if (threadIdx.x == 0) ws.fe[t] = emax;
+  int4* T = ws.fx + (int64_t)t * TS * TS + warp * QT * TS + lane;
+#pragma unroll
+  for (int u = 0; u < QT; ++u) {
+    const int4 f = fixed_point<R>(a[u], emax);
+    if constexpr (R) reinterpret_cast<int2*>(T + u * TS)[0] = make_int2(f.x, f.y);
+    else T[u * TS] = f;
+  }
+}
+__global__ void __launch_bounds__(PT) k_fixed(Grp G, int c0) {
+  __shared__ int red[PW];
+  const int g = blockIdx.y, p = G.prob[g];
+  if (!live(G, p) || c0 >= G.nvec[p] - 1) return;
+  if (is_real(G, p)) fixed_body<true>(G, g, p, c0, red);
+  else fixed_body<false>(G, g, p, c0, red);
+}
+template <bool R> SKN_DEVINL int4 ld_fixed(const int4* p) {
+  if constexpr (R) {
+    const int2 v = *reinterpret_cast<const int2*>(p);
+    return make_int4(v.x, v.y, 0, 0);
+  } else {
+    return *p;
+  }
 }
 
 // The CTAs of one problem: a cluster, or (more than 16) CTAs of a cooperative launch that meet at a counter.  A
@@ -909,11 +1075,12 @@ struct Team {
   }
 };
 
-// sv: the Householder vector; big: streamed, a quarter of a tile per warp; RES, tiles (rt), chunks of [W V] (cpc), partial
-// sums of tiles (rt x PW x 32) and of chunks (2 x cpc x PW x 32).
+// sv: the Householder vector, svf: the same in fixed point, sve: its exponents by 32 rows; big: streamed, a quarter of a
+// tile per warp; RES, tiles (rt), chunks of [W V] (cpc) and their partial sums (2 x cpc x PW x 32).
 template <bool R, bool RES>
 SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int rt, int cpc, PanelSm& sm, double2* sv,
-                           double2* big) {
+                           int4* svf, int* sve, double2* big) {
+  constexpr int NWP = RES ? PWR : PW, NTH = 32 * NWP;
   const int rank = team.rank, C = team.C;
   const int n = G.nvec[p], M = n - c0, w = min(NT, n - 1 - c0);
   const int nt = cdiv_d(M, TS), ntile = nt * (nt + 1) / 2;
@@ -922,30 +1089,35 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
   double2* W = ws.W;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   double* tri = G.tri ? G.tri + 4 * G.eig_off[p] : nullptr;
-  double2* wvs = big + (int64_t)rt * TILE_EL;      // chunk lc, column q, row r at lc TILE_EL + q TILE_LD + r
-  double2* yps = wvs + (int64_t)cpc * TILE_EL;     // tile i, quarter q, row r at (i PW + q) TS + r
-  double2* eps = yps + (int64_t)rt * PW * TS;      // chunk lc, quarter q, (y, a), row r at ((lc PW + q) 2 + part) TS + r
+  int4* wvs = reinterpret_cast<int4*>(big + (int64_t)rt * TILE_EL);      // chunk lc, column q, row r at lc TILE_EL + q TILE_LD + r
+  char* eps = reinterpret_cast<char*>(wvs + (int64_t)cpc * TILE_EL);     // chunk lc at lc EPS: y by quarters, then the integer sums
+  int* wve = reinterpret_cast<int*>(eps + (int64_t)cpc * EPS);      // chunk lc: 32 exponents, then the sums' two
   auto sync = [&]() { team.sync(); };
-  // entry (i, j) of the Hermitian trailing block, from its lower triangle
-  auto entry = [&](int i, int j) {
-    if (i >= M || j >= M) return zero2();
-    double2 a = ld<R>(i >= j ? A + i + (int64_t)j * n : A + j + (int64_t)i * n);
-    if constexpr (!R) a.y = i == j ? 0.0 : cond_flip(a.y, i < j);
-    return a;
+  // column q of chunk ch of [W V] in fixed point, lane = row
+  auto put_fixed = [&](int ch, int q, int4 f, int emax) {
+    if constexpr (RES) {
+      wvs[(ch / C) * TILE_EL + q * TILE_LD + lane] = f;
+      if (lane == 0) wve[(ch / C) * (2 * NT + 2) + q] = emax;
+    } else {
+      int4* d = ws.vf + ((int64_t)ch * 2 * NT + q) * TS + lane;
+      if constexpr (R) *reinterpret_cast<int2*>(d) = make_int2(f.x, f.y);
+      else *d = f;
+      if (lane == 0) ws.ve[ch * 2 * NT + q] = emax;
+    }
   };
+  auto fixed_exp = [&](int ch, int q) { return RES ? wve[(ch / C) * (2 * NT + 2) + q] : ws.ve[ch * 2 * NT + q]; };
   // chunks and tiles of this CTA are rank, rank + C, ...; streamed, a warp takes every PW-th of them
-  const int first = RES ? rank : rank + C * warp, stride = RES ? C : C * PW;
+  const int first = rank + C * warp, stride = C * NWP;
   if constexpr (RES) {
     for (int t = rank, i = 0; t < ntile; t += C, ++i) {
-      int I, J;
-      tile_ij(t, I, J);
-      double2* T = big + (int64_t)i * TILE_EL;
+      int4* T = reinterpret_cast<int4*>(big) + (int64_t)i * TILE_EL;
+      const int4* src = ws.fx + (int64_t)t * TS * TS;
 #pragma unroll
-      for (int u = 0; u < QT; ++u) T[(warp * QT + u) * TILE_LD + lane] = entry(I * TS + lane, J * TS + warp * QT + u);
+      for (int c = warp; c < TS; c += NWP) T[c * TILE_LD + lane] = ld_fixed<R>(src + c * TS + lane);
     }
   }
   // first column as it stands
-  for (int ch = rank + C * warp; ch < nt; ch += C * PW) {
+  for (int ch = first; ch < nt; ch += stride) {
     const int r = ch * 32 + lane;
     double2 a = zero2();
     if (r < M) {
@@ -965,8 +1137,8 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
     double2 xv[VMAX];
 #pragma unroll
     for (int u = 0; u < VMAX; ++u) {
-      const int r = tid + u * PT;
-      if (u * PT < nt * 32) xv[u] = (r > j + 1 && r < M) ? ldc<R>(ws.xc + r) : zero2();
+      const int r = tid + u * NTH;
+      if (u * NTH < nt * 32) xv[u] = (r > j + 1 && r < M) ? ldc<R>(ws.xc + r) : zero2();
     }
     if (warp < 2) {
       const double2 al = ldc<R>(ws.xc + j + 1);
@@ -1006,26 +1178,34 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
     auto put_v = [&](int r, double2 v) {
       if (r > j && r < M && (r >> 5) % C == rank) {
         st<R>(A + r + (int64_t)j * n, v);
-        if constexpr (RES) wvs[((r >> 5) / C) * TILE_EL + (NT + j) * TILE_LD + (r & 31)] = v;
         st<R>(ws.VW + (int64_t)r * 2 * NT + NT + j, v);
       }
     };
+    auto fix_v = [&](int r, double2 v) {                     // a warp's rows are a chunk
+      const int emax = __reduce_max_sync(0xffffffffu, high_word<R>(v)) >> 20;
+      const int4 f = fixed_point<R>(v, emax);
+      svf[r] = f;
+      if (lane == 0) sve[r >> 5] = emax;
+      if ((r >> 5) % C == rank) put_fixed(r >> 5, NT + j, f, emax);
+    };
 #pragma unroll
     for (int u = 0; u < VMAX; ++u) {
-      const int r = tid + u * PT;
-      if (u * PT < nt * 32 && r < nt * 32) {
+      const int r = tid + u * NTH;
+      if (u * NTH < nt * 32 && r < nt * 32) {
         double2 v = xv[u];
         if (r == j + 1) v = make_double2(1.0, 0.0);
         else if (!triv) v = mul<R>(v, scl);
         sv[r] = v;
         put_v(r, v);
+        fix_v(r, v);
       }
     }
-    for (int r = tid + VMAX * PT; r < nt * 32; r += PT) {
+    for (int r = tid + VMAX * NTH; r < nt * 32; r += NTH) {
       double2 v = r < M ? ldc<R>(ws.xc + r) : zero2();      // r > j + 1: past the entries above
       if (!triv) v = mul<R>(v, scl);
       sv[r] = v;
       put_v(r, v);
+      fix_v(r, v);
     }
     __syncthreads();
     // ---- products with v
@@ -1041,112 +1221,104 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
     };
     if (!triv) {
       if constexpr (RES) {
-        const int qc = lane & (QT - 1), qr = lane / QT;        // this lane's column and rows of the transposed quarter
-#pragma unroll 2
-        for (int t = rank, i = 0; t < ntile; t += C, ++i) {
+        for (int t = first, i = warp; t < ntile; t += stride, i += NWP) {
           int I, J;
           tile_ij(t, I, J);
-          const bool diag = I == J;
-          const double2* T = big + (int64_t)i * TILE_EL;
-          const double2 *vI = sv + I * TS, *vJ = sv + J * TS + warp * QT;
-          double2 y = zero2();
-          const double2* Tq = T + warp * QT * TILE_LD;
-          if (diag) {
-#pragma unroll
-            for (int u = 0; u < QT; ++u) y = fma_<R>(Tq[u * TILE_LD + lane], vJ[u], y);
-          } else {
-            double2 z = zero2();
-            const double2* Tc = Tq + qc * TILE_LD;
-            const int cc = warp * QT + qc;
-#pragma unroll
-            for (int u = 0; u < QT; ++u) {
-              y = fma_<R>(Tq[u * TILE_LD + lane], vJ[u], y);
-              z = fma_cja<R>(Tc[qr * QT + u], vI[qr * QT + u], z);
-            }
-            z.x += __shfl_xor_sync(0xffffffffu, z.x, QT);
-            z.x += __shfl_xor_sync(0xffffffffu, z.x, 2 * QT);
-            if constexpr (!R) {
-              z.y += __shfl_xor_sync(0xffffffffu, z.y, QT);
-              z.y += __shfl_xor_sync(0xffffffffu, z.y, 2 * QT);
-            }
-            if (lane < QT && J * TS + cc < M) st<R>(ws.Yp + (int64_t)I * n + J * TS + cc, z);
+          const int4* T = reinterpret_cast<const int4*>(big) + (int64_t)i * TILE_EL;
+          const int4 *vI = svf + I * TS, *vJ = svf + J * TS;
+          const int ea = ws.fe[t];
+          Dot<R> y;
+#pragma unroll 8
+          for (int c = 0; c < TS; ++c) y.add(T[c * TILE_LD + lane], vJ[c]);
+          y.close(false);
+          if (I != J) {
+            Dot<R> z;
+#pragma unroll 8
+            for (int r = 0; r < TS; ++r) z.add_conj(T[lane * TILE_LD + r], vI[r]);
+            z.close(true);
+            st<R>(ws.Yp + (int64_t)I * n + J * TS + lane, z.value(exp_sum(ea, sve[I])));      // J TS + 31 < I TS < M
           }
-          yps[(i * PW + warp) * TS + lane] = y;
+          put_tile(t, I, J, y.value(exp_sum(ea, sve[J])));
         }
       } else {
-        double2* T = big + (int64_t)warp * QT * TILE_LD;
+        int4* T = reinterpret_cast<int4*>(big) + (int64_t)warp * QT * TILE_LD;
         const int qc = lane & (QT - 1), qr = lane / QT;
         for (int t = first; t < ntile; t += stride) {
           int I, J;
           tile_ij(t, I, J);
-          const int gi = I * TS + lane;
           const bool diag = I == J;
-          const double2 *vI = sv + I * TS + qr * QT, *vJ = sv + J * TS;
-          const double2* col = A + gi + (int64_t)(J * TS) * n;
-          double2 y01 = zero2(), y2 = zero2(), y = zero2(), z = zero2();
+          const int4 *vI = svf + I * TS + qr * QT, *vJ = svf + J * TS;
+          const int4* src = ws.fx + (int64_t)t * TS * TS + lane;
+          const int ea = ws.fe[t];
+          Dot<R> y, z;
 #pragma unroll
           for (int q = 0; q < PW; ++q) {
-            double2 a[QT];
+            int4 a[QT];
 #pragma unroll
-            for (int u = 0; u < QT; ++u) {
-              const int gj = J * TS + q * QT + u;
-              if (diag) a[u] = entry(gi, gj);
-              else a[u] = gi < M ? ld<R>(col + (int64_t)(q * QT + u) * n) : zero2();   // gj < I TS < M
-            }
+            for (int u = 0; u < QT; ++u) a[u] = ld_fixed<R>(src + (q * QT + u) * TS);
             __syncwarp();
-            double2 yq = zero2();
 #pragma unroll
             for (int u = 0; u < QT; ++u) {
-              yq = fma_<R>(a[u], vJ[q * QT + u], yq);
+              y.add(a[u], vJ[q * QT + u]);
               if (!diag) T[u * TILE_LD + lane] = a[u];
             }
-            if (q == 0) y01 = yq;
-            if (q == 1) y01 = add<R>(y01, yq);
-            if (q == 2) y2 = yq;
-            if (q == 3) y = add<R>(y01, add<R>(y2, yq));
             if (diag) continue;
             __syncwarp();
-            double2 zq = zero2();
-            const double2* Tc = T + qc * TILE_LD + qr * QT;
+            Dot<R> zq;
+            const int4* Tc = T + qc * TILE_LD + qr * QT;
 #pragma unroll
-            for (int u = 0; u < QT; ++u) zq = fma_cja<R>(Tc[u], vI[u], zq);
-            zq.x += __shfl_xor_sync(0xffffffffu, zq.x, QT);
-            zq.x += __shfl_xor_sync(0xffffffffu, zq.x, 2 * QT);
-            if constexpr (!R) {
-              zq.y += __shfl_xor_sync(0xffffffffu, zq.y, QT);
-              zq.y += __shfl_xor_sync(0xffffffffu, zq.y, 2 * QT);
-            }
+            for (int u = 0; u < QT; ++u) zq.add_conj(Tc[u], vI[u]);
+            zq.close(true);
+            zq.sum_lanes(QT);
+            zq.sum_lanes(2 * QT);
             if (qr == q) z = zq;
           }
-          if (!diag) st<R>(ws.Yp + (int64_t)I * n + J * TS + lane, z);
-          put_tile(t, I, J, y);
+          y.close(false);
+          if (!diag) st<R>(ws.Yp + (int64_t)I * n + J * TS + lane, z.value(exp_sum(ea, sve[I])));
+          put_tile(t, I, J, y.value(exp_sum(ea, sve[J])));
         }
       }
       if (j > 0) {
-        // lane = column of [W V]: W columns 0..j-1 and V columns NT..NT+j-1; a sum per 8 rows
+        // lane = column of [W V]: W columns 0..j-1 and V columns NT..NT+j-1; a sum per chunk
         const bool on = lane < NT ? lane < j : lane - NT < j;
-        for (int ch = first; ch < nt; ch += stride) {
-          for (int q = RES ? warp : 0; q < (RES ? warp + 1 : PW); ++q) {
-            double2 s = zero2();
-            if (on) {
-              const double2* src = RES ? wvs + (ch / C) * TILE_EL + lane * TILE_LD - ch * 32 : ws.VW + lane;
-              const int64_t step = RES ? 1 : 2 * NT;
-              const int r1 = min(M, ch * 32 + (q + 1) * QT);
-#pragma unroll 4
-              for (int r = max(ch * 32 + q * QT, j + 1); r < r1; ++r)
-                s = fma_cja<R>(ld<R>(src + (int64_t)r * step), sv[r], s);
-              st<R>(ws.sD + (ch * PW + q) * 2 * NT + lane, s);
-            }
+        if constexpr (RES) {
+          const int mine = (ntile - rank + C - 1) / C;         // the chunks go on where the tiles' deal to the warps ended
+          for (int ch = rank, i = 0; ch < nt; ch += C, ++i) {
+            if ((mine + i) % NWP != warp) continue;
+            const int4 *src = wvs + (int64_t)i * TILE_EL + lane * TILE_LD, *v = svf + ch * TS;
+            Dot<R> z;
+#pragma unroll 8
+            for (int r = 0; r < TS; ++r) z.add_conj(src[r], v[r]);
+            z.close(true);
+            if (on) st<R>(ws.sD + ch * 2 * NT + lane, z.value(exp_sum(fixed_exp(ch, lane), sve[ch])));
           }
-        }
-      }
-      if constexpr (RES) {
-        __syncthreads();
-        for (int t = rank + C * warp, i = warp; t < ntile; t += C * PW, i += PW) {
-          int I, J;
-          tile_ij(t, I, J);
-          const double2* yp = yps + i * PW * TS + lane;
-          put_tile(t, I, J, sum4<R>(yp[0], yp[TS], yp[2 * TS], yp[3 * TS]));
+        } else {
+          int4* T = reinterpret_cast<int4*>(big) + (int64_t)warp * QT * TILE_LD;
+          const int qc = lane & (QT - 1), qr = lane / QT;
+          for (int ch = first; ch < nt; ch += stride) {
+            const int4 *src = ws.vf + (int64_t)ch * 2 * NT * TS + lane, *v = svf + ch * TS + qr * QT;
+            Dot<R> z;
+#pragma unroll
+            for (int q = 0; q < PW; ++q) {
+              if ((q & 1) * QT >= j) continue;                 // none of its columns is there yet
+              int4 a[QT];
+#pragma unroll
+              for (int u = 0; u < QT; ++u) a[u] = ld_fixed<R>(src + (q * QT + u) * TS);
+              __syncwarp();
+#pragma unroll
+              for (int u = 0; u < QT; ++u) T[u * TILE_LD + lane] = a[u];
+              __syncwarp();
+              Dot<R> zq;
+              const int4* Tc = T + qc * TILE_LD + qr * QT;
+#pragma unroll
+              for (int u = 0; u < QT; ++u) zq.add_conj(Tc[u], v[u]);
+              zq.close(true);
+              zq.sum_lanes(QT);
+              zq.sum_lanes(2 * QT);
+              if (qr == q) z = zq;
+            }
+            if (on) st<R>(ws.sD + ch * 2 * NT + lane, z.value(exp_sum(fixed_exp(ch, lane), sve[ch])));
+          }
         }
       }
     }
@@ -1157,35 +1329,40 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
     {
       const bool on = lane < NT ? lane < j : lane - NT < j;
       double2 s = zero2();
-      if (!triv && on) {
-#pragma unroll 8
-        for (int c = 0; c < nt; ++c) s = add<R>(s, ldc<R>(ws.sD + (c * PW + warp) * 2 * NT + lane));
+      if (!triv && on && warp < PW) {
+#pragma unroll 4
+        for (int c = warp; c < nt; c += PW) s = add<R>(s, ldc<R>(ws.sD + c * 2 * NT + lane));
       }
-      sm.part[warp][lane] = s;
-      if (!triv && warp == 1) {
+      if (warp < PW) sm.part[warp][lane] = s;
+      constexpr int W0 = RES ? PW : 1;                       // the warps past those of the sums, if there are any
+      if (!triv && warp == W0) {
         double q = 0.0;
 #pragma unroll 8
         for (int t = lane; t < ntile; t += 32) q += __ldcg(ws.sT + t);
         q = warp_sum<true>(make_double2(q, 0.0)).x;
         if (lane == 0) sm.vav = q;
-      } else if (!triv && warp == 2) {
+      } else if (!triv && warp == W0 + 1) {
         double2 q = zero2();
         for (int t = lane; t < nt; t += 32) q = add<R>(q, ldc<R>(ws.Yp + (int64_t)t * n + j + 1));
         q = warp_sum<R>(q);
         if (lane == 0) sm.yrow = q;
-      } else if (warp == 3 && lane < j) {
+      } else if (warp == W0 + 2 && lane < j) {
         sm.rowV[lane] = ldc<R>(A + (j + 1) + (int64_t)lane * n);
         sm.rowW[lane] = ldc<R>(W + (int64_t)lane * n + c0 + j + 1);
       }
     }
     __syncthreads();
-    double2* t12 = sm.t12[warp];
+    double2 tm, qm;                 // multipliers of [W V]'s column `lane` in y and in the next column
     {
       const double2 s = sum4<R>(sm.part[0][lane], sm.part[1][lane], sm.part[2][lane], sm.part[3][lane]);
-      t12[lane] = s;
-      // lane q < NT has t1_q, lane NT + q has t2_q
-      const double2 o = make_double2(__shfl_down_sync(0xffffffffu, s.x, NT),
-                                     R ? 0.0 : __shfl_down_sync(0xffffffffu, s.y, NT));
+      // lane q < NT has t1_q, lane NT + q has t2_q; W's columns take t2, V's take t1
+      const double2 o = make_double2(__shfl_xor_sync(0xffffffffu, s.x, NT),
+                                     R ? 0.0 : __shfl_xor_sync(0xffffffffu, s.y, NT));
+      const int c = lane & (NT - 1);
+      const bool on = c < j;
+      tm = on && !triv ? o : zero2();
+      qm = on && next ? (lane < NT ? sm.rowV[c] : sm.rowW[c]) : zero2();
+      if constexpr (!R) qm.y = -qm.y;
       if (!triv && warp == 0) {                            // the pivot row's tau (y - V t1 - W t2)
         double2 c = zero2();
         if (lane < j) {
@@ -1203,54 +1380,70 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
         const double t2 = R ? tau.x * tau.x : fma(tau.x, tau.x, tau.y * tau.y);
         if (lane == 0) sm.alpha = -0.5 * t2 * (sm.vav - 2.0 * dot);
       }
-      __syncwarp();
     }
-    // quarter q of a row's sums: slots q, q + 4, ... of y, and columns 4 q .. 4 q + 3 of [W V]
-    auto quarter = [&](int ch, int q, double2& y, double2& a) {
+    // the multipliers in fixed point against chunk ch, whose columns have exponents of their own: kt and kq are the
+    // largest products' exponents
+    auto multipliers = [&](int ch, int& kt, int& kq) {
+      const bool on = (lane & (NT - 1)) < j;
+      const int ev = on ? fixed_exp(ch, lane) : 0;
+      const int et = high_word<R>(tm) >> 20, eq = high_word<R>(qm) >> 20;
+      kt = __reduce_max_sync(0xffffffffu, on ? et + ev : 0);
+      kq = __reduce_max_sync(0xffffffffu, on ? eq + ev : 0);
+      sm.tf[warp][lane] = fixed_point<R>(tm, kt - ev);
+      sm.qf[warp][lane] = fixed_point<R>(qm, kq - ev);
+      if (__any_sync(0xffffffffu, on && (ev == 0x7ff || et == 0x7ff))) kt = EXP_BAD;
+      if (__any_sync(0xffffffffu, on && (ev == 0x7ff || eq == 0x7ff))) kq = EXP_BAD;
+      __syncwarp();
+    };
+    // columns c0, c0 + step, ... of W and V into a row's two sums
+    auto corrections = [&](int ch, int from, int step, Dot<R>& dy, Dot<R>& da) {
+      const int4* src = RES ? wvs + (int64_t)(ch / C) * TILE_EL + lane : ws.vf + (int64_t)ch * 2 * NT * TS + lane;
+      constexpr int LD = RES ? TILE_LD : TS;
+#pragma unroll 2
+      for (int c = from; c < j; c += step) {
+        const int4 wq = RES ? src[c * LD] : ld_fixed<R>(src + c * LD);
+        const int4 vq = RES ? src[(NT + c) * LD] : ld_fixed<R>(src + (NT + c) * LD);
+        dy.add(wq, sm.tf[warp][c]);
+        dy.add(vq, sm.tf[warp][NT + c]);
+        if (next) {
+          da.add(wq, sm.qf[warp][c]);
+          da.add(vq, sm.qf[warp][NT + c]);
+        }
+      }
+      dy.close(false);
+      da.close(false);
+    };
+    // slots q, q + 4, ... of a row's y
+    auto slots = [&](int ch, int q) {
       const int r = ch * 32 + lane;
-      y = a = zero2();
-      if (r <= j || r >= M) return;
-      if (next && q == 0) a = ld<R>(A + r + (int64_t)(j + 1) * n);
-      if (!triv) {
+      double2 y = zero2();
+      if (!triv && r > j && r < M) {
 #pragma unroll 4
         for (int s = q; s < nt; s += PW) y = add<R>(y, ldc<R>(ws.Yp + (int64_t)s * n + r));
       }
-      const double2* ws_ = RES ? wvs + (ch / C) * TILE_EL + lane : W + c0 + r;
-      const double2* vs_ = RES ? ws_ + NT * TILE_LD : A + r;
-      const int64_t step = RES ? TILE_LD : n;
-#pragma unroll
-      for (int u = 0; u < NT / PW; ++u) {
-        const int c = q * (NT / PW) + u;
-        if (c < j) {
-          const double2 vq = ld<R>(vs_ + c * step), wq = ld<R>(ws_ + c * step);
-          if (!triv) {
-            y = fms<R>(vq, t12[c], y);
-            y = fms<R>(wq, t12[NT + c], y);
-          }
-          if (next) {
-            a = fms_cj<R>(vq, sm.rowW[c], a);
-            a = fms_cj<R>(wq, sm.rowV[c], a);
-          }
-        }
-      }
+      return y;
     };
     // the row's entry of W's column j and of the next column, from the sums
-    auto finish = [&](int ch, double2 y, double2 a) {
+    auto finish = [&](int ch, double2 y, const Dot<R>& dy, int kt, const Dot<R>& da, int kq) {
       const int r = ch * 32 + lane;
       const double al = triv ? 0.0 : sm.alpha;
       const double2 wrow = triv ? zero2() : make_double2(sm.wrow.x + al, sm.wrow.y);
+      double2 wv = zero2(), a = zero2();
       if (r > j && r < M) {
         const double2 v = sv[r];
-        double2 wv = zero2();
         if (!triv) {
+          const double2 d = dy.value(kt);
+          y = make_double2(y.x - d.x, R ? 0.0 : y.y - d.y);
           wv = mul<R>(tau, y);
           wv.x = fma(al, v.x, wv.x);
           if constexpr (!R) wv.y = fma(al, v.y, wv.y);
         }
         st<R>(W + (int64_t)j * n + c0 + r, wv);
-        if constexpr (RES) wvs[(ch / C) * TILE_EL + j * TILE_LD + lane] = wv;
         st<R>(ws.VW + (int64_t)r * 2 * NT + j, wv);
         if (next) {
+          const double2 d = da.value(kq);
+          a = ld<R>(A + r + (int64_t)(j + 1) * n);
+          a = make_double2(a.x - d.x, R ? 0.0 : a.y - d.y);
           a = fms_cj<R>(v, wrow, a);
           a.x -= wv.x;                                     // V at the pivot row is 1
           if constexpr (!R) a.y -= wv.y;
@@ -1261,6 +1454,8 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
           st<R>(ws.xc + r, a);
         }
       }
+      const int emax = __reduce_max_sync(0xffffffffu, high_word<R>(wv)) >> 20;
+      put_fixed(ch, j, fixed_point<R>(wv, emax), emax);
       if (next) {
         double s = r >= j + 3 && r < M ? (R ? a.x * a.x : fma(a.x, a.x, a.y * a.y)) : 0.0;
         s = warp_sum<true>(make_double2(s, 0.0)).x;
@@ -1268,36 +1463,53 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
       }
     };
     if constexpr (RES) {
-      for (int ch = rank; ch < nt; ch += C) {
-        double2 y, a;
-        quarter(ch, warp, y, a);
-        double2* e = eps + ((ch / C) * PW + warp) * 2 * TS + lane;
-        e[0] = y;
-        e[TS] = a;
+      for (int ch = rank, i = 0; ch < nt; ch += C, ++i) {
+        char* e = eps + (int64_t)i * EPS;
+        if (warp >= PW) {                                    // half of the warps sum the slots, half the corrections
+          reinterpret_cast<double2*>(e)[(warp - PW) * TS + lane] = slots(ch, warp - PW);
+        } else {
+          int kt, kq;
+          Dot<R> dy, da;
+          multipliers(ch, kt, kq);
+          corrections(ch, warp, PW, dy, da);
+          long long* d = reinterpret_cast<long long*>(e + PW * 16 * TS) + warp * 8 * TS + lane;
+          dy.put(d, TS);
+          da.put(d + 4 * TS, TS);
+          if (warp == 0 && lane < 2) wve[i * (2 * NT + 2) + 2 * NT + lane] = lane ? kq : kt;
+          __syncwarp();
+        }
       }
       __syncthreads();
-      for (int ch = rank + C * warp; ch < nt; ch += C * PW) {
-        const double2* e = eps + (ch / C) * PW * 2 * TS + lane;
-        finish(ch, sum4<R>(e[0], e[2 * TS], e[4 * TS], e[6 * TS]), sum4<R>(e[TS], e[3 * TS], e[5 * TS], e[7 * TS]));
+      for (int ch = first, i = warp; ch < nt; ch += stride, i += NWP) {
+        const char* e = eps + (int64_t)i * EPS;
+        const double2* y = reinterpret_cast<const double2*>(e) + lane;
+        Dot<R> dy, da;
+#pragma unroll
+        for (int q = 0; q < PW; ++q) {
+          const long long* d = reinterpret_cast<const long long*>(e + PW * 16 * TS) + q * 8 * TS + lane;
+          dy.take(d, TS);
+          da.take(d + 4 * TS, TS);
+        }
+        const int* ke = wve + i * (2 * NT + 2) + 2 * NT;
+        finish(ch, sum4<R>(y[0], y[TS], y[2 * TS], y[3 * TS]), dy, ke[0], da, ke[1]);
       }
     } else {
       __syncthreads();
       for (int ch = first; ch < nt; ch += stride) {
-        double2 y0, y1, y2, y3, a0, a1, a2, a3;
-        quarter(ch, 0, y0, a0);
-        quarter(ch, 1, y1, a1);
-        y0 = add<R>(y0, y1);
-        a0 = add<R>(a0, a1);
-        quarter(ch, 2, y2, a2);
-        quarter(ch, 3, y3, a3);
-        finish(ch, add<R>(y0, add<R>(y2, y3)), add<R>(a0, add<R>(a2, a3)));
+        int kt, kq;
+        Dot<R> dy, da;
+        multipliers(ch, kt, kq);
+        corrections(ch, 0, 1, dy, da);
+        const double2 y = sum4<R>(slots(ch, 0), slots(ch, 1), slots(ch, 2), slots(ch, 3));
+        finish(ch, y, dy, kt, da, kq);
+        __syncwarp();
       }
     }
     __syncthreads();
   }
   // slices of the rows below the panel: z = [V W], both operands
   if (M - w > 1) {
-    for (int ch = rank + C * warp; ch < nt; ch += C * PW) {
+    for (int ch = first; ch < nt; ch += stride) {
       const int r = ch * 32 + lane;
       if (r < w || r >= M) continue;
       const double2* vw = ws.VW + (int64_t)r * 2 * NT;
@@ -1314,20 +1526,24 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
 }
 
 template <bool RES>
-__global__ void __launch_bounds__(PT, RES ? 1 : 4) k_tri_panel(Grp G, int c0, int C, int rt, int cpc, int grid) {
+__global__ void __launch_bounds__(RES ? PTR : PT, RES ? 1 : 4) k_tri_panel(Grp G, int c0, int C, int rt, int cpc, int grid,
+                                                                  unsigned sve_off) {
   const int g = blockIdx.x / C, p = G.prob[g];
   if (!live(G, p)) return;
   if (c0 >= G.nvec[p] - 1) return;
   extern __shared__ __align__(16) char smem_raw[];
   PanelSm& sm = *reinterpret_cast<PanelSm*>(smem_raw);
   double2* sv = reinterpret_cast<double2*>(smem_raw + sizeof(PanelSm));
-  double2* big = sv + cdiv_d(G.nmax - c0, TS) * TS;
+  const int rows = cdiv_d(G.nmax - c0, TS) * TS;
+  int4* svf = reinterpret_cast<int4*>(sv + rows);
+  double2* big = reinterpret_cast<double2*>(svf + rows);
+  int* sve = reinterpret_cast<int*>(smem_raw + sve_off);
   if (threadIdx.x == 0) sm.dead = 0;
   Team team{(int)(blockIdx.x % C), C, grid != 0, ws_of(G, g).bar + c0 / NT, 0u, G.status + p, &sm.dead};
   if (is_real(G, p))
-    panel_body<true, RES>(G, g, p, c0, team, rt, cpc, sm, sv, big);
+    panel_body<true, RES>(G, g, p, c0, team, rt, cpc, sm, sv, svf, sve, big);
   else
-    panel_body<false, RES>(G, g, p, c0, team, rt, cpc, sm, sv, big);
+    panel_body<false, RES>(G, g, p, c0, team, rt, cpc, sm, sv, svf, sve, big);
 }
 
 // ------------------------------------------------------------------ eigenvalues
@@ -1399,11 +1615,12 @@ __global__ void __launch_bounds__(64) k_eig(Grp G) {
 // ------------------------------------------------------------------ host sequence
 constexpr size_t SMEM_MAX = 227 * 1024;
 
-// Shared memory of a panel over m rows: streamed, or (rt > 0) resident with rt tiles and cpc chunks per CTA.
+// Shared memory of a panel over m rows: streamed, or (rt > 0) resident with rt tiles and cpc chunks per CTA; the exponents
+// of v are its last part.
 size_t panel_smem(int m, int rt, int cpc) {
-  const size_t head = sizeof(PanelSm) + (size_t)cdiv(m, TS) * TS * sizeof(double2);
-  if (rt == 0) return head + (size_t)PW * QT * TILE_LD * sizeof(double2);
-  return head + ((size_t)(rt + cpc) * TILE_EL + (size_t)rt * PW * TS + (size_t)cpc * PW * 2 * TS) * sizeof(double2);
+  const size_t head = sizeof(PanelSm) + (size_t)cdiv(m, TS) * (TS * (sizeof(double2) + sizeof(int4)) + sizeof(int));
+  if (rt == 0) return head + (size_t)PW * QT * TILE_LD * sizeof(int4);
+  return head + (size_t)(rt + cpc) * TILE_EL * sizeof(int4) + (size_t)cpc * (EPS + (2 * NT + 2) * sizeof(int));
 }
 
 inline int pow2_below(int v, int most) {
@@ -1412,15 +1629,45 @@ inline int pow2_below(int v, int most) {
   return c;
 }
 
+// Clusters of C CTAs that the GPU holds at once, one CTA per SM: a cluster stays within one of its processor clusters,
+// which are not all of 16 SMs or more (GB300: 7 of 16, 8 of 12, 15 of 8).
+int clusters_at_once(int C, int sms) {
+  static std::mutex lock;
+  static std::map<std::pair<int, int>, int> known;
+  int dev = 0;
+  cudaGetDevice(&dev);
+  std::lock_guard<std::mutex> hold(lock);
+  int& n = known[{dev, C}];
+  if (n == 0) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)C * sms);
+    cfg.blockDim = dim3(PTR);
+    cfg.dynamicSmemBytes = SMEM_MAX - 2048;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = C;
+    at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (cudaOccupancyMaxActiveClusters(&n, k_tri_panel<true>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = sms / (2 * C) > 1 ? sms / (2 * C) : 1;
+    }
+  }
+  return n;
+}
+
 // CTAs per problem over m rows, and the tiles of each when they are resident (0: streamed).  Resident: one CTA per SM,
-// up to one per tile, if shared memory holds its part.  A cluster's barrier takes about 1200 clocks, a counter's
-// 5000, so a grid team only from GRID_FROM CTAs.  Streamed: STREAM_PER_SM CTAs for each SM (three are resident; the
-// rest wait) even out the mixed batch's calls, which run beside one another: 305 ms at 3, 300 at 4, 289 at 6, 284 at 10.
+// up to one per tile, if shared memory holds its part and all problems run at once.  A cluster's barrier takes about 1200
+// clocks, a counter's 5000, so a grid team only from GRID_FROM CTAs.  Streamed: STREAM_PER_SM CTAs for each SM (four are
+// resident; the rest wait) even out the mixed batch's calls, which run beside one another: 204 ms at 4, 196 at 10.
 constexpr int GRID_FROM = 24, STREAM_PER_SM = 10;
 void plan_panel(int m, int n_prob, int sms, int all, int& C, int& rt) {
   const int nt = cdiv(m, TS), tiles = nt * (nt + 1) / 2;
   const int most = std::min(tiles, std::max(1, sms / n_prob));
-  C = most >= GRID_FROM ? most : pow2_below(most, 16);
+  C = most;
+  if (most < GRID_FROM)
+    for (C = std::min(most, 16); C > 1 && clusters_at_once(C, all) < n_prob;) --C;
   rt = cdiv(tiles, C);
   if ((int64_t)n_prob * C <= all && panel_smem(m, rt, cdiv(nt, C)) <= SMEM_MAX) return;
   rt = 0;
@@ -1434,7 +1681,7 @@ cudaError_t launch_panel(const Grp& G, int count, int c0, int sms, int all, cuda
   const int cpc = cdiv(cdiv(m, TS), C);
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)count * C);
-  cfg.blockDim = dim3(PT);
+  cfg.blockDim = dim3(rt ? PTR : PT);
   cfg.dynamicSmemBytes = panel_smem(m, rt, cpc);
   cfg.stream = stream;
   const int grid = C > 16;
@@ -1449,8 +1696,11 @@ cudaError_t launch_panel(const Grp& G, int count, int c0, int sms, int all, cuda
   }
   cfg.attrs = at;
   cfg.numAttrs = 1;
-  return rt ? cudaLaunchKernelEx(&cfg, k_tri_panel<true>, G, c0, C, rt, cpc, grid)
-            : cudaLaunchKernelEx(&cfg, k_tri_panel<false>, G, c0, C, rt, cpc, grid);
+  const unsigned sve_off = (unsigned)(cfg.dynamicSmemBytes - sizeof(int) * cdiv(m, TS));
+  const int nt = cdiv(m, TS);
+  k_fixed<<<dim3((unsigned)(nt * (nt + 1) / 2), (unsigned)count), PT, 0, stream>>>(G, c0);
+  return rt ? cudaLaunchKernelEx(&cfg, k_tri_panel<true>, G, c0, C, rt, cpc, grid, sve_off)
+            : cudaLaunchKernelEx(&cfg, k_tri_panel<false>, G, c0, C, rt, cpc, grid, sve_off);
 }
 
 // One update of the first `count` problems: jc column tiles per CTA, so that the GPU gets about two CTAs per SM at

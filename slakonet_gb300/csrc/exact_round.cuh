@@ -85,3 +85,28 @@ SKN_HD double round_sum28(long long hi, long long lo, int e) {
   return skn_bits_to_double((neg ? 0x8000000000000000ull : 0ull) + ((unsigned long long)be << 52) +
                             (t - 0x10000000000000ull));
 }
+
+// The double nearest to (h * 2^28 + m) * 2^k for any |h| < 2^62 and |m| < 2^62 (ties away from zero, but for bits of m
+// below 2^-64 of the sum): the sum is normalised in 64 bits. About 30 integer instructions and no FP64 one.
+SKN_HD double round_wide28(long long h, long long m, int k) {
+  long long H = h + (m >> 28);
+  unsigned long long l = (unsigned long long)m & 0xFFFFFFFull;
+  const bool neg = H < 0;
+  if (neg) {                                                  // negate the pair: l stays in [0, 2^28)
+    H = -H - (l != 0);
+    l = (0x10000000ull - l) & 0xFFFFFFFull;
+  }
+  k += 28;
+  if (H == 0) {
+    H = (long long)l;
+    l = 0;
+    k -= 28;
+    if (H == 0) return 0.0;
+  }
+  const int z = skn_clz64((unsigned long long)H);             // 1 .. 63
+  const unsigned long long top = ((unsigned long long)H << z) | ((l << 36) >> (64 - z));
+  const unsigned long long t = (top >> 11) + ((top >> 10) & 1);   // in [2^52, 2^53]: rounding up carries into the exponent
+  const int be = 1086 - z + k;                                // value = t 2^(11 - z + k)
+  if (be <= 0 || be >= 2046) return ldexp((double)(neg ? -(long long)t : (long long)t), 11 - z + k);
+  return skn_bits_to_double((neg ? 0x8000000000000000ull : 0ull) + ((unsigned long long)be << 52) + (t - 0x10000000000000ull));
+}

@@ -534,7 +534,7 @@ def panels_launches(max_n: int) -> int:
     T = -(-max_n // PANEL)
     tri = -(-(max_n - 1) // 16)
     upd = sum(1 for c0 in range(0, max_n - 1, 16) if max_n - c0 - 16 > 1)
-    return 3 + 2 * T + (T - 1) + T + (T - 1) + tri + upd + 2
+    return 3 + 2 * T + (T - 1) + T + (T - 1) + 2 * tri + upd + 2
 
 
 def panels_scratch_bytes(n: int) -> int:
@@ -562,18 +562,18 @@ def panels_parts(sizes: np.ndarray, budget: int):
 VEC_SCRATCH = 512 << 20      # device bytes of the inverse iteration's scratch per group
 
 
-SMALL_MAX_N = 96            # bound of the shared-memory eigensolver (csrc/eigh_small.cu)
-SMALL_CLASSES = (16, 24, 32, 40, 48, 56, 64, 80, 96)     # its calls' size classes: shared memory decides how many
+SMALL_MAX_N = 64            # up to here the shared-memory eigensolver (csrc/eigh_small.cu, which takes 96)
+SMALL_CLASSES = (16, 24, 32, 40, 48, 56, 64)     # its calls' size classes: shared memory decides how many
                                                          # CTAs share an SM
 
 
 def route_auto(n: int):
     """Kernel and call of a problem of n orbitals under the untuned policy: ("small", class) or ("panels", panel
-    count).  A rule on the problem alone, as route_wide.  Measured on GB300 against the one-CTA kernel:
-    panels 432 orbitals x 8 problems 18.8 ms (191 ms), 160 x 27 4.6 ms (12.6), 128 x 1000 28 ms (31),
-    200 x 500 44 ms (62), 492 x 300 208 ms (393), 96 x 3000 45 ms (38); so the small kernel as far as shared memory
-    holds a problem.  One panel call per panel count: the 600 problems of 57 to 492 orbitals of a mixed batch take
-    284 ms so, on one stream each, and 297 ms as one call that drops the smaller ones on the way."""
+    count).  A rule on the problem alone, as route_wide.  Measured on GB300, panels against the small kernel:
+    88 orbitals x 500 problems 6.2 ms (9.6), 80 x 50 1.9 (1.9), 72 x 500 5.0 (5.9), 72 x 8 1.7 (1.5), 64 x 4000 23
+    (19): the line is at 64.  Against the one-CTA kernel: 128 x 1000 19.6 ms (31), 160 x 27 3.8 (12.6), 432 x 8 11.6
+    (190), 492 x 300 130 (393).  One panel call per panel count, each on its stream: the 600 problems of 57 to 492
+    orbitals of a mixed batch took 284 ms so and 297 ms as one call that drops the smaller ones on the way."""
     if n <= SMALL_MAX_N:
         return ("small", next(c for c in SMALL_CLASSES if n <= c))
     return ("panels", -(-n // PANEL))

@@ -40,6 +40,22 @@ int main(int argc, char** argv) {
       ++bad;
     }
   }
+  for (long long it = 0; it < cases; ++it) {                    // round_wide28: within a unit of 2^-64 of the tie
+    long long h = (long long)(g() >> 1) - (1ll << 62), m = (long long)(g() >> 1) - (1ll << 62);
+    if (it % 3) h >>= (g() % 63);
+    if (it % 2) m >>= (g() % 63);
+    if (it % 7 == 0) h = (long long)(g() % 3) - 1;
+    if (it % 7 == 1) m = -(h << 28);
+    const int e = (int)(g() % 200) - 100;
+    const __int128 v = ((__int128)h << 28) + m;
+    const double got = round_wide28(h, m, e), ref = nearest(v, e);
+    const double off = std::fabs((double)(v - (__int128)std::ldexp(got, -e)));
+    const double ulp = std::ldexp(1.0, std::ilogb(v ? (double)v : 1.0) - 52);
+    if (ref != got && !(v != 0 && off <= 0.5001 * ulp)) {
+      if (bad < 5) std::printf("wide h=%lld m=%lld e=%d: expected %.17g, got %.17g\n", h, m, e, ref, got);
+      ++bad;
+    }
+  }
   std::printf("%lld mismatches in %lld cases\n", bad, cases);
   return bad != 0;
 }

@@ -1,5 +1,5 @@
-"""The panel eigensolver rounds its exact integer level sums to FP64 with round_sum28 (csrc/exact_round.cuh): built for
-the host, bit for bit the nearest double by 128-bit integers."""
+"""The panel eigensolver rounds its exact integer level sums to FP64 with round_sum28 and round_wide28
+(csrc/exact_round.cuh): built for the host, the nearest double by 128-bit integers."""
 import os
 import shutil
 import subprocess
