@@ -21,7 +21,7 @@
 // slot and is added in a fixed order, or is an integer, so a problem's results depend neither on the other problems nor
 // on the number of CTAs it is given.
 // Measured (random pencils): 492 orbitals x 300 problems 393 ms with one CTA per problem, 208 with the products in FP64,
-// 130 now (tridiagonalisation 63, updates 40, solves 16, eigenvalues 6); 432 x 8 190, 18.8, 11.6 ms (6.4 of them the
+// 123 now (tridiagonalisation 63, updates 32, solves 16, eigenvalues 6); 432 x 8 190, 18.8, 11.6 ms (6.4 of them the
 // tridiagonalisation, 15 us a column); 1152 x 2 47, 35.8 ms.
 #include <algorithm>
 #include <map>
@@ -478,20 +478,27 @@ SKN_DEVINL void tmem_ld8(uint32_t a, uint32_t* v) {
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
                : "r"(a));
 }
-// Exact sums of 8 columns over the levels: hi counts units of 2^28 of lo.  The level sums are integers below 2^22:
+SKN_DEVINL void tmem_ld4(uint32_t a, uint32_t* v) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+               : "r"(a));
+}
+// Exact sums of Q columns over the levels: hi counts units of 2^28 of lo.  The level sums are integers below 2^22:
 // the FP32 addition of 1.5 2^23 leaves them in the low bits, and two levels fit 32 bits.
+template <int Q>
 SKN_DEVINL void level_sums(uint32_t base, int level_cols, long long* hi, long long* lo) {
   auto quad = [&](int L, long long* out) {
-    uint32_t t[8], u[8], v[8], w[8];
-    tmem_ld8(base + (uint32_t)(L * level_cols), t);
-    tmem_ld8(base + (uint32_t)((L + 1) * level_cols), u);
-    tmem_ld8(base + (uint32_t)((L + 2) * level_cols), v);
-    tmem_ld8(base + (uint32_t)((L + 3) * level_cols), w);
+    uint32_t t[4][Q];
+#pragma unroll
+    for (int l = 0; l < 4; ++l) {
+      if constexpr (Q == 8) tmem_ld8(base + (uint32_t)((L + l) * level_cols), t[l]);
+      else tmem_ld4(base + (uint32_t)((L + l) * level_cols), t[l]);
+    }
     asm volatile("tcgen05.wait::ld.sync.aligned;");
     auto whole = [](uint32_t x) { return __float_as_int(__uint_as_float(x) + 12582912.0f) - 0x4B400000; };
 #pragma unroll
-    for (int q = 0; q < 8; ++q)
-      out[q] = (long long)(whole(t[q]) * 128 + whole(u[q])) * 16384 + (whole(v[q]) * 128 + whole(w[q]));
+    for (int q = 0; q < Q; ++q)
+      out[q] = (long long)(whole(t[0][q]) * 128 + whole(t[1][q])) * 16384 + (whole(t[2][q]) * 128 + whole(t[3][q]));
   };
   quad(0, hi);
   quad(4, lo);
@@ -624,8 +631,8 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
 #pragma unroll 1
     for (int cb = 0; cb < NB; cb += 8) {
       long long hr[8], lr[8], hi[8], li[8];
-      level_sums(tb + cb, 2 * NB, hr, lr);
-      level_sums(tb + NB + cb, 2 * NB, hi, li);
+      level_sums<8>(tb + cb, 2 * NB, hr, lr);
+      level_sums<8>(tb + NB + cb, 2 * NB, hi, li);
 #pragma unroll
       for (int q = 0; q < 8; ++q) {
         const int k = cb + q, ex = s_ex[k];
@@ -662,15 +669,17 @@ constexpr int B_BYTES = SLICES * 2 * BH_BYTES;       // 32 KB
 constexpr int UPD_SMEM = SLICES * A_BYTES + 2 * B_BYTES;       // 192 KB
 constexpr uint32_t BUF_COLS = SLICES * 2 * BN;       // TMEM columns of one tile
 constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
-constexpr int UPD_THREADS = 32 * 9;
+constexpr int UPD_WARPS = 16, UPD_THREADS = 32 * (UPD_WARPS + 1);
+constexpr int UC = 4;                                // columns a thread takes at once
 
 // C -= A B^T over BM x BN tiles.  SWEEP 1: blocks [0, nlow) of S22 (lower triangle, columns from sb), the rest
 // of H below the panel over all columns (sc); SWEEP 2 and 3: the trailing lower triangle of H (sb).
 // c1: first row and column of the trailing matrix.  A CTA has one 128-row block I and up to jc column tiles: its
 // 8 row slices stay in shared memory (128 KB), the column slices and the accumulators are double-buffered.
-// Thread 256 copies and issues the products of every slice pair of level < SLICES; warps 0-3 and 4-7 take the even and
-// the odd tiles: a thread has a row, fetches its entries of C while the products run, adds the levels exactly in
-// int64 and rounds once.  At n = 492 x 300 problems a tile took 39k clocks of an SM with one tile per CTA.
+// One thread copies and issues the products of every slice pair of level < SLICES; warps 0-3 and 8-11 take the halves of
+// the even tiles, the others those of the odd: a thread has a row, fetches its entries of C while the products run, adds
+// the levels exactly in int64 and rounds once.  Bound by the latency of that chain, so the warps count: at n = 492 x 300
+// problems a tile takes 39k clocks of an SM with one tile per CTA, 16k with eight warps, 12.9k with sixteen.
 // All waits are bounded; one that runs out marks the problem SKN_ERR_CUDA and leaves the tile, and the
 // copies and products that were issued are still waited for (bounded).
 template <int SWEEP>
@@ -705,10 +714,10 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
   if (tid == 0) {
     s_fail = 0;
     for (int b = 0; b < T_EMPTY; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar(b)));
-    for (int b = T_EMPTY; b < T_EMPTY + 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 4;" ::"r"(bar(b)));
+    for (int b = T_EMPTY; b < T_EMPTY + 2; ++b) asm volatile("mbarrier.init.shared::cta.b64 [%0], 8;" ::"r"(bar(b)));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  if (warp == 8) {
+  if (warp == UPD_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"(TMEM_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -717,7 +726,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
-  if (warp == 8) {
+  if (warp == UPD_WARPS) {
     if (lane == 0) {
       auto load_b = [&](int i) {
         const uint32_t bb = bar(B_FULL + (i & 1)), dst = b0 + (uint32_t)((i & 1) * B_BYTES);
@@ -785,7 +794,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
       if (!ok) s_fail = 1;
     }
   } else {
-    const int grp = warp >> 2, wq = warp & 3;        // a warp reads TMEM lanes 32 (warp mod 4) .. + 31
+    const int grp = (warp >> 2) & 1, wq = warp & 3, c0 = (warp >> 3) * (BN / 2);        // a warp reads TMEM lanes 32 (warp mod 4) .. + 31
     const int i = r0 + wq * 32 + lane;               // trailing row
     const bool rok = i < m;
     const int er = rok ? w.ea[c1 + i] : 0;
@@ -793,37 +802,34 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
     const uint32_t base = tmem + (uint32_t)grp * BUF_COLS + ((uint32_t)(wq * 32) << 16);
     for (int it = grp; it < ntile; it += 2) {
       const int q0 = (j0 + it) * BN;                 // tile's first column, counted from boff
-      double2 cv[8];
-      auto fetch = [&](int cb) {
+      double2 cv[BN / 2];
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
-          const int gc = boff + q0 + cb + q;
-          cv[q] = zero2();
-          if (rok && gc < n && (!low || i >= q0 + cb + q)) cv[q] = C[(int64_t)gc * n];
-        }
-      };
-      fetch(0);
+      for (int q = 0; q < BN / 2; ++q) {
+        const int gc = boff + q0 + c0 + q;
+        cv[q] = zero2();
+        if (rok && gc < n && (!low || i >= q0 + c0 + q)) cv[q] = C[(int64_t)gc * n];
+      }
       const bool ok = upd_wait(bar(T_FULL + grp), (uint32_t)((it >> 1) & 1), &s_fail);
       if (!ok || s_fail) {
         s_fail = 1;
         break;
       }
       asm volatile("tcgen05.fence::after_thread_sync;");
-#pragma unroll 1
-      for (int cb = 0; cb < BN; cb += 8) {
-        long long hr[8], lr[8], hi[8], li[8];
-        if (cb > 0) fetch(cb);
-        level_sums(base + cb, 2 * BN, hr, lr);
-        level_sums(base + BN + cb, 2 * BN, hi, li);
-        if (cb + 8 == BN) {                          // the accumulators have been read: the next tile may start
+#pragma unroll
+      for (int h = 0; h < BN / 2; h += UC) {
+        const int cb = c0 + h;
+        long long hr[UC], lr[UC], hi[UC], li[UC];
+        level_sums<UC>(base + cb, 2 * BN, hr, lr);
+        level_sums<UC>(base + BN + cb, 2 * BN, hi, li);
+        if (h + UC == BN / 2) {                      // the accumulators have been read: the next tile may start
           asm volatile("tcgen05.fence::before_thread_sync;");
           if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(T_EMPTY + grp)) : "memory");
         }
 #pragma unroll
-        for (int q = 0; q < 8; ++q) {
+        for (int q = 0; q < UC; ++q) {
           const int j = q0 + cb + q, gc = boff + j;
           if (rok && gc < n && (!low || i >= j)) {
-            double2 v = cv[q];
+            double2 v = cv[h + q];
             const int ec = eB[gc];
             if (er == EXP_NAN || ec == EXP_NAN) {
               v = make_double2(__longlong_as_double(0x7ff8000000000000LL), __longlong_as_double(0x7ff8000000000000LL));
@@ -841,7 +847,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   if (tid == 0 && s_fail) G.status[p] = SKN_ERR_CUDA;
-  if (warp == 8) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
+  if (warp == UPD_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
 // ------------------------------------------------------------------ tridiagonalisation panel
