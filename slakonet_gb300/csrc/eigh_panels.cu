@@ -21,8 +21,8 @@
 // slot and is added in a fixed order, or is an integer, so a problem's results depend neither on the other problems nor
 // on the number of CTAs it is given.
 // Measured (random pencils): 492 orbitals x 300 problems 393 ms with one CTA per problem, 208 with the products in FP64,
-// 123 now (tridiagonalisation 63, updates 32, solves 16, eigenvalues 6); 432 x 8 190, 18.8, 11.6 ms (6.4 of them the
-// tridiagonalisation, 15 us a column); 1152 x 2 47, 35.8 ms.
+// 114 now (tridiagonalisation 62, updates 32, solves 8, eigenvalues 6); 432 x 8 190, 18.8, 10.5 ms (6.2 of them the
+// tridiagonalisation, 15 us a column); 1152 x 2 47, 32.8 ms.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -242,62 +242,37 @@ SKN_DEVINL void slice_block(Get get, int kb, int emax, uint4* out) {
   for (int s = 0; s < SLICES; ++s) out[s] = make_uint4(w[s][0], w[s][1], w[s][2], w[s][3]);
 }
 
-// Slices of one row r: values z_k = get(k), k < 32 (zero from K on).  A form to sa (null: none) with exponent
-// ea[r]; B and B' forms of the row with its halves swapped when `swap` (z' = [z_16.. z_31, z_0.. z_15]).
-template <class Get>
-SKN_DEVINL void slice_row(Get get, int r, int64_t nr, uint16_t* sa, int* ea, uint16_t* sb, int* eb, bool swap) {
+constexpr int SE = 8;                     // entries of a row a thread slices: one block of digits per part
+SKN_DEVINL int high_word8(const double2* z) {
   int hm = 0;
-#pragma unroll 8
-  for (int k = 0; k < 32; ++k) {
-    const double2 z = get(k);
-    hm = max(hm, max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
-  }
-  const int emax = hm >> 20;                // 0x7ff: the digits mean nothing, the exponent says so
+#pragma unroll
+  for (int q = 0; q < SE; ++q)
+    hm = max(hm, max(__double2hiint(z[q].x) & 0x7fffffff, __double2hiint(z[q].y) & 0x7fffffff));
+  return hm;
+}
+// Slices of 8 of a row's 32 entries, part `part` of row r.  A form to sa (null: none) with exponent ea[r]; B and B' forms
+// to sb, of the row with its halves swapped when `swap` (z' = [z_16.. z_31, z_0.. z_15]).
+SKN_DEVINL void slice_part(const double2* z, int part, int emax, int r, int64_t nr, uint16_t* sa, int* ea, uint16_t* sb,
+                           int* eb, bool swap) {
   const int ex = emax == 0x7ff ? EXP_NAN : emax - 1022;
-  if (sa) ea[r] = ex;
-  if (sb) eb[r] = ex;
-#pragma unroll 1
-  for (int kb = 0; kb < 8; ++kb) {          // 8 entries of one part: kb < 4 real, then imaginary
+  if (part == 0) {
+    if (sa) ea[r] = ex;
+    if (sb) eb[r] = ex;
+  }
+#pragma unroll
+  for (int im = 0; im < 2; ++im) {
     uint4 out[SLICES];
-    slice_block(get, kb, emax, out);
-    const int pb = swap ? ((kb & 4) | ((kb + 2) & 3)) : kb;      // place of these entries in B
-    const bool im = kb >= 4;
+    slice_block([&](int k) { return z[k & (SE - 1)]; }, 4 * im, emax, out);
+    const int kb = part + 4 * im, pb = swap ? 4 * im + ((part + 2) & 3) : kb;      // place of these entries in A, in B
 #pragma unroll
     for (int s = 0; s < SLICES; ++s) {
       const uint4 v = out[s];
       if (sa) *reinterpret_cast<uint4*>(sa + (int64_t)s * nr * KP + tc_idx(r, kb * 8)) = v;
       if (sb) {
-        uint16_t* B = sb + (int64_t)s * nr * KP;
-        uint16_t* Bp = sb + (int64_t)(SLICES + s) * nr * KP;
-        *reinterpret_cast<uint4*>(B + tc_idx(r, pb * 8)) = v;
+        *reinterpret_cast<uint4*>(sb + (int64_t)s * nr * KP + tc_idx(r, pb * 8)) = v;
         // B' = [-Qi Qr]: the real part of Q goes to the second half, minus the imaginary part to the first
-        *reinterpret_cast<uint4*>(Bp + tc_idx(r, (pb ^ 4) * 8)) = im ? neg4(v) : v;
+        *reinterpret_cast<uint4*>(sb + (int64_t)(SLICES + s) * nr * KP + tc_idx(r, (pb ^ 4) * 8)) = im ? neg4(v) : v;
       }
-    }
-  }
-}
-
-// The same into shared memory for a product of this CTA: slice s of row r at dst + s * slice_el, form A; with prime >
-// 0 form B, and form B' at row r + prime.
-template <class Get>
-SKN_DEVINL void slice_row_to(Get get, int r, uint16_t* dst, int slice_el, int prime, int& ex) {
-  int hm = 0;
-#pragma unroll 8
-  for (int k = 0; k < 32; ++k) {
-    const double2 z = get(k);
-    hm = max(hm, max(__double2hiint(z.x) & 0x7fffffff, __double2hiint(z.y) & 0x7fffffff));
-  }
-  const int emax = hm >> 20;
-  ex = emax == 0x7ff ? EXP_NAN : emax - 1022;
-#pragma unroll 1
-  for (int kb = 0; kb < 8; ++kb) {
-    uint4 v[SLICES];
-    slice_block(get, kb, emax, v);
-#pragma unroll
-    for (int s = 0; s < SLICES; ++s) {
-      uint16_t* D = dst + (int64_t)s * slice_el;
-      *reinterpret_cast<uint4*>(D + tc_idx(r, kb * 8)) = v[s];
-      if (prime) *reinterpret_cast<uint4*>(D + tc_idx(r + prime, (kb ^ 4) * 8)) = kb >= 4 ? neg4(v[s]) : v[s];
     }
   }
 }
@@ -540,12 +515,15 @@ constexpr int A_BYTES = BM * KP * 2;                 // 16 KB: one slice of 128 
 // the panel of S, sliced as both operands of the update; the others: columns of the block row of H, sliced as column
 // operand.  MODE 2 (second sweep): blocks [0, nrow): rows from the panel's own down of H, sliced as row operand; the
 // others: rows of L21, sliced as column operand without a solve.
-// One CTA per 128 rows: a thread slices its row into shared memory, warp 4 the rows of X, thread 128 issues the
-// products, a thread rounds its row's 32 sums and slices the result.
-constexpr int SV_THREADS = 160;
+// One CTA per 128 rows, four threads a row with 8 of its 32 entries each: they slice them into shared memory (four more
+// warps the rows of X), one thread issues the products, each rounds its 8 sums and slices them for the update.  The row's
+// exponent is the only thing the four share.  Bound by the latency of that chain: with one thread a row a CTA took 53 us
+// (MODE 1) and 42 (MODE 2), 25 and 21 now.
+constexpr int SV_PARTS = 4, SV_ROW_WARPS = 4 * SV_PARTS, SV_THREADS = 32 * (SV_ROW_WARPS + SV_PARTS);
 constexpr int X_BYTES = 2 * NB * KP * 2;             // 8 KB: one slice of X, both forms
 constexpr int SV_SMEM = SLICES * (A_BYTES + X_BYTES);              // 192 KB
 constexpr uint32_t SV_COLS = SLICES * 2 * NB;        // 512 TMEM columns
+static_assert(NB / SV_PARTS == SE, "four threads slice a row");
 
 template <int MODE>
 __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow) {
@@ -560,14 +538,27 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
   const WS ws = ws_of(G, g);
   double2* S = G.S + G.hs_off[p];
   double2* H = G.H + G.hs_off[p];
-  const int r = base + tid;                          // row, or column of the block row (threads below 128)
+  const bool xwarp = warp >= SV_ROW_WARPS;
+  const int part = xwarp ? warp - SV_ROW_WARPS : warp >> 2;
+  const int row = xwarp ? lane : (warp & 3) * 32 + lane;
+  const int r = base + row;                          // row, or column of the block row (not the warps of X)
+  extern __shared__ __align__(1024) uint8_t smem[];
+  __shared__ int s_hm[SV_PARTS][BM + NB];
+  const int slot = xwarp ? BM + row : row;
+  // the exponent field of the four threads' entries
+  auto together = [&](const double2* z) {
+    s_hm[part][slot] = high_word8(z);
+    __syncthreads();
+    return max(max(s_hm[0][slot], s_hm[1][slot]), max(s_hm[2][slot], s_hm[3][slot])) >> 20;
+  };
+  double2 z[SE];
   if (MODE == 2 && !rows) {
-    if (tid >= BM || r >= n) return;
-    const double2* row = S + r + (int64_t)c0 * n;
-    slice_row([&](int k) { return row[(int64_t)k * n]; }, r, ws.nr, nullptr, nullptr, ws.sb, ws.eb, false);
+#pragma unroll
+    for (int q = 0; q < SE; ++q) z[q] = !xwarp && r < n ? S[r + (int64_t)(c0 + part * SE + q) * n] : zero2();
+    const int emax = together(z);
+    if (!xwarp && r < n) slice_part(z, part, emax, r, ws.nr, nullptr, nullptr, ws.sb, ws.eb, false);
     return;
   }
-  extern __shared__ __align__(1024) uint8_t smem[];
   __shared__ __align__(8) uint64_t s_bar;
   __shared__ uint32_t tmem_slot;
   __shared__ int s_ex[NB];
@@ -578,7 +569,7 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar));
     asm volatile("fence.mbarrier_init.release.cluster;");
   }
-  if (warp == 4) {
+  if (warp == SV_ROW_WARPS) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
                  "r"(SV_COLS));
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
@@ -587,29 +578,45 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
   const bool conj_in = !rows;
   double2* src = rows ? (MODE == 1 ? S : H) + r + (int64_t)c0 * n : H + c0 + (int64_t)r * n;
   const int64_t step = rows ? n : 1;
-  int er = 0;
-  if (warp < 4) {
-    auto in = [&](int k) {
-      if (r >= n || k >= w || (MODE == 2 && k > r - c0)) return zero2();   // above the diagonal: not updated, not needed
-      double2 z = src[k * step];
-      if (conj_in) z.y = flip_sign(z.y);
-      return z;
-    };
-    slice_row_to(in, tid, reinterpret_cast<uint16_t*>(smem), A_BYTES / 2, 0, er);
-  } else {
-    const double2* X = ws.li + (int64_t)(c0 / NB) * NB * NB + lane * NB;
-    int ex = 0;
-    // slice s: rows 0 .. 31 form B, rows 32 .. 63 form B'
-    slice_row_to([&](int k) { return X[k]; }, lane, reinterpret_cast<uint16_t*>(smem + SLICES * A_BYTES), X_BYTES / 2,
-                 NB, ex);
-    s_ex[lane] = ex;
+  const double2* X = ws.li + (int64_t)(c0 / NB) * NB * NB + lane * NB;
+#pragma unroll
+  for (int q = 0; q < SE; ++q) {
+    const int k = part * SE + q;
+    z[q] = zero2();
+    if (xwarp) {
+      z[q] = X[k];
+    } else if (r < n && k < w && !(MODE == 2 && k > r - c0)) {      // above the diagonal: not updated, not needed
+      z[q] = src[k * step];
+      if (conj_in) z[q].y = flip_sign(z[q].y);
+    }
+  }
+  int er;
+  {
+    const int emax = together(z);
+    er = emax == 0x7ff ? EXP_NAN : emax - 1022;
+    if (xwarp && part == 0) s_ex[row] = er;
+    // slice s of X: rows 0 .. 31 form B, rows 32 .. 63 form B'
+    uint16_t* dst = reinterpret_cast<uint16_t*>(smem + (xwarp ? SLICES * A_BYTES : 0));
+    const int slice_el = (xwarp ? X_BYTES : A_BYTES) / 2;
+#pragma unroll
+    for (int im = 0; im < 2; ++im) {
+      uint4 v[SLICES];
+      slice_block([&](int k) { return z[k & (SE - 1)]; }, 4 * im, emax, v);
+      const int kb = part + 4 * im;
+#pragma unroll
+      for (int s = 0; s < SLICES; ++s) {
+        uint16_t* D = dst + (int64_t)s * slice_el;
+        *reinterpret_cast<uint4*>(D + tc_idx(row, kb * 8)) = v[s];
+        if (xwarp) *reinterpret_cast<uint4*>(D + tc_idx(row + NB, (kb ^ 4) * 8)) = im ? neg4(v[s]) : v[s];
+      }
+    }
   }
   asm volatile("fence.proxy.async.shared::cta;" ::: "memory");    // the products read what the threads wrote
   asm volatile("tcgen05.fence::before_thread_sync;");
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
   const uint32_t tmem = tmem_slot;
-  if (tid == 128) {
+  if (tid == 32 * SV_ROW_WARPS) {
     for (int s = 0; s < SLICES; ++s) {
       // column slices 0 .. SLICES - 1 - s side by side give levels s .. SLICES - 1; at most 256 columns a product
       for (int t0 = 0; t0 < SLICES - s; t0 += 4) {
@@ -626,15 +633,18 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
   if (!upd_wait(bar, 0, &s_fail)) s_fail = 1;
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
-  if (!s_fail && warp < 4) {
-    const uint32_t tb = tmem + ((uint32_t)(warp * 32) << 16);
-#pragma unroll 1
-    for (int cb = 0; cb < NB; cb += 8) {
-      long long hr[8], lr[8], hi[8], li[8];
-      level_sums<8>(tb + cb, 2 * NB, hr, lr);
-      level_sums<8>(tb + NB + cb, 2 * NB, hi, li);
 #pragma unroll
-      for (int q = 0; q < 8; ++q) {
+  for (int q = 0; q < SE; ++q) z[q] = zero2();
+  if (!s_fail && !xwarp) {
+    const uint32_t tb = tmem + ((uint32_t)((warp & 3) * 32) << 16);
+#pragma unroll
+    for (int h = 0; h < SE; h += 4) {
+      const int cb = part * SE + h;
+      long long hr[4], lr[4], hi[4], li[4];
+      level_sums<4>(tb + cb, 2 * NB, hr, lr);
+      level_sums<4>(tb + NB + cb, 2 * NB, hi, li);
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
         const int k = cb + q, ex = s_ex[k];
         if (r < n && k < w) {
           double2 v;
@@ -643,24 +653,22 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
           } else {
             v = make_double2(round_sum28(hr[q], lr[q], er + ex - 63), round_sum28(hi[q], li[q], er + ex - 63));
           }
+          z[h + q] = v;
           if (conj_in) v.y = flip_sign(v.y);
           src[k * step] = v;
         }
       }
     }
-    if (r < n) {
-      if (rows && r >= c0 + NB)
-        slice_row([&](int k) { return src[k * step]; }, r, ws.nr, ws.sa, ws.ea, MODE == 1 ? ws.sb : nullptr, ws.eb,
-                  false);
-      if (!rows && c0 + NB < n)
-        slice_row([&](int k) { const double2 z = src[k]; return make_double2(z.x, flip_sign(z.y)); }, r, ws.nr, nullptr,
-                  nullptr, ws.sc, ws.ec, false);
-    }
   }
   asm volatile("tcgen05.fence::before_thread_sync;");
-  __syncthreads();
+  const int emax = together(z);                      // its barrier: the accumulators have been read
+  if (!s_fail && !xwarp && r < n) {
+    if (rows && r >= c0 + NB)
+      slice_part(z, part, emax, r, ws.nr, ws.sa, ws.ea, MODE == 1 ? ws.sb : nullptr, ws.eb, false);
+    if (!rows && c0 + NB < n) slice_part(z, part, emax, r, ws.nr, nullptr, nullptr, ws.sc, ws.ec, false);
+  }
   if (tid == 0 && s_fail) G.status[p] = SKN_ERR_CUDA;
-  if (warp == 4) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(SV_COLS));
+  if (warp == SV_ROW_WARPS) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(SV_COLS));
 }
 
 // ------------------------------------------------------------------ tensor-core update
@@ -879,6 +887,7 @@ struct PanelSm {
   double2 rowV[NT], rowW[NT];                    // V and W at the next pivot row
   double2 part[PW][2 * NT];                      // [W V]^H v by quarters of the chunks
   int4 tf[PW][2 * NT], qf[PW][2 * NT];           // multipliers of [W V]'s columns for a warp's chunk
+  int hm[PWR][32];
   double2 tau, scl, yrow, wrow;
   double vav, alpha;
   int triv, dead;
@@ -1513,20 +1522,26 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
     }
     __syncthreads();
   }
-  // slices of the rows below the panel: z = [V W], both operands
+  // slices of the rows below the panel: z = [V W], both operands; four warps a chunk
   if (M - w > 1) {
-    for (int ch = first; ch < nt; ch += stride) {
-      const int r = ch * 32 + lane;
-      if (r < w || r >= M) continue;
+    const int part = warp & 3;
+    for (int i = 0; rank + C * i < nt; i += NWP / 4) {
+      const int ch = rank + C * (i + (warp >> 2)), r = ch * 32 + lane;
+      const bool mine = ch < nt && r >= w && r < M;
       const double2* vw = ws.VW + (int64_t)r * 2 * NT;
-      slice_row(
-          [&](int q) {
-            const int u = q < NT ? NT + q : q - NT;
-            if ((q & (NT - 1)) >= w) return zero2();
-            const double2 z = vw[u];
-            return R ? make_double2(z.x, 0.0) : z;
-          },
-          c0 + r, ws.nr, ws.sa, ws.ea, ws.sb, ws.eb, true);
+      double2 z[SE];
+#pragma unroll
+      for (int e = 0; e < SE; ++e) {
+        const int q = part * SE + e;
+        z[e] = mine && (q & (NT - 1)) < w ? vw[q ^ NT] : zero2();
+        if (R) z[e].y = 0.0;
+      }
+      sm.hm[warp][lane] = high_word8(z);
+      __syncthreads();
+      const int* hm = &sm.hm[warp & ~3][lane];
+      const int emax = max(max(hm[0], hm[32]), max(hm[64], hm[96])) >> 20;
+      if (mine) slice_part(z, part, emax, c0 + r, ws.nr, ws.sa, ws.ea, ws.sb, ws.eb, true);
+      __syncthreads();
     }
   }
 }
