@@ -624,8 +624,8 @@ def launch_order(groups: Sequence[np.ndarray], prob_n: np.ndarray, prob_real: np
     small ones last; ties keep the given order."""
     def urgency(i):
         sel = groups[i]
-        cost = prob_n[sel].astype(np.float64) ** 3 * np.where(prob_real[sel], 1.0, 4.0)
-        return -float(cost.max()) / len(sel)
+        n = prob_n[sel].astype(np.float64)
+        return -float((n * n * n * np.where(prob_real[sel], 1.0, 4.0)).max()) / len(sel)
     return sorted(range(len(groups)), key=urgency)
 
 
@@ -958,7 +958,10 @@ class Engine:
         small_order = plan.order[~large]
         if len(small_order):
             tuning = self.tuning if self.tuning is not None else _default_tuning()
-            ns, at = np.unique(plan.prob_n[small_order], return_inverse=True)
+            sizes = plan.prob_n[small_order]
+            ns = np.unique(plan.nb)                  # of the structures: far fewer than problems
+            ns = ns[np.isin(ns, sizes)] if large.any() else ns
+            at = np.searchsorted(ns, sizes)
             names = ["auto" if vectors else tuning.shape_for(int(n)) for n in ns]
             names = [route_auto(int(n)) if x == "auto" else x for n, x in zip(ns, names)]
             kinds = list(dict.fromkeys(names))
@@ -966,8 +969,9 @@ class Engine:
             if self.real_path and plan.prob_real is not None:     # one-CTA shapes: real problems in a call of their own
                 own = np.array([isinstance(x, str) for x in kinds])
                 kind = kind + len(kinds) * (plan.prob_real[small_order] & own[kind])
-            for i in dict.fromkeys(kind.tolist()):
-                sel = small_order[kind == i]
+            members = [(i, np.flatnonzero(kind == i)) for i in range(int(kind.max()) + 1)]
+            for i, at in sorted((m for m in members if len(m[1])), key=lambda m: m[1][0]):     # by first appearance
+                sel = small_order[at]
                 sfx = kinds[i % len(kinds)]
                 sfx = "_real" + sfx if i >= len(kinds) else sfx
                 out.append((sfx, sel, len(sel), int(plan.prob_n[sel].max())))
