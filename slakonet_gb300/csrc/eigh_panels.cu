@@ -1618,7 +1618,8 @@ __global__ void __launch_bounds__(256) k_bounds(Grp G) {
   }
 }
 
-__global__ void __launch_bounds__(64) k_eig(Grp G) {
+// Bound by FP64 issue when a GPU is full of them; 16 CTAs per SM, so that 1000 problems of 128 orbitals are one round.
+__global__ void __launch_bounds__(64, 16) k_eig(Grp G) {
   const int g = blockIdx.y, p = G.prob[g];
   const int n = G.nvec[p], j = blockIdx.x * 64 + threadIdx.x;
   const int st = G.status[p];

@@ -2,7 +2,7 @@
 // off-diagonal e2, e2[i] coupling rows i and i+1), one eigenvalue per thread.
 // Shared by the one-CTA and the cluster eigensolvers.
 //
-//  1. FP32 bisection on the rounded matrix brackets eigenvalue j to ~1e-6 of
+//  1. FP32 trisection on the rounded matrix brackets eigenvalue j to ~1e-6 of
 //     the spectrum's scale (FP32 runs 64x faster than FP64 on GB300).
 //  2. The bracket is widened by a margin covering the FP32 rounding and
 //     checked with two FP64 Sturm counts (else the Gershgorin interval is used).
@@ -88,17 +88,31 @@ __device__ __forceinline__ double secant_step(double x0, double p0, int e0, doub
   return (x1 - x0) * (1.0 / (s - 1.0));
 }
 
-// FP32 count on the rounded tridiagonal (LDL^T pivots).  The bracket it gives is checked in FP64, so the quotient's
-// last bits do not matter: the two-instruction division.
-__device__ __forceinline__ int count32(const float* d, const float* e2, int n, float x, float pivmin) {
-  float q = d[0] - x;
-  int c = q < 0.0f;
+// FP32 counts at x0 < x1 on the rounded tridiagonal (LDL^T pivots).  The bracket they give is checked in FP64, so the
+// quotient's last bits do not matter: an approximate reciprocal.  A step is one chain of about 50 clocks; two chains side
+// by side cost little more than one while a partition has few warps.
+__device__ __forceinline__ float recip32(float q) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
+  return r;
+}
+__device__ __forceinline__ void count32(const float* d, const float* e2, int n, float x0, float x1, float pivmin, int& c0,
+                                        int& c1) {
+  float q0 = d[0] - x0, q1 = d[0] - x1;
+  if (fabsf(q0) < pivmin) q0 = -pivmin;              // before it is counted: a zero counted as positive and carried on as
+  if (fabsf(q1) < pivmin) q1 = -pivmin;              // negative loses an eigenvalue
+  c0 = q0 < 0.0f;
+  c1 = q1 < 0.0f;
+#pragma unroll 4
   for (int i = 1; i < n; ++i) {
-    if (fabsf(q) < pivmin) q = -pivmin;
-    q = (d[i] - x) - __fdividef(e2[i - 1], q);
-    c += q < 0.0f;
+    const float di = d[i], ei = e2[i - 1];
+    q0 = fmaf(-ei, recip32(q0), di - x0);
+    q1 = fmaf(-ei, recip32(q1), di - x1);
+    if (fabsf(q0) < pivmin) q0 = -pivmin;
+    if (fabsf(q1) < pivmin) q1 = -pivmin;
+    c0 += q0 < 0.0f;
+    c1 += q1 < 0.0f;
   }
-  return c;
 }
 
 // Bounds shared by the threads of one matrix: Gershgorin interval [lo, hi]
@@ -123,10 +137,15 @@ __device__ __forceinline__ Bounds make_bounds(double lo, double hi, double emax,
 __device__ double eigenvalue(const double* d, const double* e2, const float* d32, const float* e232, int n, int j,
                              const Bounds& B) {
   float a32 = (float)B.lo, b32 = (float)B.hi;
-  for (int it = 0; it < 40; ++it) {
-    const float mid = 0.5f * (a32 + b32);
-    if (!(mid > a32 && mid < b32)) break;
-    if (count32(d32, e232, n, mid, B.pivmin32) > j) b32 = mid; else a32 = mid;
+  const float enough = 0.25f * (float)B.margin;      // the bracket is widened by the margin anyway
+  for (int it = 0; it < 26 && b32 - a32 > enough; ++it) {
+    const float third = (b32 - a32) * (1.0f / 3.0f), x0 = a32 + third, x1 = b32 - third;
+    if (!(x0 > a32 && x1 < b32 && x0 < x1)) break;
+    int c0, c1;
+    count32(d32, e232, n, x0, x1, B.pivmin32, c0, c1);
+    if (c0 > j) b32 = x0;
+    else if (c1 > j) { a32 = x0; b32 = x1; }
+    else a32 = x1;
   }
   double a = (double)a32 - B.margin, b = (double)b32 + B.margin;
   if (a < B.lo) a = B.lo;
