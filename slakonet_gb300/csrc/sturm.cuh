@@ -26,6 +26,14 @@ __device__ __forceinline__ int sign_bit(double v) { return (int)((unsigned long 
 // Exponent field of |v| (biased), for power-of-two rescaling.
 __device__ __forceinline__ int exp_field(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff); }
 
+// v 2^s by its exponent field, so that the rescaling below, which a compiler may execute on every step, stays off the
+// FP64 pipe.  What falls below the normal range is zero; infinities and NaNs stay.
+__device__ __forceinline__ double shift_exp(double v, int s) {
+  const int h = __double2hiint(v), e = (h >> 20) & 0x7ff;
+  if (e == 0x7ff) return v;
+  return e == 0 || e + s <= 0 ? 0.0 : __hiloint2double(h + (s << 20), __double2loint(v));
+}
+
 // Number of eigenvalues below x: sign changes of the determinant sequence
 // p_i = (d_i - x) p_{i-1} - e2_{i-1} p_{i-2} (three FP64 operations per step, no
 // division).  (p, p_prev) are rescaled by exact powers of two when p's exponent
@@ -46,9 +54,8 @@ __device__ __forceinline__ int count64(const double* d, const double* e2, int n,
     p = pn;
     const int ex = exp_field(p);
     if (ex > 1023 + 480 || ex < 1023 - 480) {
-      const double f = __longlong_as_double((long long)(2046 - ex) << 52);  // 2^(1023 - ex)
-      p *= f;
-      pm *= f;
+      p = shift_exp(p, 1023 - ex);
+      pm = shift_exp(pm, 1023 - ex);
     }
   }
   return c;
@@ -71,9 +78,8 @@ __device__ __forceinline__ int count_value64(const double* d, const double* e2, 
     p = pn;
     const int ex = exp_field(p);
     if (ex > 1023 + 480 || ex < 1023 - 480) {
-      const double f = __longlong_as_double((long long)(2046 - ex) << 52);
-      p *= f;
-      pm *= f;
+      p = shift_exp(p, 1023 - ex);
+      pm = shift_exp(pm, 1023 - ex);
       e += ex - 1023;
     }
   }
