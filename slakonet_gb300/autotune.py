@@ -232,7 +232,6 @@ def tune_batch(engine, db, candidates: Optional[List[Tuning]] = None, reps: int 
     n_prob = len(plan.prob_n)
     eig = torch.empty(max(plan.eig_total, 1), dtype=torch.float64, device=dev)
     st = torch.empty(max(n_prob, 1), dtype=torch.int32, device=dev)
-    ctr = torch.zeros(2, dtype=torch.int32, device=dev)
     saved = engine.tuning
     best, best_t = None, float("inf")
     timings = []

@@ -21,8 +21,8 @@
 // slot and is added in a fixed order, or is an integer, so a problem's results depend neither on the other problems nor
 // on the number of CTAs it is given.
 // Measured (random pencils): 492 orbitals x 300 problems 393 ms with one CTA per problem, 208 with the products in FP64,
-// 114 now (tridiagonalisation 62, updates 32, solves 8, eigenvalues 6); 432 x 8 190, 18.8, 10.5 ms (6.2 of them the
-// tridiagonalisation, 15 us a column); 1152 x 2 47, 32.8 ms.
+// 112 now (tridiagonalisation 62, updates 32, solves 8, eigenvalues 4); 432 x 8 190, 18.8, 9.7 ms (5.7 of them the
+// tridiagonalisation, 13 us a column); 1152 x 2 47, 30.9 ms.
 #include <algorithm>
 #include <map>
 #include <mutex>
@@ -871,14 +871,15 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
 // in fixed point (below).  The FP64 unit belongs to one of the SM's four partitions: a warp issues one FP64 instruction
 // per 64 clocks, however independent its instructions are, so the FP64 work of a phase is spread over the warps.
 // RES: a CTA's tiles and its rows of [W V] fit its shared memory and stay there for the panel's 16 columns; eight warps
-// take a tile each.  The form for few problems, bound by the latency of a column: 29,700 clocks at 432 orbitals on
-// clusters of 12, 5,500 of them the products (20,000 in FP64), the rest two barriers, the reflector, the sums and the
-// row's update.  Else a warp takes whole tiles, streamed, and the CTAs of other problems fill the partitions: the form for
-// many, bound by the integer multiply-adds (4 to 5 clocks each and partition) and what FP64 is left.  Integer sums do not
-// depend on their order and FP64 sums keep theirs, so both forms give the same bits.
+// take a tile each, and two a chunk's row.  The form for few problems, bound by the latency of a column: 25,600 clocks at
+// 432 orbitals on clusters of 12, 5,500 of them the products (20,000 in FP64), the rest two barriers, the reflector, the
+// sums and the row's update.  Else a warp takes whole tiles, streamed, and the CTAs of other problems fill the partitions:
+// the form for many, bound by the integer multiply-adds (4 to 5 clocks each and partition) and what FP64 is left.  Integer
+// sums do not depend on their order and FP64 sums keep theirs, so both forms give the same bits.
 constexpr int PW = 4;                            // warps per CTA when streamed, one per partition
 constexpr int PWR = 8;                           // and when resident: two per partition hide each other's latency
 constexpr int PT = 32 * PW, PTR = 32 * PWR;
+static_assert(PWR * 32 * sizeof(double2) <= 2 * PW * 32 * sizeof(int4), "W's entries fit the multipliers");
 constexpr int TILE_LD = TS + 1;
 constexpr int TILE_EL = TS * TILE_LD;            // a resident tile, or a chunk's 32 columns of [W V]
 constexpr int QT = TS / PW;                      // columns or rows of a quarter; columns staged when streamed
@@ -887,7 +888,6 @@ struct PanelSm {
   double2 rowV[NT], rowW[NT];                    // V and W at the next pivot row
   double2 part[PW][2 * NT];                      // [W V]^H v by quarters of the chunks
   int4 tf[PW][2 * NT], qf[PW][2 * NT];           // multipliers of [W V]'s columns for a warp's chunk
-  int hm[PWR][32];
   double2 tau, scl, yrow, wrow;
   double vav, alpha;
   int triv, dead;
@@ -1378,7 +1378,8 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
       tm = on && !triv ? o : zero2();
       qm = on && next ? (lane < NT ? sm.rowV[c] : sm.rowW[c]) : zero2();
       if constexpr (!R) qm.y = -qm.y;
-      if (!triv && warp == 0) {                            // the pivot row's tau (y - V t1 - W t2)
+      // resident, by the warps that have no corrections to sum
+      if (!triv && warp == (RES ? PWR - 1 : 0)) {          // the pivot row's tau (y - V t1 - W t2)
         double2 c = zero2();
         if (lane < j) {
           c = mul<R>(sm.rowV[lane], s);
@@ -1389,7 +1390,7 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
           if constexpr (!R) c.y += __shfl_xor_sync(0xffffffffu, c.y, q);
         }
         if (lane == 0) sm.wrow = mul<R>(tau, make_double2(sm.yrow.x - c.x, R ? 0.0 : sm.yrow.y - c.y));
-      } else if (!triv && warp == 1) {                     // alpha, with Re sum_q conj(t1_q) t2_q
+      } else if (!triv && warp == (RES ? PWR - 2 : 1)) {   // alpha, with Re sum_q conj(t1_q) t2_q
         double dot = lane < j ? (R ? s.x * o.x : fma(s.x, o.x, s.y * o.y)) : 0.0;
         for (int q = 8; q > 0; q >>= 1) dot += __shfl_xor_sync(0xffffffffu, dot, q);
         const double t2 = R ? tau.x * tau.x : fma(tau.x, tau.x, tau.y * tau.y);
@@ -1438,44 +1439,58 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
       }
       return y;
     };
-    // the row's entry of W's column j and of the next column, from the sums
-    auto finish = [&](int ch, double2 y, const Dot<R>& dy, int kt, const Dot<R>& da, int kq) {
+    // the row's entry of W's column j, from the sums
+    auto w_entry = [&](int ch, double2 y, const Dot<R>& dy, int kt) {
       const int r = ch * 32 + lane;
       const double al = triv ? 0.0 : sm.alpha;
-      const double2 wrow = triv ? zero2() : make_double2(sm.wrow.x + al, sm.wrow.y);
-      double2 wv = zero2(), a = zero2();
+      double2 wv = zero2();
+      if (r > j && r < M && !triv) {
+        const double2 v = sv[r], d = dy.value(kt);
+        y = make_double2(y.x - d.x, R ? 0.0 : y.y - d.y);
+        wv = mul<R>(tau, y);
+        wv.x = fma(al, v.x, wv.x);
+        if constexpr (!R) wv.y = fma(al, v.y, wv.y);
+      }
+      return wv;
+    };
+    auto put_w = [&](int ch, double2 wv) {
+      const int r = ch * 32 + lane;
       if (r > j && r < M) {
-        const double2 v = sv[r];
-        if (!triv) {
-          const double2 d = dy.value(kt);
-          y = make_double2(y.x - d.x, R ? 0.0 : y.y - d.y);
-          wv = mul<R>(tau, y);
-          wv.x = fma(al, v.x, wv.x);
-          if constexpr (!R) wv.y = fma(al, v.y, wv.y);
-        }
         st<R>(W + (int64_t)j * n + c0 + r, wv);
         st<R>(ws.VW + (int64_t)r * 2 * NT + j, wv);
-        if (next) {
-          const double2 d = da.value(kq);
-          a = ld<R>(A + r + (int64_t)(j + 1) * n);
-          a = make_double2(a.x - d.x, R ? 0.0 : a.y - d.y);
-          a = fms_cj<R>(v, wrow, a);
-          a.x -= wv.x;                                     // V at the pivot row is 1
-          if constexpr (!R) a.y -= wv.y;
-          if (r == j + 1) {
-            a.y = 0.0;
-            ws.d[k + 1] = a.x;
-          }
-          st<R>(ws.xc + r, a);
-        }
       }
       const int emax = __reduce_max_sync(0xffffffffu, high_word<R>(wv)) >> 20;
       put_fixed(ch, j, fixed_point<R>(wv, emax), emax);
-      if (next) {
-        double s = r >= j + 3 && r < M ? (R ? a.x * a.x : fma(a.x, a.x, a.y * a.y)) : 0.0;
-        s = warp_sum<true>(make_double2(s, 0.0)).x;
-        if (lane == 0) ws.sN[ch] = s;
+    };
+    // the next column's entry but for W's column j, and with it
+    auto a_entry = [&](int ch, const Dot<R>& da, int kq) {
+      const int r = ch * 32 + lane;
+      const double al = triv ? 0.0 : sm.alpha;
+      const double2 wrow = triv ? zero2() : make_double2(sm.wrow.x + al, sm.wrow.y);
+      double2 a = zero2();
+      if (r > j && r < M && next) {
+        const double2 d = da.value(kq);
+        a = ld<R>(A + r + (int64_t)(j + 1) * n);
+        a = make_double2(a.x - d.x, R ? 0.0 : a.y - d.y);
+        a = fms_cj<R>(sv[r], wrow, a);
       }
+      return a;
+    };
+    auto put_a = [&](int ch, double2 a, double2 wv) {
+      const int r = ch * 32 + lane;
+      if (!next) return;
+      if (r > j && r < M) {
+        a.x -= wv.x;                                       // V at the pivot row is 1
+        if constexpr (!R) a.y -= wv.y;
+        if (r == j + 1) {
+          a.y = 0.0;
+          ws.d[k + 1] = a.x;
+        }
+        st<R>(ws.xc + r, a);
+      }
+      double s = r >= j + 3 && r < M ? (R ? a.x * a.x : fma(a.x, a.x, a.y * a.y)) : 0.0;
+      s = warp_sum<true>(make_double2(s, 0.0)).x;
+      if (lane == 0) ws.sN[ch] = s;
     };
     if constexpr (RES) {
       for (int ch = rank, i = 0; ch < nt; ch += C, ++i) {
@@ -1495,18 +1510,33 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
         }
       }
       __syncthreads();
-      for (int ch = first, i = warp; ch < nt; ch += stride, i += NWP) {
+      // two warps a chunk: W's column, and the next column
+      for (int i0 = 0; rank + C * i0 < nt; i0 += NWP / 2) {
+        const int i = i0 + (warp >> 1), ch = rank + C * i;
+        const bool have = ch < nt;
+        // W's entries for the other warp, in turn, where the multipliers were
+        double2* wx = reinterpret_cast<double2*>(sm.tf) + ((i0 / (NWP / 2) & 1) * (NWP / 2) + (warp >> 1)) * 32;
         const char* e = eps + (int64_t)i * EPS;
-        const double2* y = reinterpret_cast<const double2*>(e) + lane;
-        Dot<R> dy, da;
-#pragma unroll
-        for (int q = 0; q < PW; ++q) {
-          const long long* d = reinterpret_cast<const long long*>(e + PW * 16 * TS) + q * 8 * TS + lane;
-          dy.take(d, TS);
-          da.take(d + 4 * TS, TS);
-        }
         const int* ke = wve + i * (2 * NT + 2) + 2 * NT;
-        finish(ch, sum4<R>(y[0], y[TS], y[2 * TS], y[3 * TS]), dy, ke[0], da, ke[1]);
+        const long long* d = reinterpret_cast<const long long*>(e + PW * 16 * TS) + (warp & 1) * 4 * TS + lane;
+        double2 x = zero2();
+        if (have) {
+          Dot<R> z;
+#pragma unroll
+          for (int q = 0; q < PW; ++q) z.take(d + q * 8 * TS, TS);
+          if ((warp & 1) == 0) {
+            const double2* y = reinterpret_cast<const double2*>(e) + lane;
+            x = w_entry(ch, sum4<R>(y[0], y[TS], y[2 * TS], y[3 * TS]), z, ke[0]);
+            wx[lane] = x;
+          } else {
+            x = a_entry(ch, z, ke[1]);
+          }
+        }
+        __syncthreads();
+        if (have) {
+          if ((warp & 1) == 0) put_w(ch, x);
+          else put_a(ch, x, wx[lane]);
+        }
       }
     } else {
       __syncthreads();
@@ -1516,7 +1546,9 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
         multipliers(ch, kt, kq);
         corrections(ch, 0, 1, dy, da);
         const double2 y = sum4<R>(slots(ch, 0), slots(ch, 1), slots(ch, 2), slots(ch, 3));
-        finish(ch, y, dy, kt, da, kq);
+        const double2 wv = w_entry(ch, y, dy, kt), a = a_entry(ch, da, kq);
+        put_w(ch, wv);
+        put_a(ch, a, wv);
         __syncwarp();
       }
     }
@@ -1525,6 +1557,7 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
   // slices of the rows below the panel: z = [V W], both operands; four warps a chunk
   if (M - w > 1) {
     const int part = warp & 3;
+    int* hms = reinterpret_cast<int*>(sm.part);             // a warp's 32 high words
     for (int i = 0; rank + C * i < nt; i += NWP / 4) {
       const int ch = rank + C * (i + (warp >> 2)), r = ch * 32 + lane;
       const bool mine = ch < nt && r >= w && r < M;
@@ -1536,9 +1569,9 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
         z[e] = mine && (q & (NT - 1)) < w ? vw[q ^ NT] : zero2();
         if (R) z[e].y = 0.0;
       }
-      sm.hm[warp][lane] = high_word8(z);
+      hms[warp * 32 + lane] = high_word8(z);
       __syncthreads();
-      const int* hm = &sm.hm[warp & ~3][lane];
+      const int* hm = hms + (warp & ~3) * 32 + lane;
       const int emax = max(max(hm[0], hm[32]), max(hm[64], hm[96])) >> 20;
       if (mine) slice_part(z, part, emax, c0 + r, ws.nr, ws.sa, ws.ea, ws.sb, ws.eb, true);
       __syncthreads();

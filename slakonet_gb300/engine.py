@@ -568,15 +568,15 @@ SMALL_CLASSES = (16, 24, 32, 40, 48, 56, 64)     # its calls' size classes: shar
 
 
 def route_auto(n: int):
-    """Kernel and call of a problem of n orbitals under the untuned policy: ("small", class) or ("panels", panel
-    count).  A rule on the problem alone, as route_wide.  Measured on GB300, panels against the small kernel:
-    88 orbitals x 500 problems 6.2 ms (9.6), 80 x 50 1.9 (1.9), 72 x 500 5.0 (5.9), 72 x 8 1.7 (1.5), 64 x 4000 23
-    (19): the line is at 64.  Against the one-CTA kernel: 128 x 1000 19.6 ms (31), 160 x 27 3.8 (12.6), 432 x 8 11.6
-    (190), 492 x 300 130 (393).  One panel call per panel count, each on its stream: the 600 problems of 57 to 492
-    orbitals of a mixed batch took 284 ms so and 297 ms as one call that drops the smaller ones on the way."""
+    """Kernel and call of a problem of n orbitals under the untuned policy: ("small", class) or ("panels", class of
+    64 orbitals).  A rule on the problem alone, as route_wide.  Measured on GB300, panels against the small kernel:
+    88 orbitals x 500 problems 5.2 ms (9.6), 80 x 50 1.5 (1.9), 72 x 8 1.4 (1.5), 64 x 8 1.16 (1.09), 64 x 4000 18.9
+    (17.4): the line is at 64.  Against the one-CTA kernel: 128 x 1000 16.3 ms (31), 160 x 27 3.2 (12.3), 432 x 8 9.6
+    (187), 492 x 300 112 (389).  One panel call per class, each on its stream: the 600 problems of 65 to 534 orbitals
+    of a mixed batch take 156 ms so, 160 with classes of 32, 157 of 128, and took 4% longer as one call."""
     if n <= SMALL_MAX_N:
         return ("small", next(c for c in SMALL_CLASSES if n <= c))
-    return ("panels", -(-n // PANEL))
+    return ("panels", -(-n // (2 * PANEL)))
 
 
 _SIDE = threading.local()   # per-thread side streams of Engine._side_streams
@@ -930,7 +930,7 @@ class Engine:
 
     def _groups(self, db, vectors: bool = False):
         """[(launch shape suffix, the cluster size for the cluster path, ("wide", n, real) for the device-wide
-        path, or route_auto's ("small", class) or ("panels", panel count), device order, count, max_n)], cached on the batch.
+        path, or route_auto's ("small", class) or ("panels", class), device order, count, max_n)], cached on the batch.
 
         Empty when every problem takes the default single-CTA launch.  With ``vectors`` every problem takes route_auto's
         kernel: the others keep no reflectors."""
