@@ -98,9 +98,13 @@ __device__ __forceinline__ double secant_step(double x0, double p0, int e0, doub
 // quotient's last bits do not matter: an approximate reciprocal.  A step is one chain of about 50 clocks; two chains side
 // by side cost little more than one while a partition has few warps.
 __device__ __forceinline__ float recip32(float q) {
+#ifdef __CUDA_ARCH__
   float r;
   asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(q));
   return r;
+#else
+  return 1.0f / q;
+#endif
 }
 __device__ __forceinline__ void count32(const float* d, const float* e2, int n, float x0, float x1, float pivmin, int& c0,
                                         int& c1) {
@@ -167,6 +171,10 @@ __device__ double eigenvalue(const double* d, const double* e2, const float* d32
     // eigenvalue j alone in (a, b]: safeguarded secant from the bracket's ends.  A step that leaves the
     // bracket, or is not at least halving the previous step, is replaced by bisection, so the bracket keeps
     // shrinking.
+    // A line through the ends can point at an eigenvalue outside, when an end all but touches it: p is then as good as
+    // zero there, its step vanishes and would pass for convergence.  The bracket leaves its own eigenvalue well inside, so
+    // that shows as ends of very different size, and such an eigenvalue is taken only where the counts change.
+    const bool plain = abs((exp_field(p0) + e0) - (exp_field(p1) + e1)) <= 6;
     double x1 = b, xn = b + secant_step(a, p0, e0, b, p1, e1);
     double dx_old = b - a;
     for (int it = 0; it < 16; ++it) {
@@ -184,7 +192,10 @@ __device__ double eigenvalue(const double* d, const double* e2, const float* d32
       xn = x + step;
       // converged: the last step may land on the bracket's edge (the root lies within rounding of
       // the point just counted), so it is tested before the bracket, not after
-      if (fabs(step) <= B.atol && xn >= a && xn <= b) return xn;
+      if (fabs(step) <= B.atol && xn >= a && xn <= b) {
+        if (plain || (count64(d, e2, n, xn - 2.0 * B.atol) <= j && count64(d, e2, n, xn + 2.0 * B.atol) > j)) return xn;
+        xn = a - 1.0;                                // bisect
+      }
       if (xn > a && xn < b && fabs(step) <= 0.5 * dx_old) {
         dx_old = fabs(step);
       } else {
