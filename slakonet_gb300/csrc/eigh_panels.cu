@@ -1554,9 +1554,14 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
     }
     __syncthreads();
   }
-  // slices of the rows below the panel: z = [V W], both operands; four warps a chunk
+  // slices of the rows below the panel: z = [V W], both operands; four warps a chunk.  A row has one exponent, and V's
+  // entries are at most 1 while W's have the matrix's scale: V 2^k and W 2^-k meet halfway, and V W^H is the same.
   if (M - w > 1) {
     const int part = warp & 3;
+    int em = 0;
+    for (int t = lane; t < ntile; t += 32) em = max(em, ws.fe[t]);
+    em = __reduce_max_sync(0xffffffffu, em);
+    const int half = em == 0x7ff ? 0 : (em - 1022) / 2;
     int* hms = reinterpret_cast<int*>(sm.part);             // a warp's 32 high words
     for (int i = 0; rank + C * i < nt; i += NWP / 4) {
       const int ch = rank + C * (i + (warp >> 2)), r = ch * 32 + lane;
@@ -1566,8 +1571,9 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
 #pragma unroll
       for (int e = 0; e < SE; ++e) {
         const int q = part * SE + e;
+        const int k = q < NT ? half : -half;
         z[e] = mine && (q & (NT - 1)) < w ? vw[q ^ NT] : zero2();
-        if (R) z[e].y = 0.0;
+        z[e] = make_double2(skn_sturm::shift_exp(z[e].x, k), R ? 0.0 : skn_sturm::shift_exp(z[e].y, k));
       }
       hms[warp * 32 + lane] = high_word8(z);
       __syncthreads();

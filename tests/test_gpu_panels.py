@@ -140,3 +140,27 @@ def test_indefinite_overlap_and_zero_rows_and_other_sizes():
             h[40, 40] = s[40, 40] = 1.0
         r = sla.eigh(h, s, eigvals_only=True)
         assert np.abs(got[i] - r).max() <= _bound(sizes[i], r)
+
+
+def check_scaled_and_graded(n, solve):
+    """Powers of two scale exactly, so a scaled pencil's eigenvalues have the plain one's relative error (its vectors have
+    the matrix's scale beside entries of at most 1); a graded matrix has eigenvalues far below its norm, each within the
+    norm's backward error."""
+    Hs, Ss = _pairs((n,), seed=1)
+    h, s = Hs[0], Ss[0]
+    r = sla.eigh(h, s, eigvals_only=True)
+    for a, b in ((1.0, 1.0), (2.0 ** 40, 1.0), (2.0 ** -37, 1.0), (2.0 ** 300, 1.0), (1.0, 2.0 ** 100), (2.0 ** -90, 2.0 ** 90)):
+        assert np.abs(solve(h * a, s * b) * (b / a) - r).max() <= _bound(n, r), (a, b)
+    d = np.logspace(0, -6, n)
+    g = d[:, None] * h * d[None]
+    r = sla.eigh(g, s, eigvals_only=True)
+    assert np.abs(solve(g, s) - r).max() <= _bound(n, r)
+
+
+@pytest.mark.parametrize("n", [100, 200, 500])
+def test_scaled_and_graded_pencils(n):
+    check_scaled_and_graded(n, lambda h, s: _panels([h], [s])[0][0])
+
+
+def test_scaled_and_graded_pencils_on_the_one_cta_kernel():
+    check_scaled_and_graded(100, lambda h, s: _one_cta([h], [s])[0])

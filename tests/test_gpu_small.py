@@ -8,7 +8,7 @@ import scipy.linalg as sla
 import torch
 
 from slakonet_gb300._lib import call, ptr
-from test_gpu_panels import _bound, _pairs, _setup
+from test_gpu_panels import _bound, _pairs, _setup, check_scaled_and_graded
 
 pytestmark = pytest.mark.gpu
 DEV = "cuda:0"
@@ -67,3 +67,8 @@ def test_results_do_not_depend_on_the_call():
     for i in range(4):
         alone, st = _small([Hs[i]], [Ss[i]])
         assert st[0] == 0 and np.array_equal(alone[0], together[i])
+
+
+@pytest.mark.parametrize("n", [40, 96])
+def test_scaled_and_graded_pencils(n):
+    check_scaled_and_graded(n, lambda h, s: _small([h], [s])[0][0])
