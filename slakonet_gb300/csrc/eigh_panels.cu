@@ -21,9 +21,10 @@
 // slot and is added in a fixed order, or is an integer, so a problem's results depend neither on the other problems nor
 // on the number of CTAs it is given.
 // Measured (random pencils): 492 orbitals x 300 problems 393 ms with one CTA per problem, 208 with the products in FP64,
-// 112 now (tridiagonalisation 62, updates 32, solves 8, eigenvalues 4); 432 x 8 190, 18.8, 9.7 ms (5.7 of them the
+// 98 now (tridiagonalisation 48, updates 32, solves 8, eigenvalues 4); 432 x 8 190, 18.8, 9.8 ms (5.8 of them the
 // tridiagonalisation, 13 us a column); 1152 x 2 47, 30.9 ms.
 #include <algorithm>
+#include <array>
 #include <map>
 #include <mutex>
 #include <utility>
@@ -874,7 +875,8 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
 // take a tile each, and two a chunk's row.  The form for few problems, bound by the latency of a column: 25,600 clocks at
 // 432 orbitals on clusters of 12, 5,500 of them the products (20,000 in FP64), the rest two barriers, the reflector, the
 // sums and the row's update.  Else a warp takes whole tiles, streamed, and the CTAs of other problems fill the partitions:
-// the form for many, bound by the integer multiply-adds (4 to 5 clocks each and partition) and what FP64 is left.  Integer
+// the form for many, bound by latency too (at 320 x 152 a scheduler issues on 23% of its cycles, its waits split between
+// barriers, loads and fixed latencies; the integer pipe is busy 23%, FP64 14%), so residency and even rounds count.  Integer
 // sums do not depend on their order and FP64 sums keep theirs, so both forms give the same bits.
 constexpr int PW = 4;                            // warps per CTA when streamed, one per partition
 constexpr int PWR = 8;                           // and when resident: two per partition hide each other's latency
@@ -1690,29 +1692,31 @@ inline int pow2_below(int v, int most) {
   return c;
 }
 
-// Clusters of C CTAs that the GPU holds at once, one CTA per SM: a cluster stays within one of its processor clusters,
-// which are not all of 16 SMs or more (GB300: 7 of 16, 8 of 12, 15 of 8).
-int clusters_at_once(int C, int sms) {
+// Clusters of C CTAs of either form that the GPU holds at once, per_sm CTAs to an SM: a cluster stays within one of its
+// processor clusters, which are not all of 16 SMs or more (GB300, resident: 7 of 16, 8 of 12, 15 of 8).
+int clusters_at_once(bool resident, int C, int per_sm, int sms) {
   static std::mutex lock;
-  static std::map<std::pair<int, int>, int> known;
+  static std::map<std::array<int, 4>, int> known;
   int dev = 0;
   cudaGetDevice(&dev);
   std::lock_guard<std::mutex> hold(lock);
-  int& n = known[{dev, C}];
+  int& n = known[{dev, (int)resident, C, per_sm}];
   if (n == 0) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)C * sms);
-    cfg.blockDim = dim3(PTR);
-    cfg.dynamicSmemBytes = SMEM_MAX - 2048;
+    cfg.blockDim = dim3(resident ? PTR : PT);
+    cfg.dynamicSmemBytes = SMEM_MAX / per_sm - 2048;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = C;
     at[0].val.clusterDim.y = at[0].val.clusterDim.z = 1;
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&n, k_tri_panel<true>, &cfg) != cudaSuccess || n < 1) {
+    const cudaError_t e = resident ? cudaOccupancyMaxActiveClusters(&n, k_tri_panel<true>, &cfg)
+                                   : cudaOccupancyMaxActiveClusters(&n, k_tri_panel<false>, &cfg);
+    if (e != cudaSuccess || n < 1) {
       cudaGetLastError();
-      n = sms / (2 * C) > 1 ? sms / (2 * C) : 1;
+      n = std::max(1, sms * per_sm / (2 * C));
     }
   }
   return n;
@@ -1720,19 +1724,35 @@ int clusters_at_once(int C, int sms) {
 
 // CTAs per problem over m rows, and the tiles of each when they are resident (0: streamed).  Resident: one CTA per SM,
 // up to one per tile, if shared memory holds its part and all problems run at once.  A cluster's barrier takes about 1200
-// clocks, a counter's 5000, so a grid team only from GRID_FROM CTAs.  Streamed: STREAM_PER_SM CTAs for each SM (four are
-// resident; the rest wait) even out the mixed batch's calls, which run beside one another: 204 ms at 4, 196 at 10.
+// clocks, a counter's 5000, so a grid team only from GRID_FROM CTAs.  Streamed, with the GPU to itself: the size whose
+// rounds are the shortest, as a problem's time falls with its CTAs and a round that is nearly empty costs as much as a full
+// one (492 orbitals x 300 problems 98 ms, with 10 CTAs for each SM 111; 320 x 456 54 and 56).  Beside other calls there are
+// no rounds, and STREAM_PER_SM CTAs for each SM of its part (four are resident; the rest wait) even the calls out: the mixed
+// batch takes 157 ms so, 165 at 5 and 162 by rounds.
 constexpr int GRID_FROM = 24, STREAM_PER_SM = 10;
 void plan_panel(int m, int n_prob, int sms, int all, int& C, int& rt) {
   const int nt = cdiv(m, TS), tiles = nt * (nt + 1) / 2;
   const int most = std::min(tiles, std::max(1, sms / n_prob));
   C = most;
   if (most < GRID_FROM)
-    for (C = std::min(most, 16); C > 1 && clusters_at_once(C, all) < n_prob;) --C;
+    for (C = std::min(most, 16); C > 1 && clusters_at_once(true, C, 1, all) < n_prob;) --C;
   rt = cdiv(tiles, C);
   if ((int64_t)n_prob * C <= all && panel_smem(m, rt, cdiv(nt, C)) <= SMEM_MAX) return;
   rt = 0;
-  C = pow2_below(std::min(std::max(1, STREAM_PER_SM * sms / n_prob), std::max(1, tiles / (2 * PW))), 16);
+  if (sms < all) {
+    C = pow2_below(std::min(std::max(1, STREAM_PER_SM * sms / n_prob), std::max(1, tiles / (2 * PW))), 16);
+    return;
+  }
+  const int per_sm = std::max(1, std::min(4, (int)(SMEM_MAX / (panel_smem(m, 0, 0) + 1024))));
+  double best = 0.0;
+  for (int c = 1; c <= 16 && c <= std::max(1, tiles / (2 * PW)); c *= 2) {
+    const int rounds = cdiv(n_prob, clusters_at_once(false, c, per_sm, all));
+    const double cost = (double)rounds / c * (1.0 + 0.05 * (c > 1) + 0.03 * (c > 2) + 0.03 * (c > 4) + 0.03 * (c > 8));
+    if (c == 1 || cost < best) {
+      best = cost;
+      C = c;
+    }
+  }
 }
 
 cudaError_t launch_panel(const Grp& G, int count, int c0, int sms, int all, cudaStream_t stream) {

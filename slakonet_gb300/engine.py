@@ -572,7 +572,7 @@ def route_auto(n: int):
     64 orbitals).  A rule on the problem alone, as route_wide.  Measured on GB300, panels against the small kernel:
     88 orbitals x 500 problems 5.2 ms (9.6), 80 x 50 1.5 (1.9), 72 x 8 1.4 (1.5), 64 x 8 1.16 (1.09), 64 x 4000 18.9
     (17.4): the line is at 64.  Against the one-CTA kernel: 128 x 1000 16.3 ms (31), 160 x 27 3.2 (12.3), 432 x 8 9.6
-    (187), 492 x 300 112 (389).  One panel call per class, each on its stream: the 600 problems of 65 to 534 orbitals
+    (187), 492 x 300 98 (389).  One panel call per class, each on its stream: the 600 problems of 65 to 534 orbitals
     of a mixed batch take 156 ms so, 160 with classes of 32, 157 of 128, and took 4% longer as one call."""
     if n <= SMALL_MAX_N:
         return ("small", next(c for c in SMALL_CLASSES if n <= c))
