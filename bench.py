@@ -43,7 +43,7 @@ DOS_POINTS = 1000
 DOS_SIGMA = 0.1
 DOS_WINDOW = 9.0
 SAMPLE_STRIDE = 16         # CPU baseline: every 16th structure (stratified over sizes)
-# DRAM bytes (read + write) of the eigensolver launches of one execution, measured by ncu on two
+# DRAM bytes (read + write) of the one-CTA eigensolver's launches of one execution, measured by ncu on two
 # stratified samples of the default workload (profiles/k_eigh_gen_uneven_samples_dram.md):
 # `ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
 #  -k regex:k_eigh_gen -s 4 -c 4 python bench.py --path-only --sample-stride K --steps 1 --warmup 1`.
@@ -498,7 +498,7 @@ def run_gpu(args, rank, world):
         st_h = r.stats.cpu()
         e2e_times.append(time.perf_counter() - t)
         d2h = int(eig_h.numel() * 8 + dos_h.numel() * 8 + st_h.numel() * 8 + 4 * plan.n_pairs)
-        h2d = E.DeviceBatch(r.plan, dev).h2d_bytes() + 8 * (2 * plan.n_pairs + 1)
+        h2d = E.DeviceBatch(r.plan, dev).h2d_bytes() + 16 * (plan.n_pairs + 1)
     e2e = sum(e2e_times)
     e2e = max_over_ranks(e2e, world, dev)
 
@@ -531,13 +531,18 @@ def run_gpu(args, rank, world):
                             f"{1e3 * elapsed_u / args.steps:.1f} ms",
                    "autotune_s": round(t_tune, 1),
                    "autotune_batch_trials_ms": tuning.timings.get("batch_trials_ms")},
-        "roofline": {"bound": "tensor", "kernel": "k_eigh_gen (skn_eigh_gen_batched, autotuned launch shapes)",
+        "roofline": {"bound": "tensor", "kernel": "the eigensolver's launches: k_tri_panel, k_update, k_solve and the others of "
+                                                 "skn_eigh_gen_panels, k_eigh_small (or, where the autotuner prefers it, "
+                                                 "k_eigh_gen)",
+                     "note": "achieved counts the algorithm's real flops; only part of them run on the FP64 unit, the "
+                             "updates and solves are bf16 slice products and the matrix-vector products integer ones, so "
+                             "the fraction of the FP64 rate may exceed 1",
                      "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
                      "traffic": None,
                      "traffic_note": "not captured on the full batch (the capture-size rule); measured on two "
-                                     "stratified samples, see traffic_samples: DRAM bytes per execution of the "
-                                     "eigensolver launches against their H(k)+S(k) bytes. The kernel is FP64-bound: "
-                                     "its DRAM rate in the larger sample is about 1% of HBM",
+                                     "stratified samples with the one-CTA kernel, see traffic_samples: DRAM bytes per "
+                                     "execution of its launches against their H(k)+S(k) bytes, about 1% of HBM's rate "
+                                     "in the larger sample",
                      "traffic_samples": {k: dict(v, ratio=round(v["dram_bytes"] / v["hs_bytes"], 2),
                                                  dram_gbs=round(v["dram_bytes"] / v["ncu_ms"] / 1e6, 1))
                                          for k, v in EIG_TRAFFIC_SAMPLES.items()},
