@@ -27,7 +27,8 @@ constexpr double H2E = 27.211;
 // the tiles on and below the diagonal are summed and the others mirrored; bands of zero weight (outside the DOS
 // window's reach, sorted to the ends) are passed over 16 at a time; the tiles of a problem go to gridDim.y CTAs, each
 // thread with 2 x 2 entries so that a shared-memory read feeds two of them.  One CTA per problem with one entry per
-// thread over the full square took 8.4 ms for the 484 problems of 30 to 116 orbitals of a training step.
+// thread over the full square took 8.4 ms for the 484 problems of 30 to 116 orbitals of a training step, 2.8 now (1.5 at
+// the FP64 rate).
 constexpr int AT = 32, AJ = 16;
 __global__ void __launch_bounds__(256) k_adj_projectors(int n_prob, const int32_t* __restrict__ nvec,
                                                         const int64_t* __restrict__ hs_off,

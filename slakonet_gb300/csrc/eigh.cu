@@ -6,7 +6,7 @@
 //      her2, axpy, triangular solve per column),
 //   3. Householder tridiagonalisation of C (zhetd2: larfg, hemv, her2),
 //   4. eigenvalues of the real tridiagonal from Sturm counts (FP32 bracket,
-//      then FP64 Newton on the characteristic polynomial for isolated
+//      then FP64 secant steps on the characteristic polynomial for isolated
 //      eigenvalues, FP64 bisection for clusters), one thread per eigenvalue,
 //      which returns them in ascending order.
 // The reference runs torch.linalg.cholesky / solve / matmul / eigh per k
@@ -77,14 +77,6 @@ struct Vecs {
   float* e232;     // n: FP32 copy of e^2
 };
 
-// c - conj(a) * b
-__device__ __forceinline__ double2 cfms_conj_l(double2 a, double2 b, double2 c) {
-  c.x = fma(-a.x, b.x, c.x);
-  c.x = fma(-a.y, b.y, c.x);
-  c.y = fma(-a.x, b.y, c.y);
-  c.y = fma(a.y, b.x, c.y);
-  return c;
-}
 
 // Arithmetic on complex entries, or on their real parts alone when the problem
 // is real (R = true: every imaginary part of H and S is exactly zero, as at
@@ -716,7 +708,7 @@ __device__ void hetd2_lower(double2* __restrict__ A, int lda, int n, Vecs& V, do
 }
 
 // ------------------------------------------------------- tridiagonal eigenvalues
-// One thread per eigenvalue (csrc/sturm.cuh: FP32 bracket, FP64 Newton for
+// One thread per eigenvalue (csrc/sturm.cuh: FP32 bracket, FP64 secant for
 // isolated eigenvalues, FP64 bisection for clusters).  The Gershgorin bounds
 // are reduced over the CTA first.
 __device__ void tridiag_eigenvalues(int n, Vecs& V, double* out) {

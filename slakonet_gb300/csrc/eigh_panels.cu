@@ -42,7 +42,6 @@ namespace cg = cooperative_groups;
 
 constexpr int NB = 32;               // panel width of the factorisations
 constexpr int NT = 16;               // columns per tridiagonalisation panel
-constexpr int LDT = NB + 1;
 constexpr int TS = 32;               // tile edge of the matrix-vector products
 constexpr int SLICES = 8;
 constexpr int KP = 64;               // inner dimension of the sliced products (32 complex columns)
@@ -449,31 +448,23 @@ SKN_DEVINL void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t idesc, 
 SKN_DEVINL void tc_commit(uint32_t bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar));
 }
-SKN_DEVINL void tmem_ld8(uint32_t a, uint32_t* v) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
-               : "r"(a));
-}
 SKN_DEVINL void tmem_ld4(uint32_t a, uint32_t* v) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
                : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
                : "r"(a));
 }
-// Exact sums of Q columns over the levels: hi counts units of 2^28 of lo.  The level sums are integers below 2^22:
+// Exact sums of UC columns over the levels: hi counts units of 2^28 of lo.  The level sums are integers below 2^22:
 // the FP32 addition of 1.5 2^23 leaves them in the low bits, and two levels fit 32 bits.
-template <int Q>
+constexpr int UC = 4;                                // columns a thread takes at once
 SKN_DEVINL void level_sums(uint32_t base, int level_cols, long long* hi, long long* lo) {
   auto quad = [&](int L, long long* out) {
-    uint32_t t[4][Q];
+    uint32_t t[4][UC];
 #pragma unroll
-    for (int l = 0; l < 4; ++l) {
-      if constexpr (Q == 8) tmem_ld8(base + (uint32_t)((L + l) * level_cols), t[l]);
-      else tmem_ld4(base + (uint32_t)((L + l) * level_cols), t[l]);
-    }
+    for (int l = 0; l < 4; ++l) tmem_ld4(base + (uint32_t)((L + l) * level_cols), t[l]);
     asm volatile("tcgen05.wait::ld.sync.aligned;");
     auto whole = [](uint32_t x) { return __float_as_int(__uint_as_float(x) + 12582912.0f) - 0x4B400000; };
 #pragma unroll
-    for (int q = 0; q < Q; ++q)
+    for (int q = 0; q < UC; ++q)
       out[q] = (long long)(whole(t[0][q]) * 128 + whole(t[1][q])) * 16384 + (whole(t[2][q]) * 128 + whole(t[3][q]));
   };
   quad(0, hi);
@@ -642,8 +633,8 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
     for (int h = 0; h < SE; h += 4) {
       const int cb = part * SE + h;
       long long hr[4], lr[4], hi[4], li[4];
-      level_sums<4>(tb + cb, 2 * NB, hr, lr);
-      level_sums<4>(tb + NB + cb, 2 * NB, hi, li);
+      level_sums(tb + cb, 2 * NB, hr, lr);
+      level_sums(tb + NB + cb, 2 * NB, hi, li);
 #pragma unroll
       for (int q = 0; q < 4; ++q) {
         const int k = cb + q, ex = s_ex[k];
@@ -679,7 +670,6 @@ constexpr int UPD_SMEM = SLICES * A_BYTES + 2 * B_BYTES;       // 192 KB
 constexpr uint32_t BUF_COLS = SLICES * 2 * BN;       // TMEM columns of one tile
 constexpr uint32_t TMEM_COLS = 2 * BUF_COLS;
 constexpr int UPD_WARPS = 16, UPD_THREADS = 32 * (UPD_WARPS + 1);
-constexpr int UC = 4;                                // columns a thread takes at once
 
 // C -= A B^T over BM x BN tiles.  SWEEP 1: blocks [0, nlow) of S22 (lower triangle, columns from sb), the rest
 // of H below the panel over all columns (sc); SWEEP 2 and 3: the trailing lower triangle of H (sb).
@@ -828,8 +818,8 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
       for (int h = 0; h < BN / 2; h += UC) {
         const int cb = c0 + h;
         long long hr[UC], lr[UC], hi[UC], li[UC];
-        level_sums<UC>(base + cb, 2 * BN, hr, lr);
-        level_sums<UC>(base + BN + cb, 2 * BN, hi, li);
+        level_sums(base + cb, 2 * BN, hr, lr);
+        level_sums(base + BN + cb, 2 * BN, hi, li);
         if (h + UC == BN / 2) {                      // the accumulators have been read: the next tile may start
           asm volatile("tcgen05.fence::before_thread_sync;");
           if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar(T_EMPTY + grp)) : "memory");

@@ -15,7 +15,7 @@
 //      panel's earlier reflectors, the reflector, a tiled Hermitian matrix-vector product with the
 //      trailing matrix as it stood at the panel's start, the panel corrections, and w; per panel one
 //      tiled rank-2NB update A22 -= V W^H + W V^H;
-//   5. eigenvalues of the tridiagonal by Sturm counts and Newton (sturm.cuh), one thread each.
+//   5. eigenvalues of the tridiagonal by Sturm counts and secant steps (sturm.cuh), one thread each.
 // The reference calls torch.linalg.cholesky / solve / eigh per k (slakonet/utils.py:749-783,
 // slakonet/main.py:174).
 //

@@ -122,7 +122,7 @@ __global__ void __launch_bounds__(VNT) k_inverse(int n_prob, const int32_t* __re
         s_u2[(n - 1) * VNT + tid] = 0.0;   // the last row has no columns to its right: the back substitution
         s_u3[(n - 1) * VNT + tid] = 0.0;   // multiplies these by zero, and scratch may hold a NaN
         rmax = fmax(rmax, fabs(1.0 / u1));
-        // A lam exact to the last bit (the Newton step can land on the eigenvalue) leaves a pivot at the
+        // A lam exact to the last bit (the secant step can land on the eigenvalue) leaves a pivot at the
         // 1e-300 floor, and a solve then grows the vector by up to 1 / pivot: its sum of squares overflowed
         // and the eigenvector came out NaN.  Every solve's right-hand side is therefore scaled by
         // ysc = 2^-e with 2^e >= rmax, which keeps the solution near unit size; a power of two scales
@@ -200,7 +200,8 @@ __global__ void __launch_bounds__(VNT) k_inverse(int n_prob, const int32_t* __re
 // columns of one problem, one per lane, and its four warps (one per scheduler: FP64 issues at one warp instruction
 // per 64 clocks on each) every fourth row; a reflector's dot products meet in shared memory in a fixed order and
 // nowhere else.  Y stays in shared memory as long as n allows.  The problems' CTAs used to hold all n columns, one
-// per thread, in global memory: the 484 problems of 30 to 116 orbitals of a training step took 11.0 ms.
+// per thread, in global memory: the 484 problems of 30 to 116 orbitals of a training step took 11.0 ms with their inverse
+// iteration, 7.4 now (2.2 of FP64 at its rate, half of each lane's work on ragged column tiles and short reflectors).
 constexpr int BT = 32;                   // columns per CTA
 constexpr int BW = 4;                    // warps
 constexpr int SMEM_MAX = 232448 - 1024;
