@@ -35,6 +35,7 @@ static_assert(PTS == THREADS, "one thread per point in the final sums");
 constexpr double FAR_T = 36.0;              // exp(-t^2/2) and its powers stay normal up to here
 constexpr double ZERO_T = 38.8;             // beyond: exp(-t^2/2) is exactly zero
 constexpr double MAX_T = 41.0;              // exp(-t^2/2) 2^230 and its powers stay normal up to here
+constexpr int HI_INF = 0x7ff00000;          // high word of an infinity; a NaN's is no smaller
 
 // torch.linspace grid: fma(step, i, lo) for the first half, fma(-step, n-1-i, hi) after.
 SKN_DEVINL double lin_grid(double lo, double hi, int n, int i) {
@@ -90,7 +91,9 @@ SKN_DEVINL void lane_init(Lane& L, double x0, double shift, double e_lo, double 
 template <bool WINDOWED>
 SKN_DEVINL void add_band(Lane& L, double E, double w) {
   const double t = fma(-E, L.scale, L.xs) * L.inv_sigma;
+  const int ht = hi_abs(t);
   if (WINDOWED && L.masked) {
+    if (ht >= HI_INF) return;                  // a NaN is outside every window
     const int jl = near_int(fma(t, -L.inv_d, L.cl)), jh = near_int(fma(t, -L.inv_d, L.ch));
     if (jl > DG - 1 || jh < 0) return;
     double g = exp(-0.5 * (t * t)) * w;
@@ -103,9 +106,11 @@ SKN_DEVINL void add_band(Lane& L, double E, double w) {
     return;
   }
   const double te = fma((double)(DG - 1), L.d, t);
-  // all points on one side of the band and beyond the underflow
-  const int ht = hi_abs(t), he = hi_abs(te);
-  if ((__double2hiint(t) ^ __double2hiint(te)) >= 0 && ht > L.hi_zero && he > L.hi_zero) return;
+  // all points on one side of the band and beyond the underflow; an infinity or a NaN, also of the weight, is no zero:
+  // its terms are formed
+  const int he = hi_abs(te);
+  if ((__double2hiint(t) ^ __double2hiint(te)) >= 0 && min(ht, he) > L.hi_zero && max(max(ht, he), hi_abs(w)) < HI_INF)
+    return;
   if (L.fast && max(ht, he) < L.hi_max && (!WINDOWED || (fabs(t) <= L.window && fabs(te) <= L.window))) {
     // where the first factor would leave the normal range it is carried times 2^230, which leaves each term
     // as its last rounding
