@@ -16,7 +16,7 @@ import ctypes
 import math
 import threading
 from dataclasses import dataclass, field
-from typing import Dict, List, Optional, Sequence
+from typing import Dict, List, NamedTuple, Optional, Sequence
 
 import numpy as np
 import torch
@@ -476,6 +476,7 @@ class DeviceBatch:
 
     def __init__(self, plan: Plan, device):
         self.plan = plan
+        self.groups = {}                     # Engine._groups
         # work units of the Bloch-sum kernel per structure: ceil(nk_s / BLOCH_KCHUNK) k-chunks times the
         # N_s^2 ordered atom pairs (full matrices) or the N_s (N_s + 1) / 2 pairs on or below the diagonal
         # (lower triangles), numbered from an exclusive prefix sum
@@ -557,6 +558,19 @@ def panels_parts(sizes: np.ndarray, budget: int):
         parts.append((first, last, end[first:last] - per[first:last] - base, int(end[last - 1]) - base))
         first = last
     return parts
+
+
+class Group(NamedTuple):
+    """One eigensolver call's problems (a panel group's: calls).  ``kind``: the one-CTA kernel's launch shape suffix,
+    the cluster size for the cluster path, ("wide", n, real) for the device-wide path, or route_auto's ("small", class)
+    or ("panels", class).  ``order``: problem indices on the device.  Panels: ``parts`` as panels_parts has them with
+    the scratch offsets on the device and the sizes on the host, ``sms`` the SMs to plan for."""
+    kind: object
+    order: torch.Tensor
+    count: int
+    max_n: int
+    parts: tuple = ()
+    sms: int = 0
 
 
 VEC_SCRATCH = 512 << 20      # device bytes of the inverse iteration's scratch per group
@@ -838,59 +852,58 @@ class Engine:
                        ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counters), plan.max_n, stream)
             return
         scratch = {}
-        for gi, (shape, _, count, max_n) in enumerate(groups):
+        for gi, g in enumerate(groups):
             need = ctypes.c_int64(0)
-            if isinstance(shape, int):       # a cluster group
-                call("skn_eigh_large_scratch_bytes", count, max_n, shape, ctypes.addressof(need))
-            elif isinstance(shape, tuple) and shape[0] == "panels":
-                need.value = max(part[3] for part in db._panel_parts[gi])
-            elif isinstance(shape, tuple) and shape[0] == "wide":   # a device-wide group: ("wide", n, real)
-                call("skn_eigh_wide_scratch_bytes", count, max_n, ctypes.addressof(need))
+            if isinstance(g.kind, int):      # a cluster group
+                call("skn_eigh_large_scratch_bytes", g.count, g.max_n, g.kind, ctypes.addressof(need))
+            elif g.parts:
+                need.value = max(nbytes for _, _, _, nbytes, _ in g.parts)
+            elif isinstance(g.kind, tuple) and g.kind[0] == "wide":
+                call("skn_eigh_wide_scratch_bytes", g.count, g.max_n, ctypes.addressof(need))
             else:
                 continue
             scratch[gi] = torch.empty(max(need.value // 8, 1), dtype=torch.float64, device=self.device)
         vec_scratch = []
         if vec is not None:                  # the inverse iteration takes what it is given, at least one CTA's part
-            for _, _, count, max_n in groups:
+            for g in groups:
                 need, one = ctypes.c_int64(0), ctypes.c_int64(0)
-                call("skn_eigvec_scratch_bytes", count, max_n, ctypes.addressof(need))
-                call("skn_eigvec_scratch_bytes", 1, max_n, ctypes.addressof(one))
+                call("skn_eigvec_scratch_bytes", g.count, g.max_n, ctypes.addressof(need))
+                call("skn_eigvec_scratch_bytes", 1, g.max_n, ctypes.addressof(one))
                 nbytes = min(need.value, max(VEC_SCRATCH, one.value))
                 vec_scratch.append(torch.empty(nbytes // 8, dtype=torch.float64, device=self.device))
-        share = self._sm_shares(db, groups) if db._panel_parts else None
 
-        def launch(gi, sfx, order_g, count, max_n, st):
-            if isinstance(sfx, tuple) and sfx[0] == "small":
-                self._call("skn_eigh_gen_small", count, max_n, ptr(order_g), ptr(db.n),
+        def launch(gi, g, st):
+            if g.parts:
+                for first, last, ws_off, nbytes, sizes in g.parts:
+                    self._call("skn_eigh_gen_panels", last - first, sizes.ctypes.data, ptr(g.order[first:]), ptr(ws_off),
+                               ptr(db.n), ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff),
+                               ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(tri), ptr(scratch[gi]), nbytes, g.sms, st)
+                    self.launches += panels_launches(int(sizes[0])) - 1
+            elif isinstance(g.kind, tuple) and g.kind[0] == "small":
+                self._call("skn_eigh_gen_small", g.count, g.max_n, ptr(g.order), ptr(db.n),
                            ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk),
                            ptr(eig), ptr(eig_status), ptr(tri), st)
-            elif isinstance(sfx, tuple) and sfx[0] == "panels":
-                for first, last, ws_off, nbytes, sizes in db._panel_parts[gi]:
-                    self._call("skn_eigh_gen_panels", last - first, sizes.ctypes.data, ptr(order_g[first:]), ptr(ws_off),
-                               ptr(db.n), ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff),
-                               ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(tri), ptr(scratch[gi]), nbytes, share[gi],
-                               st)
-                    self.launches += panels_launches(int(sizes[0])) - 1
-            elif isinstance(sfx, tuple):
-                self._call("skn_eigh_gen_wide_tc" if self.wide_tc else "skn_eigh_gen_wide", count, max_n,
-                           ptr(order_g), ptr(db.n), ptr(db.hs_off), ptr(db.eoff),
+            elif isinstance(g.kind, tuple):
+                self._call("skn_eigh_gen_wide_tc" if self.wide_tc else "skn_eigh_gen_wide", g.count, g.max_n,
+                           ptr(g.order), ptr(db.n), ptr(db.hs_off), ptr(db.eoff),
                            ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(scratch[gi]),
-                           int(scratch[gi].numel() * 8), int(sfx[2]), st)
-            elif isinstance(sfx, int):
-                self._call("skn_eigh_gen_large", count, ptr(db.n), ptr(db.hs_off), ptr(db.eoff), ptr(order_g),
+                           int(scratch[gi].numel() * 8), g.kind[2], st)
+            elif isinstance(g.kind, int):
+                self._call("skn_eigh_gen_large", g.count, ptr(db.n), ptr(db.hs_off), ptr(db.eoff), ptr(g.order),
                            ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counters[2 * gi:]), ptr(scratch[gi]),
-                           int(scratch[gi].numel() * 8), max_n, sfx, st)
+                           int(scratch[gi].numel() * 8), g.max_n, g.kind, st)
             else:
-                self._call("skn_eigh_gen_batched" + sfx, count, ptr(db.n), ptr(db.hs_off), ptr(db.eoff),
-                           ptr(order_g), ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counters[2 * gi:]),
-                           max_n, st)
+                self._call("skn_eigh_gen_batched" + g.kind, g.count, ptr(db.n), ptr(db.hs_off), ptr(db.eoff),
+                           ptr(g.order), ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counters[2 * gi:]),
+                           g.max_n, st)
             if vec is not None:
-                self._call("skn_eigvec", count, max_n, ptr(order_g), ptr(db.n), ptr(db.real if self.real_path else None),
-                           ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk), ptr(eig), ptr(tri), ptr(eig_status), ptr(vec),
-                           ptr(vec_scratch[gi]), int(vec_scratch[gi].numel() * 8), ptr(counters[2 * gi + 1:]), st)
+                self._call("skn_eigvec", g.count, g.max_n, ptr(g.order), ptr(db.n),
+                           ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk),
+                           ptr(eig), ptr(tri), ptr(eig_status), ptr(vec), ptr(vec_scratch[gi]),
+                           int(vec_scratch[gi].numel() * 8), ptr(counters[2 * gi + 1:]), st)
 
         if len(groups) == 1:
-            launch(0, *groups[0], stream)
+            launch(0, groups[0], stream)
             return
         # one launch per group (in _groups' order) on forked streams
         main = torch.cuda.current_stream(self.device)
@@ -901,21 +914,12 @@ class Engine:
             st = self._side_streams(len(groups))[gi]
             st.wait_event(fork)
             with torch.cuda.stream(st):
-                launch(gi, *g, st.cuda_stream)
+                launch(gi, g, st.cuda_stream)
             ev = torch.cuda.Event()
             ev.record(st)
             joins.append(ev)
         for ev in joins:
             main.wait_event(ev)
-
-    def _sm_shares(self, db, groups):
-        """SMs each group plans for: its part of the batch's n^3, as the groups run beside one another."""
-        cached = getattr(db, "_shares", None)
-        if cached is None or cached[0] is not groups:
-            cost = [float((db.plan.prob_n[sel].astype(np.float64) ** 3).sum()) for sel in db._group_problems]
-            sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-            cached = db._shares = (groups, [max(1, round(sms * c / max(sum(cost), 1.0))) for c in cost])
-        return cached[1]
 
     def _side_streams(self, k):
         """k side streams for forked launches, cached per host thread and device (engines are
@@ -929,16 +933,14 @@ class Engine:
         return cur
 
     def _groups(self, db, vectors: bool = False):
-        """[(launch shape suffix, the cluster size for the cluster path, ("wide", n, real) for the device-wide
-        path, or route_auto's ("small", class) or ("panels", class), device order, count, max_n)], cached on the batch.
-
-        Empty when every problem takes the default single-CTA launch.  With ``vectors`` every problem takes route_auto's
-        kernel: the others keep no reflectors."""
+        """The batch's eigensolver groups ([Group], empty when every problem takes the default single-CTA launch), kept
+        on the batch by all that decides them.  None is ever dropped or changed: a captured graph reads their arrays.
+        With ``vectors`` every problem takes route_auto's kernel: the others keep no reflectors."""
         plan = db.plan
-        key = (vectors, id(self.tuning), self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
-        cache = getattr(db, "_groups", None)
-        if cache is not None and cache[0] == key:
-            return cache[1]
+        tuned = None if self.tuning is None else tuple(sorted(self.tuning.choice.items()))
+        key = (vectors, tuned, self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
+        if key in db.groups:
+            return db.groups[key]
         wide = route_wide(plan.prob_n, None if vectors else self.wide_threshold)[plan.order]
         csize = (np.zeros(len(plan.order), int) if vectors
                  else route_large(plan.prob_n, self.large_threshold, self.large_cluster)[plan.order])
@@ -979,23 +981,28 @@ class Engine:
             out = []     # the default launch over the batch's own order
         real = plan.prob_real if (self.real_path and plan.prob_real is not None) else np.zeros(len(plan.prob_n), bool)
         out = [out[i] for i in launch_order([g[1] for g in out], plan.prob_n, real)]
-        db._group_problems = [g[1] for g in out]
-        parts = {}
-        for gi, (sh, sel, _, _) in enumerate(out):
-            if isinstance(sh, tuple) and sh[0] == "panels":
+        cost = [float((plan.prob_n[sel].astype(np.float64) ** 3).sum()) for _, sel, _, _ in out]
+        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        groups = []
+        for (kind, sel, cnt, mx), c in zip(out, cost):
+            parts = ()
+            if isinstance(kind, tuple) and kind[0] == "panels":
                 sizes = np.ascontiguousarray(plan.prob_n[sel].astype(np.int32))
-                parts[gi] = [(a, b, w, nbytes, sizes[a:b]) for a, b, w, nbytes in panels_parts(sizes, PANELS_SCRATCH)]
-        if out:                              # problem lists and scratch offsets to the device
-            lists = [(sel, np.int32) for _, sel, _, _ in out] + [(p[2], np.int64) for g in parts.values() for p in g]
-            if len(lists) == 1 and len(lists[0][0]) == len(plan.order):      # the batch's own order
-                lists = iter([db.order])
-            else:
-                lists = iter(_to_device(lists, self.device))
-            out = [(sh, next(lists), cnt, mx) for sh, _, cnt, mx in out]
-            parts = {gi: [(a, b, next(lists), nbytes, sizes) for a, b, _, nbytes, sizes in g] for gi, g in parts.items()}
-        db._panel_parts = parts
-        db._groups = (key, out)
-        return out
+                parts = tuple((a, b, w, nbytes, sizes[a:b]) for a, b, w, nbytes in panels_parts(sizes, PANELS_SCRATCH))
+            # the groups run beside one another: each plans for the SMs of its part of the batch's n^3
+            groups.append(Group(kind, sel, cnt, mx, parts, max(1, round(sms * c / max(sum(cost), 1.0)))))
+        if not groups:
+            return db.groups.setdefault(key, groups)
+        # problem lists and scratch offsets to the device
+        lists = [(g.order, np.int32) for g in groups] + [(p[2], np.int64) for g in groups for p in g.parts]
+        if len(lists) == 1 and len(lists[0][0]) == len(plan.order):      # the batch's own order
+            lists = iter([db.order])
+        else:
+            lists = iter(_to_device(lists, self.device))
+        groups = [g._replace(order=next(lists)) for g in groups]
+        groups = [g._replace(parts=tuple((a, b, next(lists), nbytes, sizes) for a, b, _, nbytes, sizes in g.parts))
+                  for g in groups]
+        return db.groups.setdefault(key, groups)
 
     def check_tables(self):
         """Raise if the last execute() needed a table the parameter set lacks (reads one device int)."""
