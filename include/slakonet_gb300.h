@@ -342,12 +342,19 @@ int skn_eigh_gen_small(int n_prob, int max_n, const int32_t* prob, const int32_t
  *   scratch   device scratch of scratch_bytes bytes
  *   sms       SMs to plan for, as when other calls run beside this one (0: all); the
  *             results do not depend on it
+ * Waits inside the kernels are bounded; a problem one of whose waits has run out gets
+ * SKN_ERR_CUDA.  Eigenvalues are NaN where status is neither SKN_OK nor SKN_ERR_CAPACITY.
  * Results depend only on each problem.
  */
 int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
                         const int32_t* nvec, const int32_t* real, const int64_t* hs_off, const int64_t* eig_off,
                         double* H, double* S, double* eig, int32_t* status, double* tri, double* scratch,
                         int64_t scratch_bytes, int sms, cudaStream_t stream);
+/* The same with shorter waits: polls[0..2] (host) bound the polls of the solves', the updates' and the grid teams' waits. */
+int skn_eigh_gen_panels_limits(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
+                               const int32_t* nvec, const int32_t* real, const int64_t* hs_off, const int64_t* eig_off,
+                               double* H, double* S, double* eig, int32_t* status, double* tri, double* scratch,
+                               int64_t scratch_bytes, int sms, const int32_t* polls, cudaStream_t stream);
 /* Host-side query: scratch bytes of one problem of n orbitals in skn_eigh_gen_panels (written to *bytes). */
 int skn_eigh_panels_scratch_bytes(int n, int64_t* bytes);
 
@@ -356,8 +363,8 @@ int skn_eigh_panels_scratch_bytes(int n, int64_t* bytes);
  * with `tri`: inverse iteration on the tridiagonal, then the reflectors and L^-H.
  *   prob      [n_prob] problem indices, the largest first; max_n bounds their n (<= 2048)
  *   H, S, eig, tri, status, real   as that call left them (real: as it was given)
- *   vec       row-major per problem at hs_off, as skn_eigh_gen_vectors; NaN where
- *             status is SKN_ERR_NOT_SPD, untouched where it is SKN_ERR_CAPACITY
+ *   vec       row-major per problem at hs_off, as skn_eigh_gen_vectors; untouched where
+ *             status is SKN_ERR_CAPACITY, NaN where it is another error
  *   scratch   at least the query's bytes for one problem of max_n; up to the query's for n_prob
  *             lets more problems run at once, with the same results
  *   counter   one int32

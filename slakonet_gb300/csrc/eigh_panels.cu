@@ -138,8 +138,16 @@ __host__ __device__ inline Lay layout(int n) {
   return L;
 }
 
+// Polls after which the waits of a kernel give up: the solves' and the updates' on their products and copies, a grid
+// team's barriers (a poll of the last takes about half a microsecond).
+struct Limits {
+  int solve, update, team;
+};
+constexpr Limits LIMITS{1 << 26, 1 << 26, 1 << 22};
+
 struct Grp {
   int nmax, n_prob;
+  Limits limits;
   const int32_t* prob;       // [n_prob] problem of each slot, sizes descending
   const int64_t* ws_off;     // [n_prob] byte offset of each slot's scratch
   const int32_t* nvec;
@@ -471,10 +479,9 @@ SKN_DEVINL void level_sums(uint32_t base, int level_cols, long long* hi, long lo
   quad(4, lo);
 }
 
-constexpr long long WAIT_LIMIT = 1LL << 26;
-// Wait for a phase of a barrier; gives up after WAIT_LIMIT polls or once the CTA has failed.
-SKN_DEVINL bool upd_wait(uint32_t bar, uint32_t parity, volatile int* fail) {
-  for (long long it = 0; it < WAIT_LIMIT; ++it) {
+// Wait for a phase of a barrier; gives up after `limit` polls or once the CTA has failed.
+SKN_DEVINL bool upd_wait(uint32_t bar, uint32_t parity, volatile int* fail, int limit) {
+  for (int it = 0; it < limit; ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -622,9 +629,13 @@ __global__ void __launch_bounds__(SV_THREADS, 1) k_solve(Grp G, int c0, int nrow
     }
     tc_commit(bar);
   }
-  if (!upd_wait(bar, 0, &s_fail)) s_fail = 1;
+  if (!upd_wait(bar, 0, &s_fail, G.limits.solve)) s_fail = 1;
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;");
+  if (s_fail && tid == 0) {            // the products must have completed before the CTA frees its TMEM and exits
+    volatile int never = 0;
+    upd_wait(bar, 0, &never, LIMITS.solve);
+  }
 #pragma unroll
   for (int q = 0; q < SE; ++q) z[q] = zero2();
   if (!s_fail && !xwarp) {
@@ -749,16 +760,16 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
       bool ok = true;
       for (int i = 0; ok && i < ntile; ++i) {
         const int b = i & 1;
-        ok = upd_wait(bar(B_FULL + b), (uint32_t)((i >> 1) & 1), &s_fail);
+        ok = upd_wait(bar(B_FULL + b), (uint32_t)((i >> 1) & 1), &s_fail, G.limits.update);
         if (!ok) break;
         ++landed;
-        if (i >= 2) ok = upd_wait(bar(T_EMPTY + b), (uint32_t)(((i >> 1) - 1) & 1), &s_fail);
+        if (i >= 2) ok = upd_wait(bar(T_EMPTY + b), (uint32_t)(((i >> 1) - 1) & 1), &s_fail, G.limits.update);
         if (!ok) break;
         asm volatile("tcgen05.fence::after_thread_sync;");
         const uint32_t bs = b0 + (uint32_t)(b * B_BYTES), td = tmem + (uint32_t)b * BUF_COLS;
         for (int s = 0; s < SLICES; ++s) {
           if (i == 0) {
-            ok = upd_wait(bar(s), 0, &s_fail);
+            ok = upd_wait(bar(s), 0, &s_fail, G.limits.update);
             if (!ok) break;
             ++a_landed;
             asm volatile("tcgen05.fence::after_thread_sync;");
@@ -774,7 +785,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
         ++issued;
         if (!ok) break;
         if (i >= 1 && i + 1 < ntile) {                // the other column buffer, once tile i - 1 has been multiplied
-          ok = upd_wait(bar(T_FULL + (b ^ 1)), (uint32_t)(((i - 1) >> 1) & 1), &s_fail);
+          ok = upd_wait(bar(T_FULL + (b ^ 1)), (uint32_t)(((i - 1) >> 1) & 1), &s_fail, G.limits.update);
           if (!ok) break;
           finished = i;
           load_b(i + 1);
@@ -785,11 +796,11 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
       if (!ok) s_fail = 1;
       volatile int never = 0;
       for (; a_landed < SLICES; ++a_landed)
-        if (!upd_wait(bar(a_landed), 0, &never)) ok = false;
+        if (!upd_wait(bar(a_landed), 0, &never, LIMITS.update)) ok = false;
       for (; landed < loaded; ++landed)
-        if (!upd_wait(bar(B_FULL + (landed & 1)), (uint32_t)((landed >> 1) & 1), &never)) ok = false;
+        if (!upd_wait(bar(B_FULL + (landed & 1)), (uint32_t)((landed >> 1) & 1), &never, LIMITS.update)) ok = false;
       for (; finished < issued; ++finished)
-        if (!upd_wait(bar(T_FULL + (finished & 1)), (uint32_t)((finished >> 1) & 1), &never)) ok = false;
+        if (!upd_wait(bar(T_FULL + (finished & 1)), (uint32_t)((finished >> 1) & 1), &never, LIMITS.update)) ok = false;
       if (!ok) s_fail = 1;
     }
   } else {
@@ -808,7 +819,7 @@ __global__ void __launch_bounds__(UPD_THREADS, 1) k_update(Grp G, int c1, int nl
         cv[q] = zero2();
         if (rok && gc < n && (!low || i >= q0 + c0 + q)) cv[q] = C[(int64_t)gc * n];
       }
-      const bool ok = upd_wait(bar(T_FULL + grp), (uint32_t)((it >> 1) & 1), &s_fail);
+      const bool ok = upd_wait(bar(T_FULL + grp), (uint32_t)((it >> 1) & 1), &s_fail, G.limits.update);
       if (!ok || s_fail) {
         s_fail = 1;
         break;
@@ -1046,9 +1057,8 @@ template <bool R> SKN_DEVINL int4 ld_fixed(const int4* p) {
 
 // The CTAs of one problem: a cluster, or (more than 16) CTAs of a cooperative launch that meet at a counter.  A
 // wait is bounded; once one has run out the problem is marked SKN_ERR_CUDA and its CTAs no longer wait.
-constexpr int TEAM_LIMIT = 1 << 22;              // polls of about half a microsecond
 struct Team {
-  int rank, C;
+  int rank, C, limit;
   bool grid;
   unsigned* count;
   unsigned target;
@@ -1066,12 +1076,12 @@ struct Team {
         __threadfence();
         atomicAdd(count, 1u);
         int it = 0;
-        for (; it < TEAM_LIMIT; ++it) {
+        for (; it < limit; ++it) {
           unsigned v;
           asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(count) : "memory");
           if (v >= target) break;
         }
-        if (it == TEAM_LIMIT) {
+        if (it == limit) {
           *dead = 1;
           *status = SKN_ERR_CUDA;
         }
@@ -1591,7 +1601,7 @@ __global__ void __launch_bounds__(RES ? PTR : PT, RES ? 1 : 4) k_tri_panel(Grp G
   double2* big = reinterpret_cast<double2*>(svf + rows);
   int* sve = reinterpret_cast<int*>(smem_raw + sve_off);
   if (threadIdx.x == 0) sm.dead = 0;
-  Team team{(int)(blockIdx.x % C), C, grid != 0, ws_of(G, g).bar + c0 / NT, 0u, G.status + p, &sm.dead};
+  Team team{(int)(blockIdx.x % C), C, G.limits.team, grid != 0, ws_of(G, g).bar + c0 / NT, 0u, G.status + p, &sm.dead};
   if (is_real(G, p))
     panel_body<true, RES>(G, g, p, c0, team, rt, cpc, sm, sv, svf, sve, big);
   else
@@ -1656,8 +1666,8 @@ __global__ void __launch_bounds__(64, 16) k_eig(Grp G) {
   const int st = G.status[p];
   if (st == SKN_ERR_CAPACITY || j >= n) return;
   double* out = G.eig + G.eig_off[p];
-  if (st != SKN_OK) {
-    if (st == SKN_ERR_NOT_SPD) out[j] = __longlong_as_double(0x7ff8000000000000LL);
+  if (st != SKN_OK) {                        // S not positive definite, or a wait that ran out
+    out[j] = __longlong_as_double(0x7ff8000000000000LL);
     return;
   }
   const WS w = ws_of(G, g);
@@ -1852,10 +1862,10 @@ extern "C" int skn_eigh_panels_scratch_bytes(int n, int64_t* bytes) {
   return SKN_OK;
 }
 
-extern "C" int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
-                                   const int32_t* nvec, const int32_t* real, const int64_t* hs_off,
-                                   const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status,
-                                   double* tri, double* scratch, int64_t scratch_bytes, int sms, cudaStream_t stream) {
+static int panels_entry(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off, const int32_t* nvec,
+                        const int32_t* real, const int64_t* hs_off, const int64_t* eig_off, double* H, double* S,
+                        double* eig, int32_t* status, double* tri, double* scratch, int64_t scratch_bytes, int sms,
+                        Limits limits, cudaStream_t stream) {
   if (n_prob < 0 || sms < 0) return SKN_ERR_ARG;
   if (n_prob == 0) return SKN_OK;
   if (!sizes || !prob || !ws_off || !nvec || !hs_off || !eig_off || !H || !S || !eig || !status || !scratch)
@@ -1866,7 +1876,26 @@ extern "C" int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32
       (reinterpret_cast<uintptr_t>(S) & 15))
     return SKN_ERR_ARG;
   if (set_attrs() != cudaSuccess) return SKN_ERR_CUDA;
-  Grp G{sizes[0], n_prob, prob, ws_off, nvec, real, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, tri,
+  Grp G{sizes[0], n_prob, limits, prob, ws_off, nvec, real, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, tri,
         (char*)scratch, scratch_bytes};
   return run(G, sizes, sms, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
+}
+
+extern "C" int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
+                                   const int32_t* nvec, const int32_t* real, const int64_t* hs_off,
+                                   const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status,
+                                   double* tri, double* scratch, int64_t scratch_bytes, int sms, cudaStream_t stream) {
+  return panels_entry(n_prob, sizes, prob, ws_off, nvec, real, hs_off, eig_off, H, S, eig, status, tri, scratch,
+                      scratch_bytes, sms, LIMITS, stream);
+}
+
+extern "C" int skn_eigh_gen_panels_limits(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
+                                          const int32_t* nvec, const int32_t* real, const int64_t* hs_off,
+                                          const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status,
+                                          double* tri, double* scratch, int64_t scratch_bytes, int sms,
+                                          const int32_t* polls, cudaStream_t stream) {
+  if (!polls || polls[0] < 0 || polls[1] < 0 || polls[2] < 0) return SKN_ERR_ARG;
+  const Limits limits{std::min(polls[0], LIMITS.solve), std::min(polls[1], LIMITS.update), std::min(polls[2], LIMITS.team)};
+  return panels_entry(n_prob, sizes, prob, ws_off, nvec, real, hs_off, eig_off, H, S, eig, status, tri, scratch,
+                      scratch_bytes, sms, limits, stream);
 }
