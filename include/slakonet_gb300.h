@@ -297,12 +297,17 @@ int skn_eigh_wide_scratch_bytes(int n_prob, int n, int64_t* bytes);
  * integer slices of 7 bits, slice products of one level accumulate exactly in
  * FP32, and the levels are combined exactly before one FP64 rounding.  Same
  * arguments, scratch and contract as skn_eigh_gen_wide; a tensor-core stage
- * whose completion wait runs out sets the problem's status to SKN_ERR_CUDA.
+ * whose completion wait runs out sets the problem's status to SKN_ERR_CUDA
+ * and its eigenvalues to NaN.
  * No reference counterpart beyond the eighb call skn_eigh_gen_wide replaces.
  */
 int skn_eigh_gen_wide_tc(int n_prob, int n, const int32_t* prob, const int32_t* nvec, const int64_t* hs_off,
                          const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status, double* scratch,
                          int64_t scratch_bytes, int real, cudaStream_t stream);
+/* The same with shorter waits, of at most `polls` polls. */
+int skn_eigh_gen_wide_tc_limits(int n_prob, int n, const int32_t* prob, const int32_t* nvec, const int64_t* hs_off,
+                                const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status,
+                                double* scratch, int64_t scratch_bytes, int real, int polls, cudaStream_t stream);
 /*
  * Eigenvalues (and, with `tri`, the reduced form the eigenvectors start from) of
  * problems of up to 96 orbitals, one CTA per problem with both matrices in shared

@@ -58,6 +58,7 @@ SIGNATURES = {
     "skn_eigh_gen_wide": [I32, I32, P, P, P, P, P, P, P, P, P, I64, I32, P],
     "skn_eigh_wide_scratch_bytes": [I32, I32, P],
     "skn_eigh_gen_wide_tc": [I32, I32, P, P, P, P, P, P, P, P, P, I64, I32, P],
+    "skn_eigh_gen_wide_tc_limits": [I32, I32, P, P, P, P, P, P, P, P, P, I64, I32, I32, P],
     "skn_eigh_gen_small": [I32, I32, P, P, P, P, P, P, P, P, P, P, P],
     "skn_eigh_gen_panels": [I32, P, P, P, P, P, P, P, P, P, P, P, P, P, I64, I32, P],
     "skn_eigh_gen_panels_limits": [I32, P, P, P, P, P, P, P, P, P, P, P, P, P, I64, I32, P, P],

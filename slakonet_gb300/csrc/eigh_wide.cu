@@ -149,7 +149,7 @@ struct WS {
 
 // What every launch needs: the group and its buffers.
 struct Grp {
-  int n, n_prob;
+  int n, n_prob, polls;    // polls: what the tensor-core update's waits give up after
   const int32_t* prob;     // [n_prob] problem index of each slot
   const int32_t* nvec;     // [*] orbitals per problem (must equal n)
   const int64_t* hs_off;   // [*] element offset of a problem's H and S
@@ -460,10 +460,10 @@ SKN_DEVINL void tc_mma(uint32_t tmem_d, uint64_t a, uint64_t b, uint32_t accumul
       "l"(a), "l"(b), "r"(TC_IDESC), "r"(accumulate));
 }
 
-constexpr long long TC_WAIT_LIMIT = 1LL << 26;    // mbarrier polls before giving up
+constexpr int TC_WAIT_LIMIT = 1 << 26;            // mbarrier polls before giving up
 
-SKN_DEVINL bool tc_wait(uint32_t bar, uint32_t parity) {
-  for (long long it = 0; it < TC_WAIT_LIMIT; ++it) {
+SKN_DEVINL bool tc_wait(uint32_t bar, uint32_t parity, int limit = TC_WAIT_LIMIT) {
+  for (int it = 0; it < limit; ++it) {
     uint32_t done;
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
@@ -642,11 +642,11 @@ __global__ void __launch_bounds__(128) k_r2k_tc(Grp G, Mat Cm, int m) {
     // armed[b]: phases of mbarrier b armed (copies issued or MMAs committed) and not yet waited for
     int armed[5] = {1, 1, 1, 0, 0};
     int done[5] = {0, 0, 0, 0, 0};              // phases waited for
-    bool ok = tc_wait(bar_b, 0);
+    bool ok = tc_wait(bar_b, 0, G.polls);
     if (ok) done[0] = 1;
     for (int sl = 0; ok && sl < TCS; ++sl) {
       const int st = sl & 1;
-      ok = tc_wait(smem_u32(&bars[1 + st]), (uint32_t)(done[1 + st] & 1));
+      ok = tc_wait(smem_u32(&bars[1 + st]), (uint32_t)(done[1 + st] & 1), G.polls);
       if (!ok) break;
       ++done[1 + st];
       asm volatile("tcgen05.fence::after_thread_sync;");
@@ -665,7 +665,7 @@ __global__ void __launch_bounds__(128) k_r2k_tc(Grp G, Mat Cm, int m) {
           smem_u32(&bars[3 + st])));
       ++armed[3 + st];
       if (sl + 2 < TCS) {                         // refill this stage once its MMAs have read it
-        ok = tc_wait(smem_u32(&bars[3 + st]), (uint32_t)(done[3 + st] & 1));
+        ok = tc_wait(smem_u32(&bars[3 + st]), (uint32_t)(done[3 + st] & 1), G.polls);
         if (!ok) break;
         ++done[3 + st];
         load_stage(st, sl + 2);
@@ -1276,11 +1276,11 @@ __global__ void __launch_bounds__(128) k_tri_eig(Grp G) {
   if (j >= n) return;
   const int st = G.status[p];
   double* out = G.eig + G.eig_off[p];
-  if (st == SKN_ERR_NOT_SPD) {
+  if (st == SKN_ERR_CAPACITY) return;
+  if (st != SKN_OK) {                        // S not positive definite, or a wait that ran out
     out[j] = __longlong_as_double(0x7ff8000000000000LL);
     return;
   }
-  if (st != SKN_OK) return;
   const WS w = ws_of(G, g);
   const double2 lh = w.sc[3];
   const skn_sturm::Bounds B = skn_sturm::make_bounds(lh.x, lh.y, w.sc[4].x, n);
@@ -1417,7 +1417,7 @@ extern "C" int skn_eigh_wide_scratch_bytes(int n_prob, int n, int64_t* bytes) {
 
 static int wide_entry(int n_prob, int n, const int32_t* prob, const int32_t* nvec, const int64_t* hs_off,
                       const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status, double* scratch,
-                      int64_t scratch_bytes, int real, bool tc, cudaStream_t stream) {
+                      int64_t scratch_bytes, int real, bool tc, int polls, cudaStream_t stream) {
   if (n_prob < 0 || n < 1) return SKN_ERR_ARG;
   if (n_prob == 0) return SKN_OK;
   if (n_prob > 32767) return SKN_ERR_CAPACITY;   // grid z of the zero-row scan holds 2 n_prob
@@ -1428,7 +1428,7 @@ static int wide_entry(int n_prob, int n, const int32_t* prob, const int32_t* nve
       (reinterpret_cast<uintptr_t>(S) & 15) != 0)
     return SKN_ERR_ARG;
   if ((real ? set_attrs<true>() : set_attrs<false>()) != cudaSuccess) return SKN_ERR_CUDA;
-  Grp G{n, n_prob, prob, nvec, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, (double2*)scratch};
+  Grp G{n, n_prob, polls, prob, nvec, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, (double2*)scratch};
   if (real)
     run<true>(G, tc, stream);
   else
@@ -1441,7 +1441,7 @@ extern "C" int skn_eigh_gen_wide(int n_prob, int n, const int32_t* prob, const i
                                  const int64_t* eig_off, double* H, double* S, double* eig, int32_t* status,
                                  double* scratch, int64_t scratch_bytes, int real, cudaStream_t stream) {
   return wide_entry(n_prob, n, prob, nvec, hs_off, eig_off, H, S, eig, status, scratch, scratch_bytes, real, false,
-                    stream);
+                    TC_WAIT_LIMIT, stream);
 }
 
 extern "C" int skn_eigh_gen_wide_tc(int n_prob, int n, const int32_t* prob, const int32_t* nvec,
@@ -1449,5 +1449,14 @@ extern "C" int skn_eigh_gen_wide_tc(int n_prob, int n, const int32_t* prob, cons
                                     int32_t* status, double* scratch, int64_t scratch_bytes, int real,
                                     cudaStream_t stream) {
   return wide_entry(n_prob, n, prob, nvec, hs_off, eig_off, H, S, eig, status, scratch, scratch_bytes, real, true,
-                    stream);
+                    TC_WAIT_LIMIT, stream);
+}
+
+extern "C" int skn_eigh_gen_wide_tc_limits(int n_prob, int n, const int32_t* prob, const int32_t* nvec,
+                                           const int64_t* hs_off, const int64_t* eig_off, double* H, double* S,
+                                           double* eig, int32_t* status, double* scratch, int64_t scratch_bytes,
+                                           int real, int polls, cudaStream_t stream) {
+  if (polls < 0) return SKN_ERR_ARG;
+  return wide_entry(n_prob, n, prob, nvec, hs_off, eig_off, H, S, eig, status, scratch, scratch_bytes, real, true,
+                    polls < TC_WAIT_LIMIT ? polls : TC_WAIT_LIMIT, stream);
 }
