@@ -527,7 +527,11 @@ def wide_launches(n: int, nb: int = 32, tc: bool = False, tc_min: int = 512) -> 
 
 PANEL = 32                  # panel width of the blocked eigensolver (csrc/eigh_panels.cu)
 PANELS_MAX_N = 2048         # its bound
-PANELS_SCRATCH = 4 << 30    # device bytes of scratch per call; a larger group goes through in parts
+# Device bytes that one solve may hold as scratch beside H and S, all its concurrent calls together: the panel kernels'
+# (a group that needs more than its share goes through in parts) and the inverse iteration's.  Where the allocator has
+# not even that, Engine._eig_values goes on with less.
+PANELS_SCRATCH = 16 << 30
+VEC_SCRATCH = 2 << 30
 
 
 def panels_launches(max_n: int) -> int:
@@ -560,6 +564,16 @@ def panels_parts(sizes: np.ndarray, budget: int):
     return parts
 
 
+def scratch_shares(need: Sequence[int], least: Sequence[int], budget: int) -> List[int]:
+    """Bytes per group out of ``budget``: what it needs where that is no more than its fair part of what smaller needs
+    leave, else that part, but at least its ``least``."""
+    out, left = [0] * len(need), budget
+    for i, g in enumerate(sorted(range(len(need)), key=lambda g: need[g])):
+        out[g] = max(least[g], min(need[g], left // (len(need) - i)))
+        left = max(0, left - out[g])
+    return out
+
+
 class Group(NamedTuple):
     """One eigensolver call's problems (a panel group's: calls).  ``kind``: the one-CTA kernel's launch shape suffix,
     the cluster size for the cluster path, ("wide", n, real) for the device-wide path, or route_auto's ("small", class)
@@ -571,9 +585,6 @@ class Group(NamedTuple):
     max_n: int
     parts: tuple = ()
     sms: int = 0
-
-
-VEC_SCRATCH = 512 << 20      # device bytes of the inverse iteration's scratch per group
 
 
 SMALL_MAX_N = 64            # up to here the shared-memory eigensolver (csrc/eigh_small.cu, which takes 96)
@@ -619,6 +630,11 @@ def route_wide(prob_n: np.ndarray, threshold: Optional[int]) -> np.ndarray:
     if threshold is None:
         return np.zeros(len(prob_n), dtype=bool)
     return prob_n.astype(np.int64) > int(threshold)
+
+
+def _one_cta_shape(n: int) -> str:
+    from .autotune import Tuning
+    return Tuning.one_cta().shape_for(n)
 
 
 def _default_tuning():
@@ -845,32 +861,20 @@ class Engine:
         """Eigenvalues, and the eigenvectors into ``vec`` where it is given (``tri``: 4 doubles per eigenvalue)."""
         plan = db.plan
         n_prob = len(plan.prob_n)
-        groups = self._groups(db, vec is not None)
+        # a batch that leaves no room for the scratch it would have goes through with less, in the end (values) with none
+        for budget in (PANELS_SCRATCH, PANELS_SCRATCH >> 4, 0):
+            groups = self._groups(db, vec is not None, budget)
+            try:
+                scratch, vec_scratch = self._scratch(groups, vec is not None, VEC_SCRATCH * budget // PANELS_SCRATCH)
+                break
+            except torch.cuda.OutOfMemoryError:
+                if not budget:
+                    raise
         counters = torch.empty(2 * max(len(groups), 1), dtype=torch.int32, device=self.device)     # each call zeroes its own
         if not groups:
             self._call("skn_eigh_gen_batched", n_prob, ptr(db.n), ptr(db.hs_off), ptr(db.eoff), ptr(db.order),
                        ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(counters), plan.max_n, stream)
             return
-        scratch = {}
-        for gi, g in enumerate(groups):
-            need = ctypes.c_int64(0)
-            if isinstance(g.kind, int):      # a cluster group
-                call("skn_eigh_large_scratch_bytes", g.count, g.max_n, g.kind, ctypes.addressof(need))
-            elif g.parts:
-                need.value = max(nbytes for _, _, _, nbytes, _ in g.parts)
-            elif isinstance(g.kind, tuple) and g.kind[0] == "wide":
-                call("skn_eigh_wide_scratch_bytes", g.count, g.max_n, ctypes.addressof(need))
-            else:
-                continue
-            scratch[gi] = torch.empty(max(need.value // 8, 1), dtype=torch.float64, device=self.device)
-        vec_scratch = []
-        if vec is not None:                  # the inverse iteration takes what it is given, at least one CTA's part
-            for g in groups:
-                need, one = ctypes.c_int64(0), ctypes.c_int64(0)
-                call("skn_eigvec_scratch_bytes", g.count, g.max_n, ctypes.addressof(need))
-                call("skn_eigvec_scratch_bytes", 1, g.max_n, ctypes.addressof(one))
-                nbytes = min(need.value, max(VEC_SCRATCH, one.value))
-                vec_scratch.append(torch.empty(nbytes // 8, dtype=torch.float64, device=self.device))
 
         def launch(gi, g, st):
             if g.parts:
@@ -921,6 +925,31 @@ class Engine:
         for ev in joins:
             main.wait_event(ev)
 
+    def _scratch(self, groups, vectors, vec_budget):
+        """Scratch of each group's eigensolver (by group, where it needs any) and of its inverse iteration."""
+        scratch = {}
+        for gi, g in enumerate(groups):
+            need = ctypes.c_int64(0)
+            if isinstance(g.kind, int):      # a cluster group
+                call("skn_eigh_large_scratch_bytes", g.count, g.max_n, g.kind, ctypes.addressof(need))
+            elif g.parts:
+                need.value = max(nbytes for _, _, _, nbytes, _ in g.parts)
+            elif isinstance(g.kind, tuple) and g.kind[0] == "wide":
+                call("skn_eigh_wide_scratch_bytes", g.count, g.max_n, ctypes.addressof(need))
+            else:
+                continue
+            scratch[gi] = torch.empty(max(need.value // 8, 1), dtype=torch.float64, device=self.device)
+        if not vectors:
+            return scratch, []
+
+        def query(count, max_n):
+            need = ctypes.c_int64(0)
+            call("skn_eigvec_scratch_bytes", count, max_n, ctypes.addressof(need))
+            return need.value
+        # the inverse iteration takes what it is given, at least one CTA's part
+        shares = scratch_shares([query(g.count, g.max_n) for g in groups], [query(1, g.max_n) for g in groups], vec_budget)
+        return scratch, [torch.empty(n // 8, dtype=torch.float64, device=self.device) for n in shares]
+
     def _side_streams(self, k):
         """k side streams for forked launches, cached per host thread and device (engines are
         created per batch by the server; creating streams per batch would cost more than the fork)."""
@@ -932,13 +961,14 @@ class Engine:
             cur.append(torch.cuda.Stream(self.device))
         return cur
 
-    def _groups(self, db, vectors: bool = False):
+    def _groups(self, db, vectors: bool = False, budget: int = PANELS_SCRATCH):
         """The batch's eigensolver groups ([Group], empty when every problem takes the default single-CTA launch), kept
         on the batch by all that decides them.  None is ever dropped or changed: a captured graph reads their arrays.
-        With ``vectors`` every problem takes route_auto's kernel: the others keep no reflectors."""
+        With ``vectors`` every problem takes route_auto's kernel: the others keep no reflectors.  ``budget``: bytes of
+        scratch for the panel kernels; without any, values alone take the one-CTA kernel, which needs none."""
         plan = db.plan
         tuned = None if self.tuning is None else tuple(sorted(self.tuning.choice.items()))
-        key = (vectors, tuned, self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
+        key = (vectors, budget, tuned, self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
         if key in db.groups:
             return db.groups[key]
         wide = route_wide(plan.prob_n, None if vectors else self.wide_threshold)[plan.order]
@@ -966,6 +996,8 @@ class Engine:
             at = np.searchsorted(ns, sizes)
             names = ["auto" if vectors else tuning.shape_for(int(n)) for n in ns]
             names = [route_auto(int(n)) if x == "auto" else x for n, x in zip(ns, names)]
+            if not (budget or vectors):
+                names = [_one_cta_shape(int(n)) if x[0] == "panels" else x for n, x in zip(ns, names)]
             kinds = list(dict.fromkeys(names))
             kind = np.array([kinds.index(x) for x in names])[at]
             if self.real_path and plan.prob_real is not None:     # one-CTA shapes: real problems in a call of their own
@@ -983,12 +1015,16 @@ class Engine:
         out = [out[i] for i in launch_order([g[1] for g in out], plan.prob_n, real)]
         cost = [float((plan.prob_n[sel].astype(np.float64) ** 3).sum()) for _, sel, _, _ in out]
         sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+        sizes = {i: np.ascontiguousarray(plan.prob_n[sel].astype(np.int32)) for i, (kind, sel, _, _) in enumerate(out)
+                 if isinstance(kind, tuple) and kind[0] == "panels"}
+        most = [panels_parts(z, 1 << 62) for z in sizes.values()]
+        share = dict(zip(sizes, scratch_shares([sum(part[3] for part in m) for m in most],
+                                               [panels_scratch_bytes(z[0]) for z in sizes.values()], budget)))
         groups = []
-        for (kind, sel, cnt, mx), c in zip(out, cost):
+        for i, ((kind, sel, cnt, mx), c) in enumerate(zip(out, cost)):
             parts = ()
-            if isinstance(kind, tuple) and kind[0] == "panels":
-                sizes = np.ascontiguousarray(plan.prob_n[sel].astype(np.int32))
-                parts = tuple((a, b, w, nbytes, sizes[a:b]) for a, b, w, nbytes in panels_parts(sizes, PANELS_SCRATCH))
+            if i in sizes:
+                parts = tuple((a, b, w, nbytes, sizes[i][a:b]) for a, b, w, nbytes in panels_parts(sizes[i], share[i]))
             # the groups run beside one another: each plans for the SMs of its part of the batch's n^3
             groups.append(Group(kind, sel, cnt, mx, parts, max(1, round(sms * c / max(sum(cost), 1.0)))))
         if not groups:

@@ -57,3 +57,47 @@ def test_a_solve_with_vectors_leaves_what_a_captured_graph_reads():
     assert all(r() is not None and torch.equal(r(), v) for r, v in zip(first, values))
     eng.tuning = None
     assert [id(t) for t in _arrays(eng._groups(db))] == [id(r()) for r in first]
+
+
+def test_scratch_of_all_groups_stays_within_the_budget():
+    gib = 1 << 30
+    assert E.scratch_shares([3, 1, 2], [1, 1, 1], 10) == [3, 1, 2]
+    assert E.scratch_shares([8 * gib, gib, 20 * gib], [1, 1, 1], 16 * gib) == [7.5 * gib, gib, 7.5 * gib]
+    assert E.scratch_shares([8, 9], [5, 6], 0) == [5, 6]       # never less than one problem's
+    assert E.scratch_shares([], [], 5) == []
+    rng = np.random.default_rng(1)
+    for _ in range(50):
+        need = [int(x) for x in rng.integers(1, 1 << 34, rng.integers(1, 32))]
+        least = [min(n, 50 << 20) for n in need]
+        got = E.scratch_shares(need, least, 16 * gib)
+        assert sum(got) <= 16 * gib + sum(least) and all(a <= b for a, b in zip(got, need))
+
+
+@pytest.mark.parametrize("budget", [E.PANELS_SCRATCH, 64 << 20, 4 << 20])
+@pytest.mark.parametrize("vectors", [False, True])
+def test_parts_cover_every_problem_once_within_their_scratch(budget, vectors):
+    db = _batch((8, 12, 20, 40, 64), nk=20)
+    groups = _engine()._groups(db, vectors, budget)
+    seen = np.concatenate([g.order.numpy() for g in groups])
+    assert sorted(seen) == list(range(len(db.plan.prob_n)))
+    held = 0
+    for g in groups:
+        assert bool(g.parts) == (g.kind[0] == "panels")
+        at = 0
+        for first, last, off, nbytes, sizes in g.parts:
+            assert first == at and np.array_equal(sizes, db.plan.prob_n[g.order.numpy()[first:last]])
+            per = np.array([E.panels_scratch_bytes(n) for n in sizes])
+            assert off[0] == 0 and np.array_equal(off.numpy(), np.cumsum(per) - per) and nbytes == per.sum()
+            at = last
+        assert not g.parts or at == g.count
+        held += max((p[3] for p in g.parts), default=0)
+    least = sum(E.panels_scratch_bytes(g.max_n) for g in groups if g.parts)
+    assert held <= max(budget, least)
+
+
+def test_without_scratch_values_take_the_one_cta_kernel():
+    db = _batch((2, 12, 40))
+    kinds = {g.kind for g in _engine()._groups(db, False, 0)}
+    assert not any(k[0] == "panels" for k in kinds if isinstance(k, tuple))
+    assert {"_blk"} & kinds or {"_real_blk"} & kinds
+    assert any(g.parts for g in _engine()._groups(db, True, 0))        # vectors: one problem at a time
