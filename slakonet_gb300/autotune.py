@@ -1,12 +1,13 @@
-"""Launch-shape autotuner for the batched eigensolver.
+"""Autotuner of the eigensolver.
 
-The library holds the eigensolver in three launch shapes (64, 128 and 256
-threads per CTA, each with its own CTAs-per-SM, unroll and shared-memory
-staging size; see ``build.EIG_SHAPES``).  ``autotune`` times every shape on
-random Hermitian-definite problems at the upper edge of each problem-size
-bucket and keeps the fastest; the result is cached as JSON per GPU and
-library build.  ``Engine`` then runs each bucket's problems with its shape,
-the groups on forked streams so they share the GPU.
+Problems take the small or the panel kernels by default (``engine.route_auto``);
+the library also holds the one-CTA kernel in several launch shapes (threads per
+CTA, each with its own CTAs-per-SM, unroll and shared-memory staging size; see
+``build.EIG_SHAPES``).  ``autotune`` times all of them on random
+Hermitian-definite problems at the upper edge of each problem-size bucket and
+keeps the fastest; the result is cached as JSON per GPU and library build.
+``Engine`` then runs each bucket's problems so, the groups on forked streams so
+they share the GPU.
 """
 from __future__ import annotations
 
@@ -27,7 +28,7 @@ from ._lib import call, ptr
 
 SHAPES = ["", "_t32", "_t64", "_t256", "_blk"]  # export suffixes; "" is the 128-thread default, "_blk" the blocked one
 BUCKETS = [16, 32, 64, 128, 256, 512, 1024, 2048]
-# Shape of the untuned default: skn_eigh_gen_small up to 96 orbitals, skn_eigh_gen_panels above (engine.route_auto).
+# The untuned default: skn_eigh_gen_small up to 64 orbitals, skn_eigh_gen_panels above (engine.route_auto).
 AUTO = "auto"
 # The one-CTA kernel's own policy: the blocked Cholesky and reduction above 128 orbitals, where it measured 18-20%
 # faster on GB300 (n = 200-492); below, its unblocked form is faster (the panels are too short to pay).
@@ -44,6 +45,13 @@ class Tuning:
             if n <= u:
                 return self.choice.get(u, "")
         return ""
+
+    def policy_for(self, n: int) -> str:
+        """What the engine runs problems of ``n`` orbitals on: the tuned shape, AUTO where nothing was tuned."""
+        for u in BUCKETS:
+            if n <= u:
+                return self.choice.get(u, AUTO)
+        return AUTO
 
     def to_json(self) -> dict:
         return {"choice": {str(k): v for k, v in self.choice.items()}, "timings": self.timings}
@@ -83,15 +91,39 @@ def _problems(n: int, count: int, device, seed: int = 0):
     return H.transpose(1, 2).contiguous(), S.transpose(1, 2).contiguous()
 
 
-def time_shape(suffix: str, n: int, count: int, device, reps: int = 2) -> float:
-    H0, S0 = _problems(n, count, device)
+def _solver(suffix: str, n: int, count: int, device):
+    """The call that solves ``count`` problems of n orbitals, packed one after another, with ``suffix`` (a one-CTA shape
+    or AUTO): a function of H, S, eig, status and the stream."""
+    from . import engine as E
     nv = torch.full((count,), n, dtype=torch.int32, device=device)
     off = torch.arange(count, dtype=torch.int64, device=device) * n * n
     eoff = torch.arange(count, dtype=torch.int64, device=device) * n
     order = torch.arange(count, dtype=torch.int32, device=device)
+    if suffix != AUTO:
+        ctr = torch.zeros(2, dtype=torch.int32, device=device)
+        return lambda H, S, eig, st, stream: call("skn_eigh_gen_batched" + suffix, count, ptr(nv), ptr(off), ptr(eoff),
+                                                  ptr(order), ptr(H), ptr(S), ptr(eig), ptr(st), ptr(ctr), n, stream)
+    if E.route_auto(n)[0] == "small":
+        return lambda H, S, eig, st, stream: call("skn_eigh_gen_small", count, n, ptr(order), ptr(nv), 0, ptr(off),
+                                                  ptr(eoff), ptr(H), ptr(S), ptr(eig), ptr(st), 0, stream)
+    sizes = np.full(count, n, dtype=np.int32)
+    parts = [(a, b, torch.as_tensor(w, device=device), nbytes)
+             for a, b, w, nbytes in E.panels_parts(sizes, E.PANELS_SCRATCH)]
+    scratch = torch.empty(max(p[3] for p in parts) // 8, dtype=torch.float64, device=device)
+
+    def panels(H, S, eig, st, stream):
+        for a, b, w, nbytes in parts:
+            call("skn_eigh_gen_panels", b - a, sizes[a:].ctypes.data, ptr(order[a:]), ptr(w), ptr(nv), 0, ptr(off),
+                 ptr(eoff), ptr(H), ptr(S), ptr(eig), ptr(st), 0, ptr(scratch), nbytes, 0, stream)
+    return panels
+
+
+def time_shape(suffix: str, n: int, count: int, device, reps: int = 2) -> float:
+    """Seconds for ``count`` random problems of n orbitals on a one-CTA shape or AUTO, the best of ``reps``."""
+    H0, S0 = _problems(n, count, device)
+    solve = _solver(suffix, n, count, device)
     eig = torch.empty(count * n, dtype=torch.float64, device=device)
     st = torch.empty(count, dtype=torch.int32, device=device)
-    ctr = torch.zeros(2, dtype=torch.int32, device=device)
     stream = torch.cuda.current_stream(device).cuda_stream
     best = float("inf")
     for r in range(reps + 1):
@@ -101,8 +133,7 @@ def time_shape(suffix: str, n: int, count: int, device, reps: int = 2) -> float:
         a = torch.cuda.Event(enable_timing=True)
         b = torch.cuda.Event(enable_timing=True)
         a.record()
-        call("skn_eigh_gen_batched" + suffix, count, ptr(nv), ptr(off), ptr(eoff), ptr(order), ptr(H), ptr(S),
-             ptr(eig), ptr(st), ptr(ctr), n, stream)
+        solve(H, S, eig, st, stream)
         b.record()
         torch.cuda.synchronize(device)
         if r:
@@ -157,7 +188,8 @@ def buckets_up_to(max_n: int) -> List[int]:
 
 def autotune(device="cuda", cache: Optional[str] = None, budget_s: float = 0.04, use_cache: bool = True,
              buckets: Optional[List[int]] = None) -> Tuning:
-    """Fastest shape per bucket (cached per GPU and library build); buckets not tuned keep the default."""
+    """The fastest of AUTO and the one-CTA shapes per bucket (cached per GPU and library build); buckets not tuned keep
+    the default, AUTO."""
     device = torch.device(device)
     _lib.load()
     cache = cache or default_cache_path()
@@ -177,7 +209,7 @@ def autotune(device="cuda", cache: Optional[str] = None, budget_s: float = 0.04,
         # about budget_s of work at the FP64 rate, at least one problem per SM
         count = int(min(20000, max(sms, budget_s * 0.8e12 / flops)))
         reps = 2 if u <= 512 else 1
-        t = {sfx: time_shape(sfx, u, count, device, reps) for sfx in SHAPES}
+        t = {sfx: time_shape(sfx, u, count, device, reps) for sfx in [AUTO] + SHAPES}
         choice[u] = min(t, key=t.get)
         timings[str(u)] = {(sfx or "_t128"): round(v * 1e3, 3) for sfx, v in t.items()}
     tun = Tuning(choice, timings)

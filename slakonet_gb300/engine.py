@@ -607,6 +607,7 @@ def route_auto(n: int):
 _SIDE = threading.local()   # per-thread side streams of Engine._side_streams
 
 SINGLE_CTA_MAX_N = 2048   # bound of the one-CTA-per-problem eigensolver (csrc/eigh.cu)
+ONE_CTA_LARGE_N = 1024    # above, the device-wide path is 4.6 times as fast and more (cluster_for's figures)
 LARGE_MAX_N = 9216        # bound of the cluster eigensolver (csrc/eigh_cluster.cu)
 
 
@@ -971,9 +972,19 @@ class Engine:
         key = (vectors, budget, tuned, self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
         if key in db.groups:
             return db.groups[key]
-        wide = route_wide(plan.prob_n, None if vectors else self.wide_threshold)[plan.order]
-        csize = (np.zeros(len(plan.order), int) if vectors
-                 else route_large(plan.prob_n, self.large_threshold, self.large_cluster)[plan.order])
+        tuning = self.tuning if self.tuning is not None else _default_tuning()
+        # what a tuning keeps on the one-CTA kernel leaves it above ONE_CTA_LARGE_N, where the device-wide or the cluster
+        # path is on
+        own = [n for n in np.unique(plan.nb) if n > ONE_CTA_LARGE_N and not vectors and tuning.policy_for(int(n)) != "auto"]
+        own = np.isin(plan.prob_n, own) if own else np.zeros(len(plan.prob_n), bool)
+        wide = route_wide(plan.prob_n, None if vectors else self.wide_threshold)
+        wide = (wide | (own & (self.wide_threshold is not None)))[plan.order]
+        csize = np.zeros(len(plan.prob_n), int)
+        if not vectors:
+            csize = route_large(plan.prob_n, self.large_threshold, self.large_cluster)
+            if own.any() and self.large_threshold is not None:
+                csize = np.where(own, route_large(plan.prob_n, ONE_CTA_LARGE_N, self.large_cluster), csize)
+        csize = csize[plan.order]
         csize[wide] = 0
         large = (csize > 0) | wide
         out = []
@@ -989,12 +1000,11 @@ class Engine:
             out.append((int(c), sel, len(sel), int(plan.prob_n[sel].max())))
         small_order = plan.order[~large]
         if len(small_order):
-            tuning = self.tuning if self.tuning is not None else _default_tuning()
             sizes = plan.prob_n[small_order]
             ns = np.unique(plan.nb)                  # of the structures: far fewer than problems
             ns = ns[np.isin(ns, sizes)] if large.any() else ns
             at = np.searchsorted(ns, sizes)
-            names = ["auto" if vectors else tuning.shape_for(int(n)) for n in ns]
+            names = ["auto" if vectors else tuning.policy_for(int(n)) for n in ns]
             names = [route_auto(int(n)) if x == "auto" else x for n, x in zip(ns, names)]
             if not (budget or vectors):
                 names = [_one_cta_shape(int(n)) if x[0] == "panels" else x for n, x in zip(ns, names)]

@@ -101,3 +101,47 @@ def test_without_scratch_values_take_the_one_cta_kernel():
     assert not any(k[0] == "panels" for k in kinds if isinstance(k, tuple))
     assert {"_blk"} & kinds or {"_real_blk"} & kinds
     assert any(g.parts for g in _engine()._groups(db, True, 0))        # vectors: one problem at a time
+
+
+def _routes(sizes, tuning=None, **kw):
+    """{orbitals: kind of its group} of a stub batch with two problems of each size."""
+    n = np.repeat(np.array(sorted(sizes, reverse=True), np.int32), 2)
+    plan = types.SimpleNamespace(prob_n=n, nb=np.unique(n), order=np.arange(len(n)), prob_real=None)
+    db = types.SimpleNamespace(plan=plan, groups={}, order=torch.arange(len(n), dtype=torch.int32))
+    out = {}
+    for g in _engine(tuning=tuning, **kw)._groups(db):
+        out.update({int(n[p]): g.kind for p in g.order.numpy()})
+    return out
+
+
+SIZES = (10, 60, 432, 1500, 3000)
+AUTO_ROUTES = {10: ("small", 16), 60: ("small", 64), 432: ("panels", 7), 1500: ("panels", 24), 3000: ("wide", 3000, 0)}
+
+
+def test_what_was_not_tuned_keeps_the_default_route():
+    assert _routes(SIZES) == AUTO_ROUTES
+    assert _routes(SIZES, AT.Tuning({})) == AUTO_ROUTES
+    assert _routes(SIZES, AT.Tuning({16: "_t64"})) == {**AUTO_ROUTES, 10: "_t64"}
+    assert AT.Tuning({16: "_t64"}).policy_for(9000) == AT.AUTO
+
+
+def test_one_cta_problems_above_1024_orbitals_go_to_the_device_wide_or_the_cluster_path():
+    one = AT.Tuning.one_cta()
+    assert _routes(SIZES, one) == {10: "", 60: "", 432: "_blk", 1500: ("wide", 1500, 0), 3000: ("wide", 3000, 0)}
+    assert _routes(SIZES, one, wide_threshold=None) == {10: "", 60: "", 432: "_blk", 1500: 4, 3000: 8}
+    assert _routes(SIZES, one, wide_threshold=None, large_threshold=None) == {10: "", 60: "", 432: "_blk", 1500: "_blk", 3000: 8}
+    assert _routes(SIZES, None, wide_threshold=400)[432] == ("wide", 432, 0)
+
+
+def test_the_autotuner_times_the_default_route_too(monkeypatch, tmp_path):
+    asked = []
+
+    def timed(suffix, n, count, device, reps=2):
+        asked.append((suffix, n))
+        return {AT.AUTO: 1.0, "_blk": 0.5 if n == 512 else 2.0}.get(suffix, 3.0)
+    monkeypatch.setattr(AT, "time_shape", timed)
+    monkeypatch.setattr(AT, "_cache_key", lambda d: "k")
+    monkeypatch.setattr(AT._lib, "load", lambda: None)
+    tun = AT.autotune("cpu", cache=str(tmp_path / "t.json"), buckets=[64, 512])
+    assert tun.choice == {64: AT.AUTO, 512: "_blk"} and {s for s, _ in asked} == {AT.AUTO, *AT.SHAPES}
+    assert AT.autotune("cpu", cache=str(tmp_path / "t.json"), buckets=[64, 512]).choice == tun.choice
