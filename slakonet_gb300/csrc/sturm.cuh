@@ -26,12 +26,32 @@ __device__ __forceinline__ int sign_bit(double v) { return (int)((unsigned long 
 // Exponent field of |v| (biased), for power-of-two rescaling.
 __device__ __forceinline__ int exp_field(double v) { return (int)((__double_as_longlong(v) >> 52) & 0x7ff); }
 
+__device__ __forceinline__ int clz64(unsigned long long v) {
+#ifdef __CUDA_ARCH__
+  return __clzll((long long)v);
+#else
+  return __builtin_clzll(v);
+#endif
+}
+// v 2^s where v, or the result, is subnormal or out of range: what falls below is cut off, what exceeds is infinite.
+__device__ inline double shift_exp_edge(double v, int s) {
+  const unsigned long long b = (unsigned long long)__double_as_longlong(v), sign = b & 0x8000000000000000ull;
+  const int e = (int)((b >> 52) & 0x7ff);
+  unsigned long long f = b & 0xfffffffffffffull;
+  if (e == 0x7ff || (e == 0 && f == 0)) return v;
+  const int z = e == 0 ? clz64(f) - 11 : 0;
+  f = e == 0 ? f << z : f | 0x10000000000000ull;
+  const int t = (e == 0 ? 1 - z : e) + s;
+  if (t >= 0x7ff) return __longlong_as_double((long long)(sign | 0x7ff0000000000000ull));
+  if (t <= 0) return __longlong_as_double((long long)(sign | (t > -52 ? f >> (1 - t) : 0)));
+  return __longlong_as_double((long long)(sign | ((unsigned long long)t << 52) | (f & 0xfffffffffffffull)));
+}
 // v 2^s by its exponent field, so that the rescaling below, which a compiler may execute on every step, stays off the
-// FP64 pipe.  What falls below the normal range is zero; infinities and NaNs stay.
+// FP64 pipe.
 __device__ __forceinline__ double shift_exp(double v, int s) {
-  const int h = __double2hiint(v), e = (h >> 20) & 0x7ff;
-  if (e == 0x7ff) return v;
-  return e == 0 || e + s <= 0 ? 0.0 : __hiloint2double(h + (s << 20), __double2loint(v));
+  const int h = __double2hiint(v), e = (h >> 20) & 0x7ff, t = e + s;
+  if (e != 0 && e != 0x7ff && t > 0 && t < 0x7ff) return __hiloint2double(h + (int)((unsigned)s << 20), __double2loint(v));
+  return shift_exp_edge(v, s);
 }
 
 // Number of eigenvalues below x: sign changes of the determinant sequence
