@@ -14,7 +14,7 @@
 //     nearly linear, so two more evaluations (three FP64 operations per row, against
 //     five for one with the derivative) replace ~28 bisection steps.
 //  4. Clustered or degenerate eigenvalues (the bracket holds several) are
-//     bisected in FP64 to 1e-14 of the scale.
+//     bisected in FP64 to 2e-15 of the scale.
 #pragma once
 #include "skn_common.cuh"
 
@@ -157,7 +157,7 @@ __device__ __forceinline__ Bounds make_bounds(double lo, double hi, double emax,
   const double bnorm = fmax(fmax(fabs(lo), fabs(hi)), 1e-300);
   B.lo = lo - (2.2e-16 * bnorm * 4.0 * n + 1e-300);
   B.hi = hi + (2.2e-16 * bnorm * 4.0 * n + 1e-300);
-  B.atol = 1e-14 * bnorm;
+  B.atol = 2e-15 * bnorm;
   B.pivmin32 = 1.1754944e-38f * fmaxf(1.0f, (float)emax);
   B.margin = 32.0 * 5.9604645e-8 * bnorm;   // covers FP32 rounding of T and of the count
   return B;
