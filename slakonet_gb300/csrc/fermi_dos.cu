@@ -398,7 +398,7 @@ __global__ void __cluster_dims__(1, 1, skn_gauss::Z) __launch_bounds__(skn_gauss
           const double* __restrict__ muv, double e_lo, double e_hi, int npts, double sigma, double window,
           double* __restrict__ grid, double* __restrict__ dos) {
   namespace sg = skn_gauss;
-  __shared__ double part[sg::SL * sg::PTS];
+  __shared__ double part[sg::SL * sg::PTS], xg[sg::PTS];
   const int s = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int p0 = blockIdx.x * sg::PTS;
   const int nk = nkv[s], nb = nbv[s];
@@ -408,8 +408,8 @@ __global__ void __cluster_dims__(1, 1, skn_gauss::Z) __launch_bounds__(skn_gauss
   const double inv_norm = 1.0 / (sigma * sqrt(2.0 * 3.141592653589793));
   sg::Lane L;
   const int i0 = p0 + lane * sg::DG;
-  sg::lane_init(L, sg::lin_grid(e_lo, e_hi, npts, min(i0, npts - 1)), mu * H2E, e_lo, e_hi, npts, sigma, H2E,
-                WINDOWED ? window : INFINITY);
+  sg::cta_points(xg, p0, e_lo, e_hi, npts, 0.0);
+  sg::lane_init(L, xg + lane * sg::DG, mu, e_lo, e_hi, npts, sigma, H2E, WINDOWED ? window : INFINITY);
   const int slice = blockIdx.z * sg::SL + warp;
   const int parts = max(1, sg::SLICES / max(nk, 1));
   const int part_id = slice % parts;
@@ -442,9 +442,10 @@ __global__ void __cluster_dims__(1, 1, skn_gauss::Z) __launch_bounds__(skn_gauss
       }
     }
   }
-  const double v = sg::cluster_total(L, part);
+  double v = sg::cluster_total(L, part);
+  if (blockIdx.z == 0) v = sg::at_grid(L, xg, v, e_lo, e_hi, npts, part);
   if (blockIdx.z == 0 && p0 + tid < npts) {
-    if (s == 0) grid[p0 + tid] = sg::lin_grid(e_lo, e_hi, npts, p0 + tid);
+    if (s == 0) grid[p0 + tid] = xg[tid];
     dos[(int64_t)s * npts + p0 + tid] = mu == mu ? v : qnan();
   }
 }

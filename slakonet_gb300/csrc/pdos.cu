@@ -40,12 +40,12 @@ __global__ void __cluster_dims__(1, 1, skn_gauss::Z) __launch_bounds__(skn_gauss
            double e_lo, double e_hi, int npts, double sigma, double h2e, double* __restrict__ grid,
            double* __restrict__ pdos) {
   namespace sg = skn_gauss;
-  __shared__ double part[sg::SL * sg::PTS];
+  __shared__ double part[sg::SL * sg::PTS], xg[sg::PTS];
   const int g = blockIdx.y, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int p0 = blockIdx.x * sg::PTS, i0 = p0 + lane * sg::DG;
   sg::Lane L;
-  sg::lane_init(L, sg::lin_grid(e_lo, e_hi, npts, min(i0, npts - 1)), fermi_ev, e_lo, e_hi, npts, sigma, h2e,
-                INFINITY);
+  sg::cta_points(xg, p0, e_lo, e_hi, npts, fermi_ev);
+  sg::lane_init(L, xg + lane * sg::DG, 0.0, e_lo, e_hi, npts, sigma, h2e, INFINITY);
   const int slice = blockIdx.z * sg::SL + warp;
   const int parts = max(1, sg::SLICES / nk);
   if (i0 < npts) {
@@ -54,7 +54,8 @@ __global__ void __cluster_dims__(1, 1, skn_gauss::Z) __launch_bounds__(skn_gauss
       for (int b = slice % parts; b < nb; b += parts) sg::add_band<false>(L, eig[kb + b], w[(kb + b) * n_group + g]);
     }
   }
-  const double v = sg::cluster_total(L, part);
+  double v = sg::cluster_total(L, part);
+  if (blockIdx.z == 0) v = sg::at_grid(L, xg, v, e_lo, e_hi, npts, part);
   if (blockIdx.z == 0 && p0 + tid < npts) {
     if (g == 0) grid[p0 + tid] = sg::lin_grid(e_lo, e_hi, npts, p0 + tid);
     const double norm = 1.0 / (sigma * sqrt(2.0 * 3.141592653589793));
