@@ -110,3 +110,26 @@ SKN_HD double round_wide28(long long h, long long m, int k) {
   if (be <= 0 || be >= 2046) return ldexp((double)(neg ? -(long long)t : (long long)t), 11 - z + k);
   return skn_bits_to_double((neg ? 0x8000000000000000ull : 0ull) + ((unsigned long long)be << 52) + (t - 0x10000000000000ull));
 }
+
+// a / b from b's rounded reciprocal: the product corrected by its remainder (Markstein, IBM J. Res. Dev. 34, 1990), which
+// leaves the quotient's own rounding for normal operands.  An infinite or NaN product is the quotient.
+SKN_HD double skn_quotient(double a, double b, double inv_b) {
+  const double q = a * inv_b;
+  const double c = fma(fma(-q, b, a), inv_b, q);
+#ifdef __CUDA_ARCH__
+  return (__double2hiint(q) & 0x7fffffff) < 0x7ff00000 ? c : q;      // not on the FP64 pipe
+#else
+  return fabs(q) <= 1.7976931348623157e308 ? c : q;
+#endif
+}
+
+// 1 / b to twice the working precision (the remainder of the reciprocal is exact), and a / b by it for finite a: the two
+// products are rounded together, so the result is off by its own rounding alone.  Two instructions where many a share a b.
+struct SknRecip {
+  double hi, lo;
+};
+SKN_HD SknRecip skn_recip(double b) {
+  const double hi = 1.0 / b;
+  return {hi, fma(-hi, b, 1.0) * hi};
+}
+SKN_HD double skn_over(double a, SknRecip r) { return fma(a, r.hi, a * r.lo); }
