@@ -719,7 +719,7 @@ __device__ void tridiag_eigenvalues(int n, Vecs& V, double* out) {
     const double eb = (i < n - 1) ? sqrt(V.e2[i]) : 0.0;
     lo = fmin(lo, V.d[i] - ea - eb);
     hi = fmax(hi, V.d[i] + ea + eb);
-    if (i < n - 1) emax = fmax(emax, V.e2[i]);
+    emax = fmax(emax, skn_sturm::row_max(V.d[i], i < n - 1 ? V.e2[i] : 0.0));
     V.d32[i] = (float)V.d[i];
     V.e232[i] = (float)V.e2[i];
   }

@@ -496,7 +496,7 @@ __global__ void __launch_bounds__(CNT, 1) k_eigh_cluster(int n_prob, const int32
       const double eb = (i < n - 1) ? sqrt(se2[i]) : 0.0;
       lo = fmin(lo, sd[i] - ea - eb);
       hi = fmax(hi, sd[i] + ea + eb);
-      if (i < n - 1) emax = fmax(emax, se2[i]);
+      emax = fmax(emax, skn_sturm::row_max(sd[i], i < n - 1 ? se2[i] : 0.0));
     }
     for (int o = 16; o > 0; o >>= 1) {
       lo = fmin(lo, __shfl_xor_sync(0xffffffffu, lo, o));

@@ -1623,7 +1623,7 @@ __global__ void __launch_bounds__(256) k_bounds(Grp G) {
     const double eb = (i < n - 1) ? sqrt(w.e2[i]) : 0.0;
     lo = fmin(lo, w.d[i] - ea - eb);
     hi = fmax(hi, w.d[i] + ea + eb);
-    if (i < n - 1) emax = fmax(emax, w.e2[i]);
+    emax = fmax(emax, skn_sturm::row_max(w.d[i], i < n - 1 ? w.e2[i] : 0.0));
     w.d32[i] = (float)w.d[i];
     w.e232[i] = (i < n - 1) ? (float)w.e2[i] : 0.0f;
   }

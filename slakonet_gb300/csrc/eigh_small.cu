@@ -393,7 +393,7 @@ SKN_DEVINL void eigenvalues(const Shared<T>& m, int n, double* out) {
     const double eb = (i < n - 1) ? sqrt(m.e2[i]) : 0.0;
     lo = fmin(lo, m.d[i] - ea - eb);
     hi = fmax(hi, m.d[i] + ea + eb);
-    if (i < n - 1) emax = fmax(emax, m.e2[i]);
+    emax = fmax(emax, skn_sturm::row_max(m.d[i], i < n - 1 ? m.e2[i] : 0.0));
     d32[i] = (float)m.d[i];
     e232[i] = i < n - 1 ? (float)m.e2[i] : 0.0f;
   }

@@ -152,8 +152,17 @@ struct Bounds {
   float pivmin32;
 };
 
+// A row's part of `emax` below: its squared coupling, infinite where that or the diagonal is an infinity or a NaN (minima
+// and maxima pass over NaNs).
+__device__ __forceinline__ double row_max(double d, double e2) {
+  const double inf = __longlong_as_double(0x7ff0000000000000LL);
+  return exp_field(d) == 0x7ff || exp_field(e2) == 0x7ff ? inf : e2;
+}
+
+// lo, hi: Gershgorin's; emax: the largest of row_max.  An infinite emax makes every eigenvalue NaN.
 __device__ __forceinline__ Bounds make_bounds(double lo, double hi, double emax, int n) {
   Bounds B;
+  if (exp_field(emax) == 0x7ff) lo = __longlong_as_double(0x7ff8000000000000LL);
   const double bnorm = fmax(fmax(fabs(lo), fabs(hi)), 1e-300);
   B.lo = lo - (2.2e-16 * bnorm * 4.0 * n + 1e-300);
   B.hi = hi + (2.2e-16 * bnorm * 4.0 * n + 1e-300);
@@ -166,6 +175,7 @@ __device__ __forceinline__ Bounds make_bounds(double lo, double hi, double emax,
 // Eigenvalue j (0-based, ascending) of the tridiagonal.
 __device__ double eigenvalue(const double* d, const double* e2, const float* d32, const float* e232, int n, int j,
                              const Bounds& B) {
+  if (!(B.lo <= B.hi)) return __longlong_as_double(0x7ff8000000000000LL);
   float a32 = (float)B.lo, b32 = (float)B.hi;
   const float enough = 0.25f * (float)B.margin;      // the bracket is widened by the margin anyway
   for (int it = 0; it < 26 && b32 - a32 > enough; ++it) {
