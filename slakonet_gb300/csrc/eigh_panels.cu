@@ -386,6 +386,7 @@ __global__ void __launch_bounds__(256) k_potrf(Grp G, int c0) {
       const int k = kb * 8 + kq;
       if (k >= w) break;
       if (warp == kq) {
+        // root and reciprocal as in the small eigensolver: a reciprocal root and one Newton step on the root
         const double akk = __shfl_sync(0xffffffffu, a[kb].x, k);
         const bool ok = akk > 0.0 && is_finite_bits(akk);
         const double q = ok ? akk : 1.0, r = rsqrt(q), r0 = q * r;
@@ -1164,7 +1165,7 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
       const double xnorm2 = warp_sum<true>(make_double2(s, 0.0)).x;
       const bool triv = xnorm2 == 0.0 && al.y == 0.0;
       const double q = triv ? 1.0 : fma(al.x, al.x, fma(al.y, al.y, xnorm2));
-      const double inv = rsqrt(q), r0 = q * inv;                 // a root and its reciprocal from one instruction chain
+      const double inv = rsqrt(q), r0 = q * inv;                 // a root (one Newton step) and its reciprocal from one chain
       const double nrm = fma(fma(-r0, r0, q), 0.5 * inv, r0);
       const bool up = al.x >= 0.0;
       const double beta = triv ? al.x : (up ? -nrm : nrm), ib = up ? -inv : inv;

@@ -87,8 +87,9 @@ SKN_DEVINL void aux_zero_rows(const Shared<T>& m, int n) {
   }
 }
 
-// sqrt(a) and 1 / sqrt(a) from one reciprocal root (600 clocks; a root and a quotient are 830 + 550), the root
-// with one correction step.
+// sqrt(a) and 1 / sqrt(a) from one reciprocal root (600 clocks; a root and a quotient are 830 + 550): inv is off by its own
+// last place, the root a inv takes one Newton step on r^2 = a, r + (a - r^2) inv / 2, which squares that error, so the root
+// is the rounded one or its neighbour.  A column is scaled by inv: within two last places of the quotient by the root.
 SKN_DEVINL void roots(double a, double& root, double& inv) {
   inv = rsqrt(a);
   const double r = a * inv;
