@@ -1707,6 +1707,7 @@ int clusters_at_once(bool resident, int C, int per_sm, int sms) {
     cfg.gridDim = dim3((unsigned)C * sms);
     cfg.blockDim = dim3(resident ? PTR : PT);
     cfg.dynamicSmemBytes = SMEM_MAX / per_sm - 2048;
+    if (!resident) cfg.dynamicSmemBytes = std::min(cfg.dynamicSmemBytes, panel_smem(PANELS_MAX_N, 0, 0));    // its limit
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
     at[0].val.clusterDim.x = C;
