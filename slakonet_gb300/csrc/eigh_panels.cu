@@ -1093,6 +1093,14 @@ struct Team {
   }
 };
 
+// v 2^k for the two operands below, which meet near the root of the matrix's scale: no overflow; what falls below the normal
+// range is far below the row's largest entry and counts as zero.
+SKN_DEVINL double halfway(double v, int k) {
+  const int h = __double2hiint(v), e = (h >> 20) & 0x7ff;
+  if (e == 0x7ff) return v;
+  return e == 0 || e + k <= 0 ? 0.0 : __hiloint2double(h + (int)((unsigned)k << 20), __double2loint(v));
+}
+
 // sv: the Householder vector, svf: the same in fixed point, sve: its exponents by 32 rows; big: streamed, a quarter of a
 // tile per warp; RES, tiles (rt), chunks of [W V] (cpc) and their partial sums (2 x cpc x PW x 32).
 template <bool R, bool RES>
@@ -1576,7 +1584,7 @@ SKN_DEVINL void panel_body(const Grp& G, int g, int p, int c0, Team& team, int r
         const int q = part * SE + e;
         const int k = q < NT ? half : -half;
         z[e] = mine && (q & (NT - 1)) < w ? vw[q ^ NT] : zero2();
-        z[e] = make_double2(skn_sturm::shift_exp(z[e].x, k), R ? 0.0 : skn_sturm::shift_exp(z[e].y, k));
+        z[e] = make_double2(halfway(z[e].x, k), R ? 0.0 : halfway(z[e].y, k));
       }
       hms[warp * 32 + lane] = high_word8(z);
       __syncthreads();
@@ -1602,7 +1610,8 @@ __global__ void __launch_bounds__(RES ? PTR : PT, RES ? 1 : 4) k_tri_panel(Grp G
   double2* big = reinterpret_cast<double2*>(svf + rows);
   int* sve = reinterpret_cast<int*>(smem_raw + sve_off);
   if (threadIdx.x == 0) sm.dead = 0;
-  Team team{(int)(blockIdx.x % C), C, G.limits.team, grid != 0, ws_of(G, g).bar + c0 / NT, 0u, G.status + p, &sm.dead};
+  // grid teams are resident (plan_panel)
+  Team team{(int)(blockIdx.x % C), C, G.limits.team, RES && grid != 0, ws_of(G, g).bar + c0 / NT, 0u, G.status + p, &sm.dead};
   if (is_real(G, p))
     panel_body<true, RES>(G, g, p, c0, team, rt, cpc, sm, sv, svf, sve, big);
   else
