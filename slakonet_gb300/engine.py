@@ -973,18 +973,18 @@ class Engine:
         if key in db.groups:
             return db.groups[key]
         tuning = self.tuning if self.tuning is not None else _default_tuning()
-        # what a tuning keeps on the one-CTA kernel leaves it above ONE_CTA_LARGE_N, where the device-wide or the cluster
-        # path is on
-        own = [n for n in np.unique(plan.nb) if n > ONE_CTA_LARGE_N and not vectors and tuning.policy_for(int(n)) != "auto"]
-        own = np.isin(plan.prob_n, own) if own else np.zeros(len(plan.prob_n), bool)
-        wide = route_wide(plan.prob_n, None if vectors else self.wide_threshold)
-        wide = (wide | (own & (self.wide_threshold is not None)))[plan.order]
-        csize = np.zeros(len(plan.prob_n), int)
+        wide, csize = np.zeros(len(plan.prob_n), bool), np.zeros(len(plan.prob_n), int)
         if not vectors:
+            wide = route_wide(plan.prob_n, self.wide_threshold)
             csize = route_large(plan.prob_n, self.large_threshold, self.large_cluster)
-            if own.any() and self.large_threshold is not None:
-                csize = np.where(own, route_large(plan.prob_n, ONE_CTA_LARGE_N, self.large_cluster), csize)
-        csize = csize[plan.order]
+            # above ONE_CTA_LARGE_N: what a tuning keeps on the one-CTA kernel leaves it, for the cluster or the device-wide
+            # path, and what the cluster path would take goes to the device-wide one, where those are on
+            own = [n for n in np.unique(plan.nb) if n > ONE_CTA_LARGE_N and tuning.policy_for(int(n)) != "auto"]
+            if own and self.large_threshold is not None:
+                csize = np.where(np.isin(plan.prob_n, own), route_large(plan.prob_n, ONE_CTA_LARGE_N, self.large_cluster), csize)
+            if self.wide_threshold is not None:
+                wide |= (plan.prob_n > ONE_CTA_LARGE_N) & (np.isin(plan.prob_n, own) | (csize > 0))
+        wide, csize = wide[plan.order], csize[plan.order]
         csize[wide] = 0
         large = (csize > 0) | wide
         out = []

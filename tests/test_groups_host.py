@@ -131,6 +131,10 @@ def test_one_cta_problems_above_1024_orbitals_go_to_the_device_wide_or_the_clust
     assert _routes(SIZES, one, wide_threshold=None) == {10: "", 60: "", 432: "_blk", 1500: 4, 3000: 8}
     assert _routes(SIZES, one, wide_threshold=None, large_threshold=None) == {10: "", 60: "", 432: "_blk", 1500: "_blk", 3000: 8}
     assert _routes(SIZES, None, wide_threshold=400)[432] == ("wide", 432, 0)
+    # the cluster path between its threshold and 1024 orbitals, where the device-wide one is on
+    mid = SIZES + (800,)
+    assert _routes(mid, None, large_threshold=600) == {**AUTO_ROUTES, 800: 4, 1500: ("wide", 1500, 0)}
+    assert _routes(mid, None, large_threshold=600, wide_threshold=None) == {**AUTO_ROUTES, 800: 4, 1500: 4, 3000: 8}
 
 
 def test_the_autotuner_times_the_default_route_too(monkeypatch, tmp_path):
