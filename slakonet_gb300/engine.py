@@ -914,17 +914,19 @@ class Engine:
         main = torch.cuda.current_stream(self.device)
         fork = torch.cuda.Event()
         fork.record(main)
-        joins = []
-        for gi, g in enumerate(groups):
-            st = self._side_streams(len(groups))[gi]
-            st.wait_event(fork)
-            with torch.cuda.stream(st):
-                launch(gi, g, st.cuda_stream)
-            ev = torch.cuda.Event()
-            ev.record(st)
-            joins.append(ev)
-        for ev in joins:
-            main.wait_event(ev)
+        used = []
+        try:
+            for gi, g in enumerate(groups):
+                st = self._side_streams(len(groups))[gi]
+                st.wait_event(fork)
+                used.append(st)
+                with torch.cuda.stream(st):
+                    launch(gi, g, st.cuda_stream)
+        finally:                             # also where a launch was refused: the buffers are the others' until they end
+            for st in used:
+                ev = torch.cuda.Event()
+                ev.record(st)
+                main.wait_event(ev)
 
     def _scratch(self, groups, vectors, vec_budget):
         """Scratch of each group's eigensolver (by group, where it needs any) and of its inverse iteration."""

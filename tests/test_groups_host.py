@@ -149,3 +149,41 @@ def test_the_autotuner_times_the_default_route_too(monkeypatch, tmp_path):
     tun = AT.autotune("cpu", cache=str(tmp_path / "t.json"), buckets=[64, 512])
     assert tun.choice == {64: AT.AUTO, 512: "_blk"} and {s for s, _ in asked} == {AT.AUTO, *AT.SHAPES}
     assert AT.autotune("cpu", cache=str(tmp_path / "t.json"), buckets=[64, 512]).choice == tun.choice
+
+
+def test_a_refused_launch_leaves_no_side_stream_unjoined(monkeypatch):
+    """The calls of a solve run on side streams and share its buffers: also when one of them is refused, what was launched
+    before it is waited for on the solve's own stream."""
+    import contextlib
+
+    class Stream:
+        cuda_stream = 0
+
+        def __init__(self):
+            self.waits = []
+
+        def wait_event(self, ev):
+            self.waits.append(ev)
+
+    class Event:
+        def record(self, stream=None):
+            self.stream = stream
+    main, sides = Stream(), [Stream() for _ in range(8)]
+    monkeypatch.setattr(torch.cuda, "current_stream", lambda d=None: main)
+    monkeypatch.setattr(torch.cuda, "stream", lambda st: contextlib.nullcontext())
+    monkeypatch.setattr(torch.cuda, "Event", Event)
+    eng = _engine(launches=0, wide_tc=True)
+    eng._side_streams = lambda k: sides
+    calls = []
+
+    def call(name, *args):
+        calls.append(name)
+        if len(calls) == 3:
+            raise E._lib.SknError("refused")
+    eng._call = call
+    db = _batch((2, 8, 20, 40))
+    assert len(eng._groups(db)) >= 4
+    t = torch.zeros(1, dtype=torch.float64)
+    with pytest.raises(E._lib.SknError):
+        eng._eig_values(db, t, t, t, torch.zeros(1, dtype=torch.int32), 0)
+    assert [ev.stream for ev in main.waits] == sides[:3]
