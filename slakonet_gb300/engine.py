@@ -505,8 +505,8 @@ class DeviceBatch:
 
 # kernels each ABI call launches (for the launch count the bench reports)
 KERNELS_PER_CALL = {"skn_bond_counts": 1, "skn_bond_fill": 1, "skn_image_phases": 1, "skn_sk_blocks": 1,
-                    "skn_bloch": 1, "skn_bloch_pairs": 1, "skn_eigh_gen_batched": 1, "skn_eigh_gen_vectors": 2, "skn_fermi_gap": 1,
-                    "skn_dos": 2, "skn_eigvec": 2, "skn_eigh_gen_large": 1, "skn_eigh_gen_vectors_noalloc": 2}
+                    "skn_bloch": 1, "skn_bloch_pairs": 1, "skn_eigh_gen_batched": 1, "skn_eigh_gen_vectors": 3, "skn_fermi_gap": 1,
+                    "skn_dos": 2, "skn_eigvec": 2, "skn_eigh_gen_large": 1, "skn_eigh_gen_vectors_noalloc": 3}
 
 def wide_launches(n: int, nb: int = 32, tc: bool = False, tc_min: int = 512) -> int:
     """Kernel launches of one skn_eigh_gen_wide(_tc) call for problems of n orbitals (its host sequence);
