@@ -1889,7 +1889,11 @@ static int panels_entry(int n_prob, const int32_t* sizes, const int32_t* prob, c
   if (set_attrs() != cudaSuccess) return SKN_ERR_CUDA;
   Grp G{sizes[0], n_prob, limits, prob, ws_off, nvec, real, hs_off, eig_off, (double2*)H, (double2*)S, eig, status, tri,
         (char*)scratch, scratch_bytes};
-  return run(G, sizes, sms, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
+  try {                                      // the occupancy table and its lock may throw
+    return run(G, sizes, sms, stream) == cudaSuccess ? SKN_OK : SKN_ERR_CUDA;
+  } catch (...) {
+    return SKN_ERR_CUDA;
+  }
 }
 
 extern "C" int skn_eigh_gen_panels(int n_prob, const int32_t* sizes, const int32_t* prob, const int64_t* ws_off,
