@@ -46,7 +46,8 @@ def request_bytes(n_orb: int, nk: int, dos_points: int, wide_threshold: Optional
     """Device bytes one request holds while in flight (H, S, eigenvalues, DOS, slack for bonds), plus the
     device-wide eigensolver's scratch when its problems are above ``wide_threshold`` orbitals (panels,
     partial sums and the tensor-core update's integer slices: about 5.5 KB per orbital and k-point), or with
-    ``panels`` the panel kernels' scratch below it (as much again, at most PANELS_SCRATCH at a time)."""
+    ``panels`` the panel kernels' scratch below it: 11.6 times H and S at 65 orbitals, 3.3 at 128, 0.85 at 492, at most
+    PANELS_SCRATCH, which is what a whole batch holds of it."""
     nb = int(2 * 16 * n_orb * n_orb * nk + 8 * n_orb * nk + 8 * dos_points + (8 << 20))
     if wide_threshold is not None and wide_threshold < n_orb <= MAX_N and nk > 0:
         import ctypes
@@ -55,7 +56,7 @@ def request_bytes(n_orb: int, nk: int, dos_points: int, wide_threshold: Optional
         _lib.call("skn_eigh_wide_scratch_bytes", nk, n_orb, ctypes.addressof(need))
         nb += int(need.value)
     elif panels and E.SMALL_MAX_N < n_orb <= E.PANELS_MAX_N:
-        nb += min(nk * E.panels_scratch_bytes(n_orb), 2 * E.PANELS_SCRATCH)
+        nb += min(nk * E.panels_scratch_bytes(n_orb), E.PANELS_SCRATCH)
     return nb
 
 
