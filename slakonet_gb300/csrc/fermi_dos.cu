@@ -205,12 +205,13 @@ __global__ void __launch_bounds__(NT, 4)
       turn ^= 1;
     }
   };
+  const bool plain_kT = kT > 1e-290 && kT < 1e290;      // in the range of its reciprocal
   // the next mu and the energies beyond which a state is full or empty to the last bit, for all threads
   auto publish = [&](double m, int stop) {
     if (tid == 0) {
       s_mu = m;
       s_stop = stop;
-      const bool usable = fabs(m) < 1e300 && kT > 1e-290 && kT < 1e290;
+      const bool usable = fabs(m) < 1e300 && plain_kT;
       s_edge[0] = usable ? order_key(m - FULL_X * kT) : INT_MIN;
       s_edge[1] = usable ? order_key(m + FULL_X * kT) : INT_MAX;
       s_edge[2] = usable ? order_key(m + 700.0 * kT) : INT_MIN;
@@ -232,7 +233,7 @@ __global__ void __launch_bounds__(NT, 4)
   for (int it = 0; it < max_iter; ++it) {
     const double mu = s_mu;
     const int below = s_edge[0], above = s_edge[1], top = s_edge[2];
-    const bool usable = top != INT_MIN;          // mu is finite, and kT in the range of its reciprocal
+    const bool usable = top != INT_MIN;          // no diverged search: mu is finite
     double sumo = 0.0, sumg = 0.0;
     int k = k0, bb = b0;
     for (int64_t base = rank * NT; base < tot; base += (int64_t)(NEAR / NT) * stride) {      // the same trips for every thread
@@ -277,7 +278,7 @@ __global__ void __launch_bounds__(NT, 4)
       for (int q = tid; q < count; q += NT) {
         const double wk = near_w[q];
         const double d = near_e[q] - mu;
-        const double t3 = exp(usable ? skn_over(d, by_kT) : d / kT);
+        const double t3 = exp(usable ? skn_over(d, by_kT) : plain_kT ? skn_quotient(d, kT, by_kT.hi) : d / kT);
         const double occ = 1.0 / (t3 + 1.0);
         sumo = fma(occ, wk, sumo);
         sumg += ((wk * occ) * occ) * t3;
