@@ -633,6 +633,10 @@ def route_wide(prob_n: np.ndarray, threshold: Optional[int]) -> np.ndarray:
     return prob_n.astype(np.int64) > int(threshold)
 
 
+def _is(kind, name: str) -> bool:
+    return isinstance(kind, tuple) and kind[0] == name
+
+
 def _one_cta_shape(n: int) -> str:
     from .autotune import Tuning
     return Tuning.one_cta().shape_for(n)
@@ -884,7 +888,7 @@ class Engine:
                                ptr(db.n), ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff),
                                ptr(Hk), ptr(Sk), ptr(eig), ptr(eig_status), ptr(tri), ptr(scratch[gi]), nbytes, g.sms, st)
                     self.launches += panels_launches(int(sizes[0])) - 1
-            elif isinstance(g.kind, tuple) and g.kind[0] == "small":
+            elif _is(g.kind, "small"):
                 self._call("skn_eigh_gen_small", g.count, g.max_n, ptr(g.order), ptr(db.n),
                            ptr(db.real if self.real_path else None), ptr(db.hs_off), ptr(db.eoff), ptr(Hk), ptr(Sk),
                            ptr(eig), ptr(eig_status), ptr(tri), st)
@@ -937,7 +941,7 @@ class Engine:
                 call("skn_eigh_large_scratch_bytes", g.count, g.max_n, g.kind, ctypes.addressof(need))
             elif g.parts:
                 need.value = max(nbytes for _, _, _, nbytes, _ in g.parts)
-            elif isinstance(g.kind, tuple) and g.kind[0] == "wide":
+            elif _is(g.kind, "wide"):
                 call("skn_eigh_wide_scratch_bytes", g.count, g.max_n, ctypes.addressof(need))
             else:
                 continue
@@ -964,6 +968,28 @@ class Engine:
             cur.append(torch.cuda.Stream(self.device))
         return cur
 
+    def _kinds(self, ns, vectors: bool, budget: int) -> list:
+        """What problems of each size run on (Group.kind; ("wide", n) without its real part)."""
+        tuning = self.tuning if self.tuning is not None else _default_tuning()
+        policies = ["auto" if vectors else tuning.policy_for(n) for n in ns.tolist()]
+        wide, csize = np.zeros(len(ns), bool), np.zeros(len(ns), int)
+        if not vectors:
+            # above ONE_CTA_LARGE_N: what a tuning keeps on the one-CTA kernel leaves it, for the cluster or the device-wide
+            # path, and what the cluster path would take goes to the device-wide one, where those are on
+            big = ns > ONE_CTA_LARGE_N
+            own = big & np.array([x != "auto" for x in policies], bool)
+            csize = route_large(ns, self.large_threshold, self.large_cluster)
+            if own.any() and self.large_threshold is not None:
+                csize = np.where(own, route_large(ns, ONE_CTA_LARGE_N, self.large_cluster), csize)
+            wide = route_wide(ns, self.wide_threshold)
+            if self.wide_threshold is not None:
+                wide |= own | (big & (csize > 0))
+        kinds = []
+        for n, x, w, c in zip(ns.tolist(), policies, wide.tolist(), csize.tolist()):
+            kind = ("wide", n) if w else c if c else route_auto(n) if x == "auto" else x
+            kinds.append(_one_cta_shape(n) if _is(kind, "panels") and not (budget or vectors) else kind)
+        return kinds
+
     def _groups(self, db, vectors: bool = False, budget: int = PANELS_SCRATCH):
         """The batch's eigensolver groups ([Group], empty when every problem takes the default single-CTA launch), kept
         on the batch by all that decides them.  None is ever dropped or changed: a captured graph reads their arrays.
@@ -974,71 +1000,50 @@ class Engine:
         key = (vectors, budget, tuned, self.large_threshold, self.large_cluster, self.real_path, self.wide_threshold)
         if key in db.groups:
             return db.groups[key]
-        tuning = self.tuning if self.tuning is not None else _default_tuning()
-        wide, csize = np.zeros(len(plan.prob_n), bool), np.zeros(len(plan.prob_n), int)
-        if not vectors:
-            wide = route_wide(plan.prob_n, self.wide_threshold)
-            csize = route_large(plan.prob_n, self.large_threshold, self.large_cluster)
-            # above ONE_CTA_LARGE_N: what a tuning keeps on the one-CTA kernel leaves it, for the cluster or the device-wide
-            # path, and what the cluster path would take goes to the device-wide one, where those are on
-            own = [n for n in np.unique(plan.nb) if n > ONE_CTA_LARGE_N and tuning.policy_for(int(n)) != "auto"]
-            if own and self.large_threshold is not None:
-                csize = np.where(np.isin(plan.prob_n, own), route_large(plan.prob_n, ONE_CTA_LARGE_N, self.large_cluster), csize)
-            if self.wide_threshold is not None:
-                wide |= (plan.prob_n > ONE_CTA_LARGE_N) & (np.isin(plan.prob_n, own) | (csize > 0))
-        wide, csize = wide[plan.order], csize[plan.order]
-        csize[wide] = 0
-        large = (csize > 0) | wide
-        out = []
-        if wide.any():                       # one group per (n, real), largest first
-            wn = plan.prob_n[plan.order[wide]]
-            wr = (plan.prob_real[plan.order[wide]] if (self.real_path and plan.prob_real is not None)
-                  else np.zeros(len(wn), dtype=bool))
-            for n_, r_ in sorted({(int(a), bool(b)) for a, b in zip(wn, wr)}, reverse=True):
-                sel = plan.order[wide][(wn == n_) & (wr == r_)]
-                out.append((("wide", n_, int(r_)), sel, len(sel), n_))
-        for c in sorted(set(csize[csize > 0].tolist()), reverse=True):    # one launch per cluster size
-            sel = plan.order[csize == c]
-            out.append((int(c), sel, len(sel), int(plan.prob_n[sel].max())))
-        small_order = plan.order[~large]
-        if len(small_order):
-            sizes = plan.prob_n[small_order]
-            ns = np.unique(plan.nb)                  # of the structures: far fewer than problems
-            ns = ns[np.isin(ns, sizes)] if large.any() else ns
-            at = np.searchsorted(ns, sizes)
-            names = ["auto" if vectors else tuning.policy_for(int(n)) for n in ns]
-            names = [route_auto(int(n)) if x == "auto" else x for n, x in zip(ns, names)]
-            if not (budget or vectors):
-                names = [_one_cta_shape(int(n)) if x[0] == "panels" else x for n, x in zip(ns, names)]
-            kinds = list(dict.fromkeys(names))
-            kind = np.array([kinds.index(x) for x in names])[at]
-            if self.real_path and plan.prob_real is not None:     # one-CTA shapes: real problems in a call of their own
-                own = np.array([isinstance(x, str) for x in kinds])
-                kind = kind + len(kinds) * (plan.prob_real[small_order] & own[kind])
-            members = [(i, np.flatnonzero(kind == i)) for i in range(int(kind.max()) + 1)]
-            for i, at in sorted((m for m in members if len(m[1])), key=lambda m: m[1][0]):     # by first appearance
-                sel = small_order[at]
-                sfx = kinds[i % len(kinds)]
-                sfx = "_real" + sfx if i >= len(kinds) else sfx
-                out.append((sfx, sel, len(sel), int(plan.prob_n[sel].max())))
-        if len(out) == 1 and out[0][0] == "" and out[0][2] == len(plan.order):
-            out = []     # the default launch over the batch's own order
+        ns = np.unique(plan.nb)[::-1]            # of the structures: far fewer than problems, which are in this order
+        kinds = self._kinds(ns, vectors, budget)
         real = plan.prob_real if (self.real_path and plan.prob_real is not None) else np.zeros(len(plan.prob_n), bool)
-        out = [out[i] for i in launch_order([g[1] for g in out], plan.prob_n, real)]
-        cost = [float((plan.prob_n[sel].astype(np.float64) ** 3).sum()) for _, sel, _, _ in out]
-        sms = torch.cuda.get_device_properties(self.device).multi_processor_count
-        sizes = {i: np.ascontiguousarray(plan.prob_n[sel].astype(np.int32)) for i, (kind, sel, _, _) in enumerate(out)
-                 if isinstance(kind, tuple) and kind[0] == "panels"}
-        most = [panels_parts(z, 1 << 62) for z in sizes.values()]
-        share = dict(zip(sizes, scratch_shares([sum(part[3] for part in m) for m in most],
-                                               [panels_scratch_bytes(z[0]) for z in sizes.values()], budget)))
-        groups = []
-        for i, ((kind, sel, cnt, mx), c) in enumerate(zip(out, cost)):
-            parts = ()
-            if i in sizes:
-                parts = tuple((a, b, w, nbytes, sizes[i][a:b]) for a, b, w, nbytes in panels_parts(sizes[i], share[i]))
+        sizes = plan.prob_n[plan.order]
+        edges = [0, *np.searchsorted(-sizes, -ns, side="right").tolist()]
+        ranges = {}                              # kind: its ranges of plan.order, largest first
+        for i, kind in enumerate(kinds):
+            if edges[i] < edges[i + 1]:
+                ranges.setdefault(kind, []).append((edges[i], edges[i + 1]))
+        out = []                                 # [(place in the list, kind, problems)]
+        for kind, rs in ranges.items():
+            sel = np.concatenate([plan.order[a:b] for a, b in rs]) if len(rs) > 1 else plan.order[rs[0][0]:rs[0][1]]
+            if isinstance(kind, int):            # one launch per cluster size
+                out.append(((1, -kind), kind, sel))
+            elif _is(kind, "wide"):              # one group per (n, real)
+                out += [((0, -kind[1], r), (*kind, 1 - r), part) for r, part in enumerate((sel[real[sel]], sel[~real[sel]]))]
+            elif isinstance(kind, str) and real.any():     # one-CTA shapes: real problems in a call of their own
+                first = np.flatnonzero(real[sel])
+                for part, name in ((sel[~real[sel]], kind), (sel[first], "_real" + kind)):
+                    at = rs[0][0] + (int(first[0]) if name != kind and len(first) else 0)
+                    out.append(((2, at), name, part))
+            else:
+                out.append(((2, rs[0][0]), kind, sel))
+        out = [(kind, sel) for _, kind, sel in sorted((o for o in out if len(o[2])), key=lambda o: o[0])]
+        if len(out) == 1 and out[0][0] == "":
+            out = []     # the default launch over the batch's own order
+        out = [out[i] for i in launch_order([sel for _, sel in out], plan.prob_n, real)]
+        panels = {i: np.ascontiguousarray(plan.prob_n[sel], dtype=np.int32) for i, (kind, sel) in enumerate(out)
+                  if _is(kind, "panels")}
+        parts, shares = {}, {}
+        if panels:
+            parts = {i: panels_parts(z, 1 << 62) for i, z in panels.items()}
+            need = [sum(p[3] for p in parts[i]) for i in panels]
+            give = scratch_shares(need, [panels_scratch_bytes(z[0]) for z in panels.values()], budget)
+            for i, had, got in zip(panels, need, give):
+                if got < had:
+                    parts[i] = panels_parts(panels[i], got)
             # the groups run beside one another: each plans for the SMs of its part of the batch's n^3
-            groups.append(Group(kind, sel, cnt, mx, parts, max(1, round(sms * c / max(sum(cost), 1.0)))))
+            cost = [float((plan.prob_n[sel].astype(np.float64) ** 3).sum()) for _, sel in out]
+            sms = torch.cuda.get_device_properties(self.device).multi_processor_count
+            shares = {i: max(1, round(sms * cost[i] / max(sum(cost), 1.0))) for i in panels}
+        groups = [Group(kind, sel, len(sel), int(plan.prob_n[sel[0]]),
+                        tuple((a, b, w, nbytes, panels[i][a:b]) for a, b, w, nbytes in parts.get(i, ())), shares.get(i, 0))
+                  for i, (kind, sel) in enumerate(out)]
         if not groups:
             return db.groups.setdefault(key, groups)
         # problem lists and scratch offsets to the device
