@@ -59,8 +59,8 @@ _ZEROS = bytes(256)
 
 
 def _to_device(arrays, device) -> list:
-    """[(array, np.int32 / np.int64 / np.float64)] on the device, flat, in one copy: views of one buffer, each on a
-    256-byte boundary as an allocation of its own would be.  A copy each took 290 us of a one-k-point cell's call for
+    """[(array, np.int32 / np.int64 / np.float64)] on the device in one copy: views of one buffer in the arrays' shapes, each
+    on a 256-byte boundary as an allocation of its own would be.  A copy each took 290 us of a one-k-point cell's call for
     its 30 descriptor arrays, and every one waited for those before it."""
     chunks, sections, first = [], [], 0
     for dtype, (tdtype, size) in _TORCH.items():          # by type: one view and one split each
@@ -79,7 +79,8 @@ def _to_device(arrays, device) -> list:
     for tdtype, idx, sizes, start, end in sections:
         if idx:
             for i, v in zip(idx, buf[start:end].view(tdtype).split(sizes)[::2]):
-                out[i] = v
+                shape = np.shape(arrays[i][0])
+                out[i] = v if len(shape) == 1 else v.view(shape)
     return out
 
 
