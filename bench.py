@@ -43,18 +43,6 @@ DOS_POINTS = 1000
 DOS_SIGMA = 0.1
 DOS_WINDOW = 9.0
 SAMPLE_STRIDE = 16         # CPU baseline: every 16th structure (stratified over sizes)
-# DRAM bytes (read + write) of the one-CTA eigensolver's launches of one execution, measured by ncu on two
-# stratified samples of the default workload (profiles/k_eigh_gen_uneven_samples_dram.md):
-# `ncu --metrics gpu__time_duration.sum,dram__bytes_read.sum,dram__bytes_write.sum --clock-control none
-#  -k regex:k_eigh_gen -s 4 -c 4 python bench.py --path-only --sample-stride K --steps 1 --warmup 1`.
-# The ratio to the H(k)+S(k) bytes grows with the number of large problems in flight (L2 holds fewer of
-# their trailing matrices), so it is not scaled to the full batch, whose capture the size rule excludes.
-EIG_TRAFFIC_SAMPLES = {
-    "every 16th structure by size (16 structures, 1877 problems)":
-        {"hs_bytes": 659664384, "dram_bytes": 1564348928, "ncu_ms": 520.9},
-    "every 4th structure by size (64 structures, 8424 problems)":
-        {"hs_bytes": 2215006848, "dram_bytes": 37161698048, "ncu_ms": 564.8},
-}
 WORKLOAD = ("uneven batch: 256 random periodic structures, 2-64 atoms log-uniform, Z=1-65 default shells, "
             "Gamma-centred k-grids ~1000 k-atoms, FP64 generalized eigensolve per k, Fermi/gap, "
             "1000-pt DOS on [-20,10] eV")
@@ -531,21 +519,19 @@ def run_gpu(args, rank, world):
                             f"{1e3 * elapsed_u / args.steps:.1f} ms",
                    "autotune_s": round(t_tune, 1),
                    "autotune_batch_trials_ms": tuning.timings.get("batch_trials_ms")},
-        "roofline": {"bound": "tensor", "kernel": "the eigensolver's launches: k_tri_panel, k_update, k_solve and the others of "
+        "roofline": {"bound": "latency", "kernel": "the eigensolver's launches: k_tri_panel, k_update, k_solve and the others of "
                                                  "skn_eigh_gen_panels, k_eigh_small (or, where the autotuner prefers it, "
                                                  "k_eigh_gen)",
-                     "note": "achieved counts the algorithm's real flops; only part of them run on the FP64 unit, the "
-                             "updates and solves are bf16 slice products and the matrix-vector products integer ones, so "
-                             "the fraction of the FP64 rate may exceed 1",
-                     "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": achieved / peak,
-                     "traffic": None,
-                     "traffic_note": "not captured on the full batch (the capture-size rule); measured on two "
-                                     "stratified samples with the one-CTA kernel, see traffic_samples: DRAM bytes per "
-                                     "execution of its launches against their H(k)+S(k) bytes, about 1% of HBM's rate "
-                                     "in the larger sample",
-                     "traffic_samples": {k: dict(v, ratio=round(v["dram_bytes"] / v["hs_bytes"], 2),
-                                                 dram_gbs=round(v["dram_bytes"] / v["ncu_ms"] / 1e6, 1))
-                                         for k, v in EIG_TRAFFIC_SAMPLES.items()},
+                     "note": "achieved counts the algorithm's real flops as FP64; only part of them run on the FP64 unit, "
+                             "the updates and solves are bf16 slice products and the matrix-vector products integer "
+                             "ones, so no one unit's rate is the denominator and frac is null: fp64_equivalent is the "
+                             "ratio to the FP64 rate, which it may exceed. What bounds the launches is latency, see "
+                             "counters",
+                     "achieved": achieved, "peak": peak, "unit": "TFLOP/s", "frac": None, "fp64_equivalent": achieved / peak,
+                     "counters": "152 problems of 320 orbitals (profiles/k_tri_panel_n320_152.md, "
+                                 "profiles/k_update_k_solve_n320_152.md): k_tri_panel FP64 pipe 14%, integer multiply-adds "
+                                 "23%, DRAM 20%; k_update tcgen05 pipe 23-29%, DRAM 18-21%; k_solve tcgen05 9%, DRAM 20%",
+                     "traffic": None, "traffic_note": "not captured on the full batch (the capture-size rule)",
                      "peak_source": "measured in this run: FP64 FMA probe kernel (skn_fp64_probe); the FP64 "
                                     "tensor instruction (skn_fp64_probe_dmma) is measured beside it",
                      "fp64_fma_tflops": peak, "fp64_dmma_tflops": peak_dmma,

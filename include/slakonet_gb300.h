@@ -328,9 +328,10 @@ int skn_eigh_gen_small(int n_prob, int max_n, const int32_t* prob, const int32_t
  * problems of up to 2048 orbitals, in lockstep over 32-column panels: Cholesky of
  * S, C = L^-1 H L^-H by two blocked sweeps, Householder tridiagonalisation with
  * one cluster of CTAs per problem, Sturm-count eigenvalues.  Every trailing
- * update runs on the bf16 tensor cores, exact products of 8 integer slices of 7
- * bits per operand row rounded once per panel.  Replaces the same eighb call as
- * skn_eigh_gen_batched (slakonet/utils.py:741-783).
+ * update runs on the bf16 tensor cores: 8 integer slices of 7 bits per operand
+ * row, the 36 slice pairs of level below 8 added exactly and rounded once per
+ * panel, those above left out (2^-49 of the rows' scales at the very most).
+ * Replaces the same eighb call as skn_eigh_gen_batched (slakonet/utils.py:741-783).
  *   n_prob    problems of the call (<= 65535)
  *   sizes     [n_prob] (host) n of each slot's problem, descending, at most 2048
  *   prob      [n_prob] (device) problem index of each slot, into the arrays below

@@ -15,14 +15,14 @@
 // slakonet/main.py:174).
 //
 // GB300 notes.  An SM does two FP64 multiply-adds per clock, so what stays on that unit bounds everything.  The updates
-// are exact products of integer slices on the tensor cores, rounded once per panel; the matrix-vector products of the
-// tridiagonalisation are exact products of 28-bit limbs on the integer units, rounded once per tile; FP64 keeps the
-// reflectors, the O(n) work of a column and the diagonal blocks.  Every sum that crosses warps or CTAs goes to its own
+// are sums of integer slice products on the tensor cores, the leading ones added exactly and rounded once per panel; the
+// matrix-vector products of the tridiagonalisation are sums of 28-bit limb products on the integer units, rounded once per
+// tile (what each leaves out stands below); FP64 keeps the reflectors, the O(n) work of a column and the diagonal blocks.  Every sum that crosses warps or CTAs goes to its own
 // slot and is added in a fixed order, or is an integer, so a problem's results depend neither on the other problems nor
 // on the number of CTAs it is given.
 // Measured (random pencils): 492 orbitals x 300 problems 393 ms with one CTA per problem, 208 with the products in FP64,
-// 98 now (tridiagonalisation 48, updates 32, solves 8, eigenvalues 4); 432 x 8 190, 18.8, 9.8 ms (5.8 of them the
-// tridiagonalisation, 13 us a column); 1152 x 2 47, 30.9 ms.
+// 97 now (tridiagonalisation 48, updates 32, solves 8, eigenvalues 4); 432 x 8 190, 18.8, 9.8 ms (5.8 of them the
+// tridiagonalisation, 13 us a column); 1152 x 2 47, 31.3 ms.
 #include <algorithm>
 #include <array>
 #include <map>
@@ -197,10 +197,11 @@ SKN_DEVINL bool is_real(const Grp& G, int p) { return G.real != nullptr && G.rea
 // ------------------------------------------------------------------ integer slices
 // Error-free splitting (Ozaki, Ogita and Oishi, Numer. Algorithms 59, 2012).  A row of 32 complex values is
 // scaled by its exponent ex and cut into SLICES digits of 7 bits, x = 2^ex sum_s d_s 2^(-7 (s + 1)) with
-// |d_0| <= 128 and -64 <= d_s < 64 after it, each exact in bf16; what is cut off is below 2^-57 of the
-// row's largest entry.  A slice product is an integer of at most 14 bits and a 64-term sum of the at most
-// 8 slice pairs of one level s + t stays below 2^23, exact in an FP32 accumulator.  The complex product
-// P Q^H takes A = [Pr Pi], B = [Qr Qi] for the real part and B' = [-Qi Qr] for the imaginary part.
+// |d_0| <= 128 and -64 <= d_s < 64 after it, each exact in bf16; what is cut off is at most 2^-57 2^ex, 2^-56 of
+// the row's largest entry.  A slice product is an integer of at most 14 bits and a 64-term sum of the at most
+// 8 slice pairs of one level s + t < 8 stays below 2^23, exact in an FP32 accumulator.  The pairs of higher levels are left
+// out: 2^-49 of the two rows' scales if all their digits were extreme and of one sign, 2^-55 for digits without a pattern
+// (each FP64 product would be off by 2^-53 of itself).  The complex product P Q^H takes A = [Pr Pi], B = [Qr Qi] for the real part and B' = [-Qi Qr] for the imaginary part.
 // The digits are taken with integer operations: the FP64 pipe would cost more than the solves.
 constexpr int EXP_NAN = INT32_MIN;       // a row with a non-finite entry: its products become NaN
 
@@ -913,8 +914,11 @@ template <bool R> SKN_DEVINL double2 sum4(double2 a, double2 b, double2 c, doubl
 // A tile and a chunk of v are held as integers of 56 bits under one exponent, each in two limbs of 28 (balanced, so the
 // low one has a sign).  Of a product's four partial products the lowest, 2^-58 of the largest, is left out; the others are
 // exact in 64-bit accumulators over the 32 terms of a tile, and a tile's sum is rounded once.  The error per term is that
-// of the operands' last bit, 2^-57 of the largest, against 2^-53 of each product for FP64: it stays below FP64's own as
-// long as the entries of a tile are within 2^4 of each other, and relative to the matrix's norm always.
+// of the operands' last bit, at most 2^-56 of the largest, against 2^-53 of each product for FP64: it stays below FP64's own
+// as long as the entries of a tile are within 2^3 of each other, and relative to the matrix's norm always.  Entries further
+// below their tile's largest keep fewer bits than in FP64.  Measured against extended precision, eigenvalues are no further
+// off for it: physical pencils of 65 to 400 orbitals 0.3-0.5 eps of the scale (one CTA in FP64 0.9), random ones 0.16-0.23
+// (0.31-0.38), graded and block-scaled ones over 3 to 9 decades within 2% of the FP64 kernel's error or below it.
 // A partition issues a multiply-add of two 32-bit integers into 64 bits every 4.8 clocks and an FP64 instruction every 64:
 // three of the one replace one of the other.
 struct alignas(8) Limb { int h, l; };
@@ -1735,11 +1739,14 @@ int clusters_at_once(bool resident, int C, int per_sm, int sms) {
 
 // CTAs per problem over m rows, and the tiles of each when they are resident (0: streamed).  Resident: one CTA per SM,
 // up to one per tile, if shared memory holds its part and all problems run at once.  A cluster's barrier takes about 1200
-// clocks, a counter's 5000, so a grid team only from GRID_FROM CTAs.  Streamed, with the GPU to itself: the size whose
+// clocks, a counter's 5000, so a grid team only from GRID_FROM CTAs: where a cluster holds the tiles too it is 1 to 4% faster
+// (200 to 432 orbitals x 3 to 6 problems), and where it does not the grid team is 13% faster than streaming (640 x 3 to 6;
+// with the line at 17 also 640 x 7 and 8, by 8 to 12%, and 432 x 7 and 8 2 to 4% slower).  Streamed, with the GPU to itself: the size whose
 // rounds are the shortest, as a problem's time falls with its CTAs and a round that is nearly empty costs as much as a full
 // one (492 orbitals x 300 problems 98 ms, with 10 CTAs for each SM 111; 320 x 456 54 and 56).  Beside other calls there are
-// no rounds, and STREAM_PER_SM CTAs for each SM of its part (four are resident; the rest wait) even the calls out: the mixed
-// batch takes 157 ms so, 165 at 5 and 162 by rounds.
+// no rounds, and STREAM_PER_SM CTAs for each SM of its part (four are resident; the rest wait) even the calls out.  At 5, 10
+// and 20 four mixed batches take 112.8, 111.1, 112.9; 21.7, 21.9, 21.8; 25.9, 25.5, 25.6; 28.1, 28.0, 28.5 ms: a flat
+// optimum.  The terms of `cost` are estimates of what a wider cluster's barriers add, not fitted to anything.
 constexpr int GRID_FROM = 24, STREAM_PER_SM = 10;
 void plan_panel(int m, int n_prob, int sms, int all, int& C, int& rt) {
   const int nt = cdiv(m, TS), tiles = nt * (nt + 1) / 2;

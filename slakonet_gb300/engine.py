@@ -596,10 +596,11 @@ SMALL_CLASSES = (16, 24, 32, 40, 48, 56, 64)     # its calls' size classes: shar
 def route_auto(n: int):
     """Kernel and call of a problem of n orbitals under the untuned policy: ("small", class) or ("panels", class of
     64 orbitals).  A rule on the problem alone, as route_wide.  Measured on GB300, panels against the small kernel:
-    88 orbitals x 500 problems 5.2 ms (9.6), 80 x 50 1.5 (1.9), 72 x 8 1.4 (1.5), 64 x 8 1.16 (1.09), 64 x 4000 18.9
-    (17.4): the line is at 64.  Against the one-CTA kernel: 128 x 1000 16.3 ms (31), 160 x 27 3.2 (12.3), 432 x 8 9.6
-    (187), 492 x 300 98 (389).  One panel call per class, each on its stream: the 600 problems of 65 to 534 orbitals
-    of a mixed batch take 156 ms so, 160 with classes of 32, 157 of 128, and took 4% longer as one call."""
+    88 orbitals x 500 problems 5.2 ms (9.6), 80 x 50 1.6 (1.9), 72 x 8 1.4 (1.5), 64 x 8 1.17 (1.08), 64 x 4000 18.8
+    (17.4): the line is at 64.  Against the one-CTA kernel: 128 x 1000 16.4 ms (31), 160 x 27 3.2 (12.3), 432 x 8 9.8
+    (187), 492 x 300 97 (389).  One panel call per class, each on its stream: as one call the mixed batch of 600 problems
+    above 64 orbitals took 4% longer.  The class's width matters little: with 32, 64 and 128 orbitals four mixed batches
+    take 113.6, 111.1, 106.9; 21.4, 21.9, 21.8; 26.3, 25.5, 25.8; 27.5, 28.0, 28.3 ms."""
     if n <= SMALL_MAX_N:
         return ("small", next(c for c in SMALL_CLASSES if n <= c))
     return ("panels", -(-n // (2 * PANEL)))
@@ -697,7 +698,7 @@ class Engine:
         self.large_cluster = large_cluster
         # problems above wide_threshold orbitals run on the device-wide eigensolver instead (route_wide):
         # measured on GB300 it is 4.6x the 4-CTA cluster at n = 1024 and 6-7x at n = 2048-4096.  Up to the panel
-        # kernels' bound of 2048 orbitals those are faster: 2 problems of 1152 take 51 ms, 125 on this path
+        # kernels' bound of 2048 orbitals those are faster: 2 problems of 1152 take 31 ms, 125 on this path
         self.wide_threshold = wide_threshold
         # the device-wide path's rank-2k updates on the tensor cores (skn_eigh_gen_wide_tc): measured on
         # GB300, the 1000-atom structure (n = 9000, 8 real k-points) solves in 13.2 s instead of 18.9 s
