@@ -59,8 +59,8 @@ _ZEROS = bytes(256)
 
 
 def _to_device(arrays, device) -> list:
-    """[(array, np.int32 / np.int64 / np.float64)] on the device in one copy: views of one buffer in the arrays' shapes, each
-    on a 256-byte boundary as an allocation of its own would be.  A copy each took 290 us of a one-k-point cell's call for
+    """[(array, np.int32 / np.int64 / np.float64)] on the device, flat, in one copy: views of one buffer, each on a
+    256-byte boundary as an allocation of its own would be.  A copy each took 290 us of a one-k-point cell's call for
     its 30 descriptor arrays, and every one waited for those before it."""
     chunks, sections, first = [], [], 0
     for dtype, (tdtype, size) in _TORCH.items():          # by type: one view and one split each
@@ -79,8 +79,7 @@ def _to_device(arrays, device) -> list:
     for tdtype, idx, sizes, start, end in sections:
         if idx:
             for i, v in zip(idx, buf[start:end].view(tdtype).split(sizes)[::2]):
-                shape = np.shape(arrays[i][0])
-                out[i] = v if len(shape) == 1 else v.view(shape)
+                out[i] = v
     return out
 
 
@@ -499,6 +498,8 @@ class DeviceBatch:
             real=(plan.prob_real if plan.prob_real is not None else np.zeros(len(plan.prob_n)), i32),
             bloch_unit_base=(np.cumsum(full) - full, i64), bloch_unit_base_lower=(np.cumsum(lower) - lower, i64))
         self.__dict__.update(zip(arrays, _to_device(list(arrays.values()), device)))
+        self.pos, self.rng, self.kp = (t.view(-1, 3) for t in (self.pos, self.rng, self.kp))
+        self.cells = self.cells.view(-1, 3, 3)
 
     def h2d_bytes(self) -> int:
         return sum(int(v.numel() * v.element_size()) for v in vars(self).values() if isinstance(v, torch.Tensor))
@@ -642,12 +643,6 @@ def _is(kind, name: str) -> bool:
 def _one_cta_shape(n: int) -> str:
     from .autotune import Tuning
     return Tuning.one_cta().shape_for(n)
-
-
-def _default_tuning():
-    """Launch shapes per size bucket when the engine has no autotuned ones (autotune.Tuning.default)."""
-    from .autotune import Tuning
-    return Tuning.default()
 
 
 def launch_order(groups: Sequence[np.ndarray], prob_n: np.ndarray, prob_real: np.ndarray) -> List[int]:
@@ -971,11 +966,12 @@ class Engine:
         return cur
 
     def _kinds(self, ns, vectors: bool, budget: int) -> list:
-        """What problems of each size run on (Group.kind; ("wide", n) without its real part)."""
-        tuning = self.tuning if self.tuning is not None else _default_tuning()
-        policies = ["auto" if vectors else tuning.policy_for(n) for n in ns.tolist()]
+        """What problems of each size (descending) run on: Group.kind, ("wide", n) without its real part."""
+        sizes = ns.tolist()
+        policies = ["auto"] * len(sizes) if vectors or self.tuning is None else [self.tuning.policy_for(n) for n in sizes]
         wide, csize = np.zeros(len(ns), bool), np.zeros(len(ns), int)
-        if not vectors:
+        limit = min(t for t in (ONE_CTA_LARGE_N, self.large_threshold, self.wide_threshold) if t is not None)
+        if not vectors and sizes and sizes[0] > limit:
             # above ONE_CTA_LARGE_N: what a tuning keeps on the one-CTA kernel leaves it, for the cluster or the device-wide
             # path, and what the cluster path would take goes to the device-wide one, where those are on
             big = ns > ONE_CTA_LARGE_N
@@ -987,7 +983,7 @@ class Engine:
             if self.wide_threshold is not None:
                 wide |= own | (big & (csize > 0))
         kinds = []
-        for n, x, w, c in zip(ns.tolist(), policies, wide.tolist(), csize.tolist()):
+        for n, x, w, c in zip(sizes, policies, wide.tolist(), csize.tolist()):
             kind = ("wide", n) if w else c if c else route_auto(n) if x == "auto" else x
             kinds.append(_one_cta_shape(n) if _is(kind, "panels") and not (budget or vectors) else kind)
         return kinds

@@ -24,4 +24,4 @@ def test_every_type_and_empty_arrays_in_one_copy():
               (np.arange(6.0).reshape(2, 3)[:, ::-1], np.float64), (np.array([2 ** 40]), np.int64)]
     got = E._to_device(arrays, torch.device("cpu"))
     for (a, t), v in zip(arrays, got):
-        assert tuple(v.shape) == a.shape and np.array_equal(v.numpy(), a.astype(t))
+        assert tuple(v.shape) == (a.size,) and np.array_equal(v.numpy(), a.astype(t).reshape(-1))
